@@ -12,7 +12,7 @@
 // The pair update uses the structure of jac_ij (ahl21.jl:734-750): rows of
 // body i are mj*K, -mj*K on (x,v)_i, (x,v)_j and rows of body j are -mi*K,
 // mi*K, so jac_ij * [J_i; J_j] = [mj u; -mi u] with u = K (J_i - J_j), plus
-// the two mass columns (fused into the scaling FMA).  That is 54 FP64
+// the two mass columns (PREC in nbg_layout.cuh).  That is 54 FP64
 // operations per column instead of 144 for the dense 12x12 block; the
 // product is rounded differently from a dense BLAS product, which the
 // reference's BLAS leaves unspecified anyway.
@@ -92,22 +92,25 @@ __device__ __forceinline__ void pair_apply(double* J, double* E, int c, int i, i
 #pragma unroll
   for (int q = 0; q < 36; q++) K[q] = rec.get(roff + q);
   const double mi = rec.get(roff + PREC_MI), mj = rec.get(roff + PREC_MJ);
-  // the mass column of body i or j (at most one of them is this column)
-  // takes the pair's mass entries; every other column adds an exact zero
-  const int mc = (c == 7 * i + 6) ? PREC_MC6 : (c == 7 * j + 6) ? PREC_MC13 : -1;
-  double C[12];
+  // the mass columns of i and j start u from Psi and one of them adds B to
+  // each body; every other column takes exact zeros
+  const bool ci = c == 7 * i + 6, cj = c == 7 * j + 6;
+  double U[6], B[6];
 #pragma unroll
-  for (int q = 0; q < 12; q++) C[q] = (mc >= 0) ? rec.get(roff + mc + q) : 0.0;
+  for (int q = 0; q < 6; q++) {
+    U[q] = (ci || cj) ? rec.get(roff + PREC_PSI + q) : 0.0;
+    B[q] = (ci || cj) ? rec.get(roff + PREC_B + q) : 0.0;
+  }
   double D[6];
 #pragma unroll
   for (int l = 0; l < 6; l++) D[l] = J[(6 * i + l) * BS] - J[(6 * j + l) * BS];
 #pragma unroll
   for (int r = 0; r < 6; r++) {
-    double u = K[r * 6] * D[0];
+    double u = U[r];
 #pragma unroll
-    for (int l = 1; l < 6; l++) u = fma(K[r * 6 + l], D[l], u);
-    kahan(J[(6 * i + r) * BS], E[(6 * i + r) * BS], fma(mj, u, C[r]));
-    kahan(J[(6 * j + r) * BS], E[(6 * j + r) * BS], fma(-mi, u, C[6 + r]));
+    for (int l = 0; l < 6; l++) u = fma(K[r * 6 + l], D[l], u);
+    kahan(J[(6 * i + r) * BS], E[(6 * i + r) * BS], fma(mj, u, cj ? B[r] : 0.0));
+    kahan(J[(6 * j + r) * BS], E[(6 * j + r) * BS], fma(-mi, u, ci ? -B[r] : 0.0));
   }
 }
 

@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(OPS_BS) operator_pair_kernel(GroupArgs g, int 
   // step that had mass (ahl21.jl:713 returns before refilling it); zero at the
   // start of the step (zero_out!, ahl21.jl:8).
   int q = slot;
-  while (q >= 0 && cap.get(q * PCAP + 6 + 15) == 0.0) q--;
+  while (q >= 0 && cap.get(q * PCAP + PCAP_K) == 0.0) q--;
   if (q < 0) {
     for (int e = 0; e < PREC; e++) rec.put(roff + e, 0.0);
     return;
@@ -391,13 +391,44 @@ __global__ void __launch_bounds__(OPS_BS) operator_pair_kernel(GroupArgs g, int 
   int i, j;
   pair_of_slot<N>(q, g.npk, kick, &i, &j);
   const double mi = g.m[i * S + s], mj = g.m[j * S + s];
-  if (q < g.npk) pair_record_from_capture<true>(cap, q * PCAP, mi, mj, rec, roff);
-  else pair_record_from_capture<false>(cap, q * PCAP, mi, mj, rec, roff);
+  const double h2 = 0.5 * step_length(g, s, istep, g.nsteps[s], g.h[s]);
+  if (q < g.npk) pair_record_from_capture<true>(cap, q * PCAP, mi, mj, h2, rec, roff);
+  else pair_record_from_capture<false>(cap, q * PCAP, mi, mj, h2, rec, roff);
 }
 
-// Corrector (and kick) records of one chunk: one lane per (step, system).
+// Corrector records of one chunk of a group without kick pairs: one lane per
+// (step, body whose four columns it forms, system).
 template <int N>
 __global__ void __launch_bounds__(OPS_BS) operator_phi_kernel(GroupArgs g, int chunk) {
+  const int S = g.S;
+  const long long L = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (L >= (long long)g.K * N * S) return;
+  const int s = (int)(L % S);
+  const long long rest = L / S;
+  const int d = (int)(rest % N), kk = (int)(rest / N);
+  if (g.sysidx[s] < 0) return;
+  const long long istep = chunk_first_step(g, chunk, s) + kk;
+  if (istep >= g.nsteps[s] || istep < 0) return;
+  const double h = step_length(g, s, istep, g.nsteps[s], g.h[s]);
+  Rec xs{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + s, S};
+  Rec rec{g.steprec + (size_t)kk * g.R * S + s, S};
+  double x[3 * N], a[3 * N], m[N], acc[12 * N];
+  for (int q = 0; q < 3 * N; q++) {
+    x[q] = xs.get(q);
+    a[q] = xs.get(3 * N + q);
+  }
+  for (int q = 0; q < N; q++) m[q] = g.m[q * S + s];
+  for (int q = 0; q < 12 * N; q++) acc[q] = 0.0;
+  phi_columns<N>(x, a, m, h, 0, d, acc);
+  const int off_phi = g.npk * PREC;
+  for (int r = 0; r < 3 * N; r++)
+    for (int p = 0; p < 4; p++) rec.put(off_phi + r * (4 * N) + 4 * d + p, acc[4 * r + p]);
+}
+
+// Corrector and kick records of one chunk of a group with kick pairs: one lane
+// per (step, system).
+template <int N>
+__global__ void __launch_bounds__(OPS_BS) operator_kick_kernel(GroupArgs g, int chunk) {
   const int S = g.S;
   const long long L = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= (long long)g.K * S) return;
@@ -407,25 +438,24 @@ __global__ void __launch_bounds__(OPS_BS) operator_phi_kernel(GroupArgs g, int c
   if (istep >= g.nsteps[s] || istep < 0) return;
   const uint64_t kick = g.kick;
   const double h = step_length(g, s, istep, g.nsteps[s], g.h[s]);
-  Rec xs{g.xsnap + (size_t)kk * snap_count(kick != 0) * 3 * N * S + s, S};
+  Rec xs{g.xsnap + (size_t)kk * snap_count(true) * 3 * N * S + s, S};
   Rec rec{g.steprec + (size_t)kk * g.R * S + s, S};
   Sys<N> st;
   Work<N> w;
   for (int q = 0; q < N; q++) st.m[q] = g.m[q * S + s];
   for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(q), st.v[q] = st.xe[q] = st.ve[q] = 0.0;
   phic<N, true>(st, w, h, kick);
-  phisalpha<N, true>(st, w, h, 2.0, kick);
-  const int off_phi = (kick ? op_size(N) : 0) + g.npk * PREC;
+  phisalpha<N>(st, w.a, h, kick);
+  phisalpha_operator<N>(st, w, h, kick);
+  const int off_phi = op_size(N) + g.npk * PREC;
   put_op(rec, off_phi, w.op, op_size(N));
-  if (kick) {
-    const double h6 = h / 6.0;
-    for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(3 * N + q);
-    kickfast<N, true>(st, w, h6, kick);
-    put_op(rec, 0, w.op, op_size(N));
-    for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(6 * N + q);
-    kickfast<N, true>(st, w, h6, kick);
-    put_op(rec, off_phi + op_size(N) + g.npk * PREC, w.op, op_size(N));
-  }
+  const double h6 = h / 6.0;
+  for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(3 * N + q);
+  kickfast<N, true>(st, w, h6, kick);
+  put_op(rec, 0, w.op, op_size(N));
+  for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(6 * N + q);
+  kickfast<N, true>(st, w, h6, kick);
+  put_op(rec, off_phi + op_size(N) + g.npk * PREC, w.op, op_size(N));
 }
 
 // Jacobian consumer for one chunk of K steps (one lane per column).
@@ -585,11 +615,17 @@ template <int N>
 int launch_operators(const GroupArgs& g, int chunk, cudaStream_t st) {
   long long lanes = (long long)g.K * 2 * g.npk * g.S;
   allow_smem(operator_pair_kernel<N>, g.guard_smem);
-  allow_smem(operator_phi_kernel<N>, g.guard_smem);
   if (lanes > 0)
     operator_pair_kernel<N><<<(unsigned)((lanes + OPS_BS - 1) / OPS_BS), OPS_BS, g.guard_smem, st>>>(g, chunk);
-  lanes = (long long)g.K * g.S;
-  operator_phi_kernel<N><<<(unsigned)((lanes + OPS_BS - 1) / OPS_BS), OPS_BS, g.guard_smem, st>>>(g, chunk);
+  if (g.kick) {
+    lanes = (long long)g.K * g.S;
+    allow_smem(operator_kick_kernel<N>, g.guard_smem);
+    operator_kick_kernel<N><<<(unsigned)((lanes + OPS_BS - 1) / OPS_BS), OPS_BS, g.guard_smem, st>>>(g, chunk);
+  } else {
+    lanes = (long long)g.K * N * g.S;
+    allow_smem(operator_phi_kernel<N>, g.guard_smem);
+    operator_phi_kernel<N><<<(unsigned)((lanes + OPS_BS - 1) / OPS_BS), OPS_BS, g.guard_smem, st>>>(g, chunk);
+  }
   return 0;
 }
 

@@ -8,9 +8,13 @@
 
 namespace nbg {
 
-// Pair record: K[36] (row-major r*6+l), mi, mj, jac_ij[:,m_i] (12), jac_ij[:,m_j] (12)
-constexpr int PREC = 62;
-constexpr int PREC_MI = 36, PREC_MJ = 37, PREC_MC6 = 38, PREC_MC13 = 50;
+// Pair record: K[36] (row-major r*6+l), mi = m_i/(m_i+m_j), mj likewise, and
+// Psi[6] = G k d(delxv/k)/dk, B[6] = delxv/(m_i+m_j).  With D = J_i - J_j and
+// u = K D, plus Psi in the columns of m_i and m_j, the pair adds mj u to body i
+// and -mi u to body j; the column of m_i takes B off body j's rows and that of
+// m_j adds it to body i's (d(mj)/dm_i = -mj/(m_i+m_j) and so on).
+constexpr int PREC = 50;
+constexpr int PREC_MI = 36, PREC_MJ = 37, PREC_PSI = 38, PREC_B = 44;
 
 __host__ __device__ constexpr int op_size(int N) { return 12 * N * N; }
 __host__ __device__ inline int pair_bit(int i, int j, int N) { return i * N - i * (i + 1) / 2 + (j - i - 1); }
@@ -33,11 +37,13 @@ constexpr int OPS_BS = 128;     // operator kernels
 __host__ __device__ inline int trec_size(int N, int tbv) { return tbv ? 21 * N + 3 : 7 * N + 1; }
 
 // Captured Kepler-pair parameters (producer -> operator kernel): x0[3], v0[3]
-// and the 22 values jac_delxv_gamma! returns (ahl21.jl:888-889).
-constexpr int PCAP = 28;
-// Position snapshots per step: [0] at the correctors, [1] at the first and
-// [2] at the second kick (kick groups only); 3N doubles each.
-__host__ __device__ inline int snap_count(bool kick) { return kick ? 3 : 1; }
+// and the solve's 15 values (put_capture); k's place.
+constexpr int PCAP = 21;
+constexpr int PCAP_K = 17;
+// Snapshots per step, 3N doubles each: positions at the correctors, then
+// phisalpha!'s accelerations there, or in kick groups the positions at the
+// first and at the second kick.
+__host__ __device__ inline int snap_count(bool kick) { return kick ? 3 : 2; }
 
 
 struct GroupArgs {
@@ -99,8 +105,8 @@ struct GroupArgs {
   double* tscratch;  // [R][tgrid]: operator records of a search's final partial step
   int tgrid;         // threads of the transit kernel
   // producer captures for the operator kernels
-  double* pcap;   // [K][2 npk][28][S]: Kepler-pair parameters
-  double* xsnap;  // [K][snaps][3N][S]: positions at the correctors (and kicks)
+  double* pcap;   // [K][2 npk][21][S]: Kepler-pair parameters
+  double* xsnap;  // [K][snaps][3N][S]: see snap_count
 };
 
 // Length of step istep of the system in slot s (nst steps in all).

@@ -3,7 +3,7 @@
 //
 // The producer advances x, v only (the arithmetic of ahl21_no_grad.jl, bitwise
 // the x, v of the gradient step) and captures, per Kepler pair, x0, v0 and the
-// 22 values jac_delxv_gamma! returns (ahl21.jl:888-889), plus the positions at
+// values of its solve (put_capture), plus the positions and accelerations at
 // the correctors and kicks.  Everything else kepler_driftij_gamma!,
 // phic!/phisalpha! and kickfast! compute for the Jacobian depends only on
 // those values, so it runs here, off the producer's sequential chain:
@@ -38,37 +38,34 @@ __device__ __forceinline__ void pair_of_slot(int q, int npk, uint64_t kick, int*
   *pj = 1;
 }
 
-// kepler_driftij_gamma!'s Jacobian part for one pair from its capture.
+// kepler_driftij_gamma!'s Jacobian part for one pair from its capture; h2 is
+// the drift's half step.
 template <bool DRIFT_FIRST>
-__device__ void pair_record_from_capture(const Rec& cap, int coff, double m_i, double m_j, const Rec& rec,
-                                         int roff) {
-  double x0[3], v0[3];
-  for (int q = 0; q < 3; q++) {
-    x0[q] = cap.get(coff + q);
-    v0[q] = cap.get(coff + 3 + q);
-  }
+__device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int coff, double m_i, double m_j, double h2,
+                                                         const Rec& rec, int roff) {
+  double v[PCAP];
+#pragma unroll
+  for (int q = 0; q < PCAP; q++) v[q] = cap.get(coff + q);
+  const double *x0 = v, *v0 = v + 3;
   KepParams P;
-  double* pv[22] = {&P.gamma, &P.g0, &P.g1, &P.g2, &P.g3, &P.h1, &P.h2, &P.dfdt, &P.fm1, &P.gmh, &P.dgdtm1,
-                    &P.r0, &P.r, &P.r0inv, &P.rinv, &P.k, &P.h, &P.beta, &P.betainv, &P.eta, &P.sqb, &P.zeta};
-  for (int q = 0; q < 22; q++) *pv[q] = cap.get(coff + 6 + q);
-  GH gh = gh_functions<GH_H1 | GH_H2 | GH_H3 | GH_H5 | GH_H6>(P.gamma, P.beta, P.sqb);
-  P.H1v = gh.h1; P.H2v = gh.h2; P.H3v = gh.h3; P.H5v = gh.h5; P.H6v = gh.h6;
-  double jk[48], jm[6];
-  kep_jacobian<DRIFT_FIRST>(P, x0, v0, jk, jm);
-  double delxv[6];
-  for (int j = 0; j < 3; j++) delxv[j] = P.fm1 * x0[j] + P.gmh * v0[j];
-  for (int j = 0; j < 3; j++) delxv[3 + j] = P.dfdt * x0[j] + P.dgdtm1 * v0[j];
-  const double mijinv = 1.0 / (m_i + m_j);
-  const double mi = m_i * mijinv, mj = m_j * mijinv;
-  for (int r = 0; r < 6; r++)
-    for (int l = 0; l < 6; l++) rec.put(roff + r * 6 + l, jk[r + 6 * l]);
-  rec.put(roff + PREC_MI, mi);
-  rec.put(roff + PREC_MJ, mj);
-  for (int r = 0; r < 6; r++) {
-    rec.put(roff + PREC_MC6 + r, jm[r] * m_j);
-    rec.put(roff + PREC_MC13 + r, mi * delxv[r] * mijinv + GNEWT * mj * jk[r + 6 * 6]);
-    rec.put(roff + PREC_MC6 + 6 + r, (-mj) * delxv[r] * mijinv - GNEWT * mi * jk[r + 6 * 6]);
-    rec.put(roff + PREC_MC13 + 6 + r, (-jm[r]) * m_i);
+  P.s = v[6]; P.g1 = v[7]; P.g2 = v[8]; P.g3 = v[9]; P.dfdt = v[10]; P.fm1 = v[11]; P.gmh = v[12]; P.dgdtm1 = v[13];
+  P.r0 = v[14]; P.r0inv = v[15]; P.rinv = v[16]; P.k = v[PCAP_K]; P.beta = v[18]; P.eta = v[19]; P.zeta = v[20];
+  P.h = h2;
+  KepDeriv D;
+  double K[36], psi[6];
+  kep_derivatives<DRIFT_FIRST, false>(P, D);
+  kep_block<DRIFT_FIRST>(P, D, x0, v0, K, psi);
+  const double mijinv = rcp_fast(m_i + m_j);
+#pragma unroll
+  for (int q = 0; q < 36; q++) rec.put(roff + q, K[q]);
+  rec.put(roff + PREC_MI, m_i * mijinv);
+  rec.put(roff + PREC_MJ, m_j * mijinv);
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    rec.put(roff + PREC_PSI + r, psi[r]);
+    rec.put(roff + PREC_PSI + 3 + r, psi[3 + r]);
+    rec.put(roff + PREC_B + r, mijinv * fma(P.gmh, v0[r], P.fm1 * x0[r]));
+    rec.put(roff + PREC_B + 3 + r, mijinv * fma(P.dgdtm1, v0[r], P.dfdt * x0[r]));
   }
 }
 

@@ -5,8 +5,9 @@
 // reference does, and emits the step's linear operators for the Jacobian
 // consumer instead of applying them to jac_step itself:
 //   * each Kepler pair (i, j): the 6x6 block K of jac_kepler, m_i/(m_i+m_j),
-//     m_j/(m_i+m_j) and the two mass columns of jac_ij (62 doubles) -- the
-//     14x14 jac_ij of ahl21.jl:734-750 is exactly these numbers;
+//     m_j/(m_i+m_j) and two 6-vectors that make up the two mass columns of
+//     jac_ij (50 doubles) -- the 14x14 jac_ij of ahl21.jl:734-750 is exactly
+//     these numbers (see PREC in nbg_layout.cuh);
 //   * phic!/phisalpha! (ahl21.jl:392-700): jac_phi restricted to its only
 //     non-zero block, velocity rows x (position, mass) columns (3N x 4N);
 //   * kickfast! (ahl21.jl:337-386) for pair[i,j] == true: jac_kick on the
@@ -59,7 +60,7 @@ struct Work {
   double dqop[3 * N];       // dqdt_kick or dqdt_phi velocity entries
   // last pair's jac_ij (factored) and dqdt_ij: stale values are reused when
   // G (m_i + m_j) == 0, as ahl21.jl:713 returns before refilling them.
-  double lk[36], lmi, lmj, lmc6[12], lmc13[12], ldq[14];
+  double lk[36], lmi, lmj, lpsi[6], lb[6], ldq[14];
 };
 
 #define OPX(r, c) w.op[(r) * (4 * N) + (c)]
@@ -69,7 +70,7 @@ template <int N>
 __device__ __forceinline__ void reset_last(Work<N>& w) {
   for (int q = 0; q < 36; q++) w.lk[q] = 0.0;
   w.lmi = w.lmj = 0.0;
-  for (int q = 0; q < 12; q++) w.lmc6[q] = w.lmc13[q] = 0.0;
+  for (int q = 0; q < 6; q++) w.lpsi[q] = w.lb[q] = 0.0;
   for (int q = 0; q < 14; q++) w.ldq[q] = 0.0;
 }
 
@@ -77,7 +78,7 @@ __device__ __forceinline__ void reset_last(Work<N>& w) {
 template <int N>
 __device__ __forceinline__ void drift(Sys<N>& s, double h) {
 #pragma unroll
-  for (int q = 0; q < 3 * N; q++) kahan(s.x[q], s.xe[q], h * s.v[q]);
+  for (int q = 0; q < 3 * N; q++) kahan_fma(s.x[q], s.xe[q], h, s.v[q]);
 }
 
 // kickfast! (ahl21.jl:337-386 / ahl21_no_grad.jl:35-56)
@@ -271,117 +272,193 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
     }
 }
 
-// phisalpha! (ahl21.jl:558-700 / ahl21_no_grad.jl:110-158) for Kepler pairs.
-// Accumulates onto the phic! operator (jac_phi is not cleared in between).
-template <int N, bool GRADOPS>
-__device__ void phisalpha(Sys<N>& s, Work<N>& w, double h, double alpha, uint64_t kick) {
-  for (int q = 0; q < 3 * N; q++) w.a[q] = 0.0;
-  if (GRADOPS)
-    for (int q = 0; q < 12 * N * N; q++) w.dadq[q] = 0.0;
-  double coeff = alpha * (h * h * h) / 96.0 * 2.0 * GNEWT;
+// phisalpha! (ahl21.jl:558-700 / ahl21_no_grad.jl:110-158) for Kepler pairs,
+// one pair at a time: the accelerations, then the velocity corrections.
+__device__ __forceinline__ void phis_accel(const double* rij, double* f) {
+  const double rinv = rsqrt_fast(fma(rij[2], rij[2], fma(rij[1], rij[1], rij[0] * rij[0])));
+  const double f2 = (GNEWT * rinv) * (rinv * rinv);
+#pragma unroll
+  for (int k = 0; k < 3; k++) f[k] = f2 * rij[k];
+}
+__device__ __forceinline__ void phis_corr(const double* rij, const double* aij, double mij, double coeff, double* f) {
+  const double r2 = fma(rij[2], rij[2], fma(rij[1], rij[1], rij[0] * rij[0]));
+  const double rinv = rsqrt_fast(r2);
+  const double ri2 = rinv * rinv;
+  const double fac1 = (coeff * rinv) * (ri2 * ri2);
+  const double ardot = fma(aij[2], rij[2], fma(aij[1], rij[1], aij[0] * rij[0]));
+  const double fac2 = fma((2.0 * GNEWT) * mij, rinv, 3.0 * ardot);
+#pragma unroll
+  for (int k = 0; k < 3; k++) f[k] = fac1 * fma(rij[k], fac2, -(r2 * aij[k]));
+}
+__device__ __forceinline__ double phis_coeff(double h) {  // alpha = 2 (ahl21.jl:47)
+  return 2.0 * (h * h * h) / 96.0 * 2.0 * GNEWT;
+}
+template <int N>
+__device__ __forceinline__ void phis_accel_pair(const Sys<N>& s, double* a, int i, int j) {
+  double rij[3], f[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
+  phis_accel(rij, f);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    a[3 * i + k] = fma(-s.m[j], f[k], a[3 * i + k]);
+    a[3 * j + k] = fma(s.m[i], f[k], a[3 * j + k]);
+  }
+}
+template <int N>
+__device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i, int j, double coeff) {
+  double rij[3], aij[3], f[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    aij[k] = a[3 * i + k] - a[3 * j + k];
+    rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
+  }
+  phis_corr(rij, aij, s.m[i] + s.m[j], coeff, f);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], s.m[j], f[k]);
+    kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -s.m[i], f[k]);
+  }
+}
+template <int N>
+__device__ __forceinline__ void phisalpha(Sys<N>& s, double* a, double h, uint64_t kick) {
+  const double coeff = phis_coeff(h);
+#pragma unroll
+  for (int q = 0; q < 3 * N; q++) a[q] = 0.0;
   for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++)
+      if (!((kick >> pair_bit(i, j, N)) & 1)) phis_accel_pair<N>(s, a, i, j);
+  for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++)
+      if (!((kick >> pair_bit(i, j, N)) & 1)) phis_kick_pair<N>(s, a, i, j, coeff);
+}
+
+// The corrector's operator (jac_phi, ahl21.jl:558-700) for Kepler pairs: its
+// four columns of body d (position and mass), rows 3b + k, added to
+// acc[4 (3b + k) + p].  x: the positions at the corrector, a: the
+// accelerations phisalpha formed there.
+//
+// The velocity correction of pair (i, j) is m_j F, -m_i F with
+// F = fac1 (r fac2 - r^2 (a_i - a_j)), so a column is E (r's own change) plus
+// M (a_i - a_j)' with M = fac1 (3 r r^T - r^2), and only a_d and the pairs with
+// d enter the accelerations' change: one lane per (step, body) needs no
+// 3N x 4N array and no other lane, about 110 FP64 instructions a pair.
+template <int N>
+__device__ __forceinline__ void phi_columns(const double* x, const double* a, const double* m, double h,
+                                            uint64_t kick, int d, double* acc) {
+  // change of each body's acceleration by x_d (symmetric: xx, xy, xz, yy, yz, zz) and by m_d
+  double blk[N][9];
+  double own[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const double md = m[d];
+#pragma unroll 1
+  for (int i = 0; i < N; i++) {
+#pragma unroll
+    for (int q = 0; q < 9; q++) blk[i][q] = 0.0;
+    if (i == d || ((kick >> (i < d ? pair_bit(i, d, N) : pair_bit(d, i, N))) & 1)) continue;
+    double r[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) r[k] = x[3 * i + k] - x[3 * d + k];
+    const double ri = rsqrt_fast(fma(r[2], r[2], fma(r[1], r[1], r[0] * r[0])));
+    const double ri2 = ri * ri, f2 = (GNEWT * ri) * ri2, g5 = 3.0 * f2 * ri2;
+    const double gx = g5 * r[0], gy = g5 * r[1], gz = g5 * r[2];
+    const double T[6] = {fma(gx, r[0], -f2), gx * r[1], gx * r[2], fma(gy, r[1], -f2), gy * r[2], fma(gz, r[2], -f2)};
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      blk[i][q] = -(md * T[q]);
+      own[q] = fma(m[i], T[q], own[q]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) blk[i][6 + k] = -(f2 * r[k]);
+  }
+#pragma unroll
+  for (int q = 0; q < 6; q++) blk[d][q] = own[q];
+  const double coeff = phis_coeff(h);
+#pragma unroll 1
+  for (int i = 0; i < N - 1; i++)
+#pragma unroll 1
     for (int j = i + 1; j < N; j++) {
       if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      double rij[3];
-      for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-      double r2 = rij[0] * rij[0] + rij[1] * rij[1] + rij[2] * rij[2];
-      double r3 = r2 * sqrt(r2);
-      double fac2 = GNEWT / r3;
+      double r[3], aij[3], D[9];
+#pragma unroll
       for (int k = 0; k < 3; k++) {
-        double fac = fac2 * rij[k];
-        w.a[3 * i + k] = w.a[3 * i + k] - s.m[j] * fac;
-        w.a[3 * j + k] = w.a[3 * j + k] + s.m[i] * fac;
-        if (GRADOPS) {
-          DAX(3 * i + k, 4 * j + 3) -= fac;
-          DAX(3 * j + k, 4 * i + 3) += fac;
-          fac = fac * (3.0 / r2);
-          for (int p = 0; p < 3; p++) {
-            DAX(3 * i + k, 4 * i + p) += fac * s.m[j] * rij[p];
-            DAX(3 * i + k, 4 * j + p) -= fac * s.m[j] * rij[p];
-            DAX(3 * j + k, 4 * j + p) += fac * s.m[i] * rij[p];
-            DAX(3 * j + k, 4 * i + p) -= fac * s.m[i] * rij[p];
-          }
-          DAX(3 * i + k, 4 * i + k) -= fac2 * s.m[j];
-          DAX(3 * i + k, 4 * j + k) += fac2 * s.m[j];
-          DAX(3 * j + k, 4 * j + k) -= fac2 * s.m[i];
-          DAX(3 * j + k, 4 * i + k) += fac2 * s.m[i];
+        r[k] = x[3 * i + k] - x[3 * j + k];
+        aij[k] = a[3 * i + k] - a[3 * j + k];
+      }
+#pragma unroll
+      for (int q = 0; q < 9; q++) D[q] = blk[i][q] - blk[j][q];
+      const double r2 = fma(r[2], r[2], fma(r[1], r[1], r[0] * r[0]));
+      const double ri = rsqrt_fast(r2), ri2 = ri * ri;
+      const double fac1 = (coeff * ri) * (ri2 * ri2), f3 = 3.0 * fac1, fr = fac1 * r2;
+      double G[3][4];
+      const double col[4][3] = {{D[0], D[1], D[2]}, {D[1], D[3], D[4]}, {D[2], D[4], D[5]}, {D[6], D[7], D[8]}};
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const double c = f3 * fma(r[2], col[p][2], fma(r[1], col[p][1], r[0] * col[p][0]));
+#pragma unroll
+        for (int k = 0; k < 3; k++) G[k][p] = fma(r[k], c, -(fr * col[p][k]));
+      }
+      if (d == i || d == j) {
+        const double mij = m[i] + m[j];
+        const double ardot = fma(aij[2], r[2], fma(aij[1], r[1], aij[0] * r[0]));
+        const double gri = (2.0 * GNEWT) * ri, fac2 = fma(gri, mij, 3.0 * ardot);
+        const double sg = (d == i) ? 1.0 : -1.0;
+        const double q5 = -5.0 * ri2, q3 = gri * ri2 * mij, diag = sg * (fac1 * fac2), fg = fac1 * gri;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const double F = fac1 * fma(r[k], fac2, -(r2 * aij[k]));
+          const double e = sg * fma(q5, F, -(fac1 * fma(q3, r[k], 2.0 * aij[k]))), f = sg * (f3 * r[k]);
+#pragma unroll
+          for (int p = 0; p < 3; p++) G[k][p] = fma(f, aij[p], fma(e, r[p], G[k][p]));
+          G[k][k] = G[k][k] + diag;
+          G[k][3] = fma(fg, r[k], G[k][3]);
+          acc[12 * (d == i ? j : i) + 4 * k + 3] += (d == i) ? -F : F;
         }
       }
+      const double mi = -m[i], mj = m[j];
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          acc[12 * i + 4 * k + p] = fma(mj, G[k][p], acc[12 * i + 4 * k + p]);
+          acc[12 * j + 4 * k + p] = fma(mi, G[k][p], acc[12 * j + 4 * k + p]);
+        }
     }
+}
+
+// The same for every body, onto w.op, and d(v)/dh of the corrector, onto w.dqop.
+template <int N>
+__device__ void phisalpha_operator(const Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
+  for (int d = 0; d < N; d++) {
+    double acc[12 * N];
+    for (int q = 0; q < 12 * N; q++) acc[q] = 0.0;
+    phi_columns<N>(s.x, w.a, s.m, h, kick, d, acc);
+    for (int r = 0; r < 3 * N; r++)
+      for (int p = 0; p < 4; p++) OPX(r, 4 * d + p) += acc[4 * r + p];
+  }
+  const double coeff = phis_coeff(h), hi3 = 3.0 / h;
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++) {
       if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      double rij[3], aij[3];
+      double rij[3], aij[3], f[3];
       for (int k = 0; k < 3; k++) {
         aij[k] = w.a[3 * i + k] - w.a[3 * j + k];
         rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
       }
-      if (GRADOPS) {
-        for (int q = 0; q < 4 * N; q++) w.dot[q] = 0.0;
-        for (int di = 0; di < N; di++)
-          for (int p = 0; p < 4; p++)
-            for (int k = 0; k < 3; k++)
-              w.dot[4 * di + p] += rij[k] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-      }
-      double r2 = rij[0] * rij[0] + rij[1] * rij[1] + rij[2] * rij[2];
-      double r1 = sqrt(r2);
-      double ardot = aij[0] * rij[0] + aij[1] * rij[1] + aij[2] * rij[2];
-      double fac1 = coeff / (r2 * r2 * r1);
-      double mij = s.m[i] + s.m[j];
-      double fac2 = 2.0 * GNEWT * mij / r1 + 3.0 * ardot;
+      phis_corr(rij, aij, s.m[i] + s.m[j], coeff, f);
       for (int k = 0; k < 3; k++) {
-        double fac = fac1 * (rij[k] * fac2 - r2 * aij[k]);
-        kahan(s.v[3 * i + k], s.ve[3 * i + k], s.m[j] * fac);
-        kahan(s.v[3 * j + k], s.ve[3 * j + k], (-s.m[i]) * fac);
-        if (GRADOPS) {
-          w.dqop[3 * i + k] = w.dqop[3 * i + k] + 3.0 / h * s.m[j] * fac;
-          w.dqop[3 * j + k] = w.dqop[3 * j + k] - 3.0 / h * s.m[i] * fac;
-          OPX(3 * i + k, 4 * j + 3) += fac;
-          OPX(3 * j + k, 4 * i + 3) -= fac;
-          fac = fac * (5.0 / r2);
-          for (int p = 0; p < 3; p++) {
-            OPX(3 * i + k, 4 * i + p) -= fac * s.m[j] * rij[p];
-            OPX(3 * i + k, 4 * j + p) += fac * s.m[j] * rij[p];
-            OPX(3 * j + k, 4 * j + p) -= fac * s.m[i] * rij[p];
-            OPX(3 * j + k, 4 * i + p) += fac * s.m[i] * rij[p];
-          }
-          fac = 2.0 * GNEWT * fac1 * rij[k] / r1;
-          OPX(3 * i + k, 4 * i + 3) += fac * s.m[j];
-          OPX(3 * i + k, 4 * j + 3) += fac * s.m[j];
-          OPX(3 * j + k, 4 * j + 3) -= fac * s.m[i];
-          OPX(3 * j + k, 4 * i + 3) -= fac * s.m[i];
-          fac = fac1 * fac2;
-          OPX(3 * i + k, 4 * i + k) += fac * s.m[j];
-          OPX(3 * i + k, 4 * j + k) -= fac * s.m[j];
-          OPX(3 * j + k, 4 * j + k) += fac * s.m[i];
-          OPX(3 * j + k, 4 * i + k) -= fac * s.m[i];
-          fac = -2.0 * fac1 * (rij[k] * GNEWT * mij / (r2 * r1) + aij[k]);
-          for (int p = 0; p < 3; p++) {
-            double fac3 = fac * rij[p] + fac1 * 3.0 * rij[k] * aij[p];
-            OPX(3 * i + k, 4 * i + p) += s.m[j] * fac3;
-            OPX(3 * i + k, 4 * j + p) -= s.m[j] * fac3;
-            OPX(3 * j + k, 4 * j + p) += s.m[i] * fac3;
-            OPX(3 * j + k, 4 * i + p) -= s.m[i] * fac3;
-          }
-          fac = (-fac1) * r2;
-          for (int di = 0; di < N; di++) {
-            for (int p = 0; p < 3; p++)
-              OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-            for (int p = 0; p < 3; p++)
-              OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-            OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
-            OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
-          }
-          fac = 3.0 * fac1 * rij[k];
-          for (int di = 0; di < N; di++) {
-            for (int p = 0; p < 3; p++) OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * w.dot[4 * di + p];
-            for (int p = 0; p < 3; p++) OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * w.dot[4 * di + p];
-            OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * w.dot[4 * di + 3];
-            OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * w.dot[4 * di + 3];
-          }
-        }
+        w.dqop[3 * i + k] = fma(hi3 * s.m[j], f[k], w.dqop[3 * i + k]);
+        w.dqop[3 * j + k] = fma(-hi3 * s.m[i], f[k], w.dqop[3 * j + k]);
       }
     }
+}
+
+// Writes one solved pair's capture: x0, v0 and the KepParams but h.
+__device__ __forceinline__ void put_capture(const Rec& cap, int coff, const double* x0, const double* v0,
+                                            const KepParams& P) {
+  const double pv[PCAP] = {x0[0], x0[1], x0[2], v0[0],  v0[1],    v0[2], P.s, P.g1,    P.g2,   P.g3,  P.dfdt,
+                           P.fm1, P.gmh, P.dgdtm1, P.r0, P.r0inv, P.rinv, P.k, P.beta, P.eta, P.zeta};
+#pragma unroll
+  for (int q = 0; q < PCAP; q++) cap.put(coff + q, pv[q]);
 }
 
 // kepler_driftij_gamma! (ahl21.jl:706-760 with the block update of :31-42 on
@@ -390,62 +467,54 @@ template <int N, bool DRIFT_FIRST, bool GRADOPS, bool DQDT>
 __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, const Rec& rec, int roff,
                             const Rec& cap, int coff) {
   double x0[3], v0[3];
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     x0[k] = s.x[3 * i + k] - s.x[3 * j + k];
     v0[k] = s.v[3 * i + k] - s.v[3 * j + k];
   }
-  double gm = GNEWT * (s.m[i] + s.m[j]);
-  if (cap.p && gm == 0.0) cap.put(coff + 6 + 15, 0.0);  // k = 0 marks a pair that keeps the stale jac_ij
+  const double mij = s.m[i] + s.m[j];
+  const double gm = GNEWT * mij;
+  if (cap.p && gm == 0.0) cap.put(coff + PCAP_K, 0.0);  // k = 0 marks a pair that keeps the stale jac_ij
   if (gm != 0.0) {
     KepParams P;
     double delxv[6];
-    kep_delxv<DRIFT_FIRST, GRADOPS>(x0, v0, gm, h2, delxv, P);
-    if (cap.p) {
-      for (int q = 0; q < 3; q++) {
-        cap.put(coff + q, x0[q]);
-        cap.put(coff + 3 + q, v0[q]);
-      }
-      const double pv[22] = {P.gamma, P.g0, P.g1, P.g2, P.g3, P.h1, P.h2, P.dfdt, P.fm1, P.gmh, P.dgdtm1,
-                             P.r0, P.r, P.r0inv, P.rinv, P.k, P.h, P.beta, P.betainv, P.eta, P.sqb, P.zeta};
-      for (int q = 0; q < 22; q++) cap.put(coff + 6 + q, pv[q]);
-    }
-    double mijinv = 1.0 / (s.m[i] + s.m[j]);
-    double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
+    kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
+    if (cap.p) put_capture(cap, coff, x0, v0, P);
+    const double mijinv = rcp_fast(mij);
+    const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
     if (GRADOPS) {
-      double jk[48], jm[6];
-      kep_jacobian<DRIFT_FIRST>(P, x0, v0, jk, jm);
-      for (int r = 0; r < 6; r++)
-        for (int l = 0; l < 6; l++) w.lk[r * 6 + l] = jk[r + 6 * l];
+      KepDeriv D;
+      double dh[6];
+      kep_derivatives<DRIFT_FIRST, true>(P, D);
+      kep_block<DRIFT_FIRST>(P, D, x0, v0, w.lk, w.lpsi);
+      kep_by_h<DRIFT_FIRST>(P, D, x0, v0, dh);
       w.lmi = mi;
       w.lmj = mj;
       for (int r = 0; r < 6; r++) {
-        w.lmc6[r] = jm[r] * s.m[j];
-        w.lmc13[r] = mi * delxv[r] * mijinv + GNEWT * mj * jk[r + 6 * 6];
-        w.lmc6[6 + r] = (-mj) * delxv[r] * mijinv - GNEWT * mi * jk[r + 6 * 6];
-        w.lmc13[6 + r] = (-jm[r]) * s.m[i];
-      }
-      for (int r = 0; r < 6; r++) {
-        w.ldq[r] = mj * jk[r + 6 * 7];
-        w.ldq[7 + r] = (-mi) * jk[r + 6 * 7];
+        w.lb[r] = mijinv * delxv[r];
+        w.ldq[r] = mj * dh[r];
+        w.ldq[7 + r] = (-mi) * dh[r];
       }
       w.ldq[6] = w.ldq[13] = 0.0;
     }
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-      kahan(s.x[3 * i + k], s.xe[3 * i + k], mj * delxv[k]);
-      kahan(s.x[3 * j + k], s.xe[3 * j + k], (-mi) * delxv[k]);
+      kahan_fma(s.x[3 * i + k], s.xe[3 * i + k], mj, delxv[k]);
+      kahan_fma(s.x[3 * j + k], s.xe[3 * j + k], -mi, delxv[k]);
     }
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-      kahan(s.v[3 * i + k], s.ve[3 * i + k], mj * delxv[3 + k]);
-      kahan(s.v[3 * j + k], s.ve[3 * j + k], (-mi) * delxv[3 + k]);
+      kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], mj, delxv[3 + k]);
+      kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -mi, delxv[3 + k]);
     }
   }
   if (GRADOPS && rec.p) {
     for (int q = 0; q < 36; q++) rec.put(roff + q, w.lk[q]);
     rec.put(roff + PREC_MI, w.lmi);
     rec.put(roff + PREC_MJ, w.lmj);
-    for (int q = 0; q < 12; q++) {
-      rec.put(roff + PREC_MC6 + q, w.lmc6[q]);
-      rec.put(roff + PREC_MC13 + q, w.lmc13[q]);
+    for (int q = 0; q < 6; q++) {
+      rec.put(roff + PREC_PSI + q, w.lpsi[q]);
+      rec.put(roff + PREC_B + q, w.lb[q]);
     }
   }
   if (DQDT) {
@@ -518,7 +587,10 @@ __device__ __noinline__ void ahl21_step(Sys<N>& s, Work<N>& w, double h, uint64_
   if (xs.p)
     for (int q = 0; q < 3 * N; q++) xs.put(q, s.x[q]);
   phic<N, GRADOPS>(s, w, h, kick);
-  phisalpha<N, GRADOPS>(s, w, h, 2.0, kick);
+  phisalpha<N>(s, w.a, h, kick);  // moves v alone: the operator below is that of the same positions
+  if (xs.p && !kick)
+    for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, w.a[q]);
+  if (GRADOPS) phisalpha_operator<N>(s, w, h, kick);
   if (DQDT) dqdt_op(s, w, 1.0);
   if (GRADOPS) put_op(rec, roff, w.op, op_size(N));
   roff += op_size(N);
@@ -581,27 +653,26 @@ __device__ void adj_op(double* u, const Rec& rec, int roff) {
 // u <- u + A^T u for one Kepler pair record (the transpose of the factored
 // jac_ij update the consumer applies).
 __device__ __forceinline__ void adj_pair(double* u, int i, int j, const Rec& rec, int roff) {
-  double mi = rec.get(roff + PREC_MI), mj = rec.get(roff + PREC_MJ);
-  double z[6], ymi = 0.0, ymj = 0.0;
+  const double mi = rec.get(roff + PREC_MI), mj = rec.get(roff + PREC_MJ);
+  double z[6], psi = 0.0, bi = 0.0, bj = 0.0;
+#pragma unroll
   for (int r = 0; r < 6; r++) {
-    z[r] = mj * u[7 * i + r] - mi * u[7 * j + r];
-    ymi = fma(rec.get(roff + PREC_MC6 + r), u[7 * i + r], ymi);
-    ymi = fma(rec.get(roff + PREC_MC6 + 6 + r), u[7 * j + r], ymi);
-    ymj = fma(rec.get(roff + PREC_MC13 + r), u[7 * i + r], ymj);
-    ymj = fma(rec.get(roff + PREC_MC13 + 6 + r), u[7 * j + r], ymj);
+    const double ui = u[7 * i + r], uj = u[7 * j + r], b = rec.get(roff + PREC_B + r);
+    z[r] = fma(mj, ui, -(mi * uj));
+    psi = fma(rec.get(roff + PREC_PSI + r), z[r], psi);
+    bi = fma(b, uj, bi);
+    bj = fma(b, ui, bj);
   }
-  double y[6];
+#pragma unroll
   for (int l = 0; l < 6; l++) {
     double acc = 0.0;
+#pragma unroll
     for (int r = 0; r < 6; r++) acc = fma(rec.get(roff + r * 6 + l), z[r], acc);
-    y[l] = acc;
+    u[7 * i + l] = u[7 * i + l] + acc;
+    u[7 * j + l] = u[7 * j + l] - acc;
   }
-  for (int l = 0; l < 6; l++) {
-    u[7 * i + l] = u[7 * i + l] + y[l];
-    u[7 * j + l] = u[7 * j + l] - y[l];
-  }
-  u[7 * i + 6] = u[7 * i + 6] + ymi;
-  u[7 * j + 6] = u[7 * j + 6] + ymj;
+  u[7 * i + 6] = u[7 * i + 6] + (psi - bi);
+  u[7 * j + 6] = u[7 * j + 6] + (psi + bj);
 }
 
 // Adjoint of one recorded step: u^T <- u^T S where S is the step's map on

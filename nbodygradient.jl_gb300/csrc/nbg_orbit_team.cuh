@@ -30,43 +30,6 @@ namespace nbg {
 
 __host__ __device__ constexpr int team_lanes(int N) { return N / 2 > 1 ? N / 2 : 1; }
 
-// phisalpha!, first pair loop (accelerations), for one pair; the same
-// operations in the same order as phisalpha<N, false>.
-template <int N>
-__device__ __forceinline__ void phis_accel_pair(const Sys<N>& s, double* a, int i, int j) {
-  double rij[3];
-  for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-  double r2 = rij[0] * rij[0] + rij[1] * rij[1] + rij[2] * rij[2];
-  double r3 = r2 * sqrt(r2);
-  double fac2 = GNEWT / r3;
-  for (int k = 0; k < 3; k++) {
-    double fac = fac2 * rij[k];
-    a[3 * i + k] = a[3 * i + k] - s.m[j] * fac;
-    a[3 * j + k] = a[3 * j + k] + s.m[i] * fac;
-  }
-}
-
-// phisalpha!, second pair loop (velocity corrections), for one pair.
-template <int N>
-__device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i, int j, double coeff) {
-  double rij[3], aij[3];
-  for (int k = 0; k < 3; k++) {
-    aij[k] = a[3 * i + k] - a[3 * j + k];
-    rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-  }
-  double r2 = rij[0] * rij[0] + rij[1] * rij[1] + rij[2] * rij[2];
-  double r1 = sqrt(r2);
-  double ardot = aij[0] * rij[0] + aij[1] * rij[1] + aij[2] * rij[2];
-  double fac1 = coeff / (r2 * r2 * r1);
-  double mij = s.m[i] + s.m[j];
-  double fac2 = 2.0 * GNEWT * mij / r1 + 3.0 * ardot;
-  for (int k = 0; k < 3; k++) {
-    double fac = fac1 * (rij[k] * fac2 - r2 * aij[k]);
-    kahan(s.v[3 * i + k], s.ve[3 * i + k], s.m[j] * fac);
-    kahan(s.v[3 * j + k], s.ve[3 * j + k], (-s.m[i]) * fac);
-  }
-}
-
 // The pair of level `lev` (i + j == lev) that lane t of a team takes, if any.
 template <int N>
 __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {
@@ -78,45 +41,37 @@ __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {
   return true;
 }
 
-// kepler_pair<N, DRIFT_FIRST, false, false> on the two lanes of a pair slot
-// (kep_delxv2): both lanes read the pair's coordinates and solve it; role 0
-// then updates body i and writes the first half of the capture, role 1 body
-// j and the rest.  x_i and x_j are separate variables, so splitting their
-// updates between the lanes changes no value.
+// kepler_pair<N, DRIFT_FIRST, false, false> on the two lanes of a pair slot:
+// both lanes read the pair's coordinates and solve it; role 0 then updates
+// body i and writes the first half of the capture, role 1 body j and the
+// rest.  x_i and x_j are separate variables, so splitting their updates
+// between the lanes changes no value.
 template <int N, bool DRIFT_FIRST>
 __device__ __forceinline__ void kepler_pair_w2(Sys<N>& s, int i, int j, double h2, const Rec& cap, int coff,
                                                int role, unsigned mask, int base) {
   double x0[3], v0[3];
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     x0[k] = s.x[3 * i + k] - s.x[3 * j + k];
     v0[k] = s.v[3 * i + k] - s.v[3 * j + k];
   }
-  const double gm = GNEWT * (s.m[i] + s.m[j]);
+  const double mij = s.m[i] + s.m[j];
+  const double gm = GNEWT * mij;
   __syncwarp(mask);  // both lanes have read the pair before either writes
-  if (cap.p && gm == 0.0 && role == 0) cap.put(coff + 6 + 15, 0.0);
+  if (cap.p && gm == 0.0 && role == 0) cap.put(coff + PCAP_K, 0.0);
   if (gm != 0.0) {
     KepParams P;
     double delxv[6];
-    kep_delxv2<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P, role, mask, base);
-    if (cap.p) {
-      const double pv[22] = {P.gamma, P.g0, P.g1, P.g2, P.g3, P.h1, P.h2, P.dfdt, P.fm1, P.gmh, P.dgdtm1,
-                             P.r0, P.r, P.r0inv, P.rinv, P.k, P.h, P.beta, P.betainv, P.eta, P.sqb, P.zeta};
-      if (role == 0) {
-        for (int q = 0; q < 3; q++) {
-          cap.put(coff + q, x0[q]);
-          cap.put(coff + 3 + q, v0[q]);
-        }
-        for (int q = 0; q < 8; q++) cap.put(coff + 6 + q, pv[q]);
-      } else {
-        for (int q = 8; q < 22; q++) cap.put(coff + 6 + q, pv[q]);
-      }
-    }
-    const double mijinv = 1.0 / (s.m[i] + s.m[j]);
+    kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
+    if (cap.p && role == 0) put_capture(cap, coff, x0, v0, P);
+    const double mijinv = rcp_fast(mij);
     const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
     const int b = role ? j : i;
     const double f = role ? (-mi) : mj;
-    for (int k = 0; k < 3; k++) kahan(s.x[3 * b + k], s.xe[3 * b + k], f * delxv[k]);
-    for (int k = 0; k < 3; k++) kahan(s.v[3 * b + k], s.ve[3 * b + k], f * delxv[3 + k]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) kahan_fma(s.x[3 * b + k], s.xe[3 * b + k], f, delxv[k]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) kahan_fma(s.v[3 * b + k], s.ve[3 * b + k], f, delxv[3 + k]);
   }
 }
 
@@ -137,7 +92,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
   const unsigned mask = (R == 2) ? (3u << base) : 0u;
   const double h2 = 0.5 * h;
   if (run)
-    for (int q = t; q < 3 * N; q += L) kahan(s.x[q], s.xe[q], h2 * s.v[q]);
+    for (int q = t; q < 3 * N; q += L) kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
   __syncwarp();
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
@@ -153,12 +108,14 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
     for (int q = t; q < 3 * N; q += L) a[q] = 0.0;
   }
   __syncwarp();
-  const double coeff = 2.0 * (h * h * h) / 96.0 * 2.0 * GNEWT;  // alpha = 2 (ahl21.jl:47)
+  const double coeff = phis_coeff(h);
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
     if (run && role == 0 && level_pair<N>(lev, p, &i, &j)) phis_accel_pair<N>(s, a, i, j);
     __syncwarp();
   }
+  if (run && xs.p)
+    for (int q = t; q < 3 * N; q += L) xs.put(3 * N + q, a[q]);
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
     if (run && role == 0 && level_pair<N>(lev, p, &i, &j)) phis_kick_pair<N>(s, a, i, j, coeff);
@@ -174,7 +131,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
     __syncwarp();
   }
   if (run)
-    for (int q = t; q < 3 * N; q += L) kahan(s.x[q], s.xe[q], h2 * s.v[q]);
+    for (int q = t; q < 3 * N; q += L) kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
   __syncwarp();
 }
 
