@@ -139,7 +139,8 @@ __device__ __forceinline__ void drift_rows(double* J, double* E, double h) {
     for (int k = 0; k < 3; k++) kahan(J[(6 * b + k) * BS], E[(6 * b + k) * BS], h * J[(6 * b + 3 + k) * BS]);
 }
 
-// One recorded step on this column (ahl21.jl:5-95, the jac_step updates).
+// One recorded step on this column (ahl21.jl:5-95, the jac_step updates), for
+// groups with kick pairs.
 template <int N, int BS>
 __device__ void apply_step(double* J, double* E, int c, double h, uint64_t kick, const Rec& rec) {
   const double h2 = 0.5 * h;
@@ -178,6 +179,150 @@ __device__ void apply_step(double* J, double* E, int c, double h, uint64_t kick,
   } else {
     fold_all<N, BS>(J, E);
   }
+}
+
+// ------------------------------------------------- groups without kick pairs
+//
+// The same updates with the Kahan pair (S, E) normalised less often: an update
+// adds its increment to E in one FMA, J is S + E wherever it is read, and
+// (S, E) <- (S + E, (S - (S + E)) + E) follows not after every update but where
+// E holds a large increment: after the first drift (position rows), after the
+// forward sweep's pairs with body 0 (velocity rows; the pairs between planets
+// then add to a small E until the backward sweep's last pairs) and at the end
+// of the step.  An addition to E rounds at the size of the increments in it, as
+// the increment's own product does: against an extended-precision consumer of
+// the same records, 2000 steps of two 8-body systems leave 2.3e-13 and 2.5e-13
+// of jac_step where a Kahan sum at every update leaves 3.3e-13 and 2.5e-13.
+// Per column and pair 66 FP64 instructions instead of 102, and no folds; per
+// column-step at three bodies 600 instead of 864.  FP64 issue bounds the
+// kernel: 4096 three-body systems over 2000 steps went from 532 to 361 ms a
+// pass, 1024 eight-body systems over 200 steps from 273 to 202 ms.
+//
+// The corrector's operator depends on position differences alone (the sum of
+// its blocks over all bodies is zero), so it is applied to J_d - J_0.
+//
+// MASS: the column is a mass column (c % 7 == 6); the other columns, six of
+// seven, share no warp with them and carry none of their terms.
+
+__device__ __forceinline__ void normalise(double& s, double& e, double t) {  // t = s + e
+  e = (s - t) + e;
+  s = t;
+}
+
+template <int N, int BS, bool MASS>
+__device__ __forceinline__ void pair_update(double* S, double* E, int c, int i, int j, const Rec& rec, int roff) {
+  double K[36];
+#pragma unroll
+  for (int q = 0; q < 36; q++) K[q] = rec.get(roff + q);
+  const double mi = rec.get(roff + PREC_MI), mj = rec.get(roff + PREC_MJ);
+  const bool ci = MASS && c == 7 * i + 6, cj = MASS && c == 7 * j + 6;
+  double U[6], B[6];
+  if (MASS) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      U[q] = (ci || cj) ? rec.get(roff + PREC_PSI + q) : 0.0;
+      B[q] = (ci || cj) ? rec.get(roff + PREC_B + q) : 0.0;
+    }
+  }
+  double D[6];
+#pragma unroll
+  for (int l = 0; l < 6; l++)
+    D[l] = (S[(6 * i + l) * BS] + E[(6 * i + l) * BS]) - (S[(6 * j + l) * BS] + E[(6 * j + l) * BS]);
+#pragma unroll
+  for (int r = 0; r < 6; r++) {
+    double u = MASS ? fma(K[r * 6], D[0], U[r]) : K[r * 6] * D[0];
+#pragma unroll
+    for (int l = 1; l < 6; l++) u = fma(K[r * 6 + l], D[l], u);
+    double ei = fma(mj, u, E[(6 * i + r) * BS]), ej = fma(-mi, u, E[(6 * j + r) * BS]);
+    if (MASS) {
+      ei = ei + (cj ? B[r] : 0.0);
+      ej = ej - (ci ? B[r] : 0.0);
+    }
+    E[(6 * i + r) * BS] = ei;
+    E[(6 * j + r) * BS] = ej;
+  }
+}
+
+template <int N, int BS, bool MASS>
+__device__ __forceinline__ void corrector_update(const double* S, double* E, int c, const Rec& rec, int roff) {
+  double D[3 * N];  // D[3d + k]: position rows of body d less those of body 0
+#pragma unroll
+  for (int k = 0; k < 3; k++) D[k] = S[k * BS] + E[k * BS];
+#pragma unroll
+  for (int d = 1; d < N; d++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) D[3 * d + k] = (S[(6 * d + k) * BS] + E[(6 * d + k) * BS]) - D[k];
+  const int cm = c / 7;
+#pragma unroll 1
+  for (int b = 0; b < N; b++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int rb = roff + (3 * b + k) * (4 * N);
+      double acc = MASS ? fma(rec.get(rb + 4), D[3], rec.get(rb + 4 * cm + 3)) : rec.get(rb + 4) * D[3];
+#pragma unroll
+      for (int q = 1; q < 3 * (N - 1); q++) acc = fma(rec.get(rb + 4 + 4 * (q / 3) + q % 3), D[3 + q], acc);
+      E[(6 * b + 3 + k) * BS] = E[(6 * b + 3 + k) * BS] + acc;
+    }
+}
+
+// One recorded step of a kick-free group on this column.  S and E arrive and
+// leave normalised (S + E rounds to S).
+template <int N, int BS, bool MASS>
+__device__ __forceinline__ void column_step(double* S, double* E, int c, double h, const Rec& rec) {
+  const double h2 = 0.5 * h;
+#pragma unroll
+  for (int b = 0; b < N; b++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int r = (6 * b + k) * BS;
+      double s = S[r], e = fma(h2, S[r + 3 * BS], E[r]);
+      normalise(s, e, s + e);
+      S[r] = s;
+      E[r] = e;
+    }
+  int roff = 0;
+#pragma unroll 1
+  for (int i = 0; i < N - 1; i++) {
+#pragma unroll 1
+    for (int j = i + 1; j < N; j++) {
+      pair_update<N, BS, MASS>(S, E, c, i, j, rec, roff);
+      roff += PREC;
+    }
+    if (N > 2 && i == 0) {
+#pragma unroll
+      for (int q = 0; q < 3 * N; q++) {
+        const int r = (6 * (q / 3) + 3 + q % 3) * BS;
+        double s = S[r], e = E[r];
+        normalise(s, e, s + e);
+        S[r] = s;
+        E[r] = e;
+      }
+    }
+  }
+  corrector_update<N, BS, MASS>(S, E, c, rec, roff);
+  roff += op_size(N);
+#pragma unroll 1
+  for (int i = N - 2; i >= 0; i--)
+#pragma unroll 1
+    for (int j = N - 1; j > i; j--) {
+      pair_update<N, BS, MASS>(S, E, c, i, j, rec, roff);
+      roff += PREC;
+    }
+#pragma unroll
+  for (int b = 0; b < N; b++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int r = (6 * b + k) * BS, rv = r + 3 * BS;
+      double sv = S[rv], ev = E[rv];
+      const double tv = sv + ev;
+      normalise(sv, ev, tv);
+      S[rv] = sv;
+      E[rv] = ev;
+      double s = S[r], e = fma(h2, tv, E[r]);
+      normalise(s, e, s + e);
+      S[r] = s;
+      E[r] = e;
+    }
 }
 
 }  // namespace nbg

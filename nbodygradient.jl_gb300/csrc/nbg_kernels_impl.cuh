@@ -458,89 +458,118 @@ __global__ void __launch_bounds__(OPS_BS) operator_kick_kernel(GroupArgs g, int 
   put_op(rec, off_phi + op_size(N) + g.npk * PREC, w.op, op_size(N));
 }
 
-// Jacobian consumer for one chunk of K steps (one lane per column).
-template <int N>
-__global__ void __launch_bounds__(CONS_BS) jacobian_chunk_kernel(GroupArgs g, int chunk) {
-  extern __shared__ double smem[];
+// dtdq0 entries of this column for the transits of step kk (dtbvdq!,
+// timing.jl:155-193), from their adjoint rows.
+template <int N, int BS>
+__device__ __forceinline__ void column_transits(const GroupArgs& g, int s, int c, int kk, int ti, int ntt, int gsys,
+                                                const double* J, const double* E) {
+  const int S = g.S, cb = c / 7, ck = c % 7;  // column c is d/d q0[ck] of body cb
+  for (int o = 0; o < N - 1; o++) {
+    const int flag = g.tflag[(size_t)(kk * (N - 1) + o) * S + s];
+    if (flag < 0) continue;
+    const double* tr = g.trec + ((size_t)(kk * (N - 1) + o) * trec_size(N, g.tbv)) * S + s;
+    const int ib = (o < ti) ? o : o + 1;
+    if (!g.tbv) {
+      double acc = 0.0;
+      for (int b = 0; b < N; b++)
+        for (int r = 0; r < 6; r++) {
+          const double ur = tr[(size_t)(7 * b + r) * S];
+          acc = fma(ur, J[(6 * b + r) * BS], acc);
+          acc = fma(ur, E[(6 * b + r) * BS], acc);
+        }
+      if (ck == 6) acc = acc + tr[(size_t)c * S];  // unit mass row of this column
+      const double gd = tr[(size_t)(7 * N) * S];
+      g.dtdq0[g.off_dq[gsys] + ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb))] = -acc / gd;
+    } else {
+      double acc[3] = {0.0, 0.0, 0.0};
+      for (int b = 0; b < N; b++)
+        for (int r = 0; r < 6; r++) {
+          const double jv = J[(6 * b + r) * BS], ev = E[(6 * b + r) * BS];
+          for (int w = 0; w < 3; w++) {
+            const double ur = tr[(size_t)(7 * N * w + 7 * b + r) * S];
+            acc[w] = fma(ur, jv, acc[w]);
+            acc[w] = fma(ur, ev, acc[w]);
+          }
+        }
+      if (ck == 6)
+        for (int w = 0; w < 3; w++) acc[w] = acc[w] + tr[(size_t)(7 * N * w + c) * S];
+      const double gd = tr[(size_t)(21 * N) * S], vsky = tr[(size_t)(21 * N + 1) * S];
+      const double dvdt = tr[(size_t)(21 * N + 2) * S];
+      const double d1 = -acc[0] / gd;
+      double* out = g.dtdq0 + g.off_dq[gsys] + 3 * (ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb)));
+      out[0] = d1;
+      out[1] = acc[1] / vsky + dvdt * d1;
+      out[2] = 2.0 * acc[2];
+    }
+  }
+}
+
+// Jacobian consumer for one chunk of K steps (one lane per column).  A group
+// without kick pairs has its mass columns in blocks of their own: the first
+// `plain` blocks hold the other 6N columns of every system, the rest the N mass
+// columns.
+template <int N, int BS, int MODE>  // 0: kick group, every column; 1: not a mass column; 2: a mass column
+__device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int s, int c, double* smem) {
   constexpr int M = 7 * N, R6 = 6 * N;
-  const int f = blockIdx.x * CONS_BS + threadIdx.x;
-  const int s = f / M, c = f % M;
   if (s >= g.S || g.sysidx[s] < 0) return;
   const int S = g.S;
   const long long nst = g.nsteps[s];
   const long long k0 = chunk_first_step(g, chunk, s);
   if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
   double* J = smem + threadIdx.x;
-  double* E = smem + R6 * CONS_BS + threadIdx.x;
-  const double* Jg = g.Jint + (size_t)s * R6 * M + c;
-  const double* Eg = g.Eint + (size_t)s * R6 * M + c;
+  double* E = smem + R6 * BS + threadIdx.x;
+  double* Jg = g.Jint + (size_t)s * R6 * M + c;
+  double* Eg = g.Eint + (size_t)s * R6 * M + c;
   for (int r = 0; r < R6; r++) {
-    J[r * CONS_BS] = Jg[(size_t)r * M];
-    E[r * CONS_BS] = Eg[(size_t)r * M];
+    double jv = Jg[(size_t)r * M], ev = Eg[(size_t)r * M];
+    if (MODE != 0 && k0 == 0) fold(jv, ev);  // a caller's pair may not be normalised
+    J[r * BS] = jv;
+    E[r * BS] = ev;
   }
   const double h = g.h[s];
   const int ntt = g.ntt[s], ti = g.ti[s];
   const int gsys = g.sysidx[s];
-  const uint64_t kick = g.kick;
-  const int cb = c / 7, ck = c % 7;  // column c is d/d q0[ck] of body cb
   for (int kk = 0; kk < g.K; kk++) {
     const long long istep = k0 + kk;
     if (istep >= nst) break;
     Rec rec{g.steprec + (size_t)kk * g.R * S + s, S};
     if (g.trajJ) {  // column c of jac_step at the start of the step; mass rows are unit rows
       double* rj = g.trajJ + (((size_t)s * g.K + kk) * M + c) * M;
-      for (int r = 0; r < M; r++) rj[r] = (r % 7 == 6) ? ((r == c) ? 1.0 : 0.0) : J[(6 * (r / 7) + r % 7) * CONS_BS];
+      for (int r = 0; r < M; r++) rj[r] = (r % 7 == 6) ? ((r == c) ? 1.0 : 0.0) : J[(6 * (r / 7) + r % 7) * BS];
     }
-    apply_step<N, CONS_BS>(J, E, c, step_length(g, s, istep, nst, h), kick, rec);
-    if (g.notransit) continue;
-    for (int o = 0; o < N - 1; o++) {
-      const int flag = g.tflag[(size_t)(kk * (N - 1) + o) * S + s];
-      if (flag < 0) continue;
-      const double* tr = g.trec + ((size_t)(kk * (N - 1) + o) * trec_size(N, g.tbv)) * S + s;
-      const int ib = (o < ti) ? o : o + 1;
-      if (!g.tbv) {
-        double acc = 0.0;
-        for (int b = 0; b < N; b++)
-          for (int r = 0; r < 6; r++) {
-            const double ur = tr[(size_t)(7 * b + r) * S];
-            acc = fma(ur, J[(6 * b + r) * CONS_BS], acc);
-            acc = fma(ur, E[(6 * b + r) * CONS_BS], acc);
-          }
-        if (ck == 6) acc = acc + tr[(size_t)c * S];  // unit mass row of this column
-        const double gd = tr[(size_t)(7 * N) * S];
-        g.dtdq0[g.off_dq[gsys] + ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb))] = -acc / gd;
-      } else {
-        double acc[3] = {0.0, 0.0, 0.0};
-        for (int b = 0; b < N; b++)
-          for (int r = 0; r < 6; r++) {
-            const double jv = J[(6 * b + r) * CONS_BS], ev = E[(6 * b + r) * CONS_BS];
-            for (int w = 0; w < 3; w++) {
-              const double ur = tr[(size_t)(7 * N * w + 7 * b + r) * S];
-              acc[w] = fma(ur, jv, acc[w]);
-              acc[w] = fma(ur, ev, acc[w]);
-            }
-          }
-        if (ck == 6)
-          for (int w = 0; w < 3; w++) acc[w] = acc[w] + tr[(size_t)(7 * N * w + c) * S];
-        const double gd = tr[(size_t)(21 * N) * S], vsky = tr[(size_t)(21 * N + 1) * S];
-        const double dvdt = tr[(size_t)(21 * N + 2) * S];
-        const double d1 = -acc[0] / gd;
-        double* out = g.dtdq0 + g.off_dq[gsys] + 3 * (ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb)));
-        out[0] = d1;
-        out[1] = acc[1] / vsky + dvdt * d1;
-        out[2] = 2.0 * acc[2];
-      }
-    }
+    const double hs = step_length(g, s, istep, nst, h);
+    if (MODE == 0) apply_step<N, BS>(J, E, c, hs, g.kick, rec);
+    else column_step<N, BS, MODE == 2>(J, E, c, hs, rec);
+    if (!g.notransit) column_transits<N, BS>(g, s, c, kk, ti, ntt, gsys, J, E);
   }
-  double* Jw = g.Jint + (size_t)s * R6 * M + c;
-  double* Ew = g.Eint + (size_t)s * R6 * M + c;
   bool finite = true;
   for (int r = 0; r < R6; r++) {
-    Jw[(size_t)r * M] = J[r * CONS_BS];
-    Ew[(size_t)r * M] = E[r * CONS_BS];
-    finite = finite && isfinite(J[r * CONS_BS]);
+    Jg[(size_t)r * M] = J[r * BS];
+    Eg[(size_t)r * M] = E[r * BS];
+    finite = finite && isfinite(J[r * BS]);
   }
   if (!finite) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
+}
+
+template <int N>
+__global__ void __launch_bounds__(cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain) {
+  extern __shared__ double smem[];
+  constexpr int BS = cons_bs(N);
+  if ((int)blockIdx.x < plain) {
+    const int f = blockIdx.x * BS + threadIdx.x, q = f % (6 * N);
+    consume_chunk<N, BS, 1>(g, chunk, f / (6 * N), 7 * (q / 6) + q % 6, smem);
+  } else {
+    const int f = (blockIdx.x - plain) * BS + threadIdx.x;
+    consume_chunk<N, BS, 2>(g, chunk, f / N, 7 * (f % N) + 6, smem);
+  }
+}
+
+template <int N>
+__global__ void __launch_bounds__(cons_bs(N)) jacobian_kick_kernel(GroupArgs g, int chunk) {
+  extern __shared__ double smem[];
+  constexpr int BS = cons_bs(N), M = 7 * N;
+  const int f = blockIdx.x * BS + threadIdx.x;
+  consume_chunk<N, BS, 0>(g, chunk, f / M, f % M, smem);
 }
 
 // gsave[i] = g!(i, ti, x, v) for every occultor (Transits.jl:146-149).
@@ -590,11 +619,17 @@ int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
 
 template <int N>
 int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
-  long long threads = (long long)g.S * 7 * N;
-  int blocks = (int)((threads + CONS_BS - 1) / CONS_BS);
-  const int smem = 2 * 6 * N * CONS_BS * (int)sizeof(double);
-  allow_smem(jacobian_chunk_kernel<N>, smem);  // per call: the attribute belongs to the current device
-  jacobian_chunk_kernel<N><<<blocks, CONS_BS, smem, st>>>(g, chunk);
+  constexpr int BS = cons_bs(N);
+  const int smem = 2 * 6 * N * BS * (int)sizeof(double);
+  auto blocks = [](long long columns) { return (int)((columns + BS - 1) / BS); };
+  if (g.kick) {
+    allow_smem(jacobian_kick_kernel<N>, smem);  // per call: the attribute belongs to the current device
+    jacobian_kick_kernel<N><<<blocks((long long)g.S * 7 * N), BS, smem, st>>>(g, chunk);
+    return 0;
+  }
+  const int plain = blocks((long long)g.S * 6 * N);
+  allow_smem(jacobian_chunk_kernel<N>, smem);
+  jacobian_chunk_kernel<N><<<plain + blocks((long long)g.S * N), BS, smem, st>>>(g, chunk, plain);
   return 0;
 }
 

@@ -27,7 +27,10 @@ __host__ __device__ inline int step_record_size(int N, int npk, bool kick) {
 
 constexpr int PROD_BS = 32;     // orbit producer: threads per warp-sized unit of work
 constexpr int PROD_MAX_WARPS = 4;  // orbit producer: up to 4 independent warps per block
-constexpr int CONS_BS = 128;    // Jacobian consumer: four warps per block
+// Jacobian consumer: columns per block.  96 N bytes of shared memory a column:
+// four warps a block, two from nine bodies on, so that six or more warps fit an
+// SM (227 KB) at every N; every block holds 24 KB or more.
+__host__ __device__ constexpr int cons_bs(int N) { return N >= 9 ? 64 : 128; }
 constexpr int TRANSIT_BS = 32;  // transit searches: one warp per block
 constexpr int OPS_BS = 128;     // operator kernels
 
