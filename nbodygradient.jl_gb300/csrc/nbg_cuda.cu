@@ -372,8 +372,9 @@ bool use_team(int mode, int N, unsigned long long kick) {
   return mode > 0 || (mode < 0 && N >= 5);
 }
 
-// The wide team form (two lanes per pair solve): always in mode 2, in the
-// latency-bound chunks (few systems running) in modes -1 and 3.
+// The forms for latency-bound chunks (sixteen lanes per pair solve, six per
+// column of jac_step): always in mode 2, in the latency-bound chunks (few
+// systems running) in modes -1 and 3.
 bool use_wide(int mode, bool latency_bound, unsigned long long kick) {
   if (kick) return false;
   return mode == 2 || ((mode < 0 || mode == 3) && latency_bound);
@@ -730,6 +731,11 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     gx.wide = use_wide(ctx->orbit_team, tail, g.kick) ? 1 : 0;
     return gx;
   };
+  auto jac_args = [&](size_t q, const GroupArgs& g, long long c) {
+    GroupArgs gx = g;
+    gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max, g.kick) ? 1 : 0;
+    return gx;
+  };
   auto ops_args = [&](const GroupArgs& g) {
     GroupArgs gx = g;
     if (tail_any) gx.guard_smem = std::max(gx.guard_smem, 18 * 1024);
@@ -753,7 +759,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
           if ((rc = timed(3, [&] { return kOps[g.N](g, (int)c, st); }))) return rc;
           sample_now = (c == ((gmaxsteps[q] + K - 1) / K) / 2);
           sampled += (ctx->profile == 3 && sample_now) ? 1 : 0;
-          if ((rc = timed(1, [&] { return kJac[g.N](g, (int)c, st); }))) return rc;
+          if ((rc = timed(1, [&] { return kJac[g.N](jac_args(q, g, c), (int)c, st); }))) return rc;
           ctx->last_launches += 3;
           ctx->last_jac_launches++;
         }
@@ -859,7 +865,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
           NBG_CUDA(cudaStreamWaitEvent(sw, ev_tr, 0));
           sample_now = (c == ((gmaxsteps[q] + K - 1) / K) / 2);
           sampled += (ctx->profile == 3 && sample_now) ? 1 : 0;
-          if ((rc = timed_on(sw, 1, [&] { return kJac[g.N](g, (int)c, sw); }))) return rc;
+          if ((rc = timed_on(sw, 1, [&] { return kJac[g.N](jac_args(q, g, c), (int)c, sw); }))) return rc;
           ctx->last_launches += 3;
           ctx->last_jac_launches++;
         } else {

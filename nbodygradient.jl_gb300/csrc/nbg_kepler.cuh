@@ -288,6 +288,15 @@ __device__ __forceinline__ double stumpff6(double z) {
   return p;
 }
 
+// stumpff6 (even lanes) or stumpff5 (odd lanes)
+__device__ __forceinline__ double stumpff_either(double z, bool odd) {
+  constexpr double a[7] = NBG_C6_COEF, b[7] = NBG_C5_COEF;
+  double p = odd ? b[6] : a[6];
+#pragma unroll
+  for (int q = 5; q >= 0; q--) p = fma(-z, p, odd ? b[q] : a[q]);
+  return p;
+}
+
 // FP32 start of the drift's solve.  With sigma = s r0 / h Kepler's equation
 // r0 s + eta G2 + zeta G3 = h reads sigma + a sigma^2 c_2 + b sigma^3 c_3 = 1
 // at z = w sigma^2; three Halley steps from the root of its quadratic part

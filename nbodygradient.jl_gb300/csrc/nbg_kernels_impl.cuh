@@ -12,6 +12,8 @@
 // Systems are grouped by (N, grad, kick pattern) so that every warp runs one
 // control-flow path; within a group systems are sorted longest first.
 #pragma once
+#include <cuda_pipeline.h>
+
 #include <algorithm>
 
 #include "../../include/nbg.h"
@@ -50,10 +52,6 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
   const double t0 = g.t0[s], h = g.h[s], hI = g.hI[s];
   const int ntt = g.ntt[s], ti = g.ti[s];
   const uint64_t kick = g.kick;
-  // status bits raised in this chunk; or-ed into the system's word at the end
-  // (the transit searches and the consumer of the previous chunk may be
-  // or-ing theirs in meanwhile)
-  unsigned int status = 0;
   for (int kk = 0; kk < g.K; kk++) {
     const long long istep = k0 + kk;
     if (istep >= nst) break;
@@ -77,40 +75,7 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     }
     if (g.notransit) continue;
     const double t = t0 + (double)(istep + 1) * h;
-    // detect_transits! (timing.jl:3-28).  The search itself (findtransit!) is
-    // queued: it runs from a copy of this state in transit_kernel, with full
-    // warps, instead of stalling the 31 other systems of this warp.
-    for (int o = 0; o < N - 1; o++) {
-      const int ib = (o < ti) ? o : o + 1;
-      const double gi = gsky(st, ib, ti);
-      const double xi = st.x[3 * ib], yi = st.x[3 * ib + 1], zi = st.x[3 * ib + 2];
-      const double ri = sqrt(xi * xi + yi * yi + zi * zi);
-      if (g.grad) g.tflag[(size_t)(kk * (N - 1) + o) * S + s] = -1;
-      if (gi > 0.0 && gsave[ib] < 0.0 && -zi > 0.25 * ri && ri < 1e12) {
-        count[ib] += 1;
-        if (count[ib] <= ntt) {
-          const int idx = atomicAdd(g.task_count, 1);
-          if (idx < g.task_cap) {  // the capacity is the number of (step, occultor, system) slots
-            double* tf = g.task_f + (size_t)idx * (12 * N + 2);
-            for (int q = 0; q < 3 * N; q++) {
-              tf[q] = st.x[q];
-              tf[3 * N + q] = st.v[q];
-              tf[6 * N + q] = st.xe[q];
-              tf[9 * N + q] = st.ve[q];
-            }
-            tf[12 * N] = -gi * hI / (gi - gsave[ib]);  // first estimate (timing.jl:20)
-            tf[12 * N + 1] = t;
-            int* tk = g.task_i + 3 * idx;
-            tk[0] = s;
-            tk[1] = kk * (N - 1) + o;
-            tk[2] = (int)(count[ib] - 1);
-          }
-        } else {
-          status |= NBG_STATUS_NTT_OVERFLOW;
-        }
-      }
-      gsave[ib] = gi;
-    }
+    for (int o = 0; o < N - 1; o++) detect_transit<N>(g, st, s, kk, o, ti, ntt, hI, t, gsave, count);
   }
   for (int q = 0; q < 3 * N; q++) {
     g.x[q * S + s] = st.x[q];
@@ -124,8 +89,9 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     g.gsave[q * S + s] = gsave[q];
     g.count[q * S + s] = count[q];
   }
-  if (!state_finite<N>(st)) status |= NBG_STATUS_NONFINITE;
-  if (status) atomicOr(g.status + s, status);
+  // or-ed in: the transit searches and the consumer of the previous chunk may
+  // be or-ing theirs meanwhile
+  if (!state_finite<N>(st)) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
 }
 
 
@@ -458,49 +424,57 @@ __global__ void __launch_bounds__(OPS_BS) operator_kick_kernel(GroupArgs g, int 
   put_op(rec, off_phi + op_size(N) + g.npk * PREC, w.op, op_size(N));
 }
 
-// dtdq0 entries of this column for the transits of step kk (dtbvdq!,
-// timing.jl:155-193), from their adjoint rows.
+// dtdq0 entry of column c for one transit (dtbvdq!, timing.jl:155-193) from the
+// products of its adjoint rows with the column.
+template <int N>
+__device__ __forceinline__ void put_transit(const GroupArgs& g, int gsys, int ib, int flag, int ntt, int c,
+                                            const double* acc, const double* tr) {
+  const int S = g.S, cb = c / 7, ck = c % 7;  // column c is d/d q0[ck] of body cb
+  const long long at = ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb));
+  if (!g.tbv) {
+    g.dtdq0[g.off_dq[gsys] + at] = -acc[0] / tr[(size_t)(7 * N) * S];
+    return;
+  }
+  const double gd = tr[(size_t)(21 * N) * S], vsky = tr[(size_t)(21 * N + 1) * S];
+  const double dvdt = tr[(size_t)(21 * N + 2) * S];
+  const double d1 = -acc[0] / gd;
+  double* out = g.dtdq0 + g.off_dq[gsys] + 3 * at;
+  out[0] = d1;
+  out[1] = acc[1] / vsky + dvdt * d1;
+  out[2] = 2.0 * acc[2];
+}
+
+// The entries of this column for the transits of step kk.
 template <int N, int BS>
 __device__ __forceinline__ void column_transits(const GroupArgs& g, int s, int c, int kk, int ti, int ntt, int gsys,
                                                 const double* J, const double* E) {
-  const int S = g.S, cb = c / 7, ck = c % 7;  // column c is d/d q0[ck] of body cb
+  const int S = g.S, ck = c % 7;
   for (int o = 0; o < N - 1; o++) {
     const int flag = g.tflag[(size_t)(kk * (N - 1) + o) * S + s];
     if (flag < 0) continue;
     const double* tr = g.trec + ((size_t)(kk * (N - 1) + o) * trec_size(N, g.tbv)) * S + s;
     const int ib = (o < ti) ? o : o + 1;
-    if (!g.tbv) {
-      double acc = 0.0;
+    // the rows of a body in six sums, added in order (the lane form has a lane for each)
+    double acc[3];
+#pragma unroll 1
+    for (int w = 0; w < (g.tbv ? 3 : 1); w++) {
+      double part[6];
+#pragma unroll
+      for (int r = 0; r < 6; r++) part[r] = 0.0;
+#pragma unroll 1
       for (int b = 0; b < N; b++)
+#pragma unroll
         for (int r = 0; r < 6; r++) {
-          const double ur = tr[(size_t)(7 * b + r) * S];
-          acc = fma(ur, J[(6 * b + r) * BS], acc);
-          acc = fma(ur, E[(6 * b + r) * BS], acc);
+          const double ur = tr[(size_t)(7 * N * w + 7 * b + r) * S];
+          part[r] = fma(ur, E[(6 * b + r) * BS], fma(ur, J[(6 * b + r) * BS], part[r]));
         }
-      if (ck == 6) acc = acc + tr[(size_t)c * S];  // unit mass row of this column
-      const double gd = tr[(size_t)(7 * N) * S];
-      g.dtdq0[g.off_dq[gsys] + ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb))] = -acc / gd;
-    } else {
-      double acc[3] = {0.0, 0.0, 0.0};
-      for (int b = 0; b < N; b++)
-        for (int r = 0; r < 6; r++) {
-          const double jv = J[(6 * b + r) * BS], ev = E[(6 * b + r) * BS];
-          for (int w = 0; w < 3; w++) {
-            const double ur = tr[(size_t)(7 * N * w + 7 * b + r) * S];
-            acc[w] = fma(ur, jv, acc[w]);
-            acc[w] = fma(ur, ev, acc[w]);
-          }
-        }
-      if (ck == 6)
-        for (int w = 0; w < 3; w++) acc[w] = acc[w] + tr[(size_t)(7 * N * w + c) * S];
-      const double gd = tr[(size_t)(21 * N) * S], vsky = tr[(size_t)(21 * N + 1) * S];
-      const double dvdt = tr[(size_t)(21 * N + 2) * S];
-      const double d1 = -acc[0] / gd;
-      double* out = g.dtdq0 + g.off_dq[gsys] + 3 * (ib + (long long)N * (flag + (long long)ntt * (ck + 7LL * cb)));
-      out[0] = d1;
-      out[1] = acc[1] / vsky + dvdt * d1;
-      out[2] = 2.0 * acc[2];
+      double sum = part[0];
+#pragma unroll
+      for (int r = 1; r < 6; r++) sum = sum + part[r];
+      if (ck == 6) sum = sum + tr[(size_t)(7 * N * w + c) * S];  // unit mass row of this column
+      acc[w] = sum;
     }
+    put_transit<N>(g, gsys, ib, flag, ntt, c, acc, tr);
   }
 }
 
@@ -572,6 +546,229 @@ __global__ void __launch_bounds__(cons_bs(N)) jacobian_kick_kernel(GroupArgs g, 
   consume_chunk<N, BS, 0>(g, chunk, f / M, f % M, smem);
 }
 
+// Jacobian consumer for latency-bound chunks (the orbit producer's lanes form
+// runs for them): six lanes per column of jac_step, one for each row of a body,
+// five columns a warp, two warps a block.
+//
+// With few systems a column's lane is alone with its 64 cycles per FP64
+// instruction, so a step takes as long as the column's instructions.  Here a
+// pair costs 11 instead of 66 (three for D, six for its row of u, one for each
+// body) and the corrector's 3N rows go round the six lanes; lanes exchange D
+// by shuffles and the corrector's differences through shared memory.  The
+// block copies the next step's record to shared memory while it applies this
+// one (cp.async), so no trip to memory is waited out.  Per column the FP64 work
+// is that of the one-lane form within a tenth, and every value is formed by the
+// same operations in the same order: bitwise the same columns.
+// One system alone, before and after: 400 steps of eight bodies with transits
+// 121 -> 55 ms, 2000 of three 67 -> 54 ms, 203 of six 33 -> 20 ms.
+constexpr int ROWS_COLS = 5, ROWS_WARPS = 2;
+__host__ __device__ constexpr int rows_plain_warps(int N) { return (6 * N + ROWS_COLS - 1) / ROWS_COLS; }
+__host__ __device__ constexpr int rows_warps(int N) { return rows_plain_warps(N) + (N + ROWS_COLS - 1) / ROWS_COLS; }
+__host__ __device__ constexpr int rows_record(int N) { return N * (N - 1) * PREC + op_size(N); }
+template <int N>
+struct RowsShared {
+  double rec[2][rows_record(N)];
+  double S[ROWS_WARPS][6 * N * ROWS_COLS], E[ROWS_WARPS][6 * N * ROWS_COLS], D[ROWS_WARPS][3 * N * ROWS_COLS];
+  int flag[2][N];
+};
+
+template <int N, bool MASS>
+__device__ __forceinline__ void rows_pair(double* Sw, double* Ew, const double* rc, int i, int j, bool ci, bool cj,
+                                          int l, int col, bool live) {
+  const int ai = (6 * i + l) * ROWS_COLS + col, aj = (6 * j + l) * ROWS_COLS + col;
+  const double ei = Ew[ai], ej = Ew[aj];
+  const double d = (Sw[ai] + ei) - (Sw[aj] + ej);
+  const double* K = rc + 6 * l;
+  double u = 0.0;
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const double D = __shfl_sync(0xffffffffu, d, 6 * col + q);
+    if (q == 0) u = MASS ? fma(K[0], D, (ci || cj) ? rc[PREC_PSI + l] : 0.0) : K[0] * D;
+    else u = fma(K[q], D, u);
+  }
+  double ni = fma(rc[PREC_MJ], u, ei), nj = fma(-rc[PREC_MI], u, ej);
+  if (MASS) {
+    const double B = rc[PREC_B + l];
+    ni = ni + (cj ? B : 0.0);
+    nj = nj - (ci ? B : 0.0);
+  }
+  if (live) {
+    Ew[ai] = ni;
+    Ew[aj] = nj;
+  }
+}
+
+// column_step on the warp's five columns.
+template <int N, bool MASS>
+__device__ __forceinline__ void rows_step(double* Sw, double* Ew, double* Dw, const double* rec, int c, double h, int l,
+                                          int col, bool live) {
+  const double h2 = 0.5 * h;
+  const int cm = c / 7;
+  if (live && l < 3) {
+#pragma unroll
+    for (int b = 0; b < N; b++) {
+      const int r = (6 * b + l) * ROWS_COLS + col;
+      double s = Sw[r], e = fma(h2, Sw[r + 3 * ROWS_COLS], Ew[r]);
+      normalise(s, e, s + e);
+      Sw[r] = s;
+      Ew[r] = e;
+    }
+  }
+  __syncwarp();
+  const double* rc = rec;
+#pragma unroll 1
+  for (int i = 0; i < N - 1; i++) {
+#pragma unroll 1
+    for (int j = i + 1; j < N; j++, rc += PREC)
+      rows_pair<N, MASS>(Sw, Ew, rc, i, j, cm == i, cm == j, l, col, live);
+    if (N > 2 && i == 0 && live && l >= 3) {
+#pragma unroll
+      for (int b = 0; b < N; b++) {
+        const int r = (6 * b + l) * ROWS_COLS + col;
+        double s = Sw[r], e = Ew[r];
+        normalise(s, e, s + e);
+        Sw[r] = s;
+        Ew[r] = e;
+      }
+    }
+    __syncwarp();
+  }
+  if (live && l < 3) {
+    const double t0 = Sw[l * ROWS_COLS + col] + Ew[l * ROWS_COLS + col];
+#pragma unroll
+    for (int d = 1; d < N; d++) {
+      const int r = (6 * d + l) * ROWS_COLS + col;
+      Dw[(3 * d + l) * ROWS_COLS + col] = (Sw[r] + Ew[r]) - t0;
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int row = l; row < 3 * N; row += 6) {
+    const double* rb = rc + row * (4 * N);
+    const double* D = Dw + 3 * ROWS_COLS + col;
+    double acc = MASS ? fma(rb[4], D[0], rb[4 * cm + 3]) : rb[4] * D[0];
+#pragma unroll
+    for (int q = 1; q < 3 * (N - 1); q++) acc = fma(rb[4 + 4 * (q / 3) + q % 3], D[q * ROWS_COLS], acc);
+    const int r = (6 * (row / 3) + 3 + row % 3) * ROWS_COLS + col;
+    if (live) Ew[r] = Ew[r] + acc;
+  }
+  __syncwarp();
+  rc += op_size(N);
+#pragma unroll 1
+  for (int i = N - 2; i >= 0; i--)
+#pragma unroll 1
+    for (int j = N - 1; j > i; j--, rc += PREC)
+      rows_pair<N, MASS>(Sw, Ew, rc, i, j, cm == i, cm == j, l, col, live);
+#pragma unroll
+  for (int b = 0; b < N; b++) {
+    const int r = (6 * b + l) * ROWS_COLS + col;
+    double s = Sw[r], e = Ew[r], t = s + e;
+    const double tv = __shfl_sync(0xffffffffu, t, 6 * col + (l < 3 ? l + 3 : l));
+    if (l < 3) {
+      e = fma(h2, tv, e);
+      t = s + e;
+    }
+    normalise(s, e, t);
+    if (live) {
+      Sw[r] = s;
+      Ew[r] = e;
+    }
+  }
+  __syncwarp();
+}
+
+template <int N>
+__global__ void __launch_bounds__(32 * ROWS_WARPS) jacobian_rows_kernel(GroupArgs g, int chunk) {
+  extern __shared__ double smem[];
+  RowsShared<N>& sh = *reinterpret_cast<RowsShared<N>*>(smem);
+  constexpr int M = 7 * N, R6 = 6 * N, R = rows_record(N);
+  const int s = blockIdx.x, S = g.S, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (s >= S || g.sysidx[s] < 0) return;
+  const long long nst = g.nsteps[s], k0 = chunk_first_step(g, chunk, s);
+  if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
+  const int nk = (int)(nst - k0 < g.K ? nst - k0 : g.K);
+  // this lane's column: warps 0..rows_plain_warps-1 the columns that are not mass columns, then the mass columns
+  const int wid = blockIdx.y * ROWS_WARPS + warp, pw = rows_plain_warps(N);
+  const bool mass = wid >= pw;
+  const int l = lane % 6, col = lane < 30 ? lane / 6 : 0;
+  const int q = (mass ? wid - pw : wid) * ROWS_COLS + col;
+  const bool live = lane < 30 && wid < rows_warps(N) && q < (mass ? N : 6 * N);
+  const int c = !live ? 0 : mass ? 7 * q + 6 : 7 * (q / 6) + q % 6;
+  double *Sw = sh.S[warp], *Ew = sh.E[warp], *Dw = sh.D[warp];
+  double* Jg = g.Jint + (size_t)s * R6 * M + c;
+  double* Eg = g.Eint + (size_t)s * R6 * M + c;
+  if (lane < 30)
+    for (int b = 0; b < N; b++) {
+      const int r = 6 * b + l;
+      double jv = live ? Jg[(size_t)r * M] : 0.0, ev = live ? Eg[(size_t)r * M] : 0.0;
+      if (k0 == 0) fold(jv, ev);  // a caller's pair may not be normalised
+      Sw[r * ROWS_COLS + col] = jv;
+      Ew[r * ROWS_COLS + col] = ev;
+    }
+  auto fetch = [&](int kk) {
+    const double* src = g.steprec + (size_t)kk * R * S + s;
+    double* dst = sh.rec[kk & 1];
+    for (int e = tid; e < R; e += 32 * ROWS_WARPS) __pipeline_memcpy_async(dst + e, src + (size_t)e * S, sizeof(double));
+    if (!g.notransit && tid < N - 1)
+      __pipeline_memcpy_async(&sh.flag[kk & 1][tid], g.tflag + (size_t)(kk * (N - 1) + tid) * S + s, sizeof(int));
+    __pipeline_commit();
+  };
+  const double h = g.h[s];
+  const int ntt = g.ntt[s], ti = g.ti[s], gsys = g.sysidx[s];
+  fetch(0);
+#pragma unroll 1
+  for (int kk = 0; kk < nk; kk++) {
+    if (kk + 1 < nk) fetch(kk + 1);
+    else __pipeline_commit();
+    __pipeline_wait_prior(1);
+    __syncthreads();
+    if (g.trajJ && live) {  // column c of jac_step at the start of the step; mass rows are unit rows
+      double* rj = g.trajJ + (((size_t)s * g.K + kk) * M + c) * M;
+      for (int b = 0; b < N; b++) {
+        rj[7 * b + l] = Sw[(6 * b + l) * ROWS_COLS + col];
+        if (l == 0) rj[7 * b + 6] = (7 * b + 6 == c) ? 1.0 : 0.0;
+      }
+    }
+    const double hs = step_length(g, s, k0 + kk, nst, h);
+    if (mass) rows_step<N, true>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, l, col, live);
+    else rows_step<N, false>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, l, col, live);
+    if (!g.notransit)
+      for (int o = 0; o < N - 1; o++) {
+        const int flag = sh.flag[kk & 1][o];
+        if (flag < 0) continue;
+        const double* tr = g.trec + ((size_t)(kk * (N - 1) + o) * trec_size(N, g.tbv)) * S + s;
+        double acc[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int w = 0; w < (g.tbv ? 3 : 1); w++) {
+          double part = 0.0;
+          for (int b = 0; b < N; b++) {
+            const double ur = tr[(size_t)(7 * N * w + 7 * b + l) * S];
+            const int r = (6 * b + l) * ROWS_COLS + col;
+            part = fma(ur, Ew[r], fma(ur, Sw[r], part));
+          }
+          double sum = __shfl_sync(0xffffffffu, part, 6 * col);
+#pragma unroll
+          for (int r = 1; r < 6; r++) sum = sum + __shfl_sync(0xffffffffu, part, 6 * col + r);
+          if (mass) sum = sum + tr[(size_t)(7 * N * w + c) * S];  // unit mass row of this column
+          acc[w] = sum;
+        }
+        if (live && l == 0) put_transit<N>(g, gsys, (o < ti) ? o : o + 1, flag, ntt, c, acc, tr);
+      }
+    __syncthreads();  // the next fetch overwrites this step's record
+  }
+  if (live) {
+    bool finite = true;
+    for (int b = 0; b < N; b++) {
+      const int r = 6 * b + l;
+      const double jv = Sw[r * ROWS_COLS + col];
+      Jg[(size_t)r * M] = jv;
+      Eg[(size_t)r * M] = Ew[r * ROWS_COLS + col];
+      finite = finite && isfinite(jv);
+    }
+    if (!finite) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
+  }
+}
+
 // gsave[i] = g!(i, ti, x, v) for every occultor (Transits.jl:146-149).
 template <int N>
 __global__ void seed_gsave_kernel(GroupArgs g) {
@@ -598,10 +795,9 @@ template <int N>
 int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   const int W = g.pwarps > 0 ? g.pwarps : 1;
   if (g.wide && !g.kick) {
-    constexpr int T = PROD_BS / (2 * team_lanes(N));
-    const int smem = std::max(team_smem_bytes<N, 2>(W), g.prod_smem);
-    allow_smem(orbit_team_kernel<N, 2>, smem);
-    orbit_team_kernel<N, 2><<<(g.S + W * T - 1) / (W * T), PROD_BS * W, smem, st>>>(g, chunk);
+    const int smem = std::max((int)sizeof(LanesShared<N>), g.prod_smem);
+    allow_smem(orbit_lanes_kernel<N>, smem);
+    orbit_lanes_kernel<N><<<g.S, 32 * lanes_warps(N), smem, st>>>(g, chunk);
     return 0;
   }
   if (g.team && !g.kick) {
@@ -625,6 +821,13 @@ int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
   if (g.kick) {
     allow_smem(jacobian_kick_kernel<N>, smem);  // per call: the attribute belongs to the current device
     jacobian_kick_kernel<N><<<blocks((long long)g.S * 7 * N), BS, smem, st>>>(g, chunk);
+    return 0;
+  }
+  if (g.wide) {
+    const int bytes = std::max((int)sizeof(RowsShared<N>), 24 * 1024);  // as every consumer block: none fits beside a tail producer's
+    allow_smem(jacobian_rows_kernel<N>, bytes);
+    const dim3 grid(g.S, (rows_warps(N) + ROWS_WARPS - 1) / ROWS_WARPS);
+    jacobian_rows_kernel<N><<<grid, 32 * ROWS_WARPS, bytes, st>>>(g, chunk);
     return 0;
   }
   const int plain = blocks((long long)g.S * 6 * N);

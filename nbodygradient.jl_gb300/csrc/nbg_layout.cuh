@@ -58,9 +58,10 @@ struct GroupArgs {
   // that the searches are latency-bound; a full group keeps one lane per
   // search, which uses every lane of every warp
   int search_team;
-  // orbit producer in the wide team form (two lanes per pair solve,
-  // orbit_team_kernel<N, 2>) for this chunk: set by the host for latency-bound
-  // chunks (few systems running) of groups without kick pairs
+  // latency-bound chunk (few systems running) of a group without kick pairs,
+  // set by the host per chunk: the orbit producer takes its lanes form
+  // (orbit_lanes_kernel), the Jacobian consumer its rows form
+  // (jacobian_rows_kernel)
   int wide;
   // Block layout of the orbit producer: pwarps independent warps per block
   // (0 or 1: one) and prod_smem bytes of dynamic shared memory per block (at

@@ -18,6 +18,7 @@
 // Compact operator layout: row 3b + k is body b's velocity component k,
 // column 4d + p is body d's position component p (p < 3) or mass (p == 3).
 #pragma once
+#include "../../include/nbg.h"
 #include "nbg_layout.cuh"
 #include "nbg_kepler.cuh"
 
@@ -630,6 +631,43 @@ __device__ __forceinline__ double gdot(const Sys<N>& s, int i, int j) {
           (s.x[3 * j + 1] - s.x[3 * i + 1]) * (q[7 * j + 4] - q[7 * i + 4]) +
           (s.v[3 * j] - s.v[3 * i]) * (q[7 * j + 0] - q[7 * i + 0]) +
           (s.v[3 * j + 1] - s.v[3 * i + 1]) * (q[7 * j + 1] - q[7 * i + 1]));
+}
+
+// detect_transits! (timing.jl:3-28) for occultor slot o after step kk of the
+// chunk: g's sign change with the occultor in front queues a search from a copy
+// of this state (transit_kernel runs it, so that no other system of the warp
+// waits).  gsave, count: the system's N entries.
+template <int N>
+__device__ __forceinline__ void detect_transit(const GroupArgs& g, const Sys<N>& st, int s, int kk, int o, int ti,
+                                               int ntt, double hI, double t, double* gsave, long long* count) {
+  const int ib = (o < ti) ? o : o + 1, S = g.S;
+  const double gi = gsky(st, ib, ti), before = gsave[ib];
+  gsave[ib] = gi;
+  if (g.grad) g.tflag[(size_t)(kk * (N - 1) + o) * S + s] = -1;
+  if (!(gi > 0.0 && before < 0.0)) return;
+  const double xi = st.x[3 * ib], yi = st.x[3 * ib + 1], zi = st.x[3 * ib + 2];
+  const double ri = sqrt(xi * xi + yi * yi + zi * zi);
+  if (!(-zi > 0.25 * ri && ri < 1e12)) return;
+  count[ib] += 1;
+  if (count[ib] > ntt) {
+    atomicOr(g.status + s, NBG_STATUS_NTT_OVERFLOW);
+    return;
+  }
+  const int idx = atomicAdd(g.task_count, 1);
+  if (idx >= g.task_cap) return;  // the capacity is the number of (step, occultor, system) slots
+  double* tf = g.task_f + (size_t)idx * (12 * N + 2);
+  for (int q = 0; q < 3 * N; q++) {
+    tf[q] = st.x[q];
+    tf[3 * N + q] = st.v[q];
+    tf[6 * N + q] = st.xe[q];
+    tf[9 * N + q] = st.ve[q];
+  }
+  tf[12 * N] = -gi * hI / (gi - before);  // first estimate (timing.jl:20)
+  tf[12 * N + 1] = t;
+  int* tk = g.task_i + 3 * idx;
+  tk[0] = s;
+  tk[1] = kk * (N - 1) + o;
+  tk[2] = (int)(count[ib] - 1);
 }
 
 // u <- u + A^T u for the compact operator block A (velocity rows x position

@@ -41,65 +41,24 @@ __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {
   return true;
 }
 
-// kepler_pair<N, DRIFT_FIRST, false, false> on the two lanes of a pair slot:
-// both lanes read the pair's coordinates and solve it; role 0 then updates
-// body i and writes the first half of the capture, role 1 body j and the
-// rest.  x_i and x_j are separate variables, so splitting their updates
-// between the lanes changes no value.
-template <int N, bool DRIFT_FIRST>
-__device__ __forceinline__ void kepler_pair_w2(Sys<N>& s, int i, int j, double h2, const Rec& cap, int coff,
-                                               int role, unsigned mask, int base) {
-  double x0[3], v0[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    x0[k] = s.x[3 * i + k] - s.x[3 * j + k];
-    v0[k] = s.v[3 * i + k] - s.v[3 * j + k];
-  }
-  const double mij = s.m[i] + s.m[j];
-  const double gm = GNEWT * mij;
-  __syncwarp(mask);  // both lanes have read the pair before either writes
-  if (cap.p && gm == 0.0 && role == 0) cap.put(coff + PCAP_K, 0.0);
-  if (gm != 0.0) {
-    KepParams P;
-    double delxv[6];
-    kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
-    if (cap.p && role == 0) put_capture(cap, coff, x0, v0, P);
-    const double mijinv = rcp_fast(mij);
-    const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
-    const int b = role ? j : i;
-    const double f = role ? (-mi) : mj;
-#pragma unroll
-    for (int k = 0; k < 3; k++) kahan_fma(s.x[3 * b + k], s.xe[3 * b + k], f, delxv[k]);
-#pragma unroll
-    for (int k = 0; k < 3; k++) kahan_fma(s.v[3 * b + k], s.ve[3 * b + k], f, delxv[3 + k]);
-  }
-}
-
 // One AHL21 step without gradient operators for a group with no kick pairs
-// (ahl21_no_grad.jl:6-18 order), run by the R * L lanes of a team (R = 2:
-// each pair slot p on two lanes, roles 0 and 1, kepler_pair_w2); `run` is
+// (ahl21_no_grad.jl:6-18 order), run by the L lanes of a team; `run` is
 // false for lanes whose system does not step (they still meet every
 // __syncwarp).  cap / xs as in ahl21_step.  a: the team's 3N acceleration
 // scratch.
-template <int N, int R = 1>
+template <int N>
 __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int t, bool run, double h,
                                           const Rec& cap, const Rec& xs) {
-  constexpr int L = R * team_lanes(N);
+  constexpr int L = team_lanes(N);
   constexpr int P = N * (N - 1) / 2;
-  const int p = t / R, role = t % R;
-  const int lane = threadIdx.x & 31;
-  const int base = lane - role;
-  const unsigned mask = (R == 2) ? (3u << base) : 0u;
   const double h2 = 0.5 * h;
   if (run)
     for (int q = t; q < 3 * N; q += L) kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
   __syncwarp();
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
-    if (run && level_pair<N>(lev, p, &i, &j)) {
-      if (R == 1) kepler_pair<N, true, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap, pair_bit(i, j, N) * PCAP);
-      else kepler_pair_w2<N, true>(s, i, j, h2, cap, pair_bit(i, j, N) * PCAP, role, mask, base);
-    }
+    if (run && level_pair<N>(lev, t, &i, &j))
+      kepler_pair<N, true, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap, pair_bit(i, j, N) * PCAP);
     __syncwarp();
   }
   if (run) {
@@ -111,23 +70,21 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
   const double coeff = phis_coeff(h);
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
-    if (run && role == 0 && level_pair<N>(lev, p, &i, &j)) phis_accel_pair<N>(s, a, i, j);
+    if (run && level_pair<N>(lev, t, &i, &j)) phis_accel_pair<N>(s, a, i, j);
     __syncwarp();
   }
   if (run && xs.p)
     for (int q = t; q < 3 * N; q += L) xs.put(3 * N + q, a[q]);
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
-    if (run && role == 0 && level_pair<N>(lev, p, &i, &j)) phis_kick_pair<N>(s, a, i, j, coeff);
+    if (run && level_pair<N>(lev, t, &i, &j)) phis_kick_pair<N>(s, a, i, j, coeff);
     __syncwarp();
   }
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
     int i, j;
-    if (run && level_pair<N>(lev, p, &i, &j)) {
-      const int coff = (P + (P - 1 - pair_bit(i, j, N))) * PCAP;
-      if (R == 1) kepler_pair<N, false, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap, coff);
-      else kepler_pair_w2<N, false>(s, i, j, h2, cap, coff, role, mask, base);
-    }
+    if (run && level_pair<N>(lev, t, &i, &j))
+      kepler_pair<N, false, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap,
+                                          (P + (P - 1 - pair_bit(i, j, N))) * PCAP);
     __syncwarp();
   }
   if (run)
@@ -137,20 +94,19 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
 
 // Dynamic shared memory the team producer needs for W warps per block:
 // per team a Sys<N>, 3N accelerations, N g values and N transit counts.
-template <int N, int R = 1>
+template <int N>
 __host__ __device__ constexpr int team_smem_bytes(int W) {
-  return W * (PROD_BS / (R * team_lanes(N))) *
+  return W * (PROD_BS / team_lanes(N)) *
          (int)(sizeof(Sys<N>) + (3 * N + N) * sizeof(double) + N * sizeof(long long));
 }
 
-// Orbit producer, team form: L = R * team_lanes(N) lanes per system
-// (R = 2: the wide form, two lanes per pair solve), T = 32 / L systems per
-// warp (lanes beyond T * L idle), pwarps independent warps per block.  Same
-// inputs, outputs and arithmetic as orbit_chunk_kernel<N> for groups
-// without kick pairs.
-template <int N, int R = 1>
+// Orbit producer, team form: L = team_lanes(N) lanes per system, T = 32 / L
+// systems per warp (lanes beyond T * L idle), pwarps independent warps per
+// block.  Same inputs, outputs and arithmetic as orbit_chunk_kernel<N> for
+// groups without kick pairs.
+template <int N>
 __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(GroupArgs g, int chunk) {
-  constexpr int L = R * team_lanes(N);
+  constexpr int L = team_lanes(N);
   constexpr int T = PROD_BS / L;
   const int W = g.pwarps > 0 ? g.pwarps : 1;
   extern __shared__ double team_smem[];
@@ -205,45 +161,14 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
         rx[3 * N + q] = st.v[q];
       }
     }
-    team_step<N, R>(st, acc[tm], w, t, run && !last, hs, cap, xs);
+    team_step<N>(st, acc[tm], w, t, run && !last, hs, cap, xs);
     // the last step also forms dq/dt: the one-lane step, on the team's first lane
     if (last && t == 0) ahl21_step<N, true, true>(st, w, hs, 0, Rec{nullptr, 0}, cap, xs);
     __syncwarp();
-    // detect_transits! (timing.jl:3-28); occultor o on lane o % L
-    if (run && !g.notransit) {
-      const double tnow = t0 + (double)(istep + 1) * h;
-      for (int o = t; o < N - 1; o += L) {
-        const int ib = (o < ti) ? o : o + 1;
-        const double gi = gsky(st, ib, ti);
-        const double xi = st.x[3 * ib], yi = st.x[3 * ib + 1], zi = st.x[3 * ib + 2];
-        const double ri = sqrt(xi * xi + yi * yi + zi * zi);
-        if (g.grad) g.tflag[(size_t)(kk * (N - 1) + o) * S + s] = -1;
-        if (gi > 0.0 && gsv[tm][ib] < 0.0 && -zi > 0.25 * ri && ri < 1e12) {
-          cnt[tm][ib] += 1;
-          if (cnt[tm][ib] <= ntt) {
-            const int idx = atomicAdd(g.task_count, 1);
-            if (idx < g.task_cap) {
-              double* tf = g.task_f + (size_t)idx * (12 * N + 2);
-              for (int q = 0; q < 3 * N; q++) {
-                tf[q] = st.x[q];
-                tf[3 * N + q] = st.v[q];
-                tf[6 * N + q] = st.xe[q];
-                tf[9 * N + q] = st.ve[q];
-              }
-              tf[12 * N] = -gi * hI / (gi - gsv[tm][ib]);  // first estimate (timing.jl:20)
-              tf[12 * N + 1] = tnow;
-              int* tk = g.task_i + 3 * idx;
-              tk[0] = s;
-              tk[1] = kk * (N - 1) + o;
-              tk[2] = (int)(cnt[tm][ib] - 1);
-            }
-          } else {
-            atomicOr(g.status + s, NBG_STATUS_NTT_OVERFLOW);
-          }
-        }
-        gsv[tm][ib] = gi;
-      }
-    }
+    // occultor o on lane o % L
+    if (run && !g.notransit)
+      for (int o = t; o < N - 1; o += L)
+        detect_transit<N>(g, st, s, kk, o, ti, ntt, hI, t0 + (double)(istep + 1) * h, &gsv[tm][0], &cnt[tm][0]);
     __syncwarp();
   }
   if (valid) {
@@ -261,6 +186,337 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
     }
     if (t == 0 && !state_finite<N>(st)) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
   }
+}
+
+// ------------------------------------------------------------ pairs on lanes
+//
+// Orbit producer for latency-bound chunks (at most max(32, SMs / 2) systems of
+// the group still running): one block per system, sixteen lanes per pair solve.
+// A warp issues one FP64 instruction per 64 cycles however independent its
+// instructions are, and with few systems nothing else fills the SM, so a step
+// takes as long as its longest warp's FP64 instructions; spreading a solve's
+// independent pieces over lanes makes them one instruction each:
+//   * lanes 0-5 hold the pair's relative coordinates, lanes 0-5 and 6-11 the
+//     two bodies' (one subtraction, one Kahan sum instead of six and twelve);
+//   * the three dot products, the two Stumpff polynomials, G2 and G3, G0 and
+//     G1, Kepler's equation and r, and the four coefficients of the result are
+//     evaluated side by side, each by its own lanes, and shuffled to all;
+//   * the pairs of a level (equal i + j, see above) go to the block's half
+//     warps, and phisalpha!'s pair terms to one lane each before each body sums
+//     its own in pair order.
+// 57 FP64 instructions a level instead of a one-lane solve's 146.  Every value is
+// formed by the operations of kep_solve, phisalpha and kahan_fma in the same
+// order, so the results are bitwise those of the other forms.
+// One system alone, before (a pair solve on one lane or two) and after: 301 steps
+// of five bodies without derivatives 30.2 -> 15.4 ms, 2000 steps of three bodies
+// with transits 97 -> 67 ms (then bound by the consumer, jacobian_rows_kernel).
+__host__ __device__ constexpr int lanes_warps(int N) { return (N / 2 + 1) / 2 > 0 ? (N / 2 + 1) / 2 : 1; }
+
+template <int N>
+struct LanesShared {
+  Sys<N> st;
+  double a[3 * N], g[N];
+  long long cnt[N];
+  double pk[N * (N - 1) / 2], pmi[N * (N - 1) / 2], pmj[N * (N - 1) / 2];  // k, m_i / (m_i + m_j), m_j / (m_i + m_j)
+  double f[N * (N - 1) / 2][3];
+};
+
+template <int N>
+__device__ __forceinline__ void lanes_sync() {
+  if (lanes_warps(N) == 1) __syncwarp();
+  else __syncthreads();
+}
+
+// One pair of a sweep on the sixteen lanes hl = 0..15 named by `mask`.
+template <int N, bool DRIFT_FIRST>
+__device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, double h, const Rec& cap, int coff,
+                                           int hl, unsigned mask) {
+  const int pb = pair_bit(i, j, N);
+  const double k = sh.pk[pb];
+  if (k == 0.0) {
+    if (cap.p && hl == 0) cap.put(coff + PCAP_K, 0.0);
+    return;
+  }
+  auto from = [&](double v, int src) { return __shfl_sync(mask, v, src, 16); };
+  double* q = sh.st.x;  // x, v, xe, ve of Sys<N> in a row, 3N each
+  const int c = hl % 6, k3 = hl % 3;
+  const int at = (c < 3 ? 0 : 3 * N) + k3;
+  const double d = q[at + 3 * i] - q[at + 3 * j];
+  double X[3], V[3], R[3];
+#pragma unroll
+  for (int w = 0; w < 3; w++) {
+    X[w] = from(d, w);
+    V[w] = from(d, 3 + w);
+  }
+  const double xk = k3 == 0 ? X[0] : k3 == 1 ? X[1] : X[2], vk = k3 == 0 ? V[0] : k3 == 1 ? V[1] : V[2];
+  if (DRIFT_FIRST) {
+    const double rt = fma(-h, vk, xk);
+#pragma unroll
+    for (int w = 0; w < 3; w++) R[w] = from(rt, w);
+  } else {
+#pragma unroll
+    for (int w = 0; w < 3; w++) R[w] = X[w];
+  }
+  double rr, vv, eta;
+  {  // lanes by hl % 3: R.R, V.V, R.V
+    double A[3], B[3];
+#pragma unroll
+    for (int w = 0; w < 3; w++) {
+      A[w] = k3 == 1 ? V[w] : R[w];
+      B[w] = k3 == 0 ? R[w] : V[w];
+    }
+    const double dot = fma(A[2], B[2], fma(A[1], B[1], A[0] * B[0]));
+    rr = from(dot, 0);
+    vv = from(dot, 1);
+    eta = from(dot, 2);
+  }
+  const double r0inv = rsqrt_fast(rr);
+  const double r0 = rr * r0inv;
+  const double kr0 = k * r0inv;
+  const double beta = fma(2.0, kr0, -vv);
+  const double zeta = fma(-r0, beta, k);
+  float q2;
+  const float sg = kep_start((float)r0inv, (float)h, (float)beta, (float)eta, (float)zeta, &q2);
+  const double t = h * r0inv;
+  const float tinv = __fdividef(1.0f, (float)t);
+  const bool odd = hl & 1;
+  double s = t * (double)sg, ds, y, g0, g1, g2, g3, g4 = 0.0;
+  int iter = 0;
+  bool done = false;
+  do {
+    const double ss = s * s, z = beta * ss;
+    const double p = stumpff_either(z, odd);
+    const double c6 = from(p, 0), c5 = from(p, 1);
+    const double c4 = fma(-z, c6, 1.0 / 24.0);
+    const double cc = fma(-z, odd ? c5 : c4, odd ? 1.0 / 6.0 : 0.5);
+    const double sss = ss * s;
+    const double g23 = (odd ? sss : ss) * cc;
+    g2 = from(g23, 0);
+    g3 = from(g23, 1);
+    const double g01 = fma(-beta, odd ? g3 : g2, odd ? s : 1.0);
+    g0 = from(g01, 0);
+    g1 = from(g01, 1);
+    if (!DRIFT_FIRST) g4 = (ss * ss) * c4;
+    const double first = fma(r0, s, -h);
+    const double fr = fma(zeta, odd ? g2 : g3, fma(eta, odd ? g1 : g2, odd ? r0 : first));
+    const double F = from(fr, 0), r = from(fr, 1);
+    y = rcp_seed(r);
+    y = fma(y, fma(-r, y, 1.0), y);
+    const double u = F * y;
+    ds = -fma(u, (double)(q2 * ((float)u * tinv)), u);
+    s = s + ds;
+    if (!(fabs(z) <= 4.0 * KEP_ZMAX)) break;
+    done = fabs(u) <= KEP_STEP * fabs(s) && fabs(z) <= KEP_ZMAX;
+  } while (!done && ++iter < 6);
+  double del, val;  // val: fm1, gmh, dfdt, dgdtm1 by hl & 3
+  KepParams P;
+  const int w4 = hl & 3;
+  if (done) {
+    const double hd = 0.5 * ds;
+    if (!DRIFT_FIRST) g4 = fma(ds, fma(hd, g2, g3), g4);
+    const double gn = fma(ds, fma(hd, odd ? g1 : g0, odd ? g2 : g1), odd ? g3 : g2);
+    g2 = from(gn, 0);
+    g3 = from(gn, 1);
+    g1 = fma(-beta, g3, s);
+    const double r = fma(zeta, g2, fma(eta, g1, r0));
+    const double rinv = rcp_from(r, y);
+    const double krr = kr0 * rinv;
+    double pre, mul;
+    bool neg;
+    if (DRIFT_FIRST) {
+      const double ga = (w4 & 2) ? g1 : g2, gb = (w4 & 2) ? g2 : g3;
+      const double both = fma(h, ga, -(r0 * gb));
+      pre = (w4 & 2) ? krr : kr0;
+      mul = (w4 & 1) ? both : ga;
+      neg = !(w4 & 1);
+    } else {
+      const double kr = k * rinv;
+      const double h12 = fma(s, odd ? g2 : g3, odd ? -g3 : -2.0 * g4);
+      const double h1 = from(h12, 0), h2 = from(h12, 1);
+      const double eh = eta * h1;
+      const double ab = fma(w4 == 0 ? -kr0 : r0, w4 == 0 ? h1 : h2, w4 == 0 ? g2 : eh);
+      pre = (w4 == 2) ? krr : kr;
+      mul = (w4 < 2) ? ab : (w4 == 2) ? g1 : g2;
+      neg = w4 >= 2;
+    }
+    val = pre * mul;
+    if (neg) val = -val;
+    P.s = s; P.g1 = g1; P.g2 = g2; P.g3 = g3; P.r0 = r0; P.r0inv = r0inv; P.rinv = rinv; P.beta = beta; P.eta = eta;
+    P.zeta = zeta;
+    const double cx = from(val, c < 3 ? 0 : 2), cv = from(val, c < 3 ? 1 : 3);
+    del = fma(cv, vk, cx * xk);
+  } else {
+    double delxv[6];
+    kep_solve_general<DRIFT_FIRST>(X, V, k, h, delxv, P);
+    val = w4 == 0 ? P.fm1 : w4 == 1 ? P.gmh : w4 == 2 ? P.dfdt : P.dgdtm1;
+    del = delxv[0];
+#pragma unroll
+    for (int w = 1; w < 6; w++) del = (c == w) ? delxv[w] : del;
+  }
+  if (hl < 12) {
+    const int id = at + 3 * (hl < 6 ? i : j);
+    double xs = q[id], xe = q[6 * N + id];
+    kahan_fma(xs, xe, hl < 6 ? sh.pmj[pb] : -sh.pmi[pb], del);
+    q[id] = xs;
+    q[6 * N + id] = xe;
+  }
+  if (cap.p) {  // in put_capture's order, a value or two a lane
+    if (hl < 6) cap.put(coff + hl, d);
+    if (hl < 4) cap.put(coff + (hl == 0 ? 11 : hl == 1 ? 12 : hl == 2 ? 10 : 13), val);
+    const double pv[11] = {P.s, P.g1, P.g2, P.g3, P.r0, P.r0inv, P.rinv, k, P.beta, P.eta, P.zeta};
+    double own = pv[0];
+#pragma unroll
+    for (int w = 1; w < 11; w++) own = (hl == 4 + w) ? pv[w] : own;
+    if (hl >= 4 && hl < 15) cap.put(coff + (hl < 8 ? 2 + hl : 6 + hl), own);
+  }
+}
+
+// One AHL21 step of a kick-free group on the block's lanes (team_step's order).
+template <int N>
+__device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const Rec& cap, const Rec& xs) {
+  constexpr int P = N * (N - 1) / 2, T = 32 * lanes_warps(N);
+  static_assert(P <= T && 3 * N <= T, "one lane per pair and per coordinate");
+  const int t = threadIdx.x, half = t >> 4, hl = t & 15;
+  const unsigned mask = 0xffffu << (t & 16);
+  const double h2 = 0.5 * h;
+  Sys<N>& st = sh.st;
+  if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  lanes_sync<N>();
+#pragma unroll 1
+  for (int lev = 1; lev <= 2 * N - 3; lev++) {
+    int i, j;
+    if (level_pair<N>(lev, half, &i, &j)) lanes_pair<N, true>(sh, i, j, h2, cap, pair_bit(i, j, N) * PCAP, hl, mask);
+    lanes_sync<N>();
+  }
+  // pair t's bodies
+  int pi = 0, pj = t + 1;
+  while (pj >= N && pi < N - 2) {
+    pi++;
+    pj += pi + 1 - N;
+  }
+  double rij[3];
+  if (xs.p && t < 3 * N) xs.put(t, st.x[t]);
+  if (t < P) {
+#pragma unroll
+    for (int w = 0; w < 3; w++) rij[w] = st.x[3 * pi + w] - st.x[3 * pj + w];
+    phis_accel(rij, sh.f[t]);
+  }
+  lanes_sync<N>();
+  const int b = t / 3, w = t % 3;  // coordinate lane
+  if (t < 3 * N) {
+    double a = 0.0;
+    for (int o = 0; o < N; o++)
+      if (o != b) {
+        const double f = sh.f[o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)][w];
+        a = fma(o < b ? st.m[o] : -st.m[o], f, a);
+      }
+    sh.a[t] = a;
+    if (xs.p) xs.put(3 * N + t, a);
+  }
+  lanes_sync<N>();
+  if (t < P) {
+    double aij[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) aij[q] = sh.a[3 * pi + q] - sh.a[3 * pj + q];
+    phis_corr(rij, aij, st.m[pi] + st.m[pj], phis_coeff(h), sh.f[t]);
+  }
+  lanes_sync<N>();
+  if (t < 3 * N) {
+    double v = st.v[t], ve = st.ve[t];
+    for (int o = 0; o < N; o++)
+      if (o != b) kahan_fma(v, ve, o < b ? -st.m[o] : st.m[o], sh.f[o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)][w]);
+    st.v[t] = v;
+    st.ve[t] = ve;
+  }
+  lanes_sync<N>();
+#pragma unroll 1
+  for (int lev = 2 * N - 3; lev >= 1; lev--) {
+    int i, j;
+    if (level_pair<N>(lev, half, &i, &j))
+      lanes_pair<N, false>(sh, i, j, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP, hl, mask);
+    lanes_sync<N>();
+  }
+  if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  lanes_sync<N>();
+}
+
+template <int N>
+__global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupArgs g, int chunk) {
+  extern __shared__ double lanes_smem[];
+  LanesShared<N>& sh = *reinterpret_cast<LanesShared<N>*>(lanes_smem);
+  constexpr int P = N * (N - 1) / 2;
+  const int s = blockIdx.x, t = threadIdx.x, S = g.S;
+  if (s >= S || g.sysidx[s] < 0) return;
+  const long long nst = g.nsteps[s], k0 = chunk_first_step(g, chunk, s);
+  if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
+  Sys<N>& st = sh.st;
+  if (t < 3 * N) {
+    st.x[t] = g.x[t * S + s];
+    st.v[t] = g.v[t * S + s];
+    st.xe[t] = g.xe[t * S + s];
+    st.ve[t] = g.ve[t * S + s];
+  }
+  if (t < N) {
+    st.m[t] = g.m[t * S + s];
+    sh.g[t] = g.gsave[t * S + s];
+    sh.cnt[t] = g.count[t * S + s];
+  }
+  for (int q = t; q < 7 * N; q += blockDim.x) st.dqdt[q] = g.dqdt[q * S + s];
+  lanes_sync<N>();
+  if (t < P) {
+    int i = 0, j = t + 1;
+    while (j >= N && i < N - 2) {
+      i++;
+      j += i + 1 - N;
+    }
+    const double mij = st.m[i] + st.m[j], inv = rcp_fast(mij);
+    sh.pk[t] = GNEWT * mij;
+    sh.pmi[t] = st.m[i] * inv;
+    sh.pmj[t] = st.m[j] * inv;
+  }
+  lanes_sync<N>();
+  const double t0 = g.t0[s], h = g.h[s], hI = g.hI[s];
+  const int ntt = g.ntt[s], ti = g.ti[s];
+  for (int kk = 0; kk < g.K; kk++) {
+    const long long istep = k0 + kk;
+    if (istep >= nst) break;
+    Rec cap{nullptr, 0}, xs{nullptr, 0};
+    if (g.grad) {
+      cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
+      xs = Rec{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + s, S};
+    }
+    const double hs = step_length(g, s, istep, nst, h);
+    if (g.trajxv && t < 3 * N) {
+      double* rx = g.trajxv + ((size_t)s * g.K + kk) * 6 * N;
+      rx[t] = st.x[t];
+      rx[3 * N + t] = st.v[t];
+    }
+    if (g.grad && istep == nst - 1) {  // the last step also forms dq/dt: the one-lane step, on the first lane
+      if (t == 0) {
+        Work<N> w;
+        ahl21_step<N, true, true>(st, w, hs, 0, Rec{nullptr, 0}, cap, xs);
+      }
+      lanes_sync<N>();
+    } else {
+      lanes_step<N>(sh, hs, cap, xs);
+    }
+    if (!g.notransit && t < N - 1)
+      detect_transit<N>(g, st, s, kk, t, ti, ntt, hI, t0 + (double)(istep + 1) * h, sh.g, sh.cnt);
+    lanes_sync<N>();
+  }
+  if (t < 3 * N) {
+    g.x[t * S + s] = st.x[t];
+    g.v[t * S + s] = st.v[t];
+    g.xe[t * S + s] = st.xe[t];
+    g.ve[t * S + s] = st.ve[t];
+  }
+  if (g.grad && nst <= k0 + g.K)
+    for (int q = t; q < 7 * N; q += blockDim.x) g.dqdt[q * S + s] = st.dqdt[q];
+  if (t < N) {
+    g.gsave[t * S + s] = sh.g[t];
+    g.count[t * S + s] = sh.cnt[t];
+  }
+  if (t == 0 && !state_finite<N>(st)) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
 }
 
 }  // namespace nbg

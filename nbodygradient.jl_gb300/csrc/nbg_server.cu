@@ -615,12 +615,10 @@ int service_group(nbg_server* srv, int gi) {
   // searches on stt beside the operator records on sw, then the consumer
   NBG_CUDA(cudaMemsetAsync(gc.task_count, 0, sizeof(int), st));
   int rc;
-  {
-    // the wide team form while few slots are running (latency-bound chunks)
-    GroupArgs go = gc;
-    go.wide = use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2), G->kick) ? 1 : 0;
-    if ((rc = launch_group_orbit(N, go, (int)c, st))) return rc;
-  }
+  // the producer's and the consumer's forms for latency-bound chunks while few slots are running
+  GroupArgs gw = gc;
+  gw.wide = use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2), G->kick) ? 1 : 0;
+  if ((rc = launch_group_orbit(N, gw, (int)c, st))) return rc;
   NBG_CUDA(cudaEventRecord(G->ev_orb[par], st));
   NBG_CUDA(cudaStreamWaitEvent(stt, G->ev_orb[par], 0));
   NBG_CUDA(cudaStreamWaitEvent(sw, G->ev_orb[par], 0));
@@ -638,7 +636,7 @@ int service_group(nbg_server* srv, int gi) {
   }
   NBG_CUDA(cudaStreamWaitEvent(sw, G->ev_tr[par], 0));
   if (G->grad) {
-    if ((rc = launch_group_jacobian(N, gc, (int)c, sw))) return rc;
+    if ((rc = launch_group_jacobian(N, gw, (int)c, sw))) return rc;
     launches += 1;
   }
   // ---- retirement of the slots whose last step ran in this chunk, and of
