@@ -562,7 +562,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     g.tgrid = std::min(((g.task_cap + 31) / 32) * 32, std::max(1, ctx->sm_count) * 4 * 32);
     if (gp.grad) {
       GET(steprec, nb * nrec); GET(trec, nb * ntrec); GET(tflag, nb * nflag); GET(tscratch, (size_t)g.R * g.tgrid);
-      GET(pcap, nb * ncap); GET(xsnap, nb * nsnap);
+      GET(pcap, nb * ncap); GET(xsnap, nb * nsnap); GET(dh, 12 * (size_t)npk * S);
       GET(Jint, (size_t)S * 6 * N * 7 * N); GET(Eint, (size_t)S * 6 * N * 7 * N);
     }
 #undef GET
@@ -997,6 +997,7 @@ void noalloc_layout(NoallocPlan& P, ScratchArena& a, int nsys, int K, int tcap, 
       a.take(&g.tflag, (size_t)K * (N - 1) * S); a.take(&g.tscratch, (size_t)g.R * g.tgrid);
       a.take(&g.pcap, (size_t)K * 2 * g.npk * PCAP * S + 1);
       a.take(&g.xsnap, (size_t)K * snap_count(g.kick != 0) * 3 * N * S);
+      a.take(&g.dh, 12 * (size_t)g.npk * S);
       a.take(&g.Jint, (size_t)S * 6 * N * 7 * N); a.take(&g.Eint, (size_t)S * 6 * N * 7 * N);
     }
   }

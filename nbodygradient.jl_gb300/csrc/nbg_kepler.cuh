@@ -264,67 +264,56 @@ __device__ __noinline__ void kep_solve_general(const double* x0, const double* v
   P.k = k; P.h = h; P.beta = beta0; P.eta = eta; P.zeta = zeta;
 }
 
-// c_5 and c_6 of the Stumpff functions c_n(z) = sum_k (-z)^k / (n + 2k)!, to
-// degree 6 in -z: truncated below 3e-17 of c_5 and 8e-18 of c_6 at
-// |z| = KEP_ZMAX, and c_4, c_3, c_2, c_1, c_0 follow by c_n = 1/n! - z c_{n+2}
-// without a cancellation.
+// The Stumpff functions c_n(z) = sum_k (-z)^k / (n + 2k)!, n = 2..6, to degree
+// 7 in -z: truncated below 2e-17 of c_n at |z| = KEP_ZMAX.
 constexpr double KEP_ZMAX = 0.6;
-#define NBG_C5_COEF {1.0 / 120.0, 1.0 / 5040.0, 1.0 / 362880.0, 1.0 / 39916800.0, 1.0 / 6227020800.0, \
-                     1.0 / 1307674368000.0, 1.0 / 355687428096000.0}
-#define NBG_C6_COEF {1.0 / 720.0, 1.0 / 40320.0, 1.0 / 3628800.0, 1.0 / 479001600.0, 1.0 / 87178291200.0, \
-                     1.0 / 20922789888000.0, 1.0 / 6402373705728000.0}
-__device__ __forceinline__ double stumpff5(double z) {
-  constexpr double c[7] = NBG_C5_COEF;
-  double p = c[6];
+__device__ constexpr double inv_factorial(int n) {
+  double f = 1.0;
+  for (int q = 2; q <= n; q++) f *= q;  // exact up to 18!, rounded once or twice beyond
+  return 1.0 / f;
+}
+template <int NN>
+__device__ __forceinline__ double stumpff(double z) {
+  double p = inv_factorial(NN + 14);
 #pragma unroll
-  for (int q = 5; q >= 0; q--) p = fma(-z, p, c[q]);
+  for (int k = 6; k >= 0; k--) p = fma(-z, p, inv_factorial(NN + 2 * k));
   return p;
 }
-__device__ __forceinline__ double stumpff6(double z) {
-  constexpr double c[7] = NBG_C6_COEF;
-  double p = c[6];
+// c_2, c_3 or c_4, a lane's own (n = 0, 1, 2)
+__device__ __forceinline__ double stumpff234(double z, int n) {
+  double p = n == 0 ? inv_factorial(16) : n == 1 ? inv_factorial(17) : inv_factorial(18);
 #pragma unroll
-  for (int q = 5; q >= 0; q--) p = fma(-z, p, c[q]);
-  return p;
-}
-
-// stumpff6 (even lanes) or stumpff5 (odd lanes)
-__device__ __forceinline__ double stumpff_either(double z, bool odd) {
-  constexpr double a[7] = NBG_C6_COEF, b[7] = NBG_C5_COEF;
-  double p = odd ? b[6] : a[6];
-#pragma unroll
-  for (int q = 5; q >= 0; q--) p = fma(-z, p, odd ? b[q] : a[q]);
+  for (int k = 6; k >= 0; k--)
+    p = fma(-z, p, n == 0 ? inv_factorial(2 + 2 * k) : n == 1 ? inv_factorial(3 + 2 * k) : inv_factorial(4 + 2 * k));
   return p;
 }
 
 // FP32 start of the drift's solve.  With sigma = s r0 / h Kepler's equation
 // r0 s + eta G2 + zeta G3 = h reads sigma + a sigma^2 c_2 + b sigma^3 c_3 = 1
-// at z = w sigma^2; three Halley steps from the root of its quadratic part
-// leave an error of FP32 rounding.  q: half the ratio of the equation's second
-// to its first derivative at sigma, by sigma, for the FP64 step's second-order
-// term.  Nothing downstream depends on the start beyond the convergence test.
+// at z = w sigma^2; two third-order steps from 1 / (1 + a / 2) leave an error of
+// FP32 rounding for steps up to a tenth of a period.  q: half the ratio of the
+// equation's second to its first derivative at sigma, by s, for the FP64
+// step's second-order term.  Nothing downstream depends on the start beyond
+// the convergence test.
 __device__ __forceinline__ float kep_start(float r0inv, float h, float beta, float eta, float zeta, float* q) {
   const float t = h * r0inv;
   const float a = eta * t * r0inv, b = zeta * t * t * r0inv, w = beta * t * t;
-  const float disc = __fmaf_rn(2.0f, a, 1.0f);
-  float sg = disc > 0.0f ? __fdividef(2.0f, 1.0f + __fsqrt_rn(disc)) : 1.0f;
+  float sg = a > -1.0f ? __fdividef(1.0f, __fmaf_rn(0.5f, a, 1.0f)) : 1.0f;
   float half = 0.0f;
 #pragma unroll
-  for (int it = 0; it < 3; it++) {
-    const float z = w * sg * sg;
+  for (int it = 0; it < 2; it++) {
+    const float s2 = sg * sg, z = w * s2;
     const float c5 = __fmaf_rn(-z, __fmaf_rn(-z, 2.7557319e-6f, 1.9841270e-4f), 8.3333333e-3f);
     const float c4 = __fmaf_rn(-z, __fmaf_rn(-z, __fmaf_rn(-z, 2.7557319e-7f, 2.4801587e-5f), 1.3888889e-3f), 4.1666667e-2f);
     const float c3 = __fmaf_rn(-z, c5, 1.6666667e-1f), c2 = __fmaf_rn(-z, c4, 0.5f);
     const float c1 = __fmaf_rn(-z, c3, 1.0f), c0 = __fmaf_rn(-z, c2, 1.0f);
-    const float s2 = sg * sg;
     const float f = __fmaf_rn(b * s2 * sg, c3, __fmaf_rn(a * s2, c2, sg - 1.0f));
-    const float f1 = __fmaf_rn(b * s2, c2, __fmaf_rn(a * sg, c1, 1.0f));
-    const float f2 = __fmaf_rn(b * sg, c1, a * c0);
-    const float d = __fdividef(f, f1);
-    half = 0.5f * __fdividef(f2, f1);
-    sg = sg - __fdividef(d, __fmaf_rn(-d, half, 1.0f));
+    const float inv = __fdividef(1.0f, __fmaf_rn(b * s2, c2, __fmaf_rn(a * sg, c1, 1.0f)));
+    const float d = f * inv;
+    half = 0.5f * inv * __fmaf_rn(b * sg, c1, a * c0);
+    sg = __fmaf_rn(-d, __fmaf_rn(d, half, 1.0f), sg);
   }
-  *q = half;
+  *q = __fdividef(half, t);
   return sg;
 }
 
@@ -332,8 +321,8 @@ __device__ __forceinline__ float kep_start(float r0inv, float h, float beta, flo
 // (x0, v0) with k = G (m_i + m_j) over h; writes delxv (position and velocity
 // differences, finish - start minus the drift terms).
 //
-// Same quantities as the reference, other steps to them: 88 FP64 instructions
-// (99 for the drift that comes last) where the half-angle iteration took about
+// Same quantities as the reference, other steps to them: 86 FP64 instructions
+// (103 for the drift that comes last) where the half-angle iteration took about
 // 480, and 800 for a hyperbolic pair, most of them in five evaluations of sine
 // and cosine (sinh and exp) and in divisions.  FP64 step at the FP32 start:
 // F = r0 s + eta G2 + zeta G3 - h, u = F / r, ds = -(u + u^2 F'' / 2 r); the
@@ -359,28 +348,25 @@ __device__ __forceinline__ void kep_solve(const double* x0, const double* v0, do
   const double kr0 = k * r0inv;
   const double beta = fma(2.0, kr0, -vv);
   const double zeta = fma(-r0, beta, k);
+  const double t = h * r0inv;
   float q2;
   const float sg = kep_start((float)r0inv, (float)h, (float)beta, (float)eta, (float)zeta, &q2);
-  const double t = h * r0inv;
-  const float tinv = __fdividef(1.0f, (float)t);
+  const double q = (double)q2;
   double s = t * (double)sg, ds, y, g0, g1, g2, g3, g4 = 0.0;
   int iter = 0;
   bool done = false;
   do {
     const double ss = s * s, z = beta * ss;
-    const double c5 = stumpff5(z), c4 = fma(-z, stumpff6(z), 1.0 / 24.0);
-    g2 = ss * fma(-z, c4, 0.5);
-    const double sss = ss * s;
-    g3 = sss * fma(-z, c5, 1.0 / 6.0);
+    g2 = ss * stumpff<2>(z);
+    g3 = (ss * s) * stumpff<3>(z);
+    if (!DRIFT_FIRST) g4 = (ss * ss) * stumpff<4>(z);
     g0 = fma(-beta, g2, 1.0);
     g1 = fma(-beta, g3, s);
-    if (!DRIFT_FIRST) g4 = (ss * ss) * c4;
     const double F = fma(zeta, g3, fma(eta, g2, fma(r0, s, -h)));
     const double r = fma(zeta, g2, fma(eta, g1, r0));
     y = rcp_seed(r);
-    y = fma(y, fma(-r, y, 1.0), y);
     const double u = F * y;
-    ds = -fma(u, (double)(q2 * ((float)u * tinv)), u);
+    ds = -fma(u, fma(q, u, fma(-r, y, 1.0)), u);
     s = s + ds;
     if (!(fabs(z) <= 4.0 * KEP_ZMAX)) break;
     done = fabs(u) <= KEP_STEP * fabs(s) && fabs(z) <= KEP_ZMAX;
@@ -445,9 +431,9 @@ __device__ __forceinline__ void kep_derivatives(const KepParams& P, KepDeriv& o)
   const double ss = s * s, z = beta * ss, s3 = ss * s, s4 = ss * ss;
   double g4, g5, g6;
   if (fabs(z) <= 1.01 * KEP_ZMAX) {
-    const double c6 = stumpff6(z);
+    const double c6 = stumpff<6>(z);
     g4 = s4 * fma(-z, c6, 1.0 / 24.0);
-    g5 = (s4 * s) * stumpff5(z);
+    g5 = (s4 * s) * stumpff<5>(z);
     g6 = (s4 * ss) * c6;
   } else {
     const double bi = 1.0 / beta;

@@ -23,7 +23,7 @@
 namespace nbg {
 
 // Orbit producer for one chunk of K steps of one group (one lane per system).
-template <int N>
+template <int N, bool KICK>
 __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(GroupArgs g, int chunk) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane >= g.spw) return;
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
   const long long k0 = chunk_first_step(g, chunk, s);
   if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
   Sys<N> st;
-  Work<N> w;
+  double a[3 * N];
   for (int q = 0; q < 3 * N; q++) {
     st.x[q] = g.x[q * S + s];
     st.v[q] = g.v[q * S + s];
@@ -42,7 +42,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     st.ve[q] = g.ve[q * S + s];
   }
   for (int q = 0; q < N; q++) st.m[q] = g.m[q * S + s];
-  for (int q = 0; q < 7 * N; q++) st.dqdt[q] = g.dqdt[q * S + s];
+  if (KICK)
+    for (int q = 0; q < 7 * N; q++) st.dqdt[q] = g.dqdt[q * S + s];
   double gsave[N];
   long long count[N];
   for (int q = 0; q < N; q++) {
@@ -63,15 +64,23 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
         rx[3 * N + q] = st.v[q];
       }
     }
+    // x, v only; the operators are built from the captures by the operator kernels
+    Rec cap{nullptr, 0}, xs{nullptr, 0};
     if (g.grad) {
-      // x, v only; the operators are built from the captures by the operator
-      // kernels.  The last step also computes dq/dt, the State's output.
-      Rec cap{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
-      Rec xs{g.xsnap + (size_t)kk * snap_count(kick != 0) * 3 * N * S + s, S};
-      if (istep == nst - 1) ahl21_step<N, true, true>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
-      else ahl21_step<N, false, false>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
+      cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
+      xs = Rec{g.xsnap + (size_t)kk * snap_count(KICK) * 3 * N * S + s, S};
+    }
+    const bool last = g.grad && istep == nst - 1;
+    if (!KICK) {
+      if (last)  // v at the last step's start, for its dq/dt (dq_columns)
+        for (int q = 0; q < 3 * N; q++) g.dqdt[(7 * (q / 3) + 3 + q % 3) * S + s] = st.v[q];
+      plain_step<N>(st, a, hs, cap, xs);
+    } else if (last) {  // the last step also computes dq/dt, the State's output
+      Work<N> w;
+      ahl21_step<N, true, true>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
     } else {
-      ahl21_step<N, false, false>(st, w, hs, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
+      Work<N> w;
+      ahl21_step<N, false, false>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
     }
     if (g.notransit) continue;
     const double t = t0 + (double)(istep + 1) * h;
@@ -83,7 +92,7 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     g.xe[q * S + s] = st.xe[q];
     g.ve[q * S + s] = st.ve[q];
   }
-  if (g.grad && nst <= k0 + g.K)  // the chunk that ran the last step holds the final dq/dt
+  if (KICK && g.grad && nst <= k0 + g.K)  // the chunk that ran the last step holds the final dq/dt
     for (int q = 0; q < 7 * N; q++) g.dqdt[q * S + s] = st.dqdt[q];
   for (int q = 0; q < N; q++) {
     g.gsave[q * S + s] = gsave[q];
@@ -218,7 +227,8 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       tt2 = tt1;
       tt1 = dt0;
       wk = st;
-      ahl21_step<N, false, false>(wk, w, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
+      if (kick) ahl21_step<N, false, false>(wk, w, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
+      else plain_step<N>(wk, w.a, dt0, Rec{nullptr, 0}, Rec{nullptr, 0});
       const double gs = gsky(wk, ti, ib);
       const double gd = gdot_physical(wk, ti, ib);
       const double dt = -gs / gd;
@@ -306,7 +316,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_team_kernel(GroupArgs g, i
         for (int q = t; q < N; q += L) wks[tm].m[q] = st0[tm].m[q];
       }
       __syncwarp();
-      team_step<N>(wks[tm], acc[tm], w, t, active, dt0, Rec{nullptr, 0}, Rec{nullptr, 0});
+      team_step<N>(wks[tm], acc[tm], t, active, dt0, Rec{nullptr, 0}, Rec{nullptr, 0});
       __syncwarp();
       if (active) {
         const double gs = gsky(wks[tm], ti, ib);
@@ -349,7 +359,7 @@ __global__ void __launch_bounds__(OPS_BS) operator_pair_kernel(GroupArgs g, int 
   // step that had mass (ahl21.jl:713 returns before refilling it); zero at the
   // start of the step (zero_out!, ahl21.jl:8).
   int q = slot;
-  while (q >= 0 && cap.get(q * PCAP + PCAP_K) == 0.0) q--;
+  while (q >= 0 && cap.get(q * PCAP + PCAP_RINV) == 0.0) q--;
   if (q < 0) {
     for (int e = 0; e < PREC; e++) rec.put(roff + e, 0.0);
     return;
@@ -358,8 +368,10 @@ __global__ void __launch_bounds__(OPS_BS) operator_pair_kernel(GroupArgs g, int 
   pair_of_slot<N>(q, g.npk, kick, &i, &j);
   const double mi = g.m[i * S + s], mj = g.m[j * S + s];
   const double h2 = 0.5 * step_length(g, s, istep, g.nsteps[s], g.h[s]);
-  if (q < g.npk) pair_record_from_capture<true>(cap, q * PCAP, mi, mj, h2, rec, roff);
-  else pair_record_from_capture<false>(cap, q * PCAP, mi, mj, h2, rec, roff);
+  Rec dh{nullptr, 0};
+  if (!kick && q == slot && istep == g.nsteps[s] - 1) dh = Rec{g.dh + (size_t)slot * 6 * S + s, S};
+  if (q < g.npk) pair_record_from_capture<true>(cap, q * PCAP, mi, mj, h2, rec, roff, dh);
+  else pair_record_from_capture<false>(cap, q * PCAP, mi, mj, h2, rec, roff, dh);
 }
 
 // Corrector records of one chunk of a group without kick pairs: one lane per
@@ -478,10 +490,115 @@ __device__ __forceinline__ void column_transits(const GroupArgs& g, int s, int c
   }
 }
 
+// dq/dt of a system's last step (the State's dqdt; ahl21.jl:9-14, :20-24, :36-42
+// and so on), kick-free groups: one more column that the step's operators act
+// on, with the drift velocities, the drifts' derivative by h and the corrector's
+// dv/dt added on the way.  It is formed here, from the last step's record, and
+// not by the producers: there it made the last step a one-lane gradient step
+// (2.8 ms at eight bodies, 0.15 ms at two) and kept that step's working arrays
+// on every producer's stack.  Six lanes per system, one for each row of a body,
+// five systems a warp; sh: DQ_DOUBLES of the warp's own.
+template <int N>
+constexpr int DQ_DOUBLES = (9 * N + 3 * (N * (N - 1) / 2)) * 5;
+template <int N>
+__device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh) {
+  constexpr int P = N * (N - 1) / 2, C = 5;
+  const int lane = threadIdx.x & 31, l = lane % 6, col = lane < 30 ? lane / 6 : 0, S = g.S;
+  const int s = first + col;
+  bool live = lane < 30 && s < S && g.grad && g.sysidx[s] >= 0;
+  const long long nst = live ? g.nsteps[s] : 0, k0 = live ? chunk_first_step(g, chunk, s) : 0;
+  live = live && k0 >= 0 && nst > k0 && nst <= k0 + g.K;
+  if (!__any_sync(0xffffffffu, live)) return;
+  const int kk = live ? (int)(nst - 1 - k0) : 0, at = live ? s : 0;
+  const Rec rec{g.steprec + (size_t)kk * g.R * S + at, S}, dh{g.dh + at, S};
+  const Rec cap{g.pcap + (size_t)kk * 2 * P * PCAP * S + at, S}, xs{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + at, S};
+  const double h = live ? step_length(g, s, nst - 1, nst, g.h[s]) : 1.0, h2 = 0.5 * h;
+  double *Q = sh, *D = Q + 6 * N * C, *F = D + 3 * N * C;
+  for (int b = 0; b < N; b++)
+    if (live) Q[(6 * b + l) * C + col] = l < 3 ? 0.5 * g.dqdt[(7 * b + 3 + l) * S + s] : 0.0;
+  double last_i = 0.0, last_j = 0.0;
+  auto pair = [&](int i, int j, int slot, int roff) {
+    const int ai = (6 * i + l) * C + col, aj = (6 * j + l) * C + col;
+    double ti = 0.0, tj = 0.0, K[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, mi = 0.0, mj = 0.0, by_h = 0.0;
+    bool stale = false;
+    if (live) {
+#pragma unroll
+      for (int q = 0; q < 6; q++) K[q] = rec.get(roff + 6 * l + q);
+      mi = rec.get(roff + PREC_MI);
+      mj = rec.get(roff + PREC_MJ);
+      stale = cap.get(slot * PCAP + PCAP_RINV) == 0.0;
+      if (!stale) by_h = dh.get(slot * 6 + l);
+      ti = Q[ai];
+      tj = Q[aj];
+    }
+    const double d = ti - tj;
+    double u = 0.0;
+#pragma unroll
+    for (int q = 0; q < 6; q++) u = fma(K[q], __shfl_sync(0xffffffffu, d, 6 * col + q), u);
+    // a pair without mass keeps dqdt_ij, too, as the last pair left it (ahl21.jl:713)
+    const double w = fma(0.5, by_h, u);
+    last_i = fma(mj, w, stale ? fma(0.5, last_i, ti) : ti);
+    last_j = fma(-mi, w, stale ? fma(0.5, last_j, tj) : tj);
+    if (live) {
+      Q[ai] = last_i;
+      Q[aj] = last_j;
+    }
+  };
+  int slot = 0, roff = 0;
+  for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++, roff += PREC) pair(i, j, slot++, roff);
+  __syncwarp();
+  if (live) {
+    if (l < 3)
+      for (int d = 1; d < N; d++) D[(3 * d + l) * C + col] = Q[(6 * d + l) * C + col] - Q[l * C + col];
+    int p = 0;
+    for (int i = 0; i < N - 1; i++)
+      for (int j = i + 1; j < N; j++, p++) {
+        if (p % 6 != l) continue;
+        double rij[3], aij[3], f[3];
+        for (int k = 0; k < 3; k++) {
+          rij[k] = xs.get(3 * i + k) - xs.get(3 * j + k);
+          aij[k] = xs.get(3 * N + 3 * i + k) - xs.get(3 * N + 3 * j + k);
+        }
+        const double r2 = norm2(rij);
+        phis_corr(rij, r2, rsqrt_fast(r2), aij, g.m[i * S + s] + g.m[j * S + s], phis_coeff(h), f);
+        for (int k = 0; k < 3; k++) F[(3 * p + k) * C + col] = f[k];
+      }
+  }
+  __syncwarp();
+  if (live) {
+    const double hi3 = 3.0 / h;  // the correction goes with h^3
+    for (int row = l; row < 3 * N; row += 6) {
+      const int b = row / 3, k = row % 3;
+      double acc = 0.0, op = 0.0;
+      for (int q = 0; q < 3 * (N - 1); q++)
+        acc = fma(rec.get(roff + row * (4 * N) + 4 + 4 * (q / 3) + q % 3), D[(3 + q) * C + col], acc);
+      for (int o = 0; o < N; o++)
+        if (o != b)
+          op = fma(o < b ? -g.m[o * S + s] : g.m[o * S + s],
+                   F[(3 * (o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)) + k) * C + col], op);
+      const int r = (6 * b + 3 + k) * C + col;
+      Q[r] = Q[r] + fma(hi3, op, acc);
+    }
+  }
+  __syncwarp();
+  roff += op_size(N);
+  for (int i = N - 2; i >= 0; i--)
+    for (int j = N - 1; j > i; j--, roff += PREC) pair(i, j, slot++, roff);
+  __syncwarp();
+  if (live)
+    for (int b = 0; b < N; b++) {
+      double q = Q[(6 * b + l) * C + col];
+      if (l < 3) q = q + fma(h2, Q[(6 * b + 3 + l) * C + col], 0.5 * g.v[(3 * b + l) * S + s]);
+      g.dqdt[(7 * b + l) * S + s] = q;
+      if (l == 0) g.dqdt[(7 * b + 6) * S + s] = 0.0;
+    }
+}
+
 // Jacobian consumer for one chunk of K steps (one lane per column).  A group
 // without kick pairs has its mass columns in blocks of their own: the first
-// `plain` blocks hold the other 6N columns of every system, the rest the N mass
-// columns.
+// `plain` blocks hold the other 6N columns of every system, the next ones, up
+// to `all`, the N mass columns; the last ones form dq/dt.
 template <int N, int BS, int MODE>  // 0: kick group, every column; 1: not a mass column; 2: a mass column
 __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int s, int c, double* smem) {
   constexpr int M = 7 * N, R6 = 6 * N;
@@ -526,15 +643,19 @@ __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int
 }
 
 template <int N>
-__global__ void __launch_bounds__(cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain) {
+__global__ void __launch_bounds__(cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain, int all) {
   extern __shared__ double smem[];
   constexpr int BS = cons_bs(N);
   if ((int)blockIdx.x < plain) {
     const int f = blockIdx.x * BS + threadIdx.x, q = f % (6 * N);
     consume_chunk<N, BS, 1>(g, chunk, f / (6 * N), 7 * (q / 6) + q % 6, smem);
-  } else {
+  } else if ((int)blockIdx.x < all) {
     const int f = (blockIdx.x - plain) * BS + threadIdx.x;
     consume_chunk<N, BS, 2>(g, chunk, f / N, 7 * (f % N) + 6, smem);
+  } else {
+    static_assert(DQ_DOUBLES<N> * (BS / 32) <= 2 * 6 * N * BS, "dq_columns' share of the columns' shared memory");
+    const int w = (blockIdx.x - all) * (BS / 32) + threadIdx.x / 32;
+    dq_columns<N>(g, chunk, 5 * w, smem + DQ_DOUBLES<N> * (threadIdx.x / 32));
   }
 }
 
@@ -565,6 +686,7 @@ constexpr int ROWS_COLS = 5, ROWS_WARPS = 2;
 __host__ __device__ constexpr int rows_plain_warps(int N) { return (6 * N + ROWS_COLS - 1) / ROWS_COLS; }
 __host__ __device__ constexpr int rows_warps(int N) { return rows_plain_warps(N) + (N + ROWS_COLS - 1) / ROWS_COLS; }
 __host__ __device__ constexpr int rows_record(int N) { return N * (N - 1) * PREC + op_size(N); }
+__host__ __device__ constexpr int rows_blocks(int N) { return (rows_warps(N) + ROWS_WARPS - 1) / ROWS_WARPS; }
 template <int N>
 struct RowsShared {
   double rec[2][rows_record(N)];
@@ -683,6 +805,10 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) jacobian_rows_kernel(GroupArg
   RowsShared<N>& sh = *reinterpret_cast<RowsShared<N>*>(smem);
   constexpr int M = 7 * N, R6 = 6 * N, R = rows_record(N);
   const int s = blockIdx.x, S = g.S, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if ((int)blockIdx.y == rows_blocks(N)) {  // the last row of blocks forms dq/dt
+    dq_columns<N>(g, chunk, 5 * (ROWS_WARPS * s + warp), smem + DQ_DOUBLES<N> * warp);
+    return;
+  }
   if (s >= S || g.sysidx[s] < 0) return;
   const long long nst = g.nsteps[s], k0 = chunk_first_step(g, chunk, s);
   if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
@@ -808,8 +934,13 @@ int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
     return 0;
   }
   const int blocks = (g.S + W * g.spw - 1) / (W * g.spw);
-  allow_smem(orbit_chunk_kernel<N>, g.prod_smem);
-  orbit_chunk_kernel<N><<<blocks, PROD_BS * W, g.prod_smem, st>>>(g, chunk);
+  if (g.kick) {
+    allow_smem(orbit_chunk_kernel<N, true>, g.prod_smem);
+    orbit_chunk_kernel<N, true><<<blocks, PROD_BS * W, g.prod_smem, st>>>(g, chunk);
+  } else {
+    allow_smem(orbit_chunk_kernel<N, false>, g.prod_smem);
+    orbit_chunk_kernel<N, false><<<blocks, PROD_BS * W, g.prod_smem, st>>>(g, chunk);
+  }
   return 0;
 }
 
@@ -826,13 +957,15 @@ int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
   if (g.wide) {
     const int bytes = std::max((int)sizeof(RowsShared<N>), 24 * 1024);  // as every consumer block: none fits beside a tail producer's
     allow_smem(jacobian_rows_kernel<N>, bytes);
-    const dim3 grid(g.S, (rows_warps(N) + ROWS_WARPS - 1) / ROWS_WARPS);
+    static_assert(sizeof(double) * DQ_DOUBLES<N> * ROWS_WARPS <= sizeof(RowsShared<N>) || N <= 2, "dq_columns fits");
+    const dim3 grid(g.S, rows_blocks(N) + 1);
     jacobian_rows_kernel<N><<<grid, 32 * ROWS_WARPS, bytes, st>>>(g, chunk);
     return 0;
   }
   const int plain = blocks((long long)g.S * 6 * N);
   allow_smem(jacobian_chunk_kernel<N>, smem);
-  jacobian_chunk_kernel<N><<<plain + blocks((long long)g.S * N), BS, smem, st>>>(g, chunk, plain);
+  const int all = plain + blocks((long long)g.S * N), dq = (g.S + 5 * (BS / 32) - 1) / (5 * (BS / 32));
+  jacobian_chunk_kernel<N><<<all + dq, BS, smem, st>>>(g, chunk, plain, all);
   return 0;
 }
 

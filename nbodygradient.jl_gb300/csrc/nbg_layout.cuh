@@ -39,10 +39,11 @@ constexpr int OPS_BS = 128;     // operator kernels
 // v_sky and b_sky^2, v_sky and d v_sky / dt (21N + 3).
 __host__ __device__ inline int trec_size(int N, int tbv) { return tbv ? 21 * N + 3 : 7 * N + 1; }
 
-// Captured Kepler-pair parameters (producer -> operator kernel): x0[3], v0[3]
-// and the solve's 15 values (put_capture); k's place.
-constexpr int PCAP = 21;
-constexpr int PCAP_K = 17;
+// Captured Kepler-pair parameters (producer -> operator kernel), see
+// put_capture: x0[3], v0[3], eight values of the solve and the four
+// coefficients of its result.  1/r = 0 in its place marks a pair without mass.
+constexpr int PCAP = 18;
+constexpr int PCAP_RINV = 11;
 // Snapshots per step, 3N doubles each: positions at the correctors, then
 // phisalpha!'s accelerations there, or in kick groups the positions at the
 // first and at the second kick.
@@ -109,8 +110,11 @@ struct GroupArgs {
   double* tscratch;  // [R][tgrid]: operator records of a search's final partial step
   int tgrid;         // threads of the transit kernel
   // producer captures for the operator kernels
-  double* pcap;   // [K][2 npk][21][S]: Kepler-pair parameters
+  double* pcap;   // [K][2 npk][18][S]: Kepler-pair parameters
   double* xsnap;  // [K][snaps][3N][S]: see snap_count
+  // d(delxv)/dh of a system's last step, for its dq/dt: [2 npk][6][S] (groups
+  // without kick pairs)
+  double* dh;
 };
 
 // Length of step istep of the system in slot s (nst steps in all).

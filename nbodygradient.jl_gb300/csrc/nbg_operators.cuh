@@ -39,21 +39,33 @@ __device__ __forceinline__ void pair_of_slot(int q, int npk, uint64_t kick, int*
 }
 
 // kepler_driftij_gamma!'s Jacobian part for one pair from its capture; h2 is
-// the drift's half step.
+// the drift's half step.  k, zeta and G1 are formed again, as kep_solve does.
+// With dh.p the derivative by h follows there.
 template <bool DRIFT_FIRST>
 __device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int coff, double m_i, double m_j, double h2,
-                                                         const Rec& rec, int roff) {
+                                                         const Rec& rec, int roff, const Rec& dh) {
   double v[PCAP];
 #pragma unroll
   for (int q = 0; q < PCAP; q++) v[q] = cap.get(coff + q);
   const double *x0 = v, *v0 = v + 3;
   KepParams P;
-  P.s = v[6]; P.g1 = v[7]; P.g2 = v[8]; P.g3 = v[9]; P.dfdt = v[10]; P.fm1 = v[11]; P.gmh = v[12]; P.dgdtm1 = v[13];
-  P.r0 = v[14]; P.r0inv = v[15]; P.rinv = v[16]; P.k = v[PCAP_K]; P.beta = v[18]; P.eta = v[19]; P.zeta = v[20];
+  P.s = v[6]; P.g2 = v[7]; P.g3 = v[8]; P.r0 = v[9]; P.r0inv = v[10]; P.rinv = v[PCAP_RINV]; P.beta = v[12]; P.eta = v[13];
+  P.fm1 = v[14]; P.gmh = v[15]; P.dfdt = v[16]; P.dgdtm1 = v[17];
+  P.k = GNEWT * (m_i + m_j);
+  P.zeta = fma(-P.r0, P.beta, P.k);
+  P.g1 = fma(-P.beta, P.g3, P.s);
   P.h = h2;
   KepDeriv D;
   double K[36], psi[6];
-  kep_derivatives<DRIFT_FIRST, false>(P, D);
+  if (dh.p) {
+    double by_h[6];
+    kep_derivatives<DRIFT_FIRST, true>(P, D);
+    kep_by_h<DRIFT_FIRST>(P, D, x0, v0, by_h);
+#pragma unroll
+    for (int r = 0; r < 6; r++) dh.put(r, by_h[r]);
+  } else {
+    kep_derivatives<DRIFT_FIRST, false>(P, D);
+  }
   kep_block<DRIFT_FIRST>(P, D, x0, v0, K, psi);
   const double mijinv = rcp_fast(m_i + m_j);
 #pragma unroll

@@ -275,15 +275,14 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
 
 // phisalpha! (ahl21.jl:558-700 / ahl21_no_grad.jl:110-158) for Kepler pairs,
 // one pair at a time: the accelerations, then the velocity corrections.
-__device__ __forceinline__ void phis_accel(const double* rij, double* f) {
-  const double rinv = rsqrt_fast(fma(rij[2], rij[2], fma(rij[1], rij[1], rij[0] * rij[0])));
+__device__ __forceinline__ double norm2(const double* r) { return fma(r[2], r[2], fma(r[1], r[1], r[0] * r[0])); }
+__device__ __forceinline__ void phis_accel(const double* rij, double rinv, double* f) {
   const double f2 = (GNEWT * rinv) * (rinv * rinv);
 #pragma unroll
   for (int k = 0; k < 3; k++) f[k] = f2 * rij[k];
 }
-__device__ __forceinline__ void phis_corr(const double* rij, const double* aij, double mij, double coeff, double* f) {
-  const double r2 = fma(rij[2], rij[2], fma(rij[1], rij[1], rij[0] * rij[0]));
-  const double rinv = rsqrt_fast(r2);
+__device__ __forceinline__ void phis_corr(const double* rij, double r2, double rinv, const double* aij, double mij,
+                                          double coeff, double* f) {
   const double ri2 = rinv * rinv;
   const double fac1 = (coeff * rinv) * (ri2 * ri2);
   const double ardot = fma(aij[2], rij[2], fma(aij[1], rij[1], aij[0] * rij[0]));
@@ -299,7 +298,7 @@ __device__ __forceinline__ void phis_accel_pair(const Sys<N>& s, double* a, int 
   double rij[3], f[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-  phis_accel(rij, f);
+  phis_accel(rij, rsqrt_fast(norm2(rij)), f);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     a[3 * i + k] = fma(-s.m[j], f[k], a[3 * i + k]);
@@ -314,7 +313,8 @@ __device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i
     aij[k] = a[3 * i + k] - a[3 * j + k];
     rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
   }
-  phis_corr(rij, aij, s.m[i] + s.m[j], coeff, f);
+  const double r2 = norm2(rij);
+  phis_corr(rij, r2, rsqrt_fast(r2), aij, s.m[i] + s.m[j], coeff, f);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], s.m[j], f[k]);
@@ -445,7 +445,8 @@ __device__ void phisalpha_operator(const Sys<N>& s, Work<N>& w, double h, uint64
         aij[k] = w.a[3 * i + k] - w.a[3 * j + k];
         rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
       }
-      phis_corr(rij, aij, s.m[i] + s.m[j], coeff, f);
+      const double r2 = norm2(rij);
+      phis_corr(rij, r2, rsqrt_fast(r2), aij, s.m[i] + s.m[j], coeff, f);
       for (int k = 0; k < 3; k++) {
         w.dqop[3 * i + k] = fma(hi3 * s.m[j], f[k], w.dqop[3 * i + k]);
         w.dqop[3 * j + k] = fma(-hi3 * s.m[i], f[k], w.dqop[3 * j + k]);
@@ -453,21 +454,20 @@ __device__ void phisalpha_operator(const Sys<N>& s, Work<N>& w, double h, uint64
     }
 }
 
-// Writes one solved pair's capture: x0, v0 and the KepParams but h.
+// Writes one solved pair's capture (pair_record_from_capture reads it).
 __device__ __forceinline__ void put_capture(const Rec& cap, int coff, const double* x0, const double* v0,
                                             const KepParams& P) {
-  const double pv[PCAP] = {x0[0], x0[1], x0[2], v0[0],  v0[1],    v0[2], P.s, P.g1,    P.g2,   P.g3,  P.dfdt,
-                           P.fm1, P.gmh, P.dgdtm1, P.r0, P.r0inv, P.rinv, P.k, P.beta, P.eta, P.zeta};
+  const double pv[PCAP] = {x0[0], x0[1], x0[2], v0[0],  v0[1], v0[2], P.s,   P.g2,   P.g3,
+                           P.r0,  P.r0inv, P.rinv, P.beta, P.eta, P.fm1, P.gmh, P.dfdt, P.dgdtm1};
 #pragma unroll
   for (int q = 0; q < PCAP; q++) cap.put(coff + q, pv[q]);
 }
 
-// kepler_driftij_gamma! (ahl21.jl:706-760 with the block update of :31-42 on
-// dq/dt; ahl21_no_grad.jl:192-212 without Jacobian).
-template <int N, bool DRIFT_FIRST, bool GRADOPS, bool DQDT>
-__device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, const Rec& rec, int roff,
-                            const Rec& cap, int coff) {
-  double x0[3], v0[3];
+// kepler_driftij_gamma! without Jacobian (ahl21_no_grad.jl:192-212).  P and
+// delxv are left for the caller's Jacobian; false for a pair without mass.
+template <int N, bool DRIFT_FIRST>
+__device__ __forceinline__ bool kepler_pair(Sys<N>& s, int i, int j, double h2, const Rec& cap, int coff, double* x0,
+                                            double* v0, KepParams& P, double* delxv) {
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     x0[k] = s.x[3 * i + k] - s.x[3 * j + k];
@@ -475,13 +475,41 @@ __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, cons
   }
   const double mij = s.m[i] + s.m[j];
   const double gm = GNEWT * mij;
-  if (cap.p && gm == 0.0) cap.put(coff + PCAP_K, 0.0);  // k = 0 marks a pair that keeps the stale jac_ij
-  if (gm != 0.0) {
-    KepParams P;
-    double delxv[6];
-    kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
-    if (cap.p) put_capture(cap, coff, x0, v0, P);
-    const double mijinv = rcp_fast(mij);
+  if (gm == 0.0) {
+    if (cap.p) cap.put(coff + PCAP_RINV, 0.0);  // a pair that keeps the stale jac_ij
+    return false;
+  }
+  kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
+  if (cap.p) put_capture(cap, coff, x0, v0, P);
+  const double mijinv = rcp_fast(mij);
+  const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    kahan_fma(s.x[3 * i + k], s.xe[3 * i + k], mj, delxv[k]);
+    kahan_fma(s.x[3 * j + k], s.xe[3 * j + k], -mi, delxv[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], mj, delxv[3 + k]);
+    kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -mi, delxv[3 + k]);
+  }
+  return true;
+}
+template <int N, bool DRIFT_FIRST>
+__device__ __forceinline__ void kepler_pair(Sys<N>& s, int i, int j, double h2, const Rec& cap, int coff) {
+  double x0[3], v0[3], delxv[6];
+  KepParams P;
+  kepler_pair<N, DRIFT_FIRST>(s, i, j, h2, cap, coff, x0, v0, P, delxv);
+}
+
+// The same with the block update of ahl21.jl:31-42 on dq/dt (ahl21.jl:706-760).
+template <int N, bool DRIFT_FIRST, bool GRADOPS, bool DQDT>
+__device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, const Rec& rec, int roff,
+                            const Rec& cap, int coff) {
+  double x0[3], v0[3], delxv[6];
+  KepParams P;
+  if (kepler_pair<N, DRIFT_FIRST>(s, i, j, h2, cap, coff, x0, v0, P, delxv)) {
+    const double mijinv = rcp_fast(s.m[i] + s.m[j]);
     const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
     if (GRADOPS) {
       KepDeriv D;
@@ -497,16 +525,6 @@ __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, cons
         w.ldq[7 + r] = (-mi) * dh[r];
       }
       w.ldq[6] = w.ldq[13] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      kahan_fma(s.x[3 * i + k], s.xe[3 * i + k], mj, delxv[k]);
-      kahan_fma(s.x[3 * j + k], s.xe[3 * j + k], -mi, delxv[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], mj, delxv[3 + k]);
-      kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -mi, delxv[3 + k]);
     }
   }
   if (GRADOPS && rec.p) {
@@ -615,6 +633,29 @@ __device__ __noinline__ void ahl21_step(Sys<N>& s, Work<N>& w, double h, uint64_
     if (GRADOPS) put_op(rec, roff, w.op, op_size(N));
     roff += op_size(N);
   }
+}
+
+// The same step without gradient for a group with no kick pairs
+// (ahl21_no_grad.jl:6-18): x and v alone, a the accelerations at the corrector.
+template <int N>
+__device__ __forceinline__ void plain_step(Sys<N>& s, double* a, double h, const Rec& cap, const Rec& xs) {
+  const double h2 = 0.5 * h;
+  int slot = 0;
+  drift(s, h2);
+#pragma unroll 1
+  for (int i = 0; i < N - 1; i++)
+#pragma unroll 1
+    for (int j = i + 1; j < N; j++) kepler_pair<N, true>(s, i, j, h2, cap, PCAP * slot++);
+  if (xs.p)
+    for (int q = 0; q < 3 * N; q++) xs.put(q, s.x[q]);
+  phisalpha<N>(s, a, h, 0);
+  if (xs.p)
+    for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, a[q]);
+#pragma unroll 1
+  for (int i = N - 2; i >= 0; i--)
+#pragma unroll 1
+    for (int j = N - 1; j > i; j--) kepler_pair<N, false>(s, i, j, h2, cap, PCAP * slot++);
+  drift(s, h2);
 }
 
 // g! and gd! (src/transits/timing.jl:141-150) for transited body i and

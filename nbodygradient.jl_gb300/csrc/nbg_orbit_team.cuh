@@ -21,8 +21,6 @@
 // N(N-1)/2 to 2N-3 pair solves (N = 10: 45 -> 17; N = 8: 28 -> 13).
 //
 // Groups with kick pairs (pair[i,j] == true) keep the one-lane producer.
-// The last step of a grad system (which also forms dq/dt, the State's
-// output) runs the one-lane step on the team's first lane.
 #pragma once
 #include "nbg_orbit.cuh"
 
@@ -47,7 +45,7 @@ __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {
 // __syncwarp).  cap / xs as in ahl21_step.  a: the team's 3N acceleration
 // scratch.
 template <int N>
-__device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int t, bool run, double h,
+__device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run, double h,
                                           const Rec& cap, const Rec& xs) {
   constexpr int L = team_lanes(N);
   constexpr int P = N * (N - 1) / 2;
@@ -58,7 +56,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
     if (run && level_pair<N>(lev, t, &i, &j))
-      kepler_pair<N, true, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap, pair_bit(i, j, N) * PCAP);
+      kepler_pair<N, true>(s, i, j, h2, cap, pair_bit(i, j, N) * PCAP);
     __syncwarp();
   }
   if (run) {
@@ -83,8 +81,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, Work<N>& w, int 
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
     int i, j;
     if (run && level_pair<N>(lev, t, &i, &j))
-      kepler_pair<N, false, false, false>(s, w, i, j, h2, Rec{nullptr, 0}, 0, cap,
-                                          (P + (P - 1 - pair_bit(i, j, N))) * PCAP);
+      kepler_pair<N, false>(s, i, j, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP);
     __syncwarp();
   }
   if (run)
@@ -137,17 +134,14 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
       gsv[tm][q] = g.gsave[q * S + s];
       cnt[tm][q] = g.count[q * S + s];
     }
-    for (int q = t; q < 7 * N; q += L) st.dqdt[q] = g.dqdt[q * S + s];
   }
   __syncwarp();
-  Work<N> w;
   const double t0 = valid ? g.t0[s] : 0.0, h = valid ? g.h[s] : 0.0, hI = valid ? g.hI[s] : 0.0;
   const int ntt = valid ? g.ntt[s] : 0, ti = valid ? g.ti[s] : 0;
   for (int kk = 0; kk < g.K; kk++) {
     const long long istep = k0 + kk;
     const bool run = valid && istep < nst;
     if (!__any_sync(0xffffffffu, run)) break;
-    const bool last = run && g.grad && istep == nst - 1;
     Rec cap{nullptr, 0}, xs{nullptr, 0};
     if (g.grad) {
       cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
@@ -161,10 +155,9 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
         rx[3 * N + q] = st.v[q];
       }
     }
-    team_step<N>(st, acc[tm], w, t, run && !last, hs, cap, xs);
-    // the last step also forms dq/dt: the one-lane step, on the team's first lane
-    if (last && t == 0) ahl21_step<N, true, true>(st, w, hs, 0, Rec{nullptr, 0}, cap, xs);
-    __syncwarp();
+    if (run && g.grad && istep == nst - 1)  // v at the last step's start, for its dq/dt (dq_columns)
+      for (int q = t; q < 3 * N; q += L) g.dqdt[(7 * (q / 3) + 3 + q % 3) * S + s] = st.v[q];
+    team_step<N>(st, acc[tm], t, run, hs, cap, xs);
     // occultor o on lane o % L
     if (run && !g.notransit)
       for (int o = t; o < N - 1; o += L)
@@ -178,8 +171,6 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
       g.xe[q * S + s] = st.xe[q];
       g.ve[q * S + s] = st.ve[q];
     }
-    if (g.grad && nst <= k0 + g.K)
-      for (int q = t; q < 7 * N; q += L) g.dqdt[q * S + s] = st.dqdt[q];
     for (int q = t; q < N; q += L) {
       g.gsave[q * S + s] = gsv[tm][q];
       g.count[q * S + s] = cnt[tm][q];
@@ -227,21 +218,30 @@ __device__ __forceinline__ void lanes_sync() {
   else __syncthreads();
 }
 
-// One pair of a sweep on the sixteen lanes hl = 0..15 named by `mask`.
+// One pair of a sweep on the sixteen lanes hl = 0..15 of a half warp.  Both
+// halves of a warp run the same instructions, so that its two pairs share their
+// issue slots; a half without a pair (act false) repeats pair (0, 1) and writes
+// nothing.  Only a solve that needs more than one FP64 step leaves the other
+// half.
 template <int N, bool DRIFT_FIRST>
-__device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, double h, const Rec& cap, int coff,
-                                           int hl, unsigned mask) {
+__device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, bool act, double h, const Rec& cap,
+                                           int coff, int hl) {
   const int pb = pair_bit(i, j, N);
   const double k = sh.pk[pb];
   if (k == 0.0) {
-    if (cap.p && hl == 0) cap.put(coff + PCAP_K, 0.0);
-    return;
+    if (act && cap.p && hl == 0) cap.put(coff + PCAP_RINV, 0.0);
+    act = false;
   }
+  unsigned mask = 0xffffffffu;
   auto from = [&](double v, int src) { return __shfl_sync(mask, v, src, 16); };
   double* q = sh.st.x;  // x, v, xe, ve of Sys<N> in a row, 3N each
   const int c = hl % 6, k3 = hl % 3;
   const int at = (c < 3 ? 0 : 3 * N) + k3;
-  const double d = q[at + 3 * i] - q[at + 3 * j];
+  const double qi = q[at + 3 * i], qj = q[at + 3 * j], d = qi - qj;
+  // lanes 0-5 carry body i's coordinates, 6-11 body j's
+  const int id = at + 3 * (hl < 6 ? i : j);
+  double own_q = hl < 6 ? qi : qj, own_e = q[6 * N + id];
+  const double weight = hl < 6 ? sh.pmj[pb] : -sh.pmi[pb];
   double X[3], V[3], R[3];
 #pragma unroll
   for (int w = 0; w < 3; w++) {
@@ -275,43 +275,45 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, dou
   const double kr0 = k * r0inv;
   const double beta = fma(2.0, kr0, -vv);
   const double zeta = fma(-r0, beta, k);
+  const double t = h * r0inv;
   float q2;
   const float sg = kep_start((float)r0inv, (float)h, (float)beta, (float)eta, (float)zeta, &q2);
-  const double t = h * r0inv;
-  const float tinv = __fdividef(1.0f, (float)t);
+  const double q2d = (double)q2;
+  const int w4 = hl & 3;
   const bool odd = hl & 1;
   double s = t * (double)sg, ds, y, g0, g1, g2, g3, g4 = 0.0;
-  int iter = 0;
-  bool done = false;
-  do {
+  bool done = false, far = false;
+  auto iterate = [&]() {
     const double ss = s * s, z = beta * ss;
-    const double p = stumpff_either(z, odd);
-    const double c6 = from(p, 0), c5 = from(p, 1);
-    const double c4 = fma(-z, c6, 1.0 / 24.0);
-    const double cc = fma(-z, odd ? c5 : c4, odd ? 1.0 / 6.0 : 0.5);
-    const double sss = ss * s;
-    const double g23 = (odd ? sss : ss) * cc;
-    g2 = from(g23, 0);
-    g3 = from(g23, 1);
+    const double scale = ss * (w4 == 0 ? 1.0 : w4 == 1 ? s : ss);
+    const double g = scale * stumpff234(z, w4);  // G2, G3, G4 by w4
+    g2 = from(g, 0);
+    g3 = from(g, 1);
+    if (!DRIFT_FIRST) g4 = from(g, 2);
     const double g01 = fma(-beta, odd ? g3 : g2, odd ? s : 1.0);
     g0 = from(g01, 0);
     g1 = from(g01, 1);
-    if (!DRIFT_FIRST) g4 = (ss * ss) * c4;
-    const double first = fma(r0, s, -h);
+    const double first = fma(r0, s, -h);  // in the shuffles' shadow
     const double fr = fma(zeta, odd ? g2 : g3, fma(eta, odd ? g1 : g2, odd ? r0 : first));
-    const double F = from(fr, 0), r = from(fr, 1);
+    const double r = from(fr, 1);
     y = rcp_seed(r);
-    y = fma(y, fma(-r, y, 1.0), y);
-    const double u = F * y;
-    ds = -fma(u, (double)(q2 * ((float)u * tinv)), u);
+    const double ue = fma(odd ? -r : fr, y, odd ? 1.0 : 0.0);  // F / r to the seed's digits, and what they lack
+    const double u = from(ue, 0);
+    ds = -fma(u, fma(q2d, u, from(ue, 1)), u);
     s = s + ds;
-    if (!(fabs(z) <= 4.0 * KEP_ZMAX)) break;
+    far = !(fabs(z) <= 4.0 * KEP_ZMAX);
     done = fabs(u) <= KEP_STEP * fabs(s) && fabs(z) <= KEP_ZMAX;
-  } while (!done && ++iter < 6);
+  };
+  iterate();
+  if (act && !done) {
+    mask = 0xffffu << (threadIdx.x & 16);
+    for (int iter = 1; iter < 6 && !done && !far; iter++) iterate();
+    mask = 0xffffffffu;
+  }
+  __syncwarp();
   double del, val;  // val: fm1, gmh, dfdt, dgdtm1 by hl & 3
   KepParams P;
-  const int w4 = hl & 3;
-  if (done) {
+  {
     const double hd = 0.5 * ds;
     if (!DRIFT_FIRST) g4 = fma(ds, fma(hd, g2, g3), g4);
     const double gn = fma(ds, fma(hd, odd ? g1 : g0, odd ? g2 : g1), odd ? g3 : g2);
@@ -345,7 +347,8 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, dou
     P.zeta = zeta;
     const double cx = from(val, c < 3 ? 0 : 2), cv = from(val, c < 3 ? 1 : 3);
     del = fma(cv, vk, cx * xk);
-  } else {
+  }
+  if (act && !done) {
     double delxv[6];
     kep_solve_general<DRIFT_FIRST>(X, V, k, h, delxv, P);
     val = w4 == 0 ? P.fm1 : w4 == 1 ? P.gmh : w4 == 2 ? P.dfdt : P.dgdtm1;
@@ -353,21 +356,24 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, dou
 #pragma unroll
     for (int w = 1; w < 6; w++) del = (c == w) ? delxv[w] : del;
   }
-  if (hl < 12) {
-    const int id = at + 3 * (hl < 6 ? i : j);
-    double xs = q[id], xe = q[6 * N + id];
-    kahan_fma(xs, xe, hl < 6 ? sh.pmj[pb] : -sh.pmi[pb], del);
-    q[id] = xs;
-    q[6 * N + id] = xe;
+  if (act && hl < 12) {
+    kahan_fma(own_q, own_e, weight, del);
+    q[id] = own_q;
+    q[6 * N + id] = own_e;
   }
-  if (cap.p) {  // in put_capture's order, a value or two a lane
-    if (hl < 6) cap.put(coff + hl, d);
-    if (hl < 4) cap.put(coff + (hl == 0 ? 11 : hl == 1 ? 12 : hl == 2 ? 10 : 13), val);
-    const double pv[11] = {P.s, P.g1, P.g2, P.g3, P.r0, P.r0inv, P.rinv, k, P.beta, P.eta, P.zeta};
-    double own = pv[0];
-#pragma unroll
-    for (int w = 1; w < 11; w++) own = (hl == 4 + w) ? pv[w] : own;
-    if (hl >= 4 && hl < 15) cap.put(coff + (hl < 8 ? 2 + hl : 6 + hl), own);
+  if (act && cap.p) {  // in put_capture's order: lanes 0-5 x0 and v0, 6-13 the solve, then 0-3 the coefficients
+    double own = d;
+    own = hl == 6 ? P.s : own;
+    own = hl == 7 ? P.g2 : own;
+    own = hl == 8 ? P.g3 : own;
+    own = hl == 9 ? P.r0 : own;
+    own = hl == 10 ? P.r0inv : own;
+    own = hl == 11 ? P.rinv : own;
+    own = hl == 12 ? P.beta : own;
+    own = hl == 13 ? P.eta : own;
+    double* to = cap.p + (unsigned)((coff + hl) * cap.stride);  // below 2^31: 2 P PCAP slots
+    if (hl < 14) *to = own;
+    if (hl < 4) to[(unsigned)(14 * cap.stride)] = val;
   }
 }
 
@@ -377,15 +383,15 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
   constexpr int P = N * (N - 1) / 2, T = 32 * lanes_warps(N);
   static_assert(P <= T && 3 * N <= T, "one lane per pair and per coordinate");
   const int t = threadIdx.x, half = t >> 4, hl = t & 15;
-  const unsigned mask = 0xffffu << (t & 16);
   const double h2 = 0.5 * h;
   Sys<N>& st = sh.st;
   if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
   lanes_sync<N>();
 #pragma unroll 1
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
-    int i, j;
-    if (level_pair<N>(lev, half, &i, &j)) lanes_pair<N, true>(sh, i, j, h2, cap, pair_bit(i, j, N) * PCAP, hl, mask);
+    int i = 0, j = 1;
+    const bool act = level_pair<N>(lev, half, &i, &j);
+    if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, pair_bit(i, j, N) * PCAP, hl);
     lanes_sync<N>();
   }
   // pair t's bodies
@@ -394,12 +400,14 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
     pi++;
     pj += pi + 1 - N;
   }
-  double rij[3];
+  double rij[3], r2 = 0.0, rinv = 0.0;
   if (xs.p && t < 3 * N) xs.put(t, st.x[t]);
   if (t < P) {
 #pragma unroll
     for (int w = 0; w < 3; w++) rij[w] = st.x[3 * pi + w] - st.x[3 * pj + w];
-    phis_accel(rij, sh.f[t]);
+    r2 = norm2(rij);
+    rinv = rsqrt_fast(r2);
+    phis_accel(rij, rinv, sh.f[t]);
   }
   lanes_sync<N>();
   const int b = t / 3, w = t % 3;  // coordinate lane
@@ -418,7 +426,7 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
     double aij[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) aij[q] = sh.a[3 * pi + q] - sh.a[3 * pj + q];
-    phis_corr(rij, aij, st.m[pi] + st.m[pj], phis_coeff(h), sh.f[t]);
+    phis_corr(rij, r2, rinv, aij, st.m[pi] + st.m[pj], phis_coeff(h), sh.f[t]);
   }
   lanes_sync<N>();
   if (t < 3 * N) {
@@ -431,9 +439,10 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
   lanes_sync<N>();
 #pragma unroll 1
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
-    int i, j;
-    if (level_pair<N>(lev, half, &i, &j))
-      lanes_pair<N, false>(sh, i, j, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP, hl, mask);
+    int i = 0, j = 1;
+    const bool act = level_pair<N>(lev, half, &i, &j);
+    if (__any_sync(0xffffffffu, act))
+      lanes_pair<N, false>(sh, i, j, act, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP, hl);
     lanes_sync<N>();
   }
   if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
@@ -461,7 +470,6 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
     sh.g[t] = g.gsave[t * S + s];
     sh.cnt[t] = g.count[t * S + s];
   }
-  for (int q = t; q < 7 * N; q += blockDim.x) st.dqdt[q] = g.dqdt[q * S + s];
   lanes_sync<N>();
   if (t < P) {
     int i = 0, j = t + 1;
@@ -491,15 +499,9 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
       rx[t] = st.x[t];
       rx[3 * N + t] = st.v[t];
     }
-    if (g.grad && istep == nst - 1) {  // the last step also forms dq/dt: the one-lane step, on the first lane
-      if (t == 0) {
-        Work<N> w;
-        ahl21_step<N, true, true>(st, w, hs, 0, Rec{nullptr, 0}, cap, xs);
-      }
-      lanes_sync<N>();
-    } else {
-      lanes_step<N>(sh, hs, cap, xs);
-    }
+    if (g.grad && istep == nst - 1 && t < 3 * N)  // v at the last step's start, for its dq/dt (dq_columns)
+      g.dqdt[(7 * (t / 3) + 3 + t % 3) * S + s] = st.v[t];
+    lanes_step<N>(sh, hs, cap, xs);
     if (!g.notransit && t < N - 1)
       detect_transit<N>(g, st, s, kk, t, ti, ntt, hI, t0 + (double)(istep + 1) * h, sh.g, sh.cnt);
     lanes_sync<N>();
@@ -510,8 +512,6 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
     g.xe[t * S + s] = st.xe[t];
     g.ve[t * S + s] = st.ve[t];
   }
-  if (g.grad && nst <= k0 + g.K)
-    for (int q = t; q < 7 * N; q += blockDim.x) g.dqdt[q * S + s] = st.dqdt[q];
   if (t < N) {
     g.gsave[t * S + s] = sh.g[t];
     g.count[t * S + s] = sh.cnt[t];

@@ -344,7 +344,7 @@ int create_group(nbg_server* srv, int N, int grad, unsigned long long kick, Grou
     want(&g.steprec, 2 * nrec); want(&g.trec, 2 * ntrec);
     want(&g.tflag, 2 * nflag); want(&g.tscratch, (size_t)g.R * g.tgrid);
     want(&g.pcap, 2 * ncap);
-    want(&g.xsnap, 2 * nsnap);
+    want(&g.xsnap, 2 * nsnap); want(&g.dh, 12 * (size_t)npk * S);
     want(&g.Jint, S * 6 * N * 7 * N); want(&g.Eint, S * 6 * N * 7 * N);
   }
   want(&G->stage, S * G->lay.stride);
