@@ -277,11 +277,11 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
   const double zeta = fma(-r0, beta, k);
   const double t = h * r0inv;
   float q2;
-  const float sg = kep_start((float)r0inv, (float)h, (float)beta, (float)eta, (float)zeta, &q2);
-  const double q2d = (double)q2;
+  const float sg = kep_start(to_float(r0inv), to_float(h), to_float(beta), to_float(eta), to_float(zeta), &q2);
+  const double q2d = to_double(q2);
   const int w4 = hl & 3;
   const bool odd = hl & 1;
-  double s = t * (double)sg, ds, y, g0, g1, g2, g3, g4 = 0.0;
+  double s = t * to_double(sg), ds, y, g0, g1, g2, g3, g4 = 0.0;
   bool done = false, far = false;
   auto iterate = [&]() {
     const double ss = s * s, z = beta * ss;
