@@ -432,8 +432,7 @@ int nbg_last_timing(nbg_context* ctx, double* total_ms, double* orbit_ms, double
  * for T = trial_steps and 2 trial_steps, on device copies (the caller's
  * arrays are not modified) -- for each candidate mapping: steps per chunk
  * {64, 128} x orbit producer form {one lane per system, team of lanes} x
- * producer block layout {one warp; four warps holding 200 KB of shared
- * memory, operator and search blocks 32 KB} (nbg_set_producer_layout).  The
+ * producer block layout {one warp; four warps} (nbg_set_producer_layout).  The
  * two trial times give the loop's fill and drain and its time per step with
  * the whole batch active.  For a batch of uneven length (its shortest system
  * under half its longest) two more trials run only the systems with its
@@ -470,17 +469,16 @@ int nbg_set_orbit_lanes(nbg_context* ctx, int systems_per_warp);
 
 /* Form of the orbit producer for groups without kick pairs: -1 automatic
  * (default: one lane per system up to four bodies and a team of N/2 lanes
- * per system from N = 5 on, each in its wide form in latency-bound chunks),
- * 0 one lane per system, 1 a team for every N, 2 the wide team form for
+ * per system from N = 5 on, each with the wide forms in latency-bound chunks),
+ * 0 one lane per system, 1 a team for every N, 2 the wide forms for
  * every N, 3 a team for every N, wide in latency-bound chunks.  A team runs
  * the Kepler sweeps and phisalpha!'s pair loops level by level (pairs with
  * equal i + j share no body and run in parallel), which keeps every body's
- * sequence of updates and so gives bitwise the same results.  The wide form
- * runs each pair solve on two lanes, each evaluating one of its independent
- * parts (the sine and cosine series, the Newton update's numerator and
- * denominator, G3 and H1): bitwise the same results with fewer FP64
- * instructions on the system's warp.  A chunk is latency-bound when at most
- * max(32, SMs / 2) of its group's systems still run.  A tuning knob; no
+ * sequence of updates and so gives bitwise the same results.  The wide forms
+ * run each pair solve on sixteen lanes and each column of jac_step on six:
+ * bitwise the same results with fewer FP64 instructions one after the other.
+ * A chunk is latency-bound while so few of its group's systems still run that
+ * this is the faster way (some hundreds, by N and gradient).  A tuning knob; no
  * counterpart in the reference. */
 int nbg_set_orbit_team(nbg_context* ctx, int mode);
 
@@ -491,7 +489,8 @@ int nbg_set_orbit_team(nbg_context* ctx, int mode);
  * operator-record and transit-search block.  Blocks cannot share an SM when
  * their shared memory exceeds the SM's 227 KB, so smem_kb = 200 with
  * guard_kb = 32 keeps the throughput kernels off the SMs that run the
- * latency-bound producer.  Default 1, 0, 0. */
+ * latency-bound producer.  Default: no shared memory held, one warp a block,
+ * two in a one-lane group of 2048 systems or more. */
 int nbg_set_producer_layout(nbg_context* ctx, int warps_per_block, int smem_kb, int guard_kb);
 
 /* Profiling (no reference counterpart).

@@ -266,7 +266,7 @@ struct nbg_context {
   int overlap = 1;  // orbit producer on its own stream, one chunk ahead of the rest
   int orbit_spw = 0;  // 0: automatic
   int orbit_team = -1;  // -1: automatic (teams for N >= 5), 0: one lane per system, 1: teams for every N
-  int prod_warps = 1, prod_smem_kb = 0, guard_smem_kb = 0;  // orbit producer block layout
+  int prod_warps = 0, prod_smem_kb = 0, guard_smem_kb = 0;  // orbit producer block layout
   int sm_count = 0;
   double last_total_ms = 0, last_orbit_ms = 0, last_jac_ms = 0, last_transit_ms = 0, last_ops_ms = 0;
   double last_host_ms = 0;  // host time spent enqueueing the chunk loop
@@ -728,12 +728,12 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     GroupArgs gx = g;
     const bool tail = active_at(q, c) <= tail_max;
     if (tail) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
-    gx.wide = use_wide(ctx->orbit_team, tail, g.kick) ? 1 : 0;
+    gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= lanes_limit(g.N, g.grad, ctx->sm_count), g.kick) ? 1 : 0;
     return gx;
   };
   auto jac_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max, g.kick) ? 1 : 0;
+    gx.rows = use_wide(ctx->orbit_team, active_at(q, c) <= rows_limit(g.N, ctx->sm_count), g.kick) ? 1 : 0;
     return gx;
   };
   auto ops_args = [&](const GroupArgs& g) {
@@ -2022,11 +2022,11 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   for (int chunk : {64, 128})
     for (int team : {0, 1}) {
       if (team && !any_team) continue;
-      // producer blocks of one warp anywhere, or of four warps holding their
-      // SM's shared memory so that consumer, operator and search blocks run
-      // on the other SMs
+      // producer blocks of one warp or of four (4096 three-body systems over
+      // 2000 steps: 366 and 307 ms; with 200 KB of shared memory held beside
+      // the four, 317)
       cands.push_back({chunk, team, 0, 1, 0, 0});
-      cands.push_back({chunk, team, 0, 4, 200, 32});
+      cands.push_back({chunk, team, 0, 4, 0, 0});
     }
   const int save_chunk = ctx->chunk_steps, save_team = ctx->orbit_team, save_spw = ctx->orbit_spw;
   const int save_pw = ctx->prod_warps, save_sm = ctx->prod_smem_kb, save_gd = ctx->guard_smem_kb;
@@ -2046,10 +2046,13 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   // difference of two trial lengths would understate a step's time.
   int wchunk = 0;
   for (const Cand& cd : cands) wchunk = std::max(wchunk, cd.chunk);
+  // a team or one lane; the forms for latency-bound chunks beside the team and,
+  // in a batch of up to four bodies, where the choice is not between the two
+  auto mode_of = [&](bool team) { return team ? 3 : any_team ? 0 : -1; };
   for (int wteam : {0, 3}) {
     if (wteam && !any_team) continue;
     ctx->chunk_steps = wchunk;
-    ctx->orbit_team = wteam;
+    ctx->orbit_team = mode_of(wteam != 0);
     ctx->orbit_spw = cands[0].spw;
     ctx->prod_warps = cands[0].pw;
     ctx->prod_smem_kb = cands[0].smem;
@@ -2063,7 +2066,7 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   for (size_t q = 1; q <= cands.size() && !rc; q++) {
     const Cand& cd = cands[q - 1];
     ctx->chunk_steps = cd.chunk;
-    ctx->orbit_team = cd.team ? 3 : 0;  // a team, wide in latency-bound chunks
+    ctx->orbit_team = mode_of(cd.team);
     ctx->orbit_spw = cd.spw;
     ctx->prod_warps = cd.pw;
     ctx->prod_smem_kb = cd.smem;
@@ -2131,7 +2134,7 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
     return rc ? rc : set_error(NBG_EINVAL, "autotune: no candidate ran");
   }
   ctx->chunk_steps = cands[best].chunk;
-  ctx->orbit_team = cands[best].team ? 3 : 0;
+  ctx->orbit_team = mode_of(cands[best].team);
   ctx->orbit_spw = cands[best].spw;
   ctx->prod_warps = cands[best].pw;
   ctx->prod_smem_kb = cands[best].smem;

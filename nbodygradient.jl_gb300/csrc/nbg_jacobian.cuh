@@ -270,7 +270,7 @@ __device__ __forceinline__ void corrector_update(const double* S, double* E, int
 template <int N, int BS, bool MASS>
 __device__ __forceinline__ void column_step(double* S, double* E, int c, double h, const Rec& rec) {
   const double h2 = 0.5 * h;
-#pragma unroll
+#pragma unroll 2
   for (int b = 0; b < N; b++)
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -289,7 +289,7 @@ __device__ __forceinline__ void column_step(double* S, double* E, int c, double 
       roff += PREC;
     }
     if (N > 2 && i == 0) {
-#pragma unroll
+#pragma unroll 3
       for (int q = 0; q < 3 * N; q++) {
         const int r = (6 * (q / 3) + 3 + q % 3) * BS;
         double s = S[r], e = E[r];
@@ -308,7 +308,7 @@ __device__ __forceinline__ void column_step(double* S, double* E, int c, double 
       pair_update<N, BS, MASS>(S, E, c, i, j, rec, roff);
       roff += PREC;
     }
-#pragma unroll
+#pragma unroll 2
   for (int b = 0; b < N; b++)
 #pragma unroll
     for (int k = 0; k < 3; k++) {

@@ -27,7 +27,7 @@ template <int N, bool KICK>
 __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(GroupArgs g, int chunk) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane >= g.spw) return;
-  const int s = (blockIdx.x * (g.pwarps > 0 ? g.pwarps : 1) + warp) * g.spw + lane;
+  const int s = (blockIdx.x * (blockDim.x / PROD_BS) + warp) * g.spw + lane;
   if (s >= g.S || g.sysidx[s] < 0) return;
   const int S = g.S;
   const long long nst = g.nsteps[s];
@@ -642,8 +642,10 @@ __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int
   if (!finite) atomicOr(g.status + s, NBG_STATUS_NONFINITE);
 }
 
+// 168 registers a thread at most: three blocks of four warps fit an SM and leave
+// room for a producer or search warp beside them.
 template <int N>
-__global__ void __launch_bounds__(cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain, int all) {
+__global__ void __launch_bounds__(cons_bs(N), 3 * 128 / cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain, int all) {
   extern __shared__ double smem[];
   constexpr int BS = cons_bs(N);
   if ((int)blockIdx.x < plain) {
@@ -919,11 +921,16 @@ inline void allow_smem(K kernel, int bytes) {
 
 template <int N>
 int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
-  const int W = g.pwarps > 0 ? g.pwarps : 1;
+  // Without a layout of the caller's (nbg_set_producer_layout) a full group's
+  // one-lane warps go two to a block: one warp alone needs registers that three
+  // consumer blocks leave on no SM, and its block waits for one of theirs to end
+  // (4096 three-body systems over 512 steps: 94.5 -> 87.7 ms; two and four
+  // bodies within 1 %).
+  const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.S >= 2048) ? 2 : 1;
   if (g.wide && !g.kick) {
-    const int smem = std::max((int)sizeof(LanesShared<N>), g.prod_smem);
+    const int smem = std::max(lanes_systems(N) * (int)sizeof(LanesShared<N>), g.prod_smem);
     allow_smem(orbit_lanes_kernel<N>, smem);
-    orbit_lanes_kernel<N><<<g.S, 32 * lanes_warps(N), smem, st>>>(g, chunk);
+    orbit_lanes_kernel<N><<<(g.S + lanes_systems(N) - 1) / lanes_systems(N), 32 * lanes_warps(N), smem, st>>>(g, chunk);
     return 0;
   }
   if (g.team && !g.kick) {
@@ -954,7 +961,7 @@ int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
     jacobian_kick_kernel<N><<<blocks((long long)g.S * 7 * N), BS, smem, st>>>(g, chunk);
     return 0;
   }
-  if (g.wide) {
+  if (g.rows) {
     const int bytes = std::max((int)sizeof(RowsShared<N>), 24 * 1024);  // as every consumer block: none fits beside a tail producer's
     allow_smem(jacobian_rows_kernel<N>, bytes);
     static_assert(sizeof(double) * DQ_DOUBLES<N> * ROWS_WARPS <= sizeof(RowsShared<N>) || N <= 2, "dq_columns fits");

@@ -50,6 +50,26 @@ constexpr int PCAP_RINV = 11;
 __host__ __device__ inline int snap_count(bool kick) { return kick ? 3 : 2; }
 
 
+// Up to how many running systems of a kick-free group the latency-bound forms
+// are taken.  A lanes-form level costs its warp one system's pairs where the
+// one-lane and team forms carry 32 or 32 / (N/2) systems, so the line is where
+// the pairs' levels, (2N - 3) per system, fill the SMs' FP64 pipes.  Measured,
+// us a step, (one lane or team) -> lanes, rows consumer with up to four bodies:
+// N = 3 512 systems 71 -> 60, 1024 84 -> 87; N = 4 512 134 -> 107, 1024 162 -> 173;
+// N = 6 768 440 -> 380; N = 8 384 674 -> 606, 768 935 -> 933; N = 10 384 948 -> 867,
+// 768 1427 -> 1487.  Without derivatives nothing else wants the pipes: N = 3 1024
+// 57 -> 33, 2048 62 -> 58; N = 4 1024 138 -> 80, 2048 112 -> 141; N = 8 768 511 -> 296.
+__host__ inline int rows_limit(int N, int sms) {
+  // six lanes a column: level with one lane a column at 64 columns an SM (96 up
+  // to four bodies, whose lanes form it keeps company); N = 8 96 systems
+  // 417 -> 387, 192 484 -> 510; N = 10 96 627 -> 549, 192 747 -> 792
+  return (N <= 4 ? 96 : 64) * sms / (7 * N);
+}
+__host__ inline int lanes_limit(int N, bool grad, int sms) {
+  if (!grad) return N <= 4 ? (48 * sms / (2 * N - 3) < 2048 ? 48 * sms / (2 * N - 3) : 2048) : 96 * sms / (2 * N - 3);
+  return N <= 4 ? rows_limit(N, sms) : 64 * sms / (2 * N - 3);
+}
+
 struct GroupArgs {
   int N, S, nsys, grad, K, R, npk;
   int spw;   // orbit producer: systems per warp (lanes >= spw idle)
@@ -59,13 +79,13 @@ struct GroupArgs {
   // that the searches are latency-bound; a full group keeps one lane per
   // search, which uses every lane of every warp
   int search_team;
-  // latency-bound chunk (few systems running) of a group without kick pairs,
-  // set by the host per chunk: the orbit producer takes its lanes form
-  // (orbit_lanes_kernel), the Jacobian consumer its rows form
+  // forms for latency-bound chunks (few systems running) of a group without
+  // kick pairs, set by the host per chunk: the orbit producer's lanes form
+  // (orbit_lanes_kernel) and the Jacobian consumer's rows form
   // (jacobian_rows_kernel)
-  int wide;
+  int wide, rows;
   // Block layout of the orbit producer: pwarps independent warps per block
-  // (0 or 1: one) and prod_smem bytes of dynamic shared memory per block (at
+  // (0: by the group's size, launch_orbit) and prod_smem bytes of dynamic shared memory per block (at
   // least what the team form needs).  A large allocation keeps the
   // shared-memory-hungry consumer blocks, and the operator / search blocks
   // that ask for guard_smem bytes, off the SMs that run producer blocks.

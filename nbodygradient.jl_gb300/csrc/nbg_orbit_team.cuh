@@ -105,7 +105,7 @@ template <int N>
 __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(GroupArgs g, int chunk) {
   constexpr int L = team_lanes(N);
   constexpr int T = PROD_BS / L;
-  const int W = g.pwarps > 0 ? g.pwarps : 1;
+  const int W = blockDim.x / PROD_BS;
   extern __shared__ double team_smem[];
   Sys<N>* sys = reinterpret_cast<Sys<N>*>(team_smem);
   double(*acc)[3 * N] = reinterpret_cast<double(*)[3 * N]>(sys + W * T);
@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
 // ------------------------------------------------------------ pairs on lanes
 //
 // Orbit producer for latency-bound chunks (at most max(32, SMs / 2) systems of
-// the group still running): one block per system, sixteen lanes per pair solve.
+// the group still running): one block per system (two systems of two or three
+// bodies), sixteen lanes per pair solve.
 // A warp issues one FP64 instruction per 64 cycles however independent its
 // instructions are, and with few systems nothing else fills the SM, so a step
 // takes as long as its longest warp's FP64 instructions; spreading a solve's
@@ -202,6 +203,9 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
 // of five bodies without derivatives 30.2 -> 15.4 ms, 2000 steps of three bodies
 // with transits 97 -> 67 ms (then bound by the consumer, jacobian_rows_kernel).
 __host__ __device__ constexpr int lanes_warps(int N) { return (N / 2 + 1) / 2 > 0 ? (N / 2 + 1) / 2 : 1; }
+// A level of two or three bodies has one pair: a system then takes a half warp.
+__host__ __device__ constexpr int lanes_systems(int N) { return N <= 3 ? 2 : 1; }
+__host__ __device__ constexpr int lanes_each(int N) { return 32 * lanes_warps(N) / lanes_systems(N); }
 
 template <int N>
 struct LanesShared {
@@ -377,20 +381,24 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
   }
 }
 
-// One AHL21 step of a kick-free group on the block's lanes (team_step's order).
+// One AHL21 step of a kick-free group on a system's lanes t (team_step's order);
+// run is false for the lanes of a system that does not step: they keep step
+// with their warp and write nothing.
 template <int N>
-__device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const Rec& cap, const Rec& xs) {
-  constexpr int P = N * (N - 1) / 2, T = 32 * lanes_warps(N);
+__device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, double h, const Rec& cap,
+                                           const Rec& xs) {
+  constexpr int P = N * (N - 1) / 2, T = lanes_each(N);
   static_assert(P <= T && 3 * N <= T, "one lane per pair and per coordinate");
-  const int t = threadIdx.x, half = t >> 4, hl = t & 15;
+  const int half = t >> 4, hl = t & 15;
   const double h2 = 0.5 * h;
+  const bool coord = run && t < 3 * N, pair = run && t < P;
   Sys<N>& st = sh.st;
-  if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  if (coord) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
   lanes_sync<N>();
 #pragma unroll 1
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i = 0, j = 1;
-    const bool act = level_pair<N>(lev, half, &i, &j);
+    const bool act = level_pair<N>(lev, half, &i, &j) && run;
     if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, pair_bit(i, j, N) * PCAP, hl);
     lanes_sync<N>();
   }
@@ -401,8 +409,8 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
     pj += pi + 1 - N;
   }
   double rij[3], r2 = 0.0, rinv = 0.0;
-  if (xs.p && t < 3 * N) xs.put(t, st.x[t]);
-  if (t < P) {
+  if (xs.p && coord) xs.put(t, st.x[t]);
+  if (pair) {
 #pragma unroll
     for (int w = 0; w < 3; w++) rij[w] = st.x[3 * pi + w] - st.x[3 * pj + w];
     r2 = norm2(rij);
@@ -411,7 +419,7 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
   }
   lanes_sync<N>();
   const int b = t / 3, w = t % 3;  // coordinate lane
-  if (t < 3 * N) {
+  if (coord) {
     double a = 0.0;
     for (int o = 0; o < N; o++)
       if (o != b) {
@@ -422,14 +430,14 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
     if (xs.p) xs.put(3 * N + t, a);
   }
   lanes_sync<N>();
-  if (t < P) {
+  if (pair) {
     double aij[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) aij[q] = sh.a[3 * pi + q] - sh.a[3 * pj + q];
     phis_corr(rij, r2, rinv, aij, st.m[pi] + st.m[pj], phis_coeff(h), sh.f[t]);
   }
   lanes_sync<N>();
-  if (t < 3 * N) {
+  if (coord) {
     double v = st.v[t], ve = st.ve[t];
     for (int o = 0; o < N; o++)
       if (o != b) kahan_fma(v, ve, o < b ? -st.m[o] : st.m[o], sh.f[o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)][w]);
@@ -440,35 +448,39 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, double h, const R
 #pragma unroll 1
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
     int i = 0, j = 1;
-    const bool act = level_pair<N>(lev, half, &i, &j);
+    const bool act = level_pair<N>(lev, half, &i, &j) && run;
     if (__any_sync(0xffffffffu, act))
       lanes_pair<N, false>(sh, i, j, act, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP, hl);
     lanes_sync<N>();
   }
-  if (t < 3 * N) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  if (coord) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
   lanes_sync<N>();
 }
 
 template <int N>
 __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupArgs g, int chunk) {
   extern __shared__ double lanes_smem[];
-  LanesShared<N>& sh = *reinterpret_cast<LanesShared<N>*>(lanes_smem);
-  constexpr int P = N * (N - 1) / 2;
-  const int s = blockIdx.x, t = threadIdx.x, S = g.S;
-  if (s >= S || g.sysidx[s] < 0) return;
-  const long long nst = g.nsteps[s], k0 = chunk_first_step(g, chunk, s);
-  if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
+  constexpr int P = N * (N - 1) / 2, T = lanes_each(N);
+  const int t = threadIdx.x % T, S = g.S, s = blockIdx.x * lanes_systems(N) + threadIdx.x / T;
+  LanesShared<N>& sh = reinterpret_cast<LanesShared<N>*>(lanes_smem)[threadIdx.x / T];
+  bool valid = s < S && g.sysidx[s] >= 0;
+  const long long nst = valid ? g.nsteps[s] : 0, k0 = valid ? chunk_first_step(g, chunk, s) : 0;
+  valid = valid && k0 < nst && k0 >= 0;  // neither done nor admitted for a later chunk
+  // the block's systems step together until the last of them has done
+  const int nk = valid ? (int)(nst - k0 < g.K ? nst - k0 : g.K) : 0;
+  const int most = lanes_systems(N) > 1 ? max(nk, __shfl_xor_sync(0xffffffffu, nk, 16)) : nk;
+  if (most == 0) return;
   Sys<N>& st = sh.st;
   if (t < 3 * N) {
-    st.x[t] = g.x[t * S + s];
-    st.v[t] = g.v[t * S + s];
-    st.xe[t] = g.xe[t * S + s];
-    st.ve[t] = g.ve[t * S + s];
+    st.x[t] = valid ? g.x[t * S + s] : 0.0;
+    st.v[t] = valid ? g.v[t * S + s] : 0.0;
+    st.xe[t] = valid ? g.xe[t * S + s] : 0.0;
+    st.ve[t] = valid ? g.ve[t * S + s] : 0.0;
   }
   if (t < N) {
-    st.m[t] = g.m[t * S + s];
-    sh.g[t] = g.gsave[t * S + s];
-    sh.cnt[t] = g.count[t * S + s];
+    st.m[t] = valid ? g.m[t * S + s] : 0.0;
+    sh.g[t] = valid ? g.gsave[t * S + s] : 0.0;
+    sh.cnt[t] = valid ? g.count[t * S + s] : 0;
   }
   lanes_sync<N>();
   if (t < P) {
@@ -483,29 +495,30 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
     sh.pmj[t] = st.m[j] * inv;
   }
   lanes_sync<N>();
-  const double t0 = g.t0[s], h = g.h[s], hI = g.hI[s];
-  const int ntt = g.ntt[s], ti = g.ti[s];
-  for (int kk = 0; kk < g.K; kk++) {
+  const double t0 = valid ? g.t0[s] : 0.0, h = valid ? g.h[s] : 0.0, hI = valid ? g.hI[s] : 0.0;
+  const int ntt = valid ? g.ntt[s] : 0, ti = valid ? g.ti[s] : 0;
+  for (int kk = 0; kk < most; kk++) {
     const long long istep = k0 + kk;
-    if (istep >= nst) break;
+    const bool run = kk < nk;
     Rec cap{nullptr, 0}, xs{nullptr, 0};
-    if (g.grad) {
+    if (g.grad && run) {
       cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
       xs = Rec{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + s, S};
     }
-    const double hs = step_length(g, s, istep, nst, h);
-    if (g.trajxv && t < 3 * N) {
+    const double hs = run ? step_length(g, s, istep, nst, h) : h;
+    if (g.trajxv && run && t < 3 * N) {
       double* rx = g.trajxv + ((size_t)s * g.K + kk) * 6 * N;
       rx[t] = st.x[t];
       rx[3 * N + t] = st.v[t];
     }
-    if (g.grad && istep == nst - 1 && t < 3 * N)  // v at the last step's start, for its dq/dt (dq_columns)
+    if (g.grad && run && istep == nst - 1 && t < 3 * N)  // v at the last step's start, for its dq/dt (dq_columns)
       g.dqdt[(7 * (t / 3) + 3 + t % 3) * S + s] = st.v[t];
-    lanes_step<N>(sh, hs, cap, xs);
-    if (!g.notransit && t < N - 1)
+    lanes_step<N>(sh, t, run, hs, cap, xs);
+    if (!g.notransit && run && t < N - 1)
       detect_transit<N>(g, st, s, kk, t, ti, ntt, hI, t0 + (double)(istep + 1) * h, sh.g, sh.cnt);
     lanes_sync<N>();
   }
+  if (!valid) return;
   if (t < 3 * N) {
     g.x[t * S + s] = st.x[t];
     g.v[t * S + s] = st.v[t];

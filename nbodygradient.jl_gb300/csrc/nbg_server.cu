@@ -617,7 +617,8 @@ int service_group(nbg_server* srv, int gi) {
   int rc;
   // the producer's and the consumer's forms for latency-bound chunks while few slots are running
   GroupArgs gw = gc;
-  gw.wide = use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2), G->kick) ? 1 : 0;
+  gw.wide = use_wide(srv->cfg.orbit_team, G->active <= lanes_limit(N, G->grad, srv->sm_count), G->kick) ? 1 : 0;
+  gw.rows = use_wide(srv->cfg.orbit_team, G->active <= rows_limit(N, srv->sm_count), G->kick) ? 1 : 0;
   if ((rc = launch_group_orbit(N, gw, (int)c, st))) return rc;
   NBG_CUDA(cudaEventRecord(G->ev_orb[par], st));
   NBG_CUDA(cudaStreamWaitEvent(stt, G->ev_orb[par], 0));
