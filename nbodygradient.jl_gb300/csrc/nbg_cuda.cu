@@ -561,7 +561,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     }
     g.tgrid = std::min(((g.task_cap + 31) / 32) * 32, std::max(1, ctx->sm_count) * 4 * 32);
     if (gp.grad) {
-      GET(steprec, nb * nrec); GET(trec, nb * ntrec); GET(tflag, nb * nflag); GET(tscratch, (size_t)g.R * g.tgrid);
+      GET(steprec, nb * nrec); GET(trec, nb * ntrec); GET(tflag, nb * nflag); GET(tscratch, (size_t)search_scratch(N, npk, gp.kick != 0) * g.tgrid);
       GET(pcap, nb * ncap); GET(xsnap, nb * nsnap); GET(dh, 12 * (size_t)npk * S);
       GET(Jint, (size_t)S * 6 * N * 7 * N); GET(Eint, (size_t)S * 6 * N * 7 * N);
     }
@@ -720,7 +720,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   };
   auto search_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    gx.search_team = (active_at(q, c) <= tail_max) ? 1 : 0;
+    gx.search_lanes = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max, g.kick) ? 1 : 0;
     if (tail_any) gx.guard_smem = std::max(gx.guard_smem, 18 * 1024);
     return gx;
   };
@@ -994,7 +994,7 @@ void noalloc_layout(NoallocPlan& P, ScratchArena& a, int nsys, int K, int tcap, 
     a.take(&g.task_count, 1);
     if (g.grad) {
       a.take(&g.steprec, (size_t)K * g.R * S); a.take(&g.trec, (size_t)K * (N - 1) * trec_size(N, 0) * S);
-      a.take(&g.tflag, (size_t)K * (N - 1) * S); a.take(&g.tscratch, (size_t)g.R * g.tgrid);
+      a.take(&g.tflag, (size_t)K * (N - 1) * S); a.take(&g.tscratch, (size_t)search_scratch(N, g.npk, g.kick != 0) * g.tgrid);
       a.take(&g.pcap, (size_t)K * 2 * g.npk * PCAP * S + 1);
       a.take(&g.xsnap, (size_t)K * snap_count(g.kick != 0) * 3 * N * S);
       a.take(&g.dh, 12 * (size_t)g.npk * S);
@@ -2041,7 +2041,7 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   // lazy module loading (the CUDA default) the first launch of each kernel
   // loads it.  Every kernel a candidate can launch runs once here: the
   // one-lane producer, the team producer and, for an uneven batch, the chain
-  // set, whose groups take the wide form and the team searches.  Otherwise the
+  // set, whose groups take the forms for latency-bound chunks.  Otherwise the
   // first trial to allocate or to use a kernel would carry that cost, and the
   // difference of two trial lengths would understate a step's time.
   int wchunk = 0;

@@ -18,7 +18,7 @@
 
 #include "../../include/nbg.h"
 #include "nbg_jacobian.cuh"
-#include "nbg_orbit_team.cuh"
+#include "nbg_search.cuh"
 
 namespace nbg {
 
@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
 }
 
 
-// findtransit! (src/transits/timing.jl:31-109) for the searches the orbit
-// producer queued in this chunk: Newton iterations on partial AHL21 steps
+// findtransit! (src/transits/timing.jl:31-109) in groups with kick pairs (the
+// others: nbg_search.cuh), one lane per search: Newton iterations on partial AHL21 steps
 // from the end-of-step state, then (grad) the partial step at the converged
 // dt0 with its operator records and the adjoint row u^T = w^T S(dt0) that the
 // Jacobian consumer turns into dtdq0 (dtbvdq! row 1, timing.jl:155-171).
@@ -193,9 +193,8 @@ __device__ void search_finish(const GroupArgs& g, int s, int slot, int c, int ib
   ttout[0] = t + dt0;
 }
 
-// One lane per search, grid-stride over the queue.
 template <int N>
-__global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int chunk) {
+__global__ void __launch_bounds__(TRANSIT_BS) transit_kick_kernel(GroupArgs g, int chunk) {
   const int ntask = min(*g.task_count, g.task_cap);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int G = gridDim.x * blockDim.x;
@@ -227,8 +226,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       tt2 = tt1;
       tt1 = dt0;
       wk = st;
-      if (kick) ahl21_step<N, false, false>(wk, w, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
-      else plain_step<N>(wk, w.a, dt0, Rec{nullptr, 0}, Rec{nullptr, 0});
+      ahl21_step<N, false, false>(wk, w, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
       const double gs = gsky(wk, ti, ib);
       const double gd = gdot_physical(wk, ti, ib);
       const double dt = -gs / gd;
@@ -237,104 +235,6 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       if (iter >= 20 || dt0 == tt1 || dt0 == tt2) break;
     }
     search_finish<N>(g, s, slot, c, ib, ti, st, wk, dt0, t, iter, w, tid, G);
-  }
-}
-
-// Shared memory of the team search per warp: per team the search's start
-// state, the Newton iterate and the accelerations of phisalpha!.
-template <int N>
-__host__ __device__ constexpr int search_team_smem_bytes() {
-  return (PROD_BS / team_lanes(N)) * (int)(2 * sizeof(Sys<N>) + 3 * N * sizeof(double));
-}
-
-// Team form of the searches (groups without kick pairs): a team of
-// L = team_lanes(N) lanes per search, T = 32 / L searches per warp, one warp
-// per block.  The Newton iterations run the level-parallel step of the team
-// producer (team_step, bitwise the one-lane no-gradient step) on the
-// team's shared-memory copy of the state, so their critical path is
-// 2(2N - 3) pair solves per iteration instead of N(N - 1); every lane of a
-// team computes g, its derivative and the update of dt0 from the same
-// shared values, so a team stops together.  The final partial step with its
-// records and the adjoint rows run on the team's first lane
-// (search_finish), as in the one-lane kernel.  Results are bitwise those of
-// transit_kernel.
-template <int N>
-__global__ void __launch_bounds__(TRANSIT_BS) transit_team_kernel(GroupArgs g, int chunk) {
-  constexpr int L = team_lanes(N);
-  constexpr int T = PROD_BS / L;
-  extern __shared__ double search_smem[];
-  Sys<N>* st0 = reinterpret_cast<Sys<N>*>(search_smem);
-  Sys<N>* wks = st0 + T;
-  double(*acc)[3 * N] = reinterpret_cast<double(*)[3 * N]>(wks + T);
-  const int ntask = min(*g.task_count, g.task_cap);
-  const int lane = threadIdx.x & 31;
-  const int team = lane / L, t = lane % L;
-  const bool in_team = team < T;
-  const int tm = in_team ? team : 0;  // idle lanes alias team 0 but never write
-  const int S = g.S;
-  const int teams = gridDim.x * T;
-  Work<N> w;
-  for (int base = blockIdx.x * T; base < ntask; base += teams) {
-    const int idx = base + tm;
-    const bool has = in_team && idx < ntask;
-    int s = 0, slot = 0, c = 0, ti = 0, ib = 0;
-    double dt0 = 0.0, t_end = 0.0;
-    if (has) {
-      const int* tk = g.task_i + 3 * idx;
-      s = tk[0];
-      slot = tk[1];
-      c = tk[2];
-      const int o = slot % (N - 1);
-      ti = g.ti[s];
-      ib = (o < ti) ? o : o + 1;
-      const double* tf = g.task_f + (size_t)idx * (12 * N + 2);
-      for (int q = t; q < 3 * N; q += L) {
-        st0[tm].x[q] = tf[q];
-        st0[tm].v[q] = tf[3 * N + q];
-        st0[tm].xe[q] = tf[6 * N + q];
-        st0[tm].ve[q] = tf[9 * N + q];
-      }
-      for (int q = t; q < N; q += L) st0[tm].m[q] = g.m[q * S + s];
-      for (int q = t; q < 7 * N; q += L) st0[tm].dqdt[q] = 0.0;
-      dt0 = tf[12 * N];
-      t_end = tf[12 * N + 1];
-    }
-    __syncwarp();
-    double stmp = 0.0, tt1 = dt0 + 1.0, tt2 = dt0 + 2.0;
-    int iter = 0;
-    bool active = has;
-    while (__any_sync(0xffffffffu, active)) {
-      if (active) {
-        tt2 = tt1;
-        tt1 = dt0;
-        for (int q = t; q < 3 * N; q += L) {
-          wks[tm].x[q] = st0[tm].x[q];
-          wks[tm].v[q] = st0[tm].v[q];
-          wks[tm].xe[q] = st0[tm].xe[q];
-          wks[tm].ve[q] = st0[tm].ve[q];
-        }
-        for (int q = t; q < N; q += L) wks[tm].m[q] = st0[tm].m[q];
-      }
-      __syncwarp();
-      team_step<N>(wks[tm], acc[tm], t, active, dt0, Rec{nullptr, 0}, Rec{nullptr, 0});
-      __syncwarp();
-      if (active) {
-        const double gs = gsky(wks[tm], ti, ib);
-        const double gd = gdot_physical(wks[tm], ti, ib);
-        const double dt = -gs / gd;
-        kahan(dt0, stmp, dt);
-        iter += 1;
-        if (iter >= 20 || dt0 == tt1 || dt0 == tt2) active = false;
-      }
-      __syncwarp();
-    }
-    if (has && t == 0) {
-      Sys<N> st = st0[tm];
-      Sys<N> wk = wks[tm];
-      search_finish<N>(g, s, slot, c, ib, ti, st, wk, dt0, t_end, iter, w,
-                       blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-    }
-    __syncwarp();
   }
 }
 
@@ -978,14 +878,17 @@ int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
 
 template <int N>
 int launch_transit(const GroupArgs& g, int chunk, cudaStream_t st) {
-  if (team_lanes(N) > 1 && g.team && g.search_team && !g.kick) {
-    const int smem = std::max(search_team_smem_bytes<N>(), g.guard_smem);
-    allow_smem(transit_team_kernel<N>, smem);
-    transit_team_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, smem, st>>>(g, chunk);
-    return 0;
+  if (g.kick) {
+    allow_smem(transit_kick_kernel<N>, g.guard_smem);
+    transit_kick_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, g.guard_smem, st>>>(g, chunk);
+  } else if (g.search_lanes) {
+    const int smem = std::max(lanes_systems(N) * (int)sizeof(SearchShared<N>), g.guard_smem);
+    allow_smem(transit_lanes_kernel<N>, smem);
+    transit_lanes_kernel<N><<<g.tgrid / TRANSIT_BS, 32 * lanes_warps(N), smem, st>>>(g, chunk);
+  } else {
+    allow_smem(transit_kernel<N>, g.guard_smem);
+    transit_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, g.guard_smem, st>>>(g, chunk);
   }
-  allow_smem(transit_kernel<N>, g.guard_smem);
-  transit_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, g.guard_smem, st>>>(g, chunk);
   return 0;
 }
 

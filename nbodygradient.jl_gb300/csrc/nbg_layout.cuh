@@ -25,6 +25,17 @@ __host__ __device__ inline int step_record_size(int N, int npk, bool kick) {
   return (kick ? 2 * op_size(N) : 0) + 2 * npk * PREC + op_size(N);
 }
 
+// Captured Kepler-pair parameters (producer -> operator kernel), see
+// put_capture: x0[3], v0[3], eight values of the solve and the four
+// coefficients of its result.  1/r = 0 in its place marks a pair without mass.
+constexpr int PCAP = 18;
+constexpr int PCAP_RINV = 11;
+// Doubles of scratch a search needs: in kick groups its final step's record,
+// else that step's captures, snapshots and pair records with d(delxv)/dh.
+__host__ __device__ inline int search_scratch(int N, int npk, bool kick) {
+  return kick ? step_record_size(N, npk, true) : 2 * npk * (PCAP + PREC + 6) + 6 * N;
+}
+
 constexpr int PROD_BS = 32;     // orbit producer: threads per warp-sized unit of work
 constexpr int PROD_MAX_WARPS = 4;  // orbit producer: up to 4 independent warps per block
 // Jacobian consumer: columns per block.  96 N bytes of shared memory a column:
@@ -39,11 +50,6 @@ constexpr int OPS_BS = 128;     // operator kernels
 // v_sky and b_sky^2, v_sky and d v_sky / dt (21N + 3).
 __host__ __device__ inline int trec_size(int N, int tbv) { return tbv ? 21 * N + 3 : 7 * N + 1; }
 
-// Captured Kepler-pair parameters (producer -> operator kernel), see
-// put_capture: x0[3], v0[3], eight values of the solve and the four
-// coefficients of its result.  1/r = 0 in its place marks a pair without mass.
-constexpr int PCAP = 18;
-constexpr int PCAP_RINV = 11;
 // Snapshots per step, 3N doubles each: positions at the correctors, then
 // phisalpha!'s accelerations there, or in kick groups the positions at the
 // first and at the second kick.
@@ -74,11 +80,11 @@ struct GroupArgs {
   int N, S, nsys, grad, K, R, npk;
   int spw;   // orbit producer: systems per warp (lanes >= spw idle)
   int team;  // orbit producer: 1 = a team of lanes per system (orbit_team_kernel), 0 = one lane
-  // transit searches of this chunk in the team form (with team != 0): set by
-  // the host per chunk when few systems of the group are still running, so
-  // that the searches are latency-bound; a full group keeps one lane per
+  // transit searches of this chunk on a block's lanes each (transit_lanes_kernel):
+  // set by the host per chunk when few systems of the group are still running,
+  // so that the searches are latency-bound; a full group keeps one lane per
   // search, which uses every lane of every warp
-  int search_team;
+  int search_lanes;
   // forms for latency-bound chunks (few systems running) of a group without
   // kick pairs, set by the host per chunk: the orbit producer's lanes form
   // (orbit_lanes_kernel) and the Jacobian consumer's rows form
@@ -127,7 +133,7 @@ struct GroupArgs {
   int* task_i;      // [task_cap][3]: system, slot kk*(N-1)+o, transit index
   int* task_count;  // tasks queued in this chunk
   int task_cap;
-  double* tscratch;  // [R][tgrid]: operator records of a search's final partial step
+  double* tscratch;  // [search_scratch][tgrid]: captures and records of a search's final partial step
   int tgrid;         // threads of the transit kernel
   // producer captures for the operator kernels
   double* pcap;   // [K][2 npk][18][S]: Kepler-pair parameters

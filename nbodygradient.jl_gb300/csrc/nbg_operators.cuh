@@ -81,32 +81,4 @@ __device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int cof
   }
 }
 
-// Physical time derivative of the sky-plane projection g (timing.jl:141-144)
-// for transited body i and occultor j: |dv|^2 in the sky plane plus the
-// relative acceleration term.  Drives the transit Newton iterations; the
-// converged search's dtdq0 uses the reference's step derivative (gd!).
-template <int N>
-__device__ __forceinline__ double gdot_physical(const Sys<N>& s, int i, int j) {
-  double ai[2] = {0.0, 0.0}, aj[2] = {0.0, 0.0};
-  for (int b = 0; b < N; b++) {
-    if (b != i) {
-      double d0 = s.x[3 * b] - s.x[3 * i], d1 = s.x[3 * b + 1] - s.x[3 * i + 1], d2 = s.x[3 * b + 2] - s.x[3 * i + 2];
-      double r2 = d0 * d0 + d1 * d1 + d2 * d2;
-      double f = GNEWT * s.m[b] / (r2 * sqrt(r2));
-      ai[0] += f * d0;
-      ai[1] += f * d1;
-    }
-    if (b != j) {
-      double d0 = s.x[3 * b] - s.x[3 * j], d1 = s.x[3 * b + 1] - s.x[3 * j + 1], d2 = s.x[3 * b + 2] - s.x[3 * j + 2];
-      double r2 = d0 * d0 + d1 * d1 + d2 * d2;
-      double f = GNEWT * s.m[b] / (r2 * sqrt(r2));
-      aj[0] += f * d0;
-      aj[1] += f * d1;
-    }
-  }
-  const double dvx = s.v[3 * j] - s.v[3 * i], dvy = s.v[3 * j + 1] - s.v[3 * i + 1];
-  const double dx = s.x[3 * j] - s.x[3 * i], dy = s.x[3 * j + 1] - s.x[3 * i + 1];
-  return dvx * dvx + dvy * dvy + dx * (aj[0] - ai[0]) + dy * (aj[1] - ai[1]);
-}
-
 }  // namespace nbg

@@ -342,7 +342,7 @@ int create_group(nbg_server* srv, int N, int grad, unsigned long long kick, Grou
   want(&g.task_f, 2 * nf); want(&g.task_i, 2 * ni); want(&g.task_count, 2);
   if (grad) {
     want(&g.steprec, 2 * nrec); want(&g.trec, 2 * ntrec);
-    want(&g.tflag, 2 * nflag); want(&g.tscratch, (size_t)g.R * g.tgrid);
+    want(&g.tflag, 2 * nflag); want(&g.tscratch, (size_t)search_scratch(N, npk, kick != 0) * g.tgrid);
     want(&g.pcap, 2 * ncap);
     want(&g.xsnap, 2 * nsnap); want(&g.dh, 12 * (size_t)npk * S);
     want(&g.Jint, S * 6 * N * 7 * N); want(&g.Eint, S * 6 * N * 7 * N);
@@ -624,9 +624,13 @@ int service_group(nbg_server* srv, int gi) {
   NBG_CUDA(cudaStreamWaitEvent(stt, G->ev_orb[par], 0));
   NBG_CUDA(cudaStreamWaitEvent(sw, G->ev_orb[par], 0));
   {
-    // the team form of the searches while few slots are running (latency-bound searches)
+    // a block's lanes per search while few slots are running, from five bodies on:
+    // below, a search on one lane ends within the producer's next chunk (32
+    // steps by default), and the lanes would only take pipe time from the groups
+    // beside it
     GroupArgs gs = gc;
-    gs.search_team = (G->active <= std::max(32, srv->sm_count / 2)) ? 1 : 0;
+    gs.search_lanes =
+        N >= 5 && use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2), G->kick) ? 1 : 0;
     if ((rc = launch_group_transit(N, gs, (int)c, stt))) return rc;
   }
   NBG_CUDA(cudaEventRecord(G->ev_tr[par], stt));
