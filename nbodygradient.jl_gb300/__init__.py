@@ -581,23 +581,29 @@ def init_nbody_batch(ics, ctx=None):
     ctx = ctx or default_context()
     n = np.array([ic.nbody for ic in ics], dtype=np.int32)
     t0 = np.array([ic.t0 for ic in ics], dtype=np.float64)
-    el = np.concatenate([np.asfortranarray(ic.elements, dtype=np.float64).ravel(order="F") for ic in ics])
-    nested = all(np.array_equal(ic.H, hierarchy_nested(ic.nbody)) for ic in ics)
-    H = None if nested else np.concatenate(
-        [np.asfortranarray(ic.H, dtype=np.float64).ravel(order="F") for ic in ics])
-    x = np.zeros(int(3 * n.sum()))
-    v = np.zeros(int(3 * n.sum()))
-    J = np.zeros(int((49 * n.astype(np.int64) ** 2).sum()))
+    # runs of systems of one body count are packed and unpacked as one array
+    cuts = np.flatnonzero(np.diff(n)) + 1
+    runs = list(zip(np.concatenate([[0], cuts]).tolist(), np.concatenate([cuts, [len(n)]]).tolist())) if len(n) else []
+    packed = lambda mats: np.ascontiguousarray(np.array(mats, dtype=np.float64).transpose(0, 2, 1)).ravel()
+    el = np.concatenate([packed([ic.elements for ic in ics[a:b]]) for a, b in runs])
+    Hs = [packed([ic.H for ic in ics[a:b]]) for a, b in runs]
+    nested = all(np.array_equal(h.reshape(b - a, -1), np.broadcast_to(hierarchy_nested(int(n[a])).ravel(order="F"),
+                                                                      (b - a, int(n[a]) ** 2)))
+                 for h, (a, b) in zip(Hs, runs))
+    H = None if nested else np.concatenate(Hs)
+    x = np.empty(int(3 * n.sum()))
+    v = np.empty(int(3 * n.sum()))
+    J = np.empty(int((49 * n.astype(np.int64) ** 2).sum()))
     p = _lib.ptr
     _lib.check(_lib.load().nbg_batch_init_nbody(ctx.handle, len(ics), p(n, __import__("ctypes").POINTER(
         __import__("ctypes").c_int32)), p(t0), p(el), p(H), p(x), p(v), p(J)))
     out, ax, aJ = [], 0, 0
-    for k in n:
-        k = int(k)
-        out.append((x[ax:ax + 3 * k].reshape((3, k), order="F"), v[ax:ax + 3 * k].reshape((3, k), order="F"),
-                    J[aJ:aJ + 49 * k * k].reshape((7 * k, 7 * k), order="F")))
-        ax += 3 * k
-        aJ += 49 * k * k
+    for a, b in runs:
+        k, count = int(n[a]), b - a
+        cols = lambda arr, at, r, c: list(arr[at:at + count * r * c].reshape(count, c, r).transpose(0, 2, 1))
+        out += zip(cols(x, ax, 3, k), cols(v, ax, 3, k), cols(J, aJ, 7 * k, 7 * k))
+        ax += 3 * k * count
+        aJ += 49 * k * k * count
     return out
 
 

@@ -20,6 +20,7 @@
 #include <map>
 #include <tuple>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/nbg.h"
@@ -282,6 +283,28 @@ struct nbg_context {
   std::vector<cudaStream_t> hstreams;
   std::vector<cudaEvent_t> sync_events;  // cross-stream ordering, no timing
   NoallocPlan* noalloc = nullptr;         // host plan of the allocation-free entry point
+  // pinned host memory that a call's small arrays go through, one copy for all
+  // of them: 0 the plan's, 1 the caller's arrays (grow-only, kStageMax at most)
+  struct Pinned {
+    unsigned char* p = nullptr;
+    size_t bytes = 0;
+  } pinned[2];
+  int pin(int which, size_t bytes, unsigned char** out) {
+    Pinned& b = pinned[which];
+    if (b.bytes < bytes) {
+      if (b.p) cudaFreeHost(b.p);
+      b.p = nullptr;
+      b.bytes = 0;
+      const size_t want = std::max<size_t>(bytes, 64 * 1024);
+      if (cudaHostAlloc((void**)&b.p, want, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return set_error(NBG_ENOMEM, "cudaHostAlloc(%zu bytes)", want);
+      }
+      b.bytes = want;
+    }
+    *out = b.p;
+    return NBG_OK;
+  }
 
   int sync_event(size_t i, cudaEvent_t* out) {
     while (sync_events.size() <= i) {
@@ -456,24 +479,15 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     gp.systems.push_back(s);
     gp.max_steps = std::max(gp.max_steps, nsteps[s]);
   }
-  SysOff* d_off;
   int rc;
-  if ((rc = ctx->get("off", (size_t)nsys, &d_off))) return rc;
-  NBG_CUDA(cudaMemcpyAsync(d_off, off.data(), sizeof(SysOff) * nsys, cudaMemcpyHostToDevice, st));
-  long long* d_offtt;
-  long long* d_offdq;
-  if ((rc = ctx->get("offtt", (size_t)nsys, &d_offtt))) return rc;
-  if ((rc = ctx->get("offdq", (size_t)nsys, &d_offdq))) return rc;
-  {
-    std::vector<long long> a(nsys), b(nsys);
-    for (int s = 0; s < nsys; s++) { a[s] = off[s].tt; b[s] = off[s].dq; }
-    NBG_CUDA(cudaMemcpyAsync(d_offtt, a.data(), sizeof(long long) * nsys, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(d_offdq, b.data(), sizeof(long long) * nsys, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaStreamSynchronize(st));  // host vectors a, b go out of scope
-  }
   // Steps per chunk: the context's setting, shortened (not below 8) where a
   // group's operator records for one chunk would pass 4 GiB per buffer half.
+  // A short call takes a quarter of its steps, so that its producer, searches
+  // and consumer still overlap (64 steps of three bodies: SHORT_FIGURES).
   int K = std::max(1, ctx->chunk_steps);
+  long long longest = 0;
+  for (auto& kv : groups) longest = std::max(longest, kv.second.max_steps);
+  K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
   for (auto& kv : groups) {
     const GroupPlan& gp = kv.second;
     if (!gp.grad) continue;
@@ -484,6 +498,34 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     const double per_step = 8.0 * step_record_size(gp.N, npk, gp.kick != 0) * (((gp.systems.size() + 31) / 32) * 32);
     const int kmax = (int)std::min(4096.0, std::floor(4294967296.0 / per_step));
     K = std::min(K, std::max(std::min(K, 8), kmax));
+  }
+  // ---- the plan's small arrays (offsets, each group's scalars): written to
+  // pinned memory and copied as one block
+  size_t plan_bytes = 0;
+  for (auto& kv : groups) plan_bytes += ((kv.second.systems.size() + 31) / 32) * 32 * (5 * 8 + 4 * 4) + 9 * 64;
+  plan_bytes += (size_t)nsys * (sizeof(SysOff) + 24) + 4 * 64;
+  unsigned char *plan, *d_plan;
+  if ((rc = ctx->pin(0, plan_bytes, &plan)) || (rc = ctx->get("plan", plan_bytes, &d_plan))) return rc;
+  size_t plan_at = 0;
+  auto part = [&](auto** dev, size_t count) {  // room for count values; *dev their device address
+    using T = std::remove_reference_t<decltype(**dev)>;
+    T* host = (T*)(plan + plan_at);
+    *dev = (T*)(d_plan + plan_at);
+    plan_at = (plan_at + count * sizeof(T) + 63) / 64 * 64;
+    return host;
+  };
+  SysOff* d_off;
+  long long *d_offtt, *d_offdq;
+  double *d_tout, *h_tout = part(&d_tout, nsys);
+  std::vector<unsigned*> gstatus;  // each group's status words, read back at the end
+  {
+    SysOff* h_off = part(&d_off, nsys);
+    long long *h_tt = part(&d_offtt, nsys), *h_dq = part(&d_offdq, nsys);
+    for (int s = 0; s < nsys; s++) {
+      h_off[s] = off[s];
+      h_tt[s] = off[s].tt;
+      h_dq[s] = off[s].dq;
+    }
   }
   // ---- per-group device state
   std::vector<GroupArgs> gargs;
@@ -533,11 +575,15 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     auto name = [&](const char* f) { snprintf(nm, sizeof(nm), "g%d_%s", gi, f); return nm; };
 #define GET(field, cnt) if ((rc = ctx->get(name(#field), (size_t)(cnt), &g.field))) return rc
     GET(x, 3 * N * S); GET(v, 3 * N * S); GET(xe, 3 * N * S); GET(ve, 3 * N * S); GET(m, N * S);
-    GET(dqdt, 7 * N * S); GET(gsave, N * S); GET(count, N * S); GET(t0, S); GET(h, S); GET(hI, S);
-    GET(nsteps, S); GET(ntt, S); GET(ti, S); GET(sysidx, S); GET(status, S);
-    double* hlast = nullptr;
+    GET(dqdt, 7 * N * S); GET(gsave, N * S); GET(count, N * S);
+    int *h_sidx = part(&g.sysidx, S), *h_ntt = part(&g.ntt, S), *h_ti = part(&g.ti, S);
+    unsigned* h_status = part(&g.status, S);
+    gstatus.push_back(h_status);
+    double *h_t0 = part(&g.t0, S), *h_h = part(&g.h, S), *h_hI = part(&g.hI, S);
+    long long* h_ns = part(&g.nsteps, S);
+    double *hlast = nullptr, *h_hl = nullptr;
     if (plain) {
-      if ((rc = ctx->get(name("hlast"), (size_t)S, &hlast))) return rc;
+      h_hl = part(&hlast, S);
       g.hlast = hlast;
       g.notransit = 1;
     }
@@ -567,36 +613,17 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     }
 #undef GET
     g.tt = d_tt; g.off_tt = d_offtt; g.dtdq0 = d_dq0; g.off_dq = d_offdq;
-    // host-side scalars
-    std::vector<int> sidx(S, -1), vntt(S, 1), vti(S, 0);
-    std::vector<double> vt0(S, 0.0), vh(S, 0.0), vhI(S, 0.0), vhl(S, 0.0);
-    std::vector<long long> vns(S, 0);
-    for (int q = 0; q < nsg; q++) {
-      int s = gp.systems[q];
-      sidx[q] = s; vntt[q] = desc[s].ntt; vti[q] = desc[s].ti;
-      vt0[q] = t_host[s]; vh[q] = hsig[s]; vhI[q] = desc[s].h; vns[q] = nsteps[s];
-      if (plain) vhl[q] = plain[s].hlast;
-    }
-    if (plain) NBG_CUDA(cudaMemcpyAsync(hlast, vhl.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.sysidx, sidx.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.ntt, vntt.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.ti, vti.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.t0, vt0.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.h, vh.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.hI, vhI.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(g.nsteps, vns.data(), sizeof(long long) * S, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemsetAsync(g.status, 0, sizeof(unsigned) * S, st));
-    NBG_CUDA(cudaStreamSynchronize(st));
-    // gather state
-    int pb = (S + 127) / 128;
-    pack_state_kernel<<<pb, 128, 0, st>>>(N, S, g.sysidx, d_off, d_x, d_v, d_xe, d_ve, d_m, d_dqdt, d_count, g.x,
-                                          g.v, g.xe, g.ve, g.m, g.dqdt, g.count);
-    ctx->last_launches++;
-    if (gp.grad) {
-      long long tot = (long long)S * 49 * N * N;
-      pack_jac_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(N, S, g.sysidx, d_off, d_J, d_E, g.Jint, g.Eint,
-                                                                     d_bad);
-      ctx->last_launches++;
+    for (int q = 0; q < S; q++) {
+      const int s = q < nsg ? gp.systems[q] : -1;
+      h_sidx[q] = s;
+      h_status[q] = 0;
+      h_ntt[q] = s < 0 ? 1 : desc[s].ntt;
+      h_ti[q] = s < 0 ? 0 : desc[s].ti;
+      h_t0[q] = s < 0 ? 0.0 : t_host[s];
+      h_h[q] = s < 0 ? 0.0 : hsig[s];
+      h_hI[q] = s < 0 ? 0.0 : desc[s].h;
+      h_ns[q] = s < 0 ? 0 : nsteps[s];
+      if (plain) h_hl[q] = s < 0 ? 0.0 : plain[s].hlast;
     }
     gargs.push_back(g);
     {
@@ -612,14 +639,28 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     for (int sidx : gp.systems) gsteps.back().push_back(nsteps[sidx]);
     gi++;
   }
+  // gather the state
+  NBG_CUDA(cudaMemcpyAsync(d_plan, plan, plan_at, cudaMemcpyHostToDevice, st));
+  bool any_grad = false;
+  for (auto& g : gargs) {
+    launch_pack_state(g.N, g.S, g.sysidx, d_off, d_x, d_v, d_xe, d_ve, d_m, d_dqdt, d_count, g, st);
+    ctx->last_launches++;
+    if (g.grad) {
+      launch_pack_jac(g.N, g.S, g.sysidx, d_off, d_J, d_E, g, d_bad, st);
+      ctx->last_launches++;
+      any_grad = true;
+    }
+  }
   NBG_CUDA(cudaGetLastError());
-  int bad = 0;
-  NBG_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaStreamSynchronize(st));
-  if (bad)
-    return set_error(NBG_EUNSUPPORTED,
-                     "jac_step mass rows must be unit rows with zero jac_error (true for every State the reference "
-                     "builds and integrates)");
+  if (any_grad) {
+    int bad = 0;
+    NBG_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    NBG_CUDA(cudaStreamSynchronize(st));
+    if (bad)
+      return set_error(NBG_EUNSUPPORTED,
+                       "jac_step mass rows must be unit rows with zero jac_error (true for every State the reference "
+                       "builds and integrates)");
+  }
   for (auto& g : gargs) {
     kSeed[g.N](g, st);
     ctx->last_launches++;
@@ -912,13 +953,13 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   }
   // s.t = t0 + nsteps * h (Transits.jl:161 at the last step); the plain
   // drivers set it themselves (Integrator.jl:196, :228)
-  {
-    std::vector<double> tout(nsys);
-    for (int s = 0; s < nsys; s++)
-      tout[s] = plain ? plain[s].tout : (nsteps[s] > 0 ? t_host[s] + (double)nsteps[s] * hsig[s] : t_host[s]);
-    NBG_CUDA(cudaMemcpyAsync(d_t, tout.data(), sizeof(double) * nsys, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaStreamSynchronize(st));
-  }
+  for (int s = 0; s < nsys; s++)
+    h_tout[s] = plain ? plain[s].tout : (nsteps[s] > 0 ? t_host[s] + (double)nsteps[s] * hsig[s] : t_host[s]);
+  NBG_CUDA(cudaMemcpyAsync(d_t, h_tout, sizeof(double) * nsys, cudaMemcpyHostToDevice, st));
+  if (status_host)
+    for (size_t q = 0; q < gargs.size(); q++)
+      NBG_CUDA(cudaMemcpyAsync(gstatus[q], gargs[q].status, sizeof(unsigned) * gargs[q].S, cudaMemcpyDeviceToHost, st));
+  NBG_CUDA(cudaStreamSynchronize(st));
   NBG_CUDA(cudaGetLastError());
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -933,17 +974,70 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   if (ctx->profile == 3 && sampled > 0) ctx->last_jac_ms *= (double)ctx->last_jac_launches / (double)sampled;
   if (status_host) {
     std::fill(status_host, status_host + nsys, 0u);
-    for (auto& g : gargs) {
-      std::vector<unsigned> sv(g.S);
-      std::vector<int> si(g.S);
-      NBG_CUDA(cudaMemcpy(sv.data(), g.status, sizeof(unsigned) * g.S, cudaMemcpyDeviceToHost));
-      NBG_CUDA(cudaMemcpy(si.data(), g.sysidx, sizeof(int) * g.S, cudaMemcpyDeviceToHost));
-      for (int q = 0; q < g.S; q++)
-        if (si[q] >= 0) status_host[si[q]] = sv[q];
+    size_t q = 0;
+    for (auto& kv : groups) {
+      for (size_t r = 0; r < kv.second.systems.size(); r++) status_host[kv.second.systems[r]] = gstatus[q][r];
+      q++;
     }
   }
   return NBG_OK;
 }
+
+// A host call's arrays: what goes in, out or both, in one device block.  Up to
+// kStageMax in all they go through the context's pinned memory in one copy each
+// way (a copy of its own for each array of a small system costs more than the
+// bytes: 16 steps of two bodies 473 -> 358 us a call); larger ones are copied from and
+// to where they are.
+constexpr size_t kStageMax = 4u << 20;
+struct HostArrays {
+  struct Array {
+    const void* in;
+    void* out;
+    size_t bytes, at;
+  };
+  std::vector<Array> arrays;
+  size_t total = 0, out_end = 0;
+  unsigned char* dev = nullptr;
+
+  // null `in`: zeros on the device; `out` arrays first
+  void add(const void* in, void* out, size_t bytes) {
+    arrays.push_back({in, out, bytes, total});
+    total += (bytes + 255) / 256 * 256;
+    if (out) out_end = total;
+  }
+  int upload(nbg_context* ctx, const char* name) {
+    int rc;
+    if ((rc = ctx->get(name, total, &dev))) return rc;
+    if (total <= kStageMax) {
+      unsigned char* p;
+      if ((rc = ctx->pin(1, total, &p))) return rc;
+      for (auto& a : arrays)
+        if (a.in) memcpy(p + a.at, a.in, a.bytes);
+        else memset(p + a.at, 0, a.bytes);
+      NBG_CUDA(cudaMemcpyAsync(dev, p, total, cudaMemcpyHostToDevice, ctx->stream));
+      return NBG_OK;
+    }
+    for (auto& a : arrays)
+      if (a.in) NBG_CUDA(cudaMemcpyAsync(dev + a.at, a.in, a.bytes, cudaMemcpyHostToDevice, ctx->stream));
+      else NBG_CUDA(cudaMemsetAsync(dev + a.at, 0, a.bytes, ctx->stream));
+    return NBG_OK;
+  }
+  int download(nbg_context* ctx) {
+    const bool staged = total <= kStageMax;
+    if (staged)
+      NBG_CUDA(cudaMemcpyAsync(ctx->pinned[1].p, dev, out_end, cudaMemcpyDeviceToHost, ctx->stream));
+    else
+      for (auto& a : arrays)
+        if (a.out) NBG_CUDA(cudaMemcpyAsync(a.out, dev + a.at, a.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    NBG_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (staged)
+      for (auto& a : arrays)
+        if (a.out) memcpy(a.out, ctx->pinned[1].p + a.at, a.bytes);
+    return NBG_OK;
+  }
+  template <class T>
+  T* at(size_t k) const { return (T*)(dev + arrays[k].at); }
+};
 
 }  // namespace
 
@@ -1404,6 +1498,8 @@ int nbg_destroy(nbg_context* ctx) {
   for (cudaStream_t s2 : ctx->hstreams) cudaStreamSynchronize(s2);
   for (auto& kv : ctx->pool)
     if (kv.second.p) cudaFree(kv.second.p);
+  for (auto& b : ctx->pinned)
+    if (b.p) cudaFreeHost(b.p);
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
   for (auto e : ctx->prof_events) cudaEventDestroy(e);
@@ -1595,53 +1691,30 @@ static int batch_host_device(nbg_context* ctx, int nsys, const nbg_system_desc* 
   if (!copy_outputs_in)
     for (long long q = 0; q < am; q++)
       if (count[q] != 0) return set_error(NBG_EINVAL, "batched calls need fresh TransitTiming outputs (count == 0)");
-  cudaStream_t st = ctx->stream;
-  double *d_t, *d_x, *d_v, *d_m, *d_xe, *d_ve, *d_J, *d_E, *d_dq, *d_ji, *d_tt, *d_dq0, *d_del;
-  long long* d_cnt;
+  constexpr size_t D = sizeof(double);
+  HostArrays ha;
+  ha.add(t, t, D * nsys);
+  ha.add(x, x, D * ax);
+  ha.add(v, v, D * ax);
+  ha.add(xerror, xerror, D * ax);
+  ha.add(verror, verror, D * ax);
+  ha.add(jac_step, jac_step, D * aJ);
+  ha.add(jac_error, jac_error, D * aJ);
+  ha.add(dqdt, dqdt, D * adq);
+  ha.add(count, count, sizeof(int64_t) * am);
+  ha.add(copy_outputs_in ? tt : nullptr, tt, D * att);
+  ha.add(copy_outputs_in ? dtdq0 : nullptr, dtdq0, D * adq0);
+  ha.add(copy_outputs_in ? dtdelements : nullptr, dtdelements, D * adq0);
+  ha.add(m, nullptr, D * am);
+  ha.add(jac_init, nullptr, D * aJ);
   int rc;
-#define GETB(ptr, nm, cnt) if ((rc = ctx->get(nm, (size_t)(cnt), &ptr))) return rc
-  GETB(d_t, "u_t", nsys); GETB(d_x, "u_x", ax); GETB(d_v, "u_v", ax); GETB(d_m, "u_m", am);
-  GETB(d_xe, "u_xe", ax); GETB(d_ve, "u_ve", ax); GETB(d_J, "u_J", aJ); GETB(d_E, "u_E", aJ);
-  GETB(d_dq, "u_dq", adq); GETB(d_ji, "u_ji", aJ); GETB(d_tt, "u_tt", att); GETB(d_dq0, "u_dq0", adq0);
-  GETB(d_del, "u_del", adq0); GETB(d_cnt, "u_cnt", am);
-#undef GETB
-  NBG_CUDA(cudaMemcpyAsync(d_t, t, sizeof(double) * nsys, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_x, x, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_v, v, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_m, m, sizeof(double) * am, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_xe, xerror, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_ve, verror, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_J, jac_step, sizeof(double) * aJ, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_E, jac_error, sizeof(double) * aJ, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_dq, dqdt, sizeof(double) * adq, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_ji, jac_init, sizeof(double) * aJ, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_cnt, count, sizeof(long long) * am, cudaMemcpyHostToDevice, st));
-  if (copy_outputs_in) {
-    NBG_CUDA(cudaMemcpyAsync(d_tt, tt, sizeof(double) * att, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(d_dq0, dtdq0, sizeof(double) * adq0, cudaMemcpyHostToDevice, st));
-    NBG_CUDA(cudaMemcpyAsync(d_del, dtdelements, sizeof(double) * adq0, cudaMemcpyHostToDevice, st));
-  } else {
-    NBG_CUDA(cudaMemsetAsync(d_tt, 0, sizeof(double) * att, st));
-    NBG_CUDA(cudaMemsetAsync(d_dq0, 0, sizeof(double) * adq0, st));
-    NBG_CUDA(cudaMemsetAsync(d_del, 0, sizeof(double) * adq0, st));
-  }
-  rc = run_batch(ctx, nsys, desc, t, pair, d_t, d_x, d_v, d_m, d_xe, d_ve, d_J, d_E, d_dq, d_ji, d_tt, d_dq0, d_del,
-                 d_cnt, status, nullptr, tbv);
+  if ((rc = ha.upload(ctx, "u_all"))) return rc;
+  rc = run_batch(ctx, nsys, desc, t, pair, ha.at<double>(0), ha.at<double>(1), ha.at<double>(2), ha.at<double>(12),
+                 ha.at<double>(3), ha.at<double>(4), ha.at<double>(5), ha.at<double>(6), ha.at<double>(7),
+                 ha.at<double>(13), ha.at<double>(9), ha.at<double>(10), ha.at<double>(11), ha.at<long long>(8), status,
+                 nullptr, tbv);
   if (rc) return rc;
-  NBG_CUDA(cudaMemcpyAsync(t, d_t, sizeof(double) * nsys, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(x, d_x, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(v, d_v, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(xerror, d_xe, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(verror, d_ve, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(jac_step, d_J, sizeof(double) * aJ, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(jac_error, d_E, sizeof(double) * aJ, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(dqdt, d_dq, sizeof(double) * adq, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(count, d_cnt, sizeof(long long) * am, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(tt, d_tt, sizeof(double) * att, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(dtdq0, d_dq0, sizeof(double) * adq0, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(dtdelements, d_del, sizeof(double) * adq0, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaStreamSynchronize(st));
-  return NBG_OK;
+  return ha.download(ctx);
 }
 
 // Plain integration of nsys systems (host arrays, the packed layout of the
@@ -1672,37 +1745,26 @@ static int plain_host(nbg_context* ctx, int nsys, const nbg_system_desc* desc, c
       return set_error(NBG_EUNSUPPORTED, "system %d: n = %d outside %d..%d", s, n, NBG_MIN_BODIES, NBG_MAX_BODIES);
     ax += 3 * n; am += n; aJ += (long long)M * M; adq += M;
   }
-  cudaStream_t st = ctx->stream;
-  double *d_t, *d_x, *d_v, *d_m, *d_xe, *d_ve, *d_J, *d_E, *d_dq;
-  long long* d_cnt;
+  constexpr size_t D = sizeof(double);
+  HostArrays ha;
+  ha.add(t, t, D * nsys);
+  ha.add(x, x, D * ax);
+  ha.add(v, v, D * ax);
+  ha.add(xerror, xerror, D * ax);
+  ha.add(verror, verror, D * ax);
+  ha.add(jac_step, jac_step, D * aJ);
+  ha.add(jac_error, jac_error, D * aJ);
+  ha.add(dqdt, dqdt, D * adq);
+  ha.add(m, nullptr, D * am);
+  ha.add(nullptr, nullptr, sizeof(int64_t) * am);
   int rc;
-#define GETB(ptr, nm, cnt) if ((rc = ctx->get(nm, (size_t)(cnt), &ptr))) return rc
-  GETB(d_t, "p_t", nsys); GETB(d_x, "p_x", ax); GETB(d_v, "p_v", ax); GETB(d_m, "p_m", am);
-  GETB(d_xe, "p_xe", ax); GETB(d_ve, "p_ve", ax); GETB(d_J, "p_J", aJ); GETB(d_E, "p_E", aJ);
-  GETB(d_dq, "p_dq", adq); GETB(d_cnt, "p_cnt", am);
-#undef GETB
-  NBG_CUDA(cudaMemcpyAsync(d_x, x, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_v, v, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_m, m, sizeof(double) * am, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_xe, xerror, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_ve, verror, sizeof(double) * ax, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_J, jac_step, sizeof(double) * aJ, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_E, jac_error, sizeof(double) * aJ, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemcpyAsync(d_dq, dqdt, sizeof(double) * adq, cudaMemcpyHostToDevice, st));
-  NBG_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(long long) * am, st));
+  if ((rc = ha.upload(ctx, "p_all"))) return rc;
   std::vector<uint32_t> stv(nsys, 0u);
-  rc = run_batch(ctx, nsys, desc, t, pair, d_t, d_x, d_v, d_m, d_xe, d_ve, d_J, d_E, d_dq, nullptr, nullptr, nullptr,
-                 nullptr, d_cnt, stv.data(), spec, 0, traj);
+  rc = run_batch(ctx, nsys, desc, t, pair, ha.at<double>(0), ha.at<double>(1), ha.at<double>(2), ha.at<double>(8),
+                 ha.at<double>(3), ha.at<double>(4), ha.at<double>(5), ha.at<double>(6), ha.at<double>(7), nullptr,
+                 nullptr, nullptr, nullptr, ha.at<long long>(9), stv.data(), spec, 0, traj);
   if (rc) return rc;
-  NBG_CUDA(cudaMemcpyAsync(t, d_t, sizeof(double) * nsys, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(x, d_x, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(v, d_v, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(xerror, d_xe, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(verror, d_ve, sizeof(double) * ax, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(jac_step, d_J, sizeof(double) * aJ, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(jac_error, d_E, sizeof(double) * aJ, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaMemcpyAsync(dqdt, d_dq, sizeof(double) * adq, cudaMemcpyDeviceToHost, st));
-  NBG_CUDA(cudaStreamSynchronize(st));
+  if ((rc = ha.download(ctx))) return rc;
   return nonfinite_error(nsys, stv.data());
 }
 
