@@ -398,8 +398,7 @@ bool use_team(int mode, int N, unsigned long long kick) {
 // The forms for latency-bound chunks (sixteen lanes per pair solve, six per
 // column of jac_step): always in mode 2, in the latency-bound chunks (few
 // systems running) in modes -1 and 3.
-bool use_wide(int mode, bool latency_bound, unsigned long long kick) {
-  if (kick) return false;
+bool use_wide(int mode, bool latency_bound) {
   return mode == 2 || ((mode < 0 || mode == 3) && latency_bound);
 }
 }  // namespace nbg
@@ -483,7 +482,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   // Steps per chunk: the context's setting, shortened (not below 8) where a
   // group's operator records for one chunk would pass 4 GiB per buffer half.
   // A short call takes a quarter of its steps, so that its producer, searches
-  // and consumer still overlap (64 steps of three bodies: SHORT_FIGURES).
+  // and consumer still overlap (a recorded trajectory of 62 steps 2.5 -> 2.0 ms).
   int K = std::max(1, ctx->chunk_steps);
   long long longest = 0;
   for (auto& kv : groups) longest = std::max(longest, kv.second.max_steps);
@@ -608,7 +607,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     g.tgrid = std::min(((g.task_cap + 31) / 32) * 32, std::max(1, ctx->sm_count) * 4 * 32);
     if (gp.grad) {
       GET(steprec, nb * nrec); GET(trec, nb * ntrec); GET(tflag, nb * nflag); GET(tscratch, (size_t)search_scratch(N, npk, gp.kick != 0) * g.tgrid);
-      GET(pcap, nb * ncap); GET(xsnap, nb * nsnap); GET(dh, 12 * (size_t)npk * S);
+      GET(pcap, nb * ncap); GET(xsnap, nb * nsnap); GET(dh, 12 * (size_t)npk * S); GET(vsnap, 6 * N * S);
       GET(Jint, (size_t)S * 6 * N * 7 * N); GET(Eint, (size_t)S * 6 * N * 7 * N);
     }
 #undef GET
@@ -761,7 +760,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   };
   auto search_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    gx.search_lanes = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max, g.kick) ? 1 : 0;
+    gx.search_lanes = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max) ? 1 : 0;
     if (tail_any) gx.guard_smem = std::max(gx.guard_smem, 18 * 1024);
     return gx;
   };
@@ -769,12 +768,12 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     GroupArgs gx = g;
     const bool tail = active_at(q, c) <= tail_max;
     if (tail) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
-    gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= lanes_limit(g.N, g.grad, ctx->sm_count), g.kick) ? 1 : 0;
+    gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= lanes_limit(g.N, g.grad, ctx->sm_count)) ? 1 : 0;
     return gx;
   };
   auto jac_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    gx.rows = use_wide(ctx->orbit_team, active_at(q, c) <= rows_limit(g.N, ctx->sm_count), g.kick) ? 1 : 0;
+    gx.rows = use_wide(ctx->orbit_team, active_at(q, c) <= rows_limit(g.N, ctx->sm_count)) ? 1 : 0;
     return gx;
   };
   auto ops_args = [&](const GroupArgs& g) {
@@ -1091,7 +1090,7 @@ void noalloc_layout(NoallocPlan& P, ScratchArena& a, int nsys, int K, int tcap, 
       a.take(&g.tflag, (size_t)K * (N - 1) * S); a.take(&g.tscratch, (size_t)search_scratch(N, g.npk, g.kick != 0) * g.tgrid);
       a.take(&g.pcap, (size_t)K * 2 * g.npk * PCAP * S + 1);
       a.take(&g.xsnap, (size_t)K * snap_count(g.kick != 0) * 3 * N * S);
-      a.take(&g.dh, 12 * (size_t)g.npk * S);
+      a.take(&g.dh, 12 * (size_t)g.npk * S); a.take(&g.vsnap, 6 * N * S);
       a.take(&g.Jint, (size_t)S * 6 * N * 7 * N); a.take(&g.Eint, (size_t)S * 6 * N * 7 * N);
     }
   }

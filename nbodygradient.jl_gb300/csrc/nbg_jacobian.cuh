@@ -58,62 +58,6 @@ __device__ __forceinline__ void fold_rows(double* J, double* E) {
     for (int r = R0; r < R0 + NR; r++) fold(J[(6 * b + r) * BS], E[(6 * b + r) * BS]);
 }
 
-// P[vr] = (A J)[velocity row vr] for the compact operator at record offset
-// roff: one FMA chain over the position rows of J, with the exact no-op
-// terms (zero operator entries; mass rows of J, which are unit rows) reduced
-// to the single mass entry of this column, which starts the chain.  Starting
-// from it costs no FP64 instruction, where adding it inside the chain would
-// cost a warp-wide issue slot for the few mass-column lanes; the summation
-// order of the reference's BLAS product is unspecified, so any order is as
-// faithful as another.
-template <int N, int BS>
-__device__ __forceinline__ void op_product(const double* J, const Rec& rec, int roff, int c, double* P) {
-  const int cm = (c % 7 == 6) ? c / 7 : -1;  // body whose mass this column is
-#pragma unroll 1
-  for (int vr = 0; vr < 3 * N; vr++) {
-    const int rb = roff + vr * (4 * N);
-    double acc = (cm >= 0) ? rec.get(rb + 4 * cm + 3) : 0.0;
-#pragma unroll
-    for (int d = 0; d < N; d++)
-#pragma unroll
-      for (int p = 0; p < 3; p++) acc = fma(rec.get(rb + 4 * d + p), J[(6 * d + p) * BS], acc);
-    P[vr] = acc;
-  }
-}
-
-// One Kepler pair block update (ahl21.jl:31-42 / :64-75) on this column.
-// The pair's record is loaded first, all of it, so that its loads go out
-// together ahead of this pair's stores to J and E (which a load through the
-// record pointer could alias): one trip to memory per pair.  A system alone
-// on the GPU waits out every such trip, at ten bodies 90 of them per step.
-template <int N, int BS>
-__device__ __forceinline__ void pair_apply(double* J, double* E, int c, int i, int j, const Rec& rec, int roff) {
-  double K[36];
-#pragma unroll
-  for (int q = 0; q < 36; q++) K[q] = rec.get(roff + q);
-  const double mi = rec.get(roff + PREC_MI), mj = rec.get(roff + PREC_MJ);
-  // the mass columns of i and j start u from Psi and one of them adds B to
-  // each body; every other column takes exact zeros
-  const bool ci = c == 7 * i + 6, cj = c == 7 * j + 6;
-  double U[6], B[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) {
-    U[q] = (ci || cj) ? rec.get(roff + PREC_PSI + q) : 0.0;
-    B[q] = (ci || cj) ? rec.get(roff + PREC_B + q) : 0.0;
-  }
-  double D[6];
-#pragma unroll
-  for (int l = 0; l < 6; l++) D[l] = J[(6 * i + l) * BS] - J[(6 * j + l) * BS];
-#pragma unroll
-  for (int r = 0; r < 6; r++) {
-    double u = U[r];
-#pragma unroll
-    for (int l = 0; l < 6; l++) u = fma(K[r * 6 + l], D[l], u);
-    kahan(J[(6 * i + r) * BS], E[(6 * i + r) * BS], fma(mj, u, cj ? B[r] : 0.0));
-    kahan(J[(6 * j + r) * BS], E[(6 * j + r) * BS], fma(-mi, u, ci ? -B[r] : 0.0));
-  }
-}
-
 // J <- J + A J on all non-mass rows: velocity rows take the product P,
 // position rows a zero addend.  Every row is summed on its own, so the
 // position rows' folds may run first.
@@ -130,60 +74,7 @@ __device__ __forceinline__ void fold_all(double* J, double* E) {
   fold_rows<N, BS, 0, 6>(J, E);
 }
 
-// drift_grad! on jac_step (ahl21.jl:318-331): x rows += h * v rows.
-template <int N, int BS>
-__device__ __forceinline__ void drift_rows(double* J, double* E, double h) {
-#pragma unroll 1
-  for (int b = 0; b < N; b++)
-#pragma unroll
-    for (int k = 0; k < 3; k++) kahan(J[(6 * b + k) * BS], E[(6 * b + k) * BS], h * J[(6 * b + 3 + k) * BS]);
-}
-
-// One recorded step on this column (ahl21.jl:5-95, the jac_step updates), for
-// groups with kick pairs.
-template <int N, int BS>
-__device__ void apply_step(double* J, double* E, int c, double h, uint64_t kick, const Rec& rec) {
-  const double h2 = 0.5 * h;
-  double P[3 * N];
-  int roff = 0;
-  if (kick) {
-    op_product<N, BS>(J, rec, roff, c, P);  // jac_kick * jac_step before the drift
-    roff += op_size(N);
-  }
-  drift_rows<N, BS>(J, E, h2);
-  if (kick) add_velocity_rows<N, BS>(J, E, P);
-  else fold_all<N, BS>(J, E);
-#pragma unroll 1
-  for (int i = 0; i < N - 1; i++)
-#pragma unroll 1
-    for (int j = i + 1; j < N; j++) {
-      if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      pair_apply<N, BS>(J, E, c, i, j, rec, roff);
-      roff += PREC;
-    }
-  op_product<N, BS>(J, rec, roff, c, P);
-  roff += op_size(N);
-  add_velocity_rows<N, BS>(J, E, P);
-#pragma unroll 1
-  for (int i = N - 2; i >= 0; i--)
-#pragma unroll 1
-    for (int j = N - 1; j > i; j--) {
-      if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      pair_apply<N, BS>(J, E, c, i, j, rec, roff);
-      roff += PREC;
-    }
-  drift_rows<N, BS>(J, E, h2);
-  if (kick) {
-    op_product<N, BS>(J, rec, roff, c, P);
-    add_velocity_rows<N, BS>(J, E, P);
-  } else {
-    fold_all<N, BS>(J, E);
-  }
-}
-
-// ------------------------------------------------- groups without kick pairs
-//
-// The same updates with the Kahan pair (S, E) normalised less often: an update
+// The step's updates with the Kahan pair (S, E) normalised less often: an update
 // adds its increment to E in one FMA, J is S + E wherever it is read, and
 // (S, E) <- (S + E, (S - (S + E)) + E) follows not after every update but where
 // E holds a large increment: after the first drift (position rows), after the
@@ -198,8 +89,9 @@ __device__ void apply_step(double* J, double* E, int c, double h, uint64_t kick,
 // kernel: 4096 three-body systems over 2000 steps went from 532 to 361 ms a
 // pass, 1024 eight-body systems over 200 steps from 273 to 202 ms.
 //
-// The corrector's operator depends on position differences alone (the sum of
-// its blocks over all bodies is zero), so it is applied to J_d - J_0.
+// The corrector's and the kicks' operators depend on position differences alone
+// (the sum of their blocks over all bodies is zero), so they are applied to
+// J_d - J_0.
 //
 // MASS: the column is a mass column (c % 7 == 6); the other columns, six of
 // seven, share no warp with them and carry none of their terms.
@@ -265,11 +157,18 @@ __device__ __forceinline__ void corrector_update(const double* S, double* E, int
     }
 }
 
-// One recorded step of a kick-free group on this column.  S and E arrive and
-// leave normalised (S + E rounds to S).
-template <int N, int BS, bool MASS>
-__device__ __forceinline__ void column_step(double* S, double* E, int c, double h, const Rec& rec) {
+// One recorded step on this column (ahl21.jl:5-95, the jac_step updates).  S and
+// E arrive and leave normalised (S + E rounds to S).  The first kick's product is
+// formed before the drift and counts after it (ahl21.jl:16-23): it goes to E of
+// the velocity rows, whose S the drift reads.
+template <int N, int BS, bool MASS, bool KICK>
+__device__ __forceinline__ void column_step(double* S, double* E, int c, double h, uint64_t kick, const Rec& rec) {
   const double h2 = 0.5 * h;
+  int roff = 0;
+  if (KICK) {
+    corrector_update<N, BS, MASS>(S, E, c, rec, roff);
+    roff += op_size(N);
+  }
 #pragma unroll 2
   for (int b = 0; b < N; b++)
 #pragma unroll
@@ -280,11 +179,11 @@ __device__ __forceinline__ void column_step(double* S, double* E, int c, double 
       S[r] = s;
       E[r] = e;
     }
-  int roff = 0;
 #pragma unroll 1
   for (int i = 0; i < N - 1; i++) {
 #pragma unroll 1
     for (int j = i + 1; j < N; j++) {
+      if (KICK && ((kick >> pair_bit(i, j, N)) & 1)) continue;
       pair_update<N, BS, MASS>(S, E, c, i, j, rec, roff);
       roff += PREC;
     }
@@ -305,6 +204,7 @@ __device__ __forceinline__ void column_step(double* S, double* E, int c, double 
   for (int i = N - 2; i >= 0; i--)
 #pragma unroll 1
     for (int j = N - 1; j > i; j--) {
+      if (KICK && ((kick >> pair_bit(i, j, N)) & 1)) continue;
       pair_update<N, BS, MASS>(S, E, c, i, j, rec, roff);
       roff += PREC;
     }
@@ -323,6 +223,17 @@ __device__ __forceinline__ void column_step(double* S, double* E, int c, double 
       S[r] = s;
       E[r] = e;
     }
+  if (KICK) {
+    corrector_update<N, BS, MASS>(S, E, c, rec, roff);
+#pragma unroll 3
+    for (int q = 0; q < 3 * N; q++) {
+      const int r = (6 * (q / 3) + 3 + q % 3) * BS;
+      double sv = S[r], ev = E[r];
+      normalise(sv, ev, sv + ev);
+      S[r] = sv;
+      E[r] = ev;
+    }
+  }
 }
 
 }  // namespace nbg

@@ -42,8 +42,6 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     st.ve[q] = g.ve[q * S + s];
   }
   for (int q = 0; q < N; q++) st.m[q] = g.m[q * S + s];
-  if (KICK)
-    for (int q = 0; q < 7 * N; q++) st.dqdt[q] = g.dqdt[q * S + s];
   double gsave[N];
   long long count[N];
   for (int q = 0; q < N; q++) {
@@ -52,7 +50,7 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
   }
   const double t0 = g.t0[s], h = g.h[s], hI = g.hI[s];
   const int ntt = g.ntt[s], ti = g.ti[s];
-  const uint64_t kick = g.kick;
+  const uint64_t kick = KICK ? g.kick : 0;
   for (int kk = 0; kk < g.K; kk++) {
     const long long istep = k0 + kk;
     if (istep >= nst) break;
@@ -70,18 +68,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
       cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
       xs = Rec{g.xsnap + (size_t)kk * snap_count(KICK) * 3 * N * S + s, S};
     }
-    const bool last = g.grad && istep == nst - 1;
-    if (!KICK) {
-      if (last)  // v at the last step's start, for its dq/dt (dq_columns)
-        for (int q = 0; q < 3 * N; q++) g.dqdt[(7 * (q / 3) + 3 + q % 3) * S + s] = st.v[q];
-      plain_step<N>(st, a, hs, cap, xs);
-    } else if (last) {  // the last step also computes dq/dt, the State's output
-      Work<N> w;
-      ahl21_step<N, true, true>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
-    } else {
-      Work<N> w;
-      ahl21_step<N, false, false>(st, w, hs, kick, Rec{nullptr, 0}, cap, xs);
-    }
+    const Rec vs{g.grad && istep == nst - 1 ? g.vsnap + s : nullptr, S};
+    plain_step<N>(st, a, hs, kick, cap, xs, vs);
     if (g.notransit) continue;
     const double t = t0 + (double)(istep + 1) * h;
     for (int o = 0; o < N - 1; o++) detect_transit<N>(g, st, s, kk, o, ti, ntt, hI, t, gsave, count);
@@ -92,8 +80,6 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_chunk_kernel(G
     g.xe[q * S + s] = st.xe[q];
     g.ve[q * S + s] = st.ve[q];
   }
-  if (KICK && g.grad && nst <= k0 + g.K)  // the chunk that ran the last step holds the final dq/dt
-    for (int q = 0; q < 7 * N; q++) g.dqdt[q * S + s] = st.dqdt[q];
   for (int q = 0; q < N; q++) {
     g.gsave[q * S + s] = gsave[q];
     g.count[q * S + s] = count[q];
@@ -138,7 +124,7 @@ __device__ void search_finish(const GroupArgs& g, int s, int slot, int c, int ib
   if (g.grad) {
     wk = st;
     Rec rec{g.tscratch + lane_id, lanes};
-    ahl21_step<N, true, true>(wk, w, dt0, kick, rec, Rec{nullptr, 0}, Rec{nullptr, 0});
+    ahl21_step<N>(wk, w, dt0, kick, rec);
     double u[7 * N];
     for (int q = 0; q < 7 * N; q++) u[q] = 0.0;
     const double dvx = wk.v[3 * ib] - wk.v[3 * ti], dvy = wk.v[3 * ib + 1] - wk.v[3 * ti + 1];
@@ -226,7 +212,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kick_kernel(GroupArgs g, i
       tt2 = tt1;
       tt1 = dt0;
       wk = st;
-      ahl21_step<N, false, false>(wk, w, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
+      plain_step<N>(wk, w.a, dt0, kick, Rec{nullptr, 0}, Rec{nullptr, 0}, Rec{nullptr, 0});
       const double gs = gsky(wk, ti, ib);
       const double gd = gdot_physical(wk, ti, ib);
       const double dt = -gs / gd;
@@ -269,7 +255,7 @@ __global__ void __launch_bounds__(OPS_BS) operator_pair_kernel(GroupArgs g, int 
   const double mi = g.m[i * S + s], mj = g.m[j * S + s];
   const double h2 = 0.5 * step_length(g, s, istep, g.nsteps[s], g.h[s]);
   Rec dh{nullptr, 0};
-  if (!kick && q == slot && istep == g.nsteps[s] - 1) dh = Rec{g.dh + (size_t)slot * 6 * S + s, S};
+  if (q == slot && istep == g.nsteps[s] - 1) dh = Rec{g.dh + (size_t)slot * 6 * S + s, S};
   if (q < g.npk) pair_record_from_capture<true>(cap, q * PCAP, mi, mj, h2, rec, roff, dh);
   else pair_record_from_capture<false>(cap, q * PCAP, mi, mj, h2, rec, roff, dh);
 }
@@ -322,17 +308,17 @@ __global__ void __launch_bounds__(OPS_BS) operator_kick_kernel(GroupArgs g, int 
   Work<N> w;
   for (int q = 0; q < N; q++) st.m[q] = g.m[q * S + s];
   for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(q), st.v[q] = st.xe[q] = st.ve[q] = 0.0;
-  phic<N, true>(st, w, h, kick);
+  phic<N>(st, w, h, kick);
   phisalpha<N>(st, w.a, h, kick);
   phisalpha_operator<N>(st, w, h, kick);
   const int off_phi = op_size(N) + g.npk * PREC;
   put_op(rec, off_phi, w.op, op_size(N));
   const double h6 = h / 6.0;
   for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(3 * N + q);
-  kickfast<N, true>(st, w, h6, kick);
+  kickfast<N>(st, w, h6, kick);
   put_op(rec, 0, w.op, op_size(N));
   for (int q = 0; q < 3 * N; q++) st.x[q] = xs.get(6 * N + q);
-  kickfast<N, true>(st, w, h6, kick);
+  kickfast<N>(st, w, h6, kick);
   put_op(rec, off_phi + op_size(N) + g.npk * PREC, w.op, op_size(N));
 }
 
@@ -391,33 +377,81 @@ __device__ __forceinline__ void column_transits(const GroupArgs& g, int s, int c
 }
 
 // dq/dt of a system's last step (the State's dqdt; ahl21.jl:9-14, :20-24, :36-42
-// and so on), kick-free groups: one more column that the step's operators act
-// on, with the drift velocities, the drifts' derivative by h and the corrector's
+// and so on): one more column that the step's operators act on, with the drift
+// velocities, the drifts' derivative by h and the corrector's and the kicks'
 // dv/dt added on the way.  It is formed here, from the last step's record, and
 // not by the producers: there it made the last step a one-lane gradient step
 // (2.8 ms at eight bodies, 0.15 ms at two) and kept that step's working arrays
 // on every producer's stack.  Six lanes per system, one for each row of a body,
 // five systems a warp; sh: DQ_DOUBLES of the warp's own.
 template <int N>
-constexpr int DQ_DOUBLES = (9 * N + 3 * (N * (N - 1) / 2)) * 5;
-template <int N>
+constexpr int DQ_DOUBLES = (15 * N + 6 * (N * (N - 1) / 2)) * 5;
+template <int N, bool KICK>
 __device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh) {
   constexpr int P = N * (N - 1) / 2, C = 5;
   const int lane = threadIdx.x & 31, l = lane % 6, col = lane < 30 ? lane / 6 : 0, S = g.S;
   const int s = first + col;
+  const uint64_t kick = KICK ? g.kick : 0;
   bool live = lane < 30 && s < S && g.grad && g.sysidx[s] >= 0;
   const long long nst = live ? g.nsteps[s] : 0, k0 = live ? chunk_first_step(g, chunk, s) : 0;
   live = live && k0 >= 0 && nst > k0 && nst <= k0 + g.K;
   if (!__any_sync(0xffffffffu, live)) return;
   const int kk = live ? (int)(nst - 1 - k0) : 0, at = live ? s : 0;
-  const Rec rec{g.steprec + (size_t)kk * g.R * S + at, S}, dh{g.dh + at, S};
-  const Rec cap{g.pcap + (size_t)kk * 2 * P * PCAP * S + at, S}, xs{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + at, S};
+  const Rec rec{g.steprec + (size_t)kk * g.R * S + at, S}, dh{g.dh + at, S}, vs{g.vsnap + at, S};
+  const Rec cap{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + at, S};
+  const Rec xs{g.xsnap + (size_t)kk * snap_count(KICK) * 3 * N * S + at, S};
   const double h = live ? step_length(g, s, nst - 1, nst, g.h[s]) : 1.0, h2 = 0.5 * h;
-  double *Q = sh, *D = Q + 6 * N * C, *F = D + 3 * N * C;
+  // Q: dq/dt [6b + r]; D: position differences; A: accelerations by Kepler and
+  // by kicked pairs; F, G: a pair's force and correction
+  double *Q = sh, *D = Q + 6 * N * C, *A = D + 3 * N * C, *F = A + 6 * N * C, *G = F + 3 * P * C;
+  auto mass = [&](int b) { return g.m[b * S + s]; };
+  auto pair_at = [](int o, int b) { return o < b ? pair_bit(o, b, N) : pair_bit(b, o, N); };
+  auto is_kick = [&](int pb) { return KICK && ((kick >> pb) & 1); };
+  // G r / r^3 of every pair at the positions of snapshot `snap`, in F
+  auto forces = [&](int snap) {
+    int p = 0;
+    for (int i = 0; i < N - 1; i++)
+      for (int j = i + 1; j < N; j++, p++) {
+        if (p % 6 != l || !live) continue;
+        double rij[3], f[3];
+        for (int k = 0; k < 3; k++) rij[k] = xs.get(3 * N * snap + 3 * i + k) - xs.get(3 * N * snap + 3 * j + k);
+        phis_accel(rij, rsqrt_fast(norm2(rij)), f);
+        for (int k = 0; k < 3; k++) F[(3 * p + k) * C + col] = f[k];
+      }
+    __syncwarp();
+  };
+  // a kick over h / 6: its dv/dt and, on dq/dt, its operator at roff (the first: dq/dt is zero)
+  auto kick_rows = [&](int snap, int roff) {
+    forces(snap);
+    if (roff >= 0 && live && l < 3)
+      for (int d = 1; d < N; d++) D[(3 * d + l) * C + col] = Q[(6 * d + l) * C + col] - Q[l * C + col];
+    __syncwarp();
+    if (live)
+      for (int row = l; row < 3 * N; row += 6) {
+        const int b = row / 3, k = row % 3;
+        double acc = 0.0, op = 0.0;
+        if (roff >= 0)
+          for (int q = 0; q < 3 * (N - 1); q++)
+            acc = fma(rec.get(roff + row * (4 * N) + 4 + 4 * (q / 3) + q % 3), D[(3 + q) * C + col], acc);
+        for (int o = 0; o < N; o++)
+          if (o != b && is_kick(pair_at(o, b))) op = fma(o < b ? mass(o) : -mass(o), F[(3 * pair_at(o, b) + k) * C + col], op);
+        const int r = (6 * b + 3 + k) * C + col;
+        Q[r] = Q[r] + fma(1.0 / 6.0, op, acc);
+      }
+    __syncwarp();
+  };
   for (int b = 0; b < N; b++)
-    if (live) Q[(6 * b + l) * C + col] = l < 3 ? 0.5 * g.dqdt[(7 * b + 3 + l) * S + s] : 0.0;
+    if (live) Q[(6 * b + l) * C + col] = 0.0;
+  int roff = 0;
+  if (KICK) {
+    kick_rows(1, -1);
+    roff += op_size(N);
+  }
+  __syncwarp();
+  for (int b = 0; b < N; b++)
+    if (live && l < 3) Q[(6 * b + l) * C + col] = fma(h2, Q[(6 * b + 3 + l) * C + col], 0.5 * vs.get(3 * b + l));
   double last_i = 0.0, last_j = 0.0;
-  auto pair = [&](int i, int j, int slot, int roff) {
+  auto pair = [&](int i, int j, int slot) {
     const int ai = (6 * i + l) * C + col, aj = (6 * j + l) * C + col;
     double ti = 0.0, tj = 0.0, K[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, mi = 0.0, mj = 0.0, by_h = 0.0;
     bool stale = false;
@@ -444,39 +478,63 @@ __device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh)
       Q[aj] = last_j;
     }
   };
-  int slot = 0, roff = 0;
+  int slot = 0;
   for (int i = 0; i < N - 1; i++)
-    for (int j = i + 1; j < N; j++, roff += PREC) pair(i, j, slot++, roff);
+    for (int j = i + 1; j < N; j++)
+      if (!is_kick(pair_bit(i, j, N))) {
+        pair(i, j, slot++);
+        roff += PREC;
+      }
+  __syncwarp();
+  if (live && l < 3)
+    for (int d = 1; d < N; d++) D[(3 * d + l) * C + col] = Q[(6 * d + l) * C + col] - Q[l * C + col];
+  forces(0);
+  if (live)
+    for (int row = l; row < 3 * N; row += 6) {  // accelerations, as the producer sums them
+      const int b = row / 3, k = row % 3;
+      double a = 0.0, ac = 0.0;
+      for (int o = 0; o < N; o++)
+        if (o != b) {
+          const double f = F[(3 * pair_at(o, b) + k) * C + col], m = o < b ? mass(o) : -mass(o);
+          if (is_kick(pair_at(o, b))) ac = fma(m, f, ac);
+          else a = fma(m, f, a);
+        }
+      A[row * C + col] = a;
+      A[(3 * N + row) * C + col] = ac;
+    }
   __syncwarp();
   if (live) {
-    if (l < 3)
-      for (int d = 1; d < N; d++) D[(3 * d + l) * C + col] = Q[(6 * d + l) * C + col] - Q[l * C + col];
     int p = 0;
     for (int i = 0; i < N - 1; i++)
       for (int j = i + 1; j < N; j++, p++) {
         if (p % 6 != l) continue;
+        const double* a = A + (is_kick(p) ? 3 * N * C : 0) + col;
         double rij[3], aij[3], f[3];
         for (int k = 0; k < 3; k++) {
           rij[k] = xs.get(3 * i + k) - xs.get(3 * j + k);
-          aij[k] = xs.get(3 * N + 3 * i + k) - xs.get(3 * N + 3 * j + k);
+          aij[k] = a[(3 * i + k) * C] - a[(3 * j + k) * C];
         }
         const double r2 = norm2(rij);
-        phis_corr(rij, r2, rsqrt_fast(r2), aij, g.m[i * S + s] + g.m[j * S + s], phis_coeff(h), f);
-        for (int k = 0; k < 3; k++) F[(3 * p + k) * C + col] = f[k];
+        phis_corr(rij, r2, rsqrt_fast(r2), aij, is_kick(p) ? 0.0 : mass(i) + mass(j),
+                  is_kick(p) ? phic_coeff(h) : phis_coeff(h), f);
+        for (int k = 0; k < 3; k++) G[(3 * p + k) * C + col] = f[k];
       }
   }
   __syncwarp();
   if (live) {
-    const double hi3 = 3.0 / h;  // the correction goes with h^3
+    const double hi3 = 3.0 / h;  // the corrections go with h^3, phic!'s kick with 2h / 3
     for (int row = l; row < 3 * N; row += 6) {
       const int b = row / 3, k = row % 3;
-      double acc = 0.0, op = 0.0;
+      double acc = 0.0, op = 0.0, kv = 0.0;
       for (int q = 0; q < 3 * (N - 1); q++)
         acc = fma(rec.get(roff + row * (4 * N) + 4 + 4 * (q / 3) + q % 3), D[(3 + q) * C + col], acc);
       for (int o = 0; o < N; o++)
-        if (o != b)
-          op = fma(o < b ? -g.m[o * S + s] : g.m[o * S + s],
-                   F[(3 * (o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)) + k) * C + col], op);
+        if (o != b) {
+          const int at3 = (3 * pair_at(o, b) + k) * C + col;
+          op = fma(o < b ? -mass(o) : mass(o), G[at3], op);
+          if (is_kick(pair_at(o, b))) kv = fma(o < b ? mass(o) : -mass(o), F[at3], kv);
+        }
+      if (KICK) acc = fma(2.0 / 3.0, kv, acc);
       const int r = (6 * b + 3 + k) * C + col;
       Q[r] = Q[r] + fma(hi3, op, acc);
     }
@@ -484,22 +542,31 @@ __device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh)
   __syncwarp();
   roff += op_size(N);
   for (int i = N - 2; i >= 0; i--)
-    for (int j = N - 1; j > i; j--, roff += PREC) pair(i, j, slot++, roff);
+    for (int j = N - 1; j > i; j--)
+      if (!is_kick(pair_bit(i, j, N))) {
+        pair(i, j, slot++);
+        roff += PREC;
+      }
   __syncwarp();
+  if (live && l < 3)
+    for (int b = 0; b < N; b++) {
+      const int r = (6 * b + l) * C + col;
+      Q[r] = Q[r] + fma(h2, Q[r + 3 * C], 0.5 * vs.get(3 * N + 3 * b + l));
+    }
+  __syncwarp();
+  if (KICK) kick_rows(2, roff);
   if (live)
     for (int b = 0; b < N; b++) {
-      double q = Q[(6 * b + l) * C + col];
-      if (l < 3) q = q + fma(h2, Q[(6 * b + 3 + l) * C + col], 0.5 * g.v[(3 * b + l) * S + s]);
-      g.dqdt[(7 * b + l) * S + s] = q;
+      g.dqdt[(7 * b + l) * S + s] = Q[(6 * b + l) * C + col];
       if (l == 0) g.dqdt[(7 * b + 6) * S + s] = 0.0;
     }
 }
 
-// Jacobian consumer for one chunk of K steps (one lane per column).  A group
-// without kick pairs has its mass columns in blocks of their own: the first
-// `plain` blocks hold the other 6N columns of every system, the next ones, up
-// to `all`, the N mass columns; the last ones form dq/dt.
-template <int N, int BS, int MODE>  // 0: kick group, every column; 1: not a mass column; 2: a mass column
+// Jacobian consumer for one chunk of K steps (one lane per column).  The mass
+// columns have blocks of their own: the first `plain` blocks hold the other 6N
+// columns of every system, the next ones, up to `all`, the N mass columns; the
+// last ones form dq/dt.
+template <int N, int BS, bool MASS, bool KICK>
 __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int s, int c, double* smem) {
   constexpr int M = 7 * N, R6 = 6 * N;
   if (s >= g.S || g.sysidx[s] < 0) return;
@@ -513,7 +580,7 @@ __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int
   double* Eg = g.Eint + (size_t)s * R6 * M + c;
   for (int r = 0; r < R6; r++) {
     double jv = Jg[(size_t)r * M], ev = Eg[(size_t)r * M];
-    if (MODE != 0 && k0 == 0) fold(jv, ev);  // a caller's pair may not be normalised
+    if (k0 == 0) fold(jv, ev);  // a caller's pair may not be normalised
     J[r * BS] = jv;
     E[r * BS] = ev;
   }
@@ -529,8 +596,7 @@ __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int
       for (int r = 0; r < M; r++) rj[r] = (r % 7 == 6) ? ((r == c) ? 1.0 : 0.0) : J[(6 * (r / 7) + r % 7) * BS];
     }
     const double hs = step_length(g, s, istep, nst, h);
-    if (MODE == 0) apply_step<N, BS>(J, E, c, hs, g.kick, rec);
-    else column_step<N, BS, MODE == 2>(J, E, c, hs, rec);
+    column_step<N, BS, MASS, KICK>(J, E, c, hs, KICK ? g.kick : 0, rec);
     if (!g.notransit) column_transits<N, BS>(g, s, c, kk, ti, ntt, gsys, J, E);
   }
   bool finite = true;
@@ -544,29 +610,21 @@ __device__ __forceinline__ void consume_chunk(const GroupArgs& g, int chunk, int
 
 // 168 registers a thread at most: three blocks of four warps fit an SM and leave
 // room for a producer or search warp beside them.
-template <int N>
+template <int N, bool KICK>
 __global__ void __launch_bounds__(cons_bs(N), 3 * 128 / cons_bs(N)) jacobian_chunk_kernel(GroupArgs g, int chunk, int plain, int all) {
   extern __shared__ double smem[];
   constexpr int BS = cons_bs(N);
   if ((int)blockIdx.x < plain) {
     const int f = blockIdx.x * BS + threadIdx.x, q = f % (6 * N);
-    consume_chunk<N, BS, 1>(g, chunk, f / (6 * N), 7 * (q / 6) + q % 6, smem);
+    consume_chunk<N, BS, false, KICK>(g, chunk, f / (6 * N), 7 * (q / 6) + q % 6, smem);
   } else if ((int)blockIdx.x < all) {
     const int f = (blockIdx.x - plain) * BS + threadIdx.x;
-    consume_chunk<N, BS, 2>(g, chunk, f / N, 7 * (f % N) + 6, smem);
+    consume_chunk<N, BS, true, KICK>(g, chunk, f / N, 7 * (f % N) + 6, smem);
   } else {
     static_assert(DQ_DOUBLES<N> * (BS / 32) <= 2 * 6 * N * BS, "dq_columns' share of the columns' shared memory");
     const int w = (blockIdx.x - all) * (BS / 32) + threadIdx.x / 32;
-    dq_columns<N>(g, chunk, 5 * w, smem + DQ_DOUBLES<N> * (threadIdx.x / 32));
+    dq_columns<N, KICK>(g, chunk, 5 * w, smem + DQ_DOUBLES<N> * (threadIdx.x / 32));
   }
-}
-
-template <int N>
-__global__ void __launch_bounds__(cons_bs(N)) jacobian_kick_kernel(GroupArgs g, int chunk) {
-  extern __shared__ double smem[];
-  constexpr int BS = cons_bs(N), M = 7 * N;
-  const int f = blockIdx.x * BS + threadIdx.x;
-  consume_chunk<N, BS, 0>(g, chunk, f / M, f % M, smem);
 }
 
 // Jacobian consumer for latency-bound chunks (the orbit producer's lanes form
@@ -587,11 +645,13 @@ __global__ void __launch_bounds__(cons_bs(N)) jacobian_kick_kernel(GroupArgs g, 
 constexpr int ROWS_COLS = 5, ROWS_WARPS = 2;
 __host__ __device__ constexpr int rows_plain_warps(int N) { return (6 * N + ROWS_COLS - 1) / ROWS_COLS; }
 __host__ __device__ constexpr int rows_warps(int N) { return rows_plain_warps(N) + (N + ROWS_COLS - 1) / ROWS_COLS; }
-__host__ __device__ constexpr int rows_record(int N) { return N * (N - 1) * PREC + op_size(N); }
+__host__ __device__ constexpr int rows_record(int N, bool kick) {  // at most
+  return N * (N - 1) * PREC + (kick ? 3 : 1) * op_size(N);
+}
 __host__ __device__ constexpr int rows_blocks(int N) { return (rows_warps(N) + ROWS_WARPS - 1) / ROWS_WARPS; }
-template <int N>
+template <int N, bool KICK>
 struct RowsShared {
-  double rec[2][rows_record(N)];
+  double rec[2][rows_record(N, KICK)];
   double S[ROWS_WARPS][6 * N * ROWS_COLS], E[ROWS_WARPS][6 * N * ROWS_COLS], D[ROWS_WARPS][3 * N * ROWS_COLS];
   int flag[2][N];
 };
@@ -622,41 +682,11 @@ __device__ __forceinline__ void rows_pair(double* Sw, double* Ew, const double* 
   }
 }
 
-// column_step on the warp's five columns.
+// corrector_update on the warp's columns: velocity rows of an operator that acts
+// on position differences.
 template <int N, bool MASS>
-__device__ __forceinline__ void rows_step(double* Sw, double* Ew, double* Dw, const double* rec, int c, double h, int l,
-                                          int col, bool live) {
-  const double h2 = 0.5 * h;
-  const int cm = c / 7;
-  if (live && l < 3) {
-#pragma unroll
-    for (int b = 0; b < N; b++) {
-      const int r = (6 * b + l) * ROWS_COLS + col;
-      double s = Sw[r], e = fma(h2, Sw[r + 3 * ROWS_COLS], Ew[r]);
-      normalise(s, e, s + e);
-      Sw[r] = s;
-      Ew[r] = e;
-    }
-  }
-  __syncwarp();
-  const double* rc = rec;
-#pragma unroll 1
-  for (int i = 0; i < N - 1; i++) {
-#pragma unroll 1
-    for (int j = i + 1; j < N; j++, rc += PREC)
-      rows_pair<N, MASS>(Sw, Ew, rc, i, j, cm == i, cm == j, l, col, live);
-    if (N > 2 && i == 0 && live && l >= 3) {
-#pragma unroll
-      for (int b = 0; b < N; b++) {
-        const int r = (6 * b + l) * ROWS_COLS + col;
-        double s = Sw[r], e = Ew[r];
-        normalise(s, e, s + e);
-        Sw[r] = s;
-        Ew[r] = e;
-      }
-    }
-    __syncwarp();
-  }
+__device__ __forceinline__ void rows_operator(const double* Sw, double* Ew, double* Dw, const double* rc, int cm, int l,
+                                              int col, bool live) {
   if (live && l < 3) {
     const double t0 = Sw[l * ROWS_COLS + col] + Ew[l * ROWS_COLS + col];
 #pragma unroll
@@ -677,12 +707,60 @@ __device__ __forceinline__ void rows_step(double* Sw, double* Ew, double* Dw, co
     if (live) Ew[r] = Ew[r] + acc;
   }
   __syncwarp();
+}
+
+// column_step on the warp's five columns.
+template <int N, bool MASS, bool KICK>
+__device__ __forceinline__ void rows_step(double* Sw, double* Ew, double* Dw, const double* rec, int c, double h,
+                                          uint64_t kick, int l, int col, bool live) {
+  const double h2 = 0.5 * h;
+  const int cm = c / 7;
+  const double* rc = rec;
+  if (KICK) {
+    rows_operator<N, MASS>(Sw, Ew, Dw, rc, cm, l, col, live);
+    rc += op_size(N);
+  }
+  if (live && l < 3) {
+#pragma unroll
+    for (int b = 0; b < N; b++) {
+      const int r = (6 * b + l) * ROWS_COLS + col;
+      double s = Sw[r], e = fma(h2, Sw[r + 3 * ROWS_COLS], Ew[r]);
+      normalise(s, e, s + e);
+      Sw[r] = s;
+      Ew[r] = e;
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int i = 0; i < N - 1; i++) {
+#pragma unroll 1
+    for (int j = i + 1; j < N; j++) {
+      if (KICK && ((kick >> pair_bit(i, j, N)) & 1)) continue;
+      rows_pair<N, MASS>(Sw, Ew, rc, i, j, cm == i, cm == j, l, col, live);
+      rc += PREC;
+    }
+    if (N > 2 && i == 0 && live && l >= 3) {
+#pragma unroll
+      for (int b = 0; b < N; b++) {
+        const int r = (6 * b + l) * ROWS_COLS + col;
+        double s = Sw[r], e = Ew[r];
+        normalise(s, e, s + e);
+        Sw[r] = s;
+        Ew[r] = e;
+      }
+    }
+    __syncwarp();
+  }
+  rows_operator<N, MASS>(Sw, Ew, Dw, rc, cm, l, col, live);
   rc += op_size(N);
 #pragma unroll 1
   for (int i = N - 2; i >= 0; i--)
 #pragma unroll 1
-    for (int j = N - 1; j > i; j--, rc += PREC)
+    for (int j = N - 1; j > i; j--) {
+      if (KICK && ((kick >> pair_bit(i, j, N)) & 1)) continue;
       rows_pair<N, MASS>(Sw, Ew, rc, i, j, cm == i, cm == j, l, col, live);
+      rc += PREC;
+    }
 #pragma unroll
   for (int b = 0; b < N; b++) {
     const int r = (6 * b + l) * ROWS_COLS + col;
@@ -699,19 +777,32 @@ __device__ __forceinline__ void rows_step(double* Sw, double* Ew, double* Dw, co
     }
   }
   __syncwarp();
+  if (KICK) {
+    rows_operator<N, MASS>(Sw, Ew, Dw, rc, cm, l, col, live);
+    if (live && l >= 3)
+      for (int b = 0; b < N; b++) {
+        const int r = (6 * b + l) * ROWS_COLS + col;
+        double s = Sw[r], e = Ew[r];
+        normalise(s, e, s + e);
+        Sw[r] = s;
+        Ew[r] = e;
+      }
+    __syncwarp();
+  }
 }
 
-template <int N>
+template <int N, bool KICK>
 __global__ void __launch_bounds__(32 * ROWS_WARPS) jacobian_rows_kernel(GroupArgs g, int chunk) {
   extern __shared__ double smem[];
-  RowsShared<N>& sh = *reinterpret_cast<RowsShared<N>*>(smem);
-  constexpr int M = 7 * N, R6 = 6 * N, R = rows_record(N);
+  RowsShared<N, KICK>& sh = *reinterpret_cast<RowsShared<N, KICK>*>(smem);
+  constexpr int M = 7 * N, R6 = 6 * N;
   const int s = blockIdx.x, S = g.S, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if ((int)blockIdx.y == rows_blocks(N)) {  // the last row of blocks forms dq/dt
-    dq_columns<N>(g, chunk, 5 * (ROWS_WARPS * s + warp), smem + DQ_DOUBLES<N> * warp);
+    dq_columns<N, KICK>(g, chunk, 5 * (ROWS_WARPS * s + warp), smem + DQ_DOUBLES<N> * warp);
     return;
   }
   if (s >= S || g.sysidx[s] < 0) return;
+  const int R = KICK ? g.R : rows_record(N, false);  // a kick group's record is shorter by its kicked pairs
   const long long nst = g.nsteps[s], k0 = chunk_first_step(g, chunk, s);
   if (k0 >= nst || k0 < 0) return;  // done, or admitted for a later chunk
   const int nk = (int)(nst - k0 < g.K ? nst - k0 : g.K);
@@ -758,8 +849,8 @@ __global__ void __launch_bounds__(32 * ROWS_WARPS) jacobian_rows_kernel(GroupArg
       }
     }
     const double hs = step_length(g, s, k0 + kk, nst, h);
-    if (mass) rows_step<N, true>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, l, col, live);
-    else rows_step<N, false>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, l, col, live);
+    if (mass) rows_step<N, true, KICK>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, g.kick, l, col, live);
+    else rows_step<N, false, KICK>(Sw, Ew, Dw, sh.rec[kk & 1], c, hs, g.kick, l, col, live);
     if (!g.notransit)
       for (int o = 0; o < N - 1; o++) {
         const int flag = sh.flag[kk & 1][o];
@@ -819,6 +910,14 @@ inline void allow_smem(K kernel, int bytes) {
   if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
+template <int N, bool KICK>
+void launch_lanes(const GroupArgs& g, int chunk, cudaStream_t st) {
+  const int smem = std::max(lanes_systems(N) * (int)sizeof(LanesShared<N>), g.prod_smem);
+  allow_smem(orbit_lanes_kernel<N, KICK>, smem);
+  orbit_lanes_kernel<N, KICK>
+      <<<(g.S + lanes_systems(N) - 1) / lanes_systems(N), 32 * lanes_warps(N), smem, st>>>(g, chunk);
+}
+
 template <int N>
 int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   // Without a layout of the caller's (nbg_set_producer_layout) a full group's
@@ -827,10 +926,9 @@ int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   // (4096 three-body systems over 512 steps: 94.5 -> 87.7 ms; two and four
   // bodies within 1 %).
   const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.S >= 2048) ? 2 : 1;
-  if (g.wide && !g.kick) {
-    const int smem = std::max(lanes_systems(N) * (int)sizeof(LanesShared<N>), g.prod_smem);
-    allow_smem(orbit_lanes_kernel<N>, smem);
-    orbit_lanes_kernel<N><<<(g.S + lanes_systems(N) - 1) / lanes_systems(N), 32 * lanes_warps(N), smem, st>>>(g, chunk);
+  if (g.wide) {
+    if (g.kick) launch_lanes<N, true>(g, chunk, st);
+    else launch_lanes<N, false>(g, chunk, st);
     return 0;
   }
   if (g.team && !g.kick) {
@@ -851,28 +949,32 @@ int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   return 0;
 }
 
-template <int N>
-int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
+template <int N, bool KICK>
+void launch_consumer(const GroupArgs& g, int chunk, cudaStream_t st) {
+  // the attributes are set per call: they belong to the current device
+  if (g.rows) {
+    // as every consumer block: none fits beside a tail producer's
+    const int bytes = std::max((int)sizeof(RowsShared<N, KICK>), 24 * 1024);
+    static_assert(sizeof(double) * DQ_DOUBLES<N> * ROWS_WARPS <= std::max<size_t>(sizeof(RowsShared<N, KICK>), 24 * 1024),
+                  "dq_columns fits");
+    allow_smem(jacobian_rows_kernel<N, KICK>, bytes);
+    const dim3 grid(g.S, rows_blocks(N) + 1);
+    jacobian_rows_kernel<N, KICK><<<grid, 32 * ROWS_WARPS, bytes, st>>>(g, chunk);
+    return;
+  }
   constexpr int BS = cons_bs(N);
   const int smem = 2 * 6 * N * BS * (int)sizeof(double);
   auto blocks = [](long long columns) { return (int)((columns + BS - 1) / BS); };
-  if (g.kick) {
-    allow_smem(jacobian_kick_kernel<N>, smem);  // per call: the attribute belongs to the current device
-    jacobian_kick_kernel<N><<<blocks((long long)g.S * 7 * N), BS, smem, st>>>(g, chunk);
-    return 0;
-  }
-  if (g.rows) {
-    const int bytes = std::max((int)sizeof(RowsShared<N>), 24 * 1024);  // as every consumer block: none fits beside a tail producer's
-    allow_smem(jacobian_rows_kernel<N>, bytes);
-    static_assert(sizeof(double) * DQ_DOUBLES<N> * ROWS_WARPS <= sizeof(RowsShared<N>) || N <= 2, "dq_columns fits");
-    const dim3 grid(g.S, rows_blocks(N) + 1);
-    jacobian_rows_kernel<N><<<grid, 32 * ROWS_WARPS, bytes, st>>>(g, chunk);
-    return 0;
-  }
-  const int plain = blocks((long long)g.S * 6 * N);
-  allow_smem(jacobian_chunk_kernel<N>, smem);
-  const int all = plain + blocks((long long)g.S * N), dq = (g.S + 5 * (BS / 32) - 1) / (5 * (BS / 32));
-  jacobian_chunk_kernel<N><<<all + dq, BS, smem, st>>>(g, chunk, plain, all);
+  const int plain = blocks((long long)g.S * 6 * N), all = plain + blocks((long long)g.S * N);
+  const int dq = (g.S + 5 * (BS / 32) - 1) / (5 * (BS / 32));
+  allow_smem(jacobian_chunk_kernel<N, KICK>, smem);
+  jacobian_chunk_kernel<N, KICK><<<all + dq, BS, smem, st>>>(g, chunk, plain, all);
+}
+
+template <int N>
+int launch_jac(const GroupArgs& g, int chunk, cudaStream_t st) {
+  if (g.kick) launch_consumer<N, true>(g, chunk, st);
+  else launch_consumer<N, false>(g, chunk, st);
   return 0;
 }
 

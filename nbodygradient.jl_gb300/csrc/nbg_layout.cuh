@@ -56,8 +56,7 @@ __host__ __device__ inline int trec_size(int N, int tbv) { return tbv ? 21 * N +
 __host__ __device__ inline int snap_count(bool kick) { return kick ? 3 : 2; }
 
 
-// Up to how many running systems of a kick-free group the latency-bound forms
-// are taken.  A lanes-form level costs its warp one system's pairs where the
+// Up to how many running systems of a group the latency-bound forms are taken.  A lanes-form level costs its warp one system's pairs where the
 // one-lane and team forms carry 32 or 32 / (N/2) systems, so the line is where
 // the pairs' levels, (2N - 3) per system, fill the SMs' FP64 pipes.  Measured,
 // us a step, (one lane or team) -> lanes, rows consumer with up to four bodies:
@@ -85,8 +84,8 @@ struct GroupArgs {
   // so that the searches are latency-bound; a full group keeps one lane per
   // search, which uses every lane of every warp
   int search_lanes;
-  // forms for latency-bound chunks (few systems running) of a group without
-  // kick pairs, set by the host per chunk: the orbit producer's lanes form
+  // forms for latency-bound chunks (few systems running), set by the host per
+  // chunk: the orbit producer's lanes form
   // (orbit_lanes_kernel) and the Jacobian consumer's rows form
   // (jacobian_rows_kernel)
   int wide, rows;
@@ -138,9 +137,9 @@ struct GroupArgs {
   // producer captures for the operator kernels
   double* pcap;   // [K][2 npk][18][S]: Kepler-pair parameters
   double* xsnap;  // [K][snaps][3N][S]: see snap_count
-  // d(delxv)/dh of a system's last step, for its dq/dt: [2 npk][6][S] (groups
-  // without kick pairs)
+  // d(delxv)/dh of a system's last step, for its dq/dt: [2 npk][6][S]
   double* dh;
+  double* vsnap;  // [2][3N][S]: v at the two drifts of a system's last step, for its dq/dt
 };
 
 // Length of step istep of the system in slot s (nst steps in all).

@@ -83,12 +83,10 @@ __device__ __forceinline__ void drift(Sys<N>& s, double h) {
 }
 
 // kickfast! (ahl21.jl:337-386 / ahl21_no_grad.jl:35-56)
-template <int N, bool GRADOPS>
+template <int N>
 __device__ void kickfast(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
-  if (GRADOPS) {
-    for (int q = 0; q < 12 * N * N; q++) w.op[q] = 0.0;
-    for (int q = 0; q < 3 * N; q++) w.dqop[q] = 0.0;
-  }
+  for (int q = 0; q < 12 * N * N; q++) w.op[q] = 0.0;
+  for (int q = 0; q < 3 * N; q++) w.dqop[q] = 0.0;
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++) {
       if (!((kick >> pair_bit(i, j, N)) & 1)) continue;
@@ -101,23 +99,21 @@ __device__ void kickfast(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
         double fac = fac2 * rij[k];
         kahan(s.v[3 * i + k], s.ve[3 * i + k], (-s.m[j]) * fac);
         kahan(s.v[3 * j + k], s.ve[3 * j + k], s.m[i] * fac);
-        if (GRADOPS) {
-          w.dqop[3 * i + k] = w.dqop[3 * i + k] - s.m[j] * fac / h;
-          w.dqop[3 * j + k] = w.dqop[3 * j + k] + s.m[i] * fac / h;
-          OPX(3 * i + k, 4 * j + 3) -= fac;
-          OPX(3 * j + k, 4 * i + 3) += fac;
-          fac = fac * (3.0 * r2inv);
-          for (int p = 0; p < 3; p++) {
-            OPX(3 * i + k, 4 * i + p) += fac * s.m[j] * rij[p];
-            OPX(3 * i + k, 4 * j + p) -= fac * s.m[j] * rij[p];
-            OPX(3 * j + k, 4 * j + p) += fac * s.m[i] * rij[p];
-            OPX(3 * j + k, 4 * i + p) -= fac * s.m[i] * rij[p];
-          }
-          OPX(3 * i + k, 4 * i + k) -= fac2 * s.m[j];
-          OPX(3 * i + k, 4 * j + k) += fac2 * s.m[j];
-          OPX(3 * j + k, 4 * j + k) -= fac2 * s.m[i];
-          OPX(3 * j + k, 4 * i + k) += fac2 * s.m[i];
+        w.dqop[3 * i + k] = w.dqop[3 * i + k] - s.m[j] * fac / h;
+        w.dqop[3 * j + k] = w.dqop[3 * j + k] + s.m[i] * fac / h;
+        OPX(3 * i + k, 4 * j + 3) -= fac;
+        OPX(3 * j + k, 4 * i + 3) += fac;
+        fac = fac * (3.0 * r2inv);
+        for (int p = 0; p < 3; p++) {
+          OPX(3 * i + k, 4 * i + p) += fac * s.m[j] * rij[p];
+          OPX(3 * i + k, 4 * j + p) -= fac * s.m[j] * rij[p];
+          OPX(3 * j + k, 4 * j + p) += fac * s.m[i] * rij[p];
+          OPX(3 * j + k, 4 * i + p) -= fac * s.m[i] * rij[p];
         }
+        OPX(3 * i + k, 4 * i + k) -= fac2 * s.m[j];
+        OPX(3 * i + k, 4 * j + k) += fac2 * s.m[j];
+        OPX(3 * j + k, 4 * j + k) -= fac2 * s.m[i];
+        OPX(3 * j + k, 4 * i + k) += fac2 * s.m[i];
       }
     }
 }
@@ -144,13 +140,11 @@ __device__ __forceinline__ void put_op(const Rec& rec, int off, const double* op
 }
 
 // phic! (ahl21.jl:392-552 / ahl21_no_grad.jl:62-104): corrector for kick pairs
-template <int N, bool GRADOPS>
+template <int N>
 __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
   for (int q = 0; q < 3 * N; q++) w.a[q] = 0.0;
-  if (GRADOPS) {
-    for (int q = 0; q < 12 * N * N; q++) { w.dadq[q] = 0.0; w.op[q] = 0.0; }
-    for (int q = 0; q < 3 * N; q++) w.dqop[q] = 0.0;
-  }
+  for (int q = 0; q < 12 * N * N; q++) { w.dadq[q] = 0.0; w.op[q] = 0.0; }
+  for (int q = 0; q < 3 * N; q++) w.dqop[q] = 0.0;
   if (!kick) return;
   double coeff = h * h * h / 36.0 * GNEWT;
   for (int i = 0; i < N - 1; i++)
@@ -167,38 +161,36 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
         kahan(s.v[3 * j + k], s.ve[3 * j + k], s.m[i] * facv);
         w.a[3 * i + k] = w.a[3 * i + k] - s.m[j] * fac;
         w.a[3 * j + k] = w.a[3 * j + k] + s.m[i] * fac;
-        if (GRADOPS) {
-          w.dqop[3 * i + k] = w.dqop[3 * i + k] - 1.0 / h * s.m[j] * facv;
-          w.dqop[3 * j + k] = w.dqop[3 * j + k] + 1.0 / h * s.m[i] * facv;
-          OPX(3 * i + k, 4 * j + 3) -= facv;
-          OPX(3 * j + k, 4 * i + 3) += facv;
-          facv = facv * (3.0 * r2inv);
-          for (int p = 0; p < 3; p++) {
-            OPX(3 * i + k, 4 * i + p) += facv * s.m[j] * rij[p];
-            OPX(3 * i + k, 4 * j + p) -= facv * s.m[j] * rij[p];
-            OPX(3 * j + k, 4 * j + p) += facv * s.m[i] * rij[p];
-            OPX(3 * j + k, 4 * i + p) -= facv * s.m[i] * rij[p];
-          }
-          facv = 2.0 * h / 3.0 * GNEWT * r3inv;
-          OPX(3 * i + k, 4 * i + k) -= facv * s.m[j];
-          OPX(3 * i + k, 4 * j + k) += facv * s.m[j];
-          OPX(3 * j + k, 4 * j + k) -= facv * s.m[i];
-          OPX(3 * j + k, 4 * i + k) += facv * s.m[i];
-          DAX(3 * i + k, 4 * j + 3) -= fac;
-          DAX(3 * j + k, 4 * i + 3) += fac;
-          fac = fac * (3.0 * r2inv);
-          for (int p = 0; p < 3; p++) {
-            DAX(3 * i + k, 4 * i + p) += fac * s.m[j] * rij[p];
-            DAX(3 * i + k, 4 * j + p) -= fac * s.m[j] * rij[p];
-            DAX(3 * j + k, 4 * j + p) += fac * s.m[i] * rij[p];
-            DAX(3 * j + k, 4 * i + p) -= fac * s.m[i] * rij[p];
-          }
-          fac = GNEWT * r3inv;
-          DAX(3 * i + k, 4 * i + k) -= fac * s.m[j];
-          DAX(3 * i + k, 4 * j + k) += fac * s.m[j];
-          DAX(3 * j + k, 4 * j + k) -= fac * s.m[i];
-          DAX(3 * j + k, 4 * i + k) += fac * s.m[i];
+        w.dqop[3 * i + k] = w.dqop[3 * i + k] - 1.0 / h * s.m[j] * facv;
+        w.dqop[3 * j + k] = w.dqop[3 * j + k] + 1.0 / h * s.m[i] * facv;
+        OPX(3 * i + k, 4 * j + 3) -= facv;
+        OPX(3 * j + k, 4 * i + 3) += facv;
+        facv = facv * (3.0 * r2inv);
+        for (int p = 0; p < 3; p++) {
+          OPX(3 * i + k, 4 * i + p) += facv * s.m[j] * rij[p];
+          OPX(3 * i + k, 4 * j + p) -= facv * s.m[j] * rij[p];
+          OPX(3 * j + k, 4 * j + p) += facv * s.m[i] * rij[p];
+          OPX(3 * j + k, 4 * i + p) -= facv * s.m[i] * rij[p];
         }
+        facv = 2.0 * h / 3.0 * GNEWT * r3inv;
+        OPX(3 * i + k, 4 * i + k) -= facv * s.m[j];
+        OPX(3 * i + k, 4 * j + k) += facv * s.m[j];
+        OPX(3 * j + k, 4 * j + k) -= facv * s.m[i];
+        OPX(3 * j + k, 4 * i + k) += facv * s.m[i];
+        DAX(3 * i + k, 4 * j + 3) -= fac;
+        DAX(3 * j + k, 4 * i + 3) += fac;
+        fac = fac * (3.0 * r2inv);
+        for (int p = 0; p < 3; p++) {
+          DAX(3 * i + k, 4 * i + p) += fac * s.m[j] * rij[p];
+          DAX(3 * i + k, 4 * j + p) -= fac * s.m[j] * rij[p];
+          DAX(3 * j + k, 4 * j + p) += fac * s.m[i] * rij[p];
+          DAX(3 * j + k, 4 * i + p) -= fac * s.m[i] * rij[p];
+        }
+        fac = GNEWT * r3inv;
+        DAX(3 * i + k, 4 * i + k) -= fac * s.m[j];
+        DAX(3 * i + k, 4 * j + k) += fac * s.m[j];
+        DAX(3 * j + k, 4 * j + k) -= fac * s.m[i];
+        DAX(3 * j + k, 4 * i + k) += fac * s.m[i];
       }
     }
   for (int i = 0; i < N - 1; i++)
@@ -209,13 +201,11 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
         aij[k] = w.a[3 * i + k] - w.a[3 * j + k];
         rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
       }
-      if (GRADOPS) {
-        for (int q = 0; q < 4 * N; q++) w.dot[q] = 0.0;
-        for (int di = 0; di < N; di++)
-          for (int p = 0; p < 4; p++)
-            for (int k = 0; k < 3; k++)
-              w.dot[4 * di + p] += rij[k] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-      }
+      for (int q = 0; q < 4 * N; q++) w.dot[q] = 0.0;
+      for (int di = 0; di < N; di++)
+        for (int p = 0; p < 4; p++)
+          for (int k = 0; k < 3; k++)
+            w.dot[4 * di + p] += rij[k] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
       double r2 = rij[0] * rij[0] + rij[1] * rij[1] + rij[2] * rij[2];
       double r1 = sqrt(r2);
       double ardot = aij[0] * rij[0] + aij[1] * rij[1] + aij[2] * rij[2];
@@ -225,49 +215,47 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
         double fac = fac1 * (rij[k] * fac2 - r2 * aij[k]);
         kahan(s.v[3 * i + k], s.ve[3 * i + k], s.m[j] * fac);
         kahan(s.v[3 * j + k], s.ve[3 * j + k], (-s.m[i]) * fac);
-        if (GRADOPS) {
-          w.dqop[3 * i + k] = w.dqop[3 * i + k] + 3.0 / h * s.m[j] * fac;
-          w.dqop[3 * j + k] = w.dqop[3 * j + k] - 3.0 / h * s.m[i] * fac;
-          OPX(3 * i + k, 4 * j + 3) += fac;
-          OPX(3 * j + k, 4 * i + 3) -= fac;
-          fac = fac * (5.0 / r2);
+        w.dqop[3 * i + k] = w.dqop[3 * i + k] + 3.0 / h * s.m[j] * fac;
+        w.dqop[3 * j + k] = w.dqop[3 * j + k] - 3.0 / h * s.m[i] * fac;
+        OPX(3 * i + k, 4 * j + 3) += fac;
+        OPX(3 * j + k, 4 * i + 3) -= fac;
+        fac = fac * (5.0 / r2);
+        for (int p = 0; p < 3; p++) {
+          OPX(3 * i + k, 4 * i + p) -= fac * s.m[j] * rij[p];
+          OPX(3 * i + k, 4 * j + p) += fac * s.m[j] * rij[p];
+          OPX(3 * j + k, 4 * j + p) -= fac * s.m[i] * rij[p];
+          OPX(3 * j + k, 4 * i + p) += fac * s.m[i] * rij[p];
+        }
+        fac = fac1 * fac2;
+        OPX(3 * i + k, 4 * i + k) += fac * s.m[j];
+        OPX(3 * i + k, 4 * j + k) -= fac * s.m[j];
+        OPX(3 * j + k, 4 * j + k) += fac * s.m[i];
+        OPX(3 * j + k, 4 * i + k) -= fac * s.m[i];
+        fac = -2.0 * fac1 * aij[k];
+        for (int p = 0; p < 3; p++) {
+          double fac3 = fac * rij[p] + fac1 * 3.0 * rij[k] * aij[p];
+          OPX(3 * i + k, 4 * i + p) += s.m[j] * fac3;
+          OPX(3 * i + k, 4 * j + p) -= s.m[j] * fac3;
+          OPX(3 * j + k, 4 * j + p) += s.m[i] * fac3;
+          OPX(3 * j + k, 4 * i + p) -= s.m[i] * fac3;
+        }
+        fac = (-fac1) * r2;
+        for (int di = 0; di < N; di++) {
           for (int p = 0; p < 3; p++) {
-            OPX(3 * i + k, 4 * i + p) -= fac * s.m[j] * rij[p];
-            OPX(3 * i + k, 4 * j + p) += fac * s.m[j] * rij[p];
-            OPX(3 * j + k, 4 * j + p) -= fac * s.m[i] * rij[p];
-            OPX(3 * j + k, 4 * i + p) += fac * s.m[i] * rij[p];
+            OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
+            OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
           }
-          fac = fac1 * fac2;
-          OPX(3 * i + k, 4 * i + k) += fac * s.m[j];
-          OPX(3 * i + k, 4 * j + k) -= fac * s.m[j];
-          OPX(3 * j + k, 4 * j + k) += fac * s.m[i];
-          OPX(3 * j + k, 4 * i + k) -= fac * s.m[i];
-          fac = -2.0 * fac1 * aij[k];
+          OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
+          OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
+        }
+        fac = 3.0 * fac1 * rij[k];
+        for (int di = 0; di < N; di++) {
           for (int p = 0; p < 3; p++) {
-            double fac3 = fac * rij[p] + fac1 * 3.0 * rij[k] * aij[p];
-            OPX(3 * i + k, 4 * i + p) += s.m[j] * fac3;
-            OPX(3 * i + k, 4 * j + p) -= s.m[j] * fac3;
-            OPX(3 * j + k, 4 * j + p) += s.m[i] * fac3;
-            OPX(3 * j + k, 4 * i + p) -= s.m[i] * fac3;
+            OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * w.dot[4 * di + p];
+            OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * w.dot[4 * di + p];
           }
-          fac = (-fac1) * r2;
-          for (int di = 0; di < N; di++) {
-            for (int p = 0; p < 3; p++) {
-              OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-              OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + p) - DAX(3 * j + k, 4 * di + p));
-            }
-            OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
-            OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * (DAX(3 * i + k, 4 * di + 3) - DAX(3 * j + k, 4 * di + 3));
-          }
-          fac = 3.0 * fac1 * rij[k];
-          for (int di = 0; di < N; di++) {
-            for (int p = 0; p < 3; p++) {
-              OPX(3 * i + k, 4 * di + p) += fac * s.m[j] * w.dot[4 * di + p];
-              OPX(3 * j + k, 4 * di + p) -= fac * s.m[i] * w.dot[4 * di + p];
-            }
-            OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * w.dot[4 * di + 3];
-            OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * w.dot[4 * di + 3];
-          }
+          OPX(3 * i + k, 4 * di + 3) += fac * s.m[j] * w.dot[4 * di + 3];
+          OPX(3 * j + k, 4 * di + 3) -= fac * s.m[i] * w.dot[4 * di + 3];
         }
       }
     }
@@ -306,7 +294,7 @@ __device__ __forceinline__ void phis_accel_pair(const Sys<N>& s, double* a, int 
   }
 }
 template <int N>
-__device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i, int j, double coeff) {
+__device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i, int j, double mij, double coeff) {
   double rij[3], aij[3], f[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
@@ -314,7 +302,7 @@ __device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i
     rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
   }
   const double r2 = norm2(rij);
-  phis_corr(rij, r2, rsqrt_fast(r2), aij, s.m[i] + s.m[j], coeff, f);
+  phis_corr(rij, r2, rsqrt_fast(r2), aij, mij, coeff, f);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], s.m[j], f[k]);
@@ -331,7 +319,41 @@ __device__ __forceinline__ void phisalpha(Sys<N>& s, double* a, double h, uint64
       if (!((kick >> pair_bit(i, j, N)) & 1)) phis_accel_pair<N>(s, a, i, j);
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++)
-      if (!((kick >> pair_bit(i, j, N)) & 1)) phis_kick_pair<N>(s, a, i, j, coeff);
+      if (!((kick >> pair_bit(i, j, N)) & 1)) phis_kick_pair<N>(s, a, i, j, s.m[i] + s.m[j], coeff);
+}
+
+// kickfast! without gradient (ahl21_no_grad.jl:35-56): kicks over h between the
+// pairs of the mask.
+template <int N>
+__device__ __forceinline__ void plain_kick(Sys<N>& s, double h, uint64_t kick) {
+  for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++) {
+      if (!((kick >> pair_bit(i, j, N)) & 1)) continue;
+      double rij[3], f[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
+      phis_accel(rij, rsqrt_fast(norm2(rij)), f);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], -(h * s.m[j]), f[k]);
+        kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], h * s.m[i], f[k]);
+      }
+    }
+}
+// phic! without gradient (ahl21_no_grad.jl:62-104): a kick over 2h/3 and the
+// correction, between the pairs of the mask.
+__device__ __forceinline__ double phic_coeff(double h) { return h * h * h / 36.0 * GNEWT; }
+template <int N>
+__device__ __forceinline__ void plain_phic(Sys<N>& s, double* a, double h, uint64_t kick) {
+  plain_kick<N>(s, 2.0 * h / 3.0, kick);
+#pragma unroll
+  for (int q = 0; q < 3 * N; q++) a[q] = 0.0;
+  for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++)
+      if ((kick >> pair_bit(i, j, N)) & 1) phis_accel_pair<N>(s, a, i, j);
+  for (int i = 0; i < N - 1; i++)
+    for (int j = i + 1; j < N; j++)
+      if ((kick >> pair_bit(i, j, N)) & 1) phis_kick_pair<N>(s, a, i, j, 0.0, phic_coeff(h));
 }
 
 // The corrector's operator (jac_phi, ahl21.jl:558-700) for Kepler pairs: its
@@ -503,15 +525,14 @@ __device__ __forceinline__ void kepler_pair(Sys<N>& s, int i, int j, double h2, 
 }
 
 // The same with the block update of ahl21.jl:31-42 on dq/dt (ahl21.jl:706-760).
-template <int N, bool DRIFT_FIRST, bool GRADOPS, bool DQDT>
-__device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, const Rec& rec, int roff,
-                            const Rec& cap, int coff) {
+template <int N, bool DRIFT_FIRST>
+__device__ void kepler_pair_grad(Sys<N>& s, Work<N>& w, int i, int j, double h2, const Rec& rec, int roff) {
   double x0[3], v0[3], delxv[6];
   KepParams P;
-  if (kepler_pair<N, DRIFT_FIRST>(s, i, j, h2, cap, coff, x0, v0, P, delxv)) {
+  if (kepler_pair<N, DRIFT_FIRST>(s, i, j, h2, Rec{nullptr, 0}, 0, x0, v0, P, delxv)) {
     const double mijinv = rcp_fast(s.m[i] + s.m[j]);
     const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
-    if (GRADOPS) {
+    {
       KepDeriv D;
       double dh[6];
       kep_derivatives<DRIFT_FIRST, true>(P, D);
@@ -527,7 +548,7 @@ __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, cons
       w.ldq[6] = w.ldq[13] = 0.0;
     }
   }
-  if (GRADOPS && rec.p) {
+  if (rec.p) {
     for (int q = 0; q < 36; q++) rec.put(roff + q, w.lk[q]);
     rec.put(roff + PREC_MI, w.lmi);
     rec.put(roff + PREC_MJ, w.lmj);
@@ -536,7 +557,7 @@ __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, cons
       rec.put(roff + PREC_B + q, w.lb[q]);
     }
   }
-  if (DQDT) {
+  {
     // d.dqdt_ij .*= 1/2; d.dqdt_ij .+= dqdt_tmp1 .+ jac_ij * dqdt_tmp1 (ahl21.jl:38-40)
     double t1[14];
     for (int q = 0; q < 7; q++) {
@@ -570,92 +591,93 @@ __device__ void kepler_pair(Sys<N>& s, Work<N>& w, int i, int j, double h2, cons
   }
 }
 
-// One AHL21 step (ahl21.jl:5-95 / ahl21_no_grad.jl:6-18).
-//   GRADOPS: build the operators (needed for records and for dq/dt);
-//   DQDT:    compute dq/dt as the reference does;
-//   rec:     where the operator record goes (rec.p == nullptr: nowhere).
-//   cap, xs: where the Kepler-pair parameters and the position snapshots go
-//            for the operator kernel (p == nullptr: nowhere).
-template <int N, bool GRADOPS, bool DQDT>
-__device__ __noinline__ void ahl21_step(Sys<N>& s, Work<N>& w, double h, uint64_t kick, const Rec& rec,
-                                        const Rec& cap, const Rec& xs) {
+// One AHL21 step with its gradient (ahl21.jl:5-95): x, v, dq/dt as the reference
+// forms it, and the operator record at rec.
+template <int N>
+__device__ __noinline__ void ahl21_step(Sys<N>& s, Work<N>& w, double h, uint64_t kick, const Rec& rec) {
   const double h2 = 0.5 * h, h6 = h / 6.0;
-  if (GRADOPS) reset_last(w);
-  if (DQDT)
-    for (int q = 0; q < 7 * N; q++) s.dqdt[q] = 0.0;
-  int roff = 0, slot = 0;
-  if (kick && xs.p)
-    for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, s.x[q]);
+  reset_last(w);
+  for (int q = 0; q < 7 * N; q++) s.dqdt[q] = 0.0;
+  int roff = 0;
   if (kick) {
-    kickfast<N, GRADOPS>(s, w, h6, kick);
-    if (DQDT) dqdt_op(s, w, 6.0);
-    if (GRADOPS) { put_op(rec, roff, w.op, op_size(N)); }
+    kickfast<N>(s, w, h6, kick);
+    dqdt_op(s, w, 6.0);
+    put_op(rec, roff, w.op, op_size(N));
     roff += op_size(N);
   }
   drift(s, h2);
-  if (DQDT)
-    for (int b = 0; b < N; b++)
-      for (int k = 0; k < 3; k++) s.dqdt[7 * b + k] = 0.5 * s.v[3 * b + k] + h2 * s.dqdt[7 * b + 3 + k];
+  for (int b = 0; b < N; b++)
+    for (int k = 0; k < 3; k++) s.dqdt[7 * b + k] = 0.5 * s.v[3 * b + k] + h2 * s.dqdt[7 * b + 3 + k];
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++) {
       if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      kepler_pair<N, true, GRADOPS, DQDT>(s, w, i, j, h2, rec, roff, cap, slot * PCAP);
+      kepler_pair_grad<N, true>(s, w, i, j, h2, rec, roff);
       roff += PREC;
-      slot++;
     }
-  if (xs.p)
-    for (int q = 0; q < 3 * N; q++) xs.put(q, s.x[q]);
-  phic<N, GRADOPS>(s, w, h, kick);
+  phic<N>(s, w, h, kick);
   phisalpha<N>(s, w.a, h, kick);  // moves v alone: the operator below is that of the same positions
-  if (xs.p && !kick)
-    for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, w.a[q]);
-  if (GRADOPS) phisalpha_operator<N>(s, w, h, kick);
-  if (DQDT) dqdt_op(s, w, 1.0);
-  if (GRADOPS) put_op(rec, roff, w.op, op_size(N));
+  phisalpha_operator<N>(s, w, h, kick);
+  dqdt_op(s, w, 1.0);
+  put_op(rec, roff, w.op, op_size(N));
   roff += op_size(N);
   for (int i = N - 2; i >= 0; i--)
     for (int j = N - 1; j > i; j--) {
       if ((kick >> pair_bit(i, j, N)) & 1) continue;
-      kepler_pair<N, false, GRADOPS, DQDT>(s, w, i, j, h2, rec, roff, cap, slot * PCAP);
+      kepler_pair_grad<N, false>(s, w, i, j, h2, rec, roff);
       roff += PREC;
-      slot++;
     }
   drift(s, h2);
-  if (DQDT)
-    for (int b = 0; b < N; b++)
-      for (int k = 0; k < 3; k++)
-        s.dqdt[7 * b + k] = s.dqdt[7 * b + k] + (0.5 * s.v[3 * b + k] + h2 * s.dqdt[7 * b + 3 + k]);
+  for (int b = 0; b < N; b++)
+    for (int k = 0; k < 3; k++)
+      s.dqdt[7 * b + k] = s.dqdt[7 * b + k] + (0.5 * s.v[3 * b + k] + h2 * s.dqdt[7 * b + 3 + k]);
   if (kick) {
-    if (xs.p)
-      for (int q = 0; q < 3 * N; q++) xs.put(6 * N + q, s.x[q]);
-    kickfast<N, GRADOPS>(s, w, h6, kick);
-    if (DQDT) dqdt_op(s, w, 6.0);
-    if (GRADOPS) put_op(rec, roff, w.op, op_size(N));
-    roff += op_size(N);
+    kickfast<N>(s, w, h6, kick);
+    dqdt_op(s, w, 6.0);
+    put_op(rec, roff, w.op, op_size(N));
   }
 }
 
-// The same step without gradient for a group with no kick pairs
-// (ahl21_no_grad.jl:6-18): x and v alone, a the accelerations at the corrector.
+// The same step without gradient (ahl21_no_grad.jl:6-18): x and v alone, a the
+// accelerations at the corrector.  cap, xs, vs: where the captures and
+// snapshots go (snap_count) and, for dq/dt, v at the first drift and at the
+// second (3N each); p == nullptr: nowhere.
 template <int N>
-__device__ __forceinline__ void plain_step(Sys<N>& s, double* a, double h, const Rec& cap, const Rec& xs) {
+__device__ __forceinline__ void plain_step(Sys<N>& s, double* a, double h, uint64_t kick, const Rec& cap,
+                                           const Rec& xs, const Rec& vs) {
   const double h2 = 0.5 * h;
   int slot = 0;
+  if (kick) {
+    if (xs.p)
+      for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, s.x[q]);
+    plain_kick<N>(s, h / 6.0, kick);
+  }
+  if (vs.p)
+    for (int q = 0; q < 3 * N; q++) vs.put(q, s.v[q]);
   drift(s, h2);
 #pragma unroll 1
   for (int i = 0; i < N - 1; i++)
 #pragma unroll 1
-    for (int j = i + 1; j < N; j++) kepler_pair<N, true>(s, i, j, h2, cap, PCAP * slot++);
+    for (int j = i + 1; j < N; j++)
+      if (!((kick >> pair_bit(i, j, N)) & 1)) kepler_pair<N, true>(s, i, j, h2, cap, PCAP * slot++);
   if (xs.p)
     for (int q = 0; q < 3 * N; q++) xs.put(q, s.x[q]);
-  phisalpha<N>(s, a, h, 0);
-  if (xs.p)
+  if (kick) plain_phic<N>(s, a, h, kick);
+  phisalpha<N>(s, a, h, kick);
+  if (xs.p && !kick)
     for (int q = 0; q < 3 * N; q++) xs.put(3 * N + q, a[q]);
 #pragma unroll 1
   for (int i = N - 2; i >= 0; i--)
 #pragma unroll 1
-    for (int j = N - 1; j > i; j--) kepler_pair<N, false>(s, i, j, h2, cap, PCAP * slot++);
+    for (int j = N - 1; j > i; j--)
+      if (!((kick >> pair_bit(i, j, N)) & 1)) kepler_pair<N, false>(s, i, j, h2, cap, PCAP * slot++);
+  if (vs.p)
+    for (int q = 0; q < 3 * N; q++) vs.put(3 * N + q, s.v[q]);
   drift(s, h2);
+  if (kick) {
+    if (xs.p)
+      for (int q = 0; q < 3 * N; q++) xs.put(6 * N + q, s.x[q]);
+    plain_kick<N>(s, h / 6.0, kick);
+  }
 }
 
 // g! and gd! (src/transits/timing.jl:141-150) for transited body i and

@@ -20,7 +20,7 @@
 // masses in shared memory.  The critical path of a sweep drops from
 // N(N-1)/2 to 2N-3 pair solves (N = 10: 45 -> 17; N = 8: 28 -> 13).
 //
-// Groups with kick pairs (pair[i,j] == true) keep the one-lane producer.
+// Groups with kick pairs (pair[i,j] == true) take one lane or the lanes form.
 #pragma once
 #include "nbg_orbit.cuh"
 
@@ -46,12 +46,15 @@ __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {
 // scratch.
 template <int N>
 __device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run, double h,
-                                          const Rec& cap, const Rec& xs) {
+                                          const Rec& cap, const Rec& xs, const Rec& vs) {
   constexpr int L = team_lanes(N);
   constexpr int P = N * (N - 1) / 2;
   const double h2 = 0.5 * h;
   if (run)
-    for (int q = t; q < 3 * N; q += L) kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+    for (int q = t; q < 3 * N; q += L) {
+      if (vs.p) vs.put(q, s.v[q]);
+      kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+    }
   __syncwarp();
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
@@ -75,7 +78,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run,
     for (int q = t; q < 3 * N; q += L) xs.put(3 * N + q, a[q]);
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i, j;
-    if (run && level_pair<N>(lev, t, &i, &j)) phis_kick_pair<N>(s, a, i, j, coeff);
+    if (run && level_pair<N>(lev, t, &i, &j)) phis_kick_pair<N>(s, a, i, j, s.m[i] + s.m[j], coeff);
     __syncwarp();
   }
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
@@ -85,7 +88,10 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run,
     __syncwarp();
   }
   if (run)
-    for (int q = t; q < 3 * N; q += L) kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+    for (int q = t; q < 3 * N; q += L) {
+      if (vs.p) vs.put(3 * N + q, s.v[q]);
+      kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+    }
   __syncwarp();
 }
 
@@ -155,9 +161,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
         rx[3 * N + q] = st.v[q];
       }
     }
-    if (run && g.grad && istep == nst - 1)  // v at the last step's start, for its dq/dt (dq_columns)
-      for (int q = t; q < 3 * N; q += L) g.dqdt[(7 * (q / 3) + 3 + q % 3) * S + s] = st.v[q];
-    team_step<N>(st, acc[tm], t, run, hs, cap, xs);
+    const Rec vs{run && g.grad && istep == nst - 1 ? g.vsnap + s : nullptr, S};
+    team_step<N>(st, acc[tm], t, run, hs, cap, xs, vs);
     // occultor o on lane o % L
     if (run && !g.notransit)
       for (int o = t; o < N - 1; o += L)
@@ -210,7 +215,7 @@ __host__ __device__ constexpr int lanes_each(int N) { return 32 * lanes_warps(N)
 template <int N>
 struct LanesShared {
   Sys<N> st;
-  double a[3 * N], g[N];
+  double a[3 * N], ac[3 * N], g[N];
   long long cnt[N];
   double pk[N * (N - 1) / 2], pmi[N * (N - 1) / 2], pmj[N * (N - 1) / 2];  // k, m_i / (m_i + m_j), m_j / (m_i + m_j)
   double f[N * (N - 1) / 2][3];
@@ -381,66 +386,97 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
   }
 }
 
-// One AHL21 step of a kick-free group on a system's lanes t (team_step's order);
-// run is false for the lanes of a system that does not step: they keep step
-// with their warp and write nothing.
-template <int N>
-__device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, double h, const Rec& cap,
-                                           const Rec& xs) {
+// One AHL21 step on a system's lanes t (plain_step's values); run is false for
+// the lanes of a system that does not step: they keep step with their warp and
+// write nothing.  KICK: the group has kick pairs (kick).
+template <int N, bool KICK>
+__device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, double h, uint64_t kick,
+                                           const Rec& cap, const Rec& xs, const Rec& vs) {
   constexpr int P = N * (N - 1) / 2, T = lanes_each(N);
   static_assert(P <= T && 3 * N <= T, "one lane per pair and per coordinate");
   const int half = t >> 4, hl = t & 15;
   const double h2 = 0.5 * h;
   const bool coord = run && t < 3 * N, pair = run && t < P;
   Sys<N>& st = sh.st;
-  if (coord) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
-  lanes_sync<N>();
-#pragma unroll 1
-  for (int lev = 1; lev <= 2 * N - 3; lev++) {
-    int i = 0, j = 1;
-    const bool act = level_pair<N>(lev, half, &i, &j) && run;
-    if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, pair_bit(i, j, N) * PCAP, hl);
-    lanes_sync<N>();
-  }
-  // pair t's bodies
-  int pi = 0, pj = t + 1;
+  int pi = 0, pj = t + 1;  // pair t's bodies
   while (pj >= N && pi < N - 2) {
     pi++;
     pj += pi + 1 - N;
   }
+  const int b = t / 3, w = t % 3;  // coordinate lane
+  const bool kicked = KICK && pair && ((kick >> t) & 1);
+  auto pair_at = [&](int o) { return o < b ? pair_bit(o, b, N) : pair_bit(b, o, N); };
+  auto is_kick = [&](int o) { return KICK && ((kick >> pair_at(o)) & 1); };
   double rij[3], r2 = 0.0, rinv = 0.0;
-  if (xs.p && coord) xs.put(t, st.x[t]);
-  if (pair) {
+  auto force = [&](bool which) {  // G r / r^3 of pair t
+    if (!which) return;
 #pragma unroll
-    for (int w = 0; w < 3; w++) rij[w] = st.x[3 * pi + w] - st.x[3 * pj + w];
+    for (int q = 0; q < 3; q++) rij[q] = st.x[3 * pi + q] - st.x[3 * pj + q];
     r2 = norm2(rij);
     rinv = rsqrt_fast(r2);
     phis_accel(rij, rinv, sh.f[t]);
+  };
+  auto kick_v = [&](double hk) {  // the kicked pairs' velocity changes, by body and in pair order
+    if (!coord) return;
+    double v = st.v[t], ve = st.ve[t];
+    for (int o = 0; o < N; o++)
+      if (o != b && is_kick(o)) kahan_fma(v, ve, o < b ? hk * st.m[o] : -(hk * st.m[o]), sh.f[pair_at(o)][w]);
+    st.v[t] = v;
+    st.ve[t] = ve;
+  };
+  if (KICK) {
+    if (xs.p && coord) xs.put(3 * N + t, st.x[t]);
+    force(kicked);
+    lanes_sync<N>();
+    kick_v(h / 6.0);
+  }
+  if (coord) {
+    if (vs.p) vs.put(t, st.v[t]);
+    kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
   }
   lanes_sync<N>();
-  const int b = t / 3, w = t % 3;  // coordinate lane
+  // a Kepler pair's capture slot: the ones before it in sweep order
+  auto slot_of = [&](int pb) { return KICK ? pb - __popcll(kick & ((1ull << pb) - 1)) : pb; };
+  const int npk = KICK ? P - __popcll(kick) : P;
+#pragma unroll 1
+  for (int lev = 1; lev <= 2 * N - 3; lev++) {
+    int i = 0, j = 1;
+    bool act = level_pair<N>(lev, half, &i, &j) && run;
+    const int pb = pair_bit(i, j, N);
+    if (KICK) act = act && !((kick >> pb) & 1);
+    if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, slot_of(pb) * PCAP, hl);
+    lanes_sync<N>();
+  }
+  if (xs.p && coord) xs.put(t, st.x[t]);
+  force(pair);
+  lanes_sync<N>();
+  if (KICK) kick_v(2.0 * h / 3.0);
   if (coord) {
-    double a = 0.0;
+    double a = 0.0, ac = 0.0;  // by the Kepler pairs and by the kicked ones
     for (int o = 0; o < N; o++)
       if (o != b) {
-        const double f = sh.f[o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)][w];
-        a = fma(o < b ? st.m[o] : -st.m[o], f, a);
+        const double f = sh.f[pair_at(o)][w], m = o < b ? st.m[o] : -st.m[o];
+        if (is_kick(o)) ac = fma(m, f, ac);
+        else a = fma(m, f, a);
       }
     sh.a[t] = a;
-    if (xs.p) xs.put(3 * N + t, a);
+    if (KICK) sh.ac[t] = ac;
+    if (xs.p && !KICK) xs.put(3 * N + t, a);
   }
   lanes_sync<N>();
   if (pair) {
+    const double* a = kicked ? sh.ac : sh.a;
     double aij[3];
 #pragma unroll
-    for (int q = 0; q < 3; q++) aij[q] = sh.a[3 * pi + q] - sh.a[3 * pj + q];
-    phis_corr(rij, r2, rinv, aij, st.m[pi] + st.m[pj], phis_coeff(h), sh.f[t]);
+    for (int q = 0; q < 3; q++) aij[q] = a[3 * pi + q] - a[3 * pj + q];
+    phis_corr(rij, r2, rinv, aij, kicked ? 0.0 : st.m[pi] + st.m[pj], kicked ? phic_coeff(h) : phis_coeff(h), sh.f[t]);
   }
   lanes_sync<N>();
   if (coord) {
     double v = st.v[t], ve = st.ve[t];
-    for (int o = 0; o < N; o++)
-      if (o != b) kahan_fma(v, ve, o < b ? -st.m[o] : st.m[o], sh.f[o < b ? pair_bit(o, b, N) : pair_bit(b, o, N)][w]);
+    for (int pass = KICK ? 0 : 1; pass < 2; pass++)  // the kicked pairs' corrections, then the Kepler pairs'
+      for (int o = 0; o < N; o++)
+        if (o != b && is_kick(o) == (pass == 0)) kahan_fma(v, ve, o < b ? -st.m[o] : st.m[o], sh.f[pair_at(o)][w]);
     st.v[t] = v;
     st.ve[t] = ve;
   }
@@ -448,16 +484,28 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
 #pragma unroll 1
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
     int i = 0, j = 1;
-    const bool act = level_pair<N>(lev, half, &i, &j) && run;
+    bool act = level_pair<N>(lev, half, &i, &j) && run;
+    const int pb = pair_bit(i, j, N);
+    if (KICK) act = act && !((kick >> pb) & 1);
     if (__any_sync(0xffffffffu, act))
-      lanes_pair<N, false>(sh, i, j, act, h2, cap, (P + (P - 1 - pair_bit(i, j, N))) * PCAP, hl);
+      lanes_pair<N, false>(sh, i, j, act, h2, cap, (npk + (npk - 1 - slot_of(pb))) * PCAP, hl);
     lanes_sync<N>();
   }
-  if (coord) kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  if (coord) {
+    if (vs.p) vs.put(3 * N + t, st.v[t]);
+    kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+  }
   lanes_sync<N>();
+  if (KICK) {
+    if (xs.p && coord) xs.put(6 * N + t, st.x[t]);
+    force(kicked);
+    lanes_sync<N>();
+    kick_v(h / 6.0);
+    lanes_sync<N>();
+  }
 }
 
-template <int N>
+template <int N, bool KICK>
 __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupArgs g, int chunk) {
   extern __shared__ double lanes_smem[];
   constexpr int P = N * (N - 1) / 2, T = lanes_each(N);
@@ -503,7 +551,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
     Rec cap{nullptr, 0}, xs{nullptr, 0};
     if (g.grad && run) {
       cap = Rec{g.pcap + (size_t)kk * 2 * g.npk * PCAP * S + s, S};
-      xs = Rec{g.xsnap + (size_t)kk * snap_count(false) * 3 * N * S + s, S};
+      xs = Rec{g.xsnap + (size_t)kk * snap_count(KICK) * 3 * N * S + s, S};
     }
     const double hs = run ? step_length(g, s, istep, nst, h) : h;
     if (g.trajxv && run && t < 3 * N) {
@@ -511,9 +559,8 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
       rx[t] = st.x[t];
       rx[3 * N + t] = st.v[t];
     }
-    if (g.grad && run && istep == nst - 1 && t < 3 * N)  // v at the last step's start, for its dq/dt (dq_columns)
-      g.dqdt[(7 * (t / 3) + 3 + t % 3) * S + s] = st.v[t];
-    lanes_step<N>(sh, t, run, hs, cap, xs);
+    const Rec vs{g.grad && run && istep == nst - 1 ? g.vsnap + s : nullptr, S};
+    lanes_step<N, KICK>(sh, t, run, hs, g.kick, cap, xs, vs);
     if (!g.notransit && run && t < N - 1)
       detect_transit<N>(g, st, s, kk, t, ti, ntt, hI, t0 + (double)(istep + 1) * h, sh.g, sh.cnt);
     lanes_sync<N>();

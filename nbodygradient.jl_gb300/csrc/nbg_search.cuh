@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       tt2 = tt1;
       tt1 = dt0;
       start();
-      plain_step<N>(wk, a, dt0, none, none);
+      plain_step<N>(wk, a, dt0, 0, none, none, none);
       const double gs = gsky(wk, k.ti, k.ib), gd = gdot_physical(wk, k.ti, k.ib);
       const double dt = -gs / gd;
       kahan(dt0, stmp, dt);
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
     double* ttout = g.tt + g.off_tt[g.sysidx[k.s]] + (long long)(g.tbv ? 3 : 1) * (k.ib + (long long)N * k.c);
     if (g.grad) {
       start();
-      plain_step<N>(wk, a, dt0, scr, Rec{scr.p + (size_t)SearchAt<N>::xs * G, G});
+      plain_step<N>(wk, a, dt0, 0, scr, Rec{scr.p + (size_t)SearchAt<N>::xs * G, G}, none);
 #pragma unroll 1
       for (int slot = 0; slot < 2 * SearchAt<N>::P; slot++) search_record<N>(scr, wk.m, slot, 0.5 * dt0);
       const double dvx = wk.v[3 * k.ib] - wk.v[3 * k.ti], dvy = wk.v[3 * k.ib + 1] - wk.v[3 * k.ti + 1];
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
     // every search of the block steps until the last has converged
     while (SYS > 1 ? __any_sync(0xffffffffu, active) : active) {
       start(active);
-      lanes_step<N>(sh.l, t, active, dt0, none, none);
+      lanes_step<N, false>(sh.l, t, active, dt0, 0, none, none, none);
       if (t < N) {
         if (t != k.ti) sky_pull(wk, t, k.ti, sh.pull[0][t]);
         if (t != k.ib) sky_pull(wk, t, k.ib, sh.pull[1][t]);
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
     double* ttout = g.tt + g.off_tt[g.sysidx[k.s]] + (long long)(g.tbv ? 3 : 1) * (k.ib + (long long)N * k.c);
     if (g.grad) {
       start(true);
-      lanes_step<N>(sh.l, t, true, dt0, Rec{sh.scr + At::cap, 1}, Rec{sh.scr + At::xs, 1});
+      lanes_step<N, false>(sh.l, t, true, dt0, 0, Rec{sh.scr + At::cap, 1}, Rec{sh.scr + At::xs, 1}, none);
       for (int slot = t; slot < 2 * P; slot += T) search_record<N>(Rec{sh.scr, 1}, wk.m, slot, 0.5 * dt0);
       const double h2 = 0.5 * dt0, coeff = phis_coeff(dt0);
       double r[3], a[3], r2 = 0.0, ri = 0.0;  // pair t at the corrector

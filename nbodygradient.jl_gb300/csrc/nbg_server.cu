@@ -344,7 +344,7 @@ int create_group(nbg_server* srv, int N, int grad, unsigned long long kick, Grou
     want(&g.steprec, 2 * nrec); want(&g.trec, 2 * ntrec);
     want(&g.tflag, 2 * nflag); want(&g.tscratch, (size_t)search_scratch(N, npk, kick != 0) * g.tgrid);
     want(&g.pcap, 2 * ncap);
-    want(&g.xsnap, 2 * nsnap); want(&g.dh, 12 * (size_t)npk * S);
+    want(&g.xsnap, 2 * nsnap); want(&g.dh, 12 * (size_t)npk * S); want(&g.vsnap, 6 * N * S);
     want(&g.Jint, S * 6 * N * 7 * N); want(&g.Eint, S * 6 * N * 7 * N);
   }
   want(&G->stage, S * G->lay.stride);
@@ -617,8 +617,8 @@ int service_group(nbg_server* srv, int gi) {
   int rc;
   // the producer's and the consumer's forms for latency-bound chunks while few slots are running
   GroupArgs gw = gc;
-  gw.wide = use_wide(srv->cfg.orbit_team, G->active <= lanes_limit(N, G->grad, srv->sm_count), G->kick) ? 1 : 0;
-  gw.rows = use_wide(srv->cfg.orbit_team, G->active <= rows_limit(N, srv->sm_count), G->kick) ? 1 : 0;
+  gw.wide = use_wide(srv->cfg.orbit_team, G->active <= lanes_limit(N, G->grad, srv->sm_count)) ? 1 : 0;
+  gw.rows = use_wide(srv->cfg.orbit_team, G->active <= rows_limit(N, srv->sm_count)) ? 1 : 0;
   if ((rc = launch_group_orbit(N, gw, (int)c, st))) return rc;
   NBG_CUDA(cudaEventRecord(G->ev_orb[par], st));
   NBG_CUDA(cudaStreamWaitEvent(stt, G->ev_orb[par], 0));
@@ -630,7 +630,7 @@ int service_group(nbg_server* srv, int gi) {
     // beside it
     GroupArgs gs = gc;
     gs.search_lanes =
-        N >= 5 && use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2), G->kick) ? 1 : 0;
+        N >= 5 && use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2)) ? 1 : 0;
     if ((rc = launch_group_transit(N, gs, (int)c, stt))) return rc;
   }
   NBG_CUDA(cudaEventRecord(G->ev_tr[par], stt));
