@@ -119,7 +119,7 @@ __device__ __forceinline__ void pair_update(double* S, double* E, int c, int i, 
   double D[6];
 #pragma unroll
   for (int l = 0; l < 6; l++)
-    D[l] = (S[(6 * i + l) * BS] + E[(6 * i + l) * BS]) - (S[(6 * j + l) * BS] + E[(6 * j + l) * BS]);
+    D[l] = (S[(6 * i + l) * BS] - S[(6 * j + l) * BS]) + (E[(6 * i + l) * BS] - E[(6 * j + l) * BS]);
 #pragma unroll
   for (int r = 0; r < 6; r++) {
     double u = MASS ? fma(K[r * 6], D[0], U[r]) : K[r * 6] * D[0];

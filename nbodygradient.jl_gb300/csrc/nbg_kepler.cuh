@@ -344,7 +344,7 @@ __device__ __forceinline__ float kep_start(float r0inv, float h, float beta, flo
 // next term is below u^3 / s^2, so the step that is at most KEP_STEP s long is
 // the last and the G_n move to s + ds by their Taylor series,
 // dG_n / ds = G_{n-1}.  Against binary128 over 3000 draws delxv is off by
-// 2.9e-16 rms (the half-angle iteration: 4.2e-16), star-planet and planet pairs
+// 2.8e-16 rms (the half-angle iteration: 4.2e-16), star-planet and planet pairs
 // alike.  With kep_derivatives and phi_columns a lone 3-body system's 2000
 // steps went from 241 to 120 ms, a lone 8-body system's 400 from 261 to 167 ms,
 // 4096 three-body systems over 2000 steps from 745 to 532 ms.
@@ -411,10 +411,11 @@ __device__ __forceinline__ void kep_solve(const double* x0, const double* v0, do
     gmh = kr * fma(r0, h2, eta * h1);
     dgdtm1 = -(kr * g2);
   }
+  // the large product (v0's is smaller by h's order) is the one that is not rounded
 #pragma unroll
   for (int q = 0; q < 3; q++) {
-    delxv[q] = fma(gmh, v0[q], fm1 * x0[q]);
-    delxv[3 + q] = fma(dgdtm1, v0[q], dfdt * x0[q]);
+    delxv[q] = fma(fm1, x0[q], gmh * v0[q]);
+    delxv[3 + q] = fma(dfdt, x0[q], dgdtm1 * v0[q]);
   }
   P.s = s; P.g1 = g1; P.g2 = g2; P.g3 = g3;
   P.dfdt = dfdt; P.fm1 = fm1; P.gmh = gmh; P.dgdtm1 = dgdtm1; P.r0 = r0; P.r = r; P.r0inv = r0inv; P.rinv = rinv;

@@ -661,7 +661,7 @@ __device__ __forceinline__ void rows_pair(double* Sw, double* Ew, const double* 
                                           int l, int col, bool live) {
   const int ai = (6 * i + l) * ROWS_COLS + col, aj = (6 * j + l) * ROWS_COLS + col;
   const double ei = Ew[ai], ej = Ew[aj];
-  const double d = (Sw[ai] + ei) - (Sw[aj] + ej);
+  const double d = (Sw[ai] - Sw[aj]) + (ei - ej);
   const double* K = rc + 6 * l;
   double u = 0.0;
 #pragma unroll

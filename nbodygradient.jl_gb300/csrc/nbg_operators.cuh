@@ -76,8 +76,8 @@ __device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int cof
   for (int r = 0; r < 3; r++) {
     rec.put(roff + PREC_PSI + r, psi[r]);
     rec.put(roff + PREC_PSI + 3 + r, psi[3 + r]);
-    rec.put(roff + PREC_B + r, mijinv * fma(P.gmh, v0[r], P.fm1 * x0[r]));
-    rec.put(roff + PREC_B + 3 + r, mijinv * fma(P.dgdtm1, v0[r], P.dfdt * x0[r]));
+    rec.put(roff + PREC_B + r, mijinv * fma(P.fm1, x0[r], P.gmh * v0[r]));
+    rec.put(roff + PREC_B + 3 + r, mijinv * fma(P.dfdt, x0[r], P.dgdtm1 * v0[r]));
   }
 }
 

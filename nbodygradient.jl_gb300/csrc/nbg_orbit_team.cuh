@@ -355,7 +355,7 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
     P.s = s; P.g1 = g1; P.g2 = g2; P.g3 = g3; P.r0 = r0; P.r0inv = r0inv; P.rinv = rinv; P.beta = beta; P.eta = eta;
     P.zeta = zeta;
     const double cx = from(val, c < 3 ? 0 : 2), cv = from(val, c < 3 ? 1 : 3);
-    del = fma(cv, vk, cx * xk);
+    del = fma(cx, xk, cv * vk);
   }
   if (act && !done) {
     double delxv[6];
