@@ -59,16 +59,15 @@ def load_package():
 def flops_per_system_step(n):
     """Algorithmic FP64 flops of the Jacobian consumer per system-step (FMA = 2).
 
-    Per column of jac_step and step: 2P pair updates of 132 flops (6 differences,
-    a 6x6 product u = K D (66), the two mass-ratio scalings (12) and the Kahan
-    sums of 12 rows (48)); the phi block 3N x 3N (18 N^2) with its Kahan sums
-    (12 N); two drifts (30 N).  The zero-addend folds of 6N, 3N and 6N rows
-    count one add per row (15 N): the warp tests s + e and runs the fold's
-    other two adds only when one would change a row, which after a
-    compensated add it almost never does.  7N columns.
+    Per column of jac_step and step: 2P pair updates of 108 flops (the
+    differences of six rows' pairs (S, E) 18, a 6x6 product u = K D 66, the
+    increments of twelve rows 24); the phi block on position differences,
+    3N x 3(N - 1), with its sums (18 N^2 - 12 N - 3); the first drift with its
+    rows' normalisation 15 N, the second with all rows' 24 N, and from three
+    bodies on one more normalisation of the velocity rows 9 N.  7N columns.
     """
     P = n * (n - 1) // 2
-    per_col = 2 * P * 132 + 18 * n * n + 57 * n
+    per_col = 2 * P * 108 + 18 * n * n + (36 if n > 2 else 27) * n - 3
     return per_col * 7 * n
 
 

@@ -1,6 +1,6 @@
 // nbg_jacobian.cuh -- the Jacobian consumer: one GPU lane owns one column of
 // jac_step (and of jac_error) of one system and applies the operator stream
-// the orbit producer recorded, with the reference's compensated summation.
+// the orbit producer's captures were turned into.
 //
 // Every update of ahl21! on jac_step (src/integrator/ahl21/ahl21.jl:5-95) has
 // the form J <- J + A J followed by comp_sum_matrix!(J, J_err, A J)
@@ -12,15 +12,17 @@
 // The pair update uses the structure of jac_ij (ahl21.jl:734-750): rows of
 // body i are mj*K, -mj*K on (x,v)_i, (x,v)_j and rows of body j are -mi*K,
 // mi*K, so jac_ij * [J_i; J_j] = [mj u; -mi u] with u = K (J_i - J_j), plus
-// the two mass columns (PREC in nbg_layout.cuh).  That is 54 FP64
-// operations per column instead of 144 for the dense 12x12 block; the
-// product is rounded differently from a dense BLAS product, which the
-// reference's BLAS leaves unspecified anyway.
+// the two mass columns (PREC in nbg_layout.cuh): 36 products instead of 144
+// for the dense 12x12 block; the product is rounded differently from a dense
+// BLAS product, which the reference's BLAS leaves unspecified anyway.
 #pragma once
 #include "nbg_operators.cuh"
 
 namespace nbg {
 
+// The reference's folds and compensated row updates as it has them: what the
+// tests hold against; the consumer's steps below normalise instead.
+//
 // Kahan fold with a zero addend (comp_sum_matrix! on a zero entry).
 __device__ __forceinline__ void fold(double& s, double& e) {
   double t = s + e;

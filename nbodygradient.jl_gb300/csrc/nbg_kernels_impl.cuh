@@ -2,13 +2,18 @@
 // launchers.  Included only by nbg_inst.cu, which instantiates them for one
 // body count N per translation unit (the units compile in parallel).
 //
-// Work decomposition (one launch pair per chunk of K steps):
-//   orbit_chunk_kernel<N>     one lane per system: x, v, dq/dt, transit search
-//                             (src/transits/timing.jl:3-109); writes the step
-//                             operator records, tt and per-transit adjoint rows
-//   jacobian_chunk_kernel<N>  one lane per (system, column of jac_step): applies
-//                             the records with Kahan summation and turns each
-//                             transit's adjoint row into dtdq0 entries
+// Work decomposition, per chunk of K steps:
+//   orbit_chunk_kernel<N>     one lane per system (nbg_orbit_team.cuh: a team, or a
+//                             block's lanes): x, v, transit detection
+//                             (src/transits/timing.jl:3-28); writes the pairs'
+//                             captures, the snapshots and the search tasks
+//   transit_kernel<N>         one lane per search (nbg_search.cuh: a block's lanes;
+//                             transit_kick_kernel with kick pairs): tt and the
+//                             per-transit adjoint rows (timing.jl:31-193)
+//   operator_*_kernel<N>      captures and snapshots into the step's records
+//   jacobian_chunk_kernel<N>  one lane per (system, column of jac_step), or
+//   jacobian_rows_kernel<N>   six: apply the records, form dq/dt of the last
+//                             step and each transit's dtdq0 entries
 // Systems are grouped by (N, grad, kick pattern) so that every warp runs one
 // control-flow path; within a group systems are sorted longest first.
 #pragma once

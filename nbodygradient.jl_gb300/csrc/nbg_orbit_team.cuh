@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
 
 // ------------------------------------------------------------ pairs on lanes
 //
-// Orbit producer for latency-bound chunks (at most max(32, SMs / 2) systems of
-// the group still running): one block per system (two systems of two or three
+// Orbit producer for latency-bound chunks (up to lanes_limit systems of the
+// group still running): one block per system (two systems of two or three
 // bodies), sixteen lanes per pair solve.
 // A warp issues one FP64 instruction per 64 cycles however independent its
 // instructions are, and with few systems nothing else fills the SM, so a step
