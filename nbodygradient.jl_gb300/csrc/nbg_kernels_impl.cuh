@@ -926,11 +926,17 @@ void launch_lanes(const GroupArgs& g, int chunk, cudaStream_t st) {
 template <int N>
 int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   // Without a layout of the caller's (nbg_set_producer_layout) a full group's
-  // one-lane warps go two to a block: one warp alone needs registers that three
-  // consumer blocks leave on no SM, and its block waits for one of theirs to end
-  // (4096 three-body systems over 512 steps: 94.5 -> 87.7 ms; two and four
-  // bodies within 1 %).
-  const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.S >= 2048) ? 2 : 1;
+  // one-lane warps go three to a block: one warp alone needs registers that three
+  // consumer blocks leave on no SM, and its block waits for one of theirs to end;
+  // which sizes that hits depends on how the consumer's last wave ends. One, two,
+  // three, four warps a block, ms, with derivatives:
+  // N = 3 512 steps 1600 systems 44.3, 44.3, 43.1, 40.4, 1900 61.6, 46.9, 47.0, 47.2,
+  // 2300 63.3, 63.4, 48.9, 49.0, 3100 75.6, 75.9, 76.0, 77.1, 4096 92.1, 85.5, 81.4, 80.2;
+  // N = 2 1024 steps 3000 systems 53.5, 53.6, 40.8, 40.9, 4096 59.0, 59.2, 59.5, 60.2;
+  // N = 4 256 steps 1700 systems 58.8, 47.7, 47.3, 47.6, 2048 66.9, 67.3, 67.2, 68.6.
+  // Without derivatives there is no consumer, and one warp a block is the fastest:
+  // N = 3 1024 steps 4096 systems 53.8, 54.3, 55.5, 58.7; N = 4 512 steps 53.3, 53.9, 54.7, 56.9.
+  const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.grad && g.S >= 1024) ? 3 : 1;
   if (g.wide) {
     if (g.kick) launch_lanes<N, true>(g, chunk, st);
     else launch_lanes<N, false>(g, chunk, st);

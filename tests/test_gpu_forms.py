@@ -106,9 +106,9 @@ def test_sizes_where_the_form_changes(n, systems_per_sm, beside):
             assert np.array_equal(full.view(k, q), small.view(k, q % 5)), (k, q)
 
 
-@pytest.mark.parametrize("count", [2047, 2048, 2051])
+@pytest.mark.parametrize("count", [1023, 1024, 2051])
 def test_full_group_of_one_lane_producers(count):
-    """From 2048 systems on the one-lane producer takes two warps a block."""
+    """From 1024 systems on, with derivatives, the one-lane producer takes three warps a block."""
     few, hs = systems(3, 7)
     states, hh = [few[q % 7] for q in range(count)], [hs[q % 7] for q in range(count)]
     same(run(states, hh, 9, -1, ntt=2), run(states, hh, 9, 0, ntt=2, layout=(1, 0, 0)))
