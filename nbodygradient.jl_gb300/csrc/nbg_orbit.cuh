@@ -366,13 +366,15 @@ __device__ __forceinline__ void plain_phic(Sys<N>& s, double* a, double h, uint6
 // M (a_i - a_j)' with M = fac1 (3 r r^T - r^2), and only a_d and the pairs with
 // d enter the accelerations' change: one lane per (step, body) needs no
 // 3N x 4N array and no other lane, about 110 FP64 instructions a pair.
-template <int N>
+// POS = false: the mass column alone.
+template <int N, bool POS = true>
 __device__ __forceinline__ void phi_columns(const double* x, const double* a, const double* m, double h,
                                             uint64_t kick, int d, double* acc) {
   // change of each body's acceleration by x_d (symmetric: xx, xy, xz, yy, yz, zz) and by m_d
   double blk[N][9];
   double own[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   const double md = m[d];
+  constexpr int P0 = POS ? 0 : 3;
 #pragma unroll 1
   for (int i = 0; i < N; i++) {
 #pragma unroll
@@ -386,7 +388,7 @@ __device__ __forceinline__ void phi_columns(const double* x, const double* a, co
     const double gx = g5 * r[0], gy = g5 * r[1], gz = g5 * r[2];
     const double T[6] = {fma(gx, r[0], -f2), gx * r[1], gx * r[2], fma(gy, r[1], -f2), gy * r[2], fma(gz, r[2], -f2)};
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
+    for (int q = 0; q < (POS ? 6 : 0); q++) {
       blk[i][q] = -(md * T[q]);
       own[q] = fma(m[i], T[q], own[q]);
     }
@@ -408,14 +410,14 @@ __device__ __forceinline__ void phi_columns(const double* x, const double* a, co
         aij[k] = a[3 * i + k] - a[3 * j + k];
       }
 #pragma unroll
-      for (int q = 0; q < 9; q++) D[q] = blk[i][q] - blk[j][q];
+      for (int q = P0 ? 6 : 0; q < 9; q++) D[q] = blk[i][q] - blk[j][q];
       const double r2 = fma(r[2], r[2], fma(r[1], r[1], r[0] * r[0]));
       const double ri = rsqrt_fast(r2), ri2 = ri * ri;
       const double fac1 = (coeff * ri) * (ri2 * ri2), f3 = 3.0 * fac1, fr = fac1 * r2;
       double G[3][4];
       const double col[4][3] = {{D[0], D[1], D[2]}, {D[1], D[3], D[4]}, {D[2], D[4], D[5]}, {D[6], D[7], D[8]}};
 #pragma unroll
-      for (int p = 0; p < 4; p++) {
+      for (int p = P0; p < 4; p++) {
         const double c = f3 * fma(r[2], col[p][2], fma(r[1], col[p][1], r[0] * col[p][0]));
 #pragma unroll
         for (int k = 0; k < 3; k++) G[k][p] = fma(r[k], c, -(fr * col[p][k]));
@@ -431,8 +433,8 @@ __device__ __forceinline__ void phi_columns(const double* x, const double* a, co
           const double F = fac1 * fma(r[k], fac2, -(r2 * aij[k]));
           const double e = sg * fma(q5, F, -(fac1 * fma(q3, r[k], 2.0 * aij[k]))), f = sg * (f3 * r[k]);
 #pragma unroll
-          for (int p = 0; p < 3; p++) G[k][p] = fma(f, aij[p], fma(e, r[p], G[k][p]));
-          G[k][k] = G[k][k] + diag;
+          for (int p = P0; p < 3; p++) G[k][p] = fma(f, aij[p], fma(e, r[p], G[k][p]));
+          if (POS) G[k][k] = G[k][k] + diag;
           G[k][3] = fma(fg, r[k], G[k][3]);
           acc[12 * (d == i ? j : i) + 4 * k + 3] += (d == i) ? -F : F;
         }
@@ -441,7 +443,7 @@ __device__ __forceinline__ void phi_columns(const double* x, const double* a, co
 #pragma unroll
       for (int k = 0; k < 3; k++)
 #pragma unroll
-        for (int p = 0; p < 4; p++) {
+        for (int p = P0; p < 4; p++) {
           acc[12 * i + 4 * k + p] = fma(mj, G[k][p], acc[12 * i + 4 * k + p]);
           acc[12 * j + 4 * k + p] = fma(mi, G[k][p], acc[12 * j + 4 * k + p]);
         }
