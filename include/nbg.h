@@ -467,7 +467,7 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc_
  * warps per SM).  A tuning knob; results do not depend on it. */
 int nbg_set_orbit_lanes(nbg_context* ctx, int systems_per_warp);
 
-/* Form of the orbit producer for groups without kick pairs: -1 automatic
+/* Forms of the kernels (a team in groups without kick pairs only): -1 automatic
  * (default: one lane per system up to four bodies and a team of N/2 lanes
  * per system from N = 5 on, each with the wide forms in latency-bound chunks),
  * 0 one lane per system, 1 a team for every N, 2 the wide forms for
@@ -490,7 +490,7 @@ int nbg_set_orbit_team(nbg_context* ctx, int mode);
  * their shared memory exceeds the SM's 227 KB, so smem_kb = 200 with
  * guard_kb = 32 keeps the throughput kernels off the SMs that run the
  * latency-bound producer.  Default: no shared memory held, one warp a block,
- * two in a one-lane group of 2048 systems or more. */
+ * three in a one-lane group with derivatives of 1024 systems or more. */
 int nbg_set_producer_layout(nbg_context* ctx, int warps_per_block, int smem_kb, int guard_kb);
 
 /* Profiling (no reference counterpart).

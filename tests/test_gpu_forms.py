@@ -140,3 +140,26 @@ def test_initial_conditions_packed_and_alone():
     for got, ic in zip(nbg.init_nbody_batch(ics), ics):
         for a, b in zip(got, nbg.init_nbody_batch([ic])[0]):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 8])
+@pytest.mark.parametrize("grad", [True, False])
+def test_search_forms_agree_on_transit_parameters(n, grad):
+    """The three adjoint rows of a search on one lane and on a block's lanes."""
+    els, hs, _ = W.batch_uneven(1, seed=600 + n, nmin=n, nmax=n)
+    h, tmax = hs[0], 70 * hs[0]
+    ctx, out = nbg.default_context(), []
+    try:
+        for mode in (0, 2):
+            ctx.set_orbit_team(mode)
+            ic = W.ic_of(els[0])
+            s, tp = nbg.State(ic), nbg.TransitParameters(tmax, ic)
+            nbg.Integrator(nbg.ahl21, h, 0.0, tmax)(s, tp, grad=grad)
+            out.append((s, tp))
+    finally:
+        ctx.set_orbit_team(-1)
+    (s0, a), (s1, b) = out
+    assert a.count.sum() > 0 and np.array_equal(a.count, b.count)
+    assert np.array_equal(s0.x, s1.x) and np.array_equal(a.ttbv, b.ttbv)
+    if grad:
+        assert np.array_equal(a.dtbvdq0, b.dtbvdq0) and np.array_equal(a.dtbvdelements, b.dtbvdelements)
