@@ -767,8 +767,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   };
   auto orbit_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    const bool tail = active_at(q, c) <= tail_max;
-    if (tail) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
+    if (active_at(q, c) <= tail_limit(g.N, ctx->sm_count)) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
     gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= lanes_limit(g.N, g.grad, ctx->sm_count)) ? 1 : 0;
     return gx;
   };
@@ -891,7 +890,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
           return rc;
         if (c >= 2) NBG_CUDA(cudaStreamWaitEvent(sp, ev_done, 0));
         NBG_CUDA(cudaMemsetAsync(g.task_count, 0, sizeof(int), sp));
-        if (active_at(q, c) <= tail_max) tail_any = true;
+        if (active_at(q, c) <= tail_limit(g.N, ctx->sm_count)) tail_any = true;
         if ((rc = timed_on(sp, 0, [&] { return kOrbit[g.N](orbit_args(q, g, c), (int)c, sp); }))) return rc;
         NBG_CUDA(cudaEventRecord(ev_orb, sp));
         NBG_CUDA(cudaStreamWaitEvent(stt, ev_orb, 0));

@@ -8,12 +8,13 @@
 // The translation unit is compiled with --fmad=false: every product and sum
 // rounds on its own but where fma() is written.
 //
-// GPU-specific structure: this chip issues one FP64 instruction per SM and
-// about 20 clocks, and one warp at most one per 64, so a drift costs what its
-// FP64 instructions cost.  kep_solve writes it in the universal variable s
-// with the functions G_n(beta, s) = s^n c_n(beta s^2) from two short
-// polynomials, takes its start from an FP32 solve (the FP32 pipes are idle
-// beside the FP64 one) and needs one FP64 evaluation of Kepler's equation.
+// What moves x and v (kep_solve, and the steps in nbg_orbit.cuh) rounds
+// operation by operation as the reference's expressions do, with correctly
+// rounded division and square root: whether a transit search's iterates repeat
+// within their limit hangs on the last digit of x and v, and with it the
+// status word NBG_STATUS_NEWTON_ITMAX.  What only the Jacobian reads
+// (kep_derivatives and on) is free in its rounding and takes fused products and
+// reciprocals of one ulp.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -29,14 +30,6 @@ __device__ __forceinline__ double jsign(double x) { return x > 0.0 ? 1.0 : (x < 
 // comp_sum (src/utils.jl:16-23)
 __device__ __forceinline__ void kahan(double& s, double& e, double a) {
   e = e + a;
-  double t = s + e;
-  e = (s - t) + e;
-  s = t;
-}
-
-// The same for the product f a, which is not rounded on its own.
-__device__ __forceinline__ void kahan_fma(double& s, double& e, double f, double a) {
-  e = fma(f, a, e);
   double t = s + e;
   e = (s - t) + e;
   s = t;
@@ -176,18 +169,17 @@ __device__ __forceinline__ GH gh_functions(double gamma, double beta, double sqb
 }
 
 // What a drift leaves for its Jacobian (jac_delxv_gamma! returns the same
-// quantities, ahl21.jl:888): the universal variable s = gamma / sqrt|beta|
-// and the functions of it.
+// quantities, ahl21.jl:888): gamma = s sqrt|beta| and the functions of it.
 struct KepParams {
-  double s, g1, g2, g3, dfdt, fm1, gmh, dgdtm1, r0, r, r0inv, rinv, k, h, beta, eta, zeta;
+  double gamma, g1, g2, g3, dfdt, fm1, gmh, dgdtm1, r0, r, r0inv, rinv, k, h, beta, eta, zeta;
 };
 
-// Drift over |beta| s^2 > KEP_ZMAX (a step of an eighth of the period or
-// more), or one whose solve below has not converged: the half-angle iteration
-// of jac_delxv_gamma! (ahl21.jl:766-890) with its closed forms.
+// jac_delxv_gamma! (ahl21.jl:766-890): Kepler drift of the relative orbit
+// (x0, v0) with k = G (m_i + m_j) over h; writes delxv (position and velocity
+// differences, finish - start minus the drift terms).
 template <bool DRIFT_FIRST>
-__device__ __noinline__ void kep_solve_general(const double* x0, const double* v0, double k, double h, double* delxv,
-                                               KepParams& P) {
+__device__ __noinline__ void kep_solve(const double* x0, const double* v0, double k, double h, double* delxv,
+                                       KepParams& P) {
   double rt0 = x0[0] - h * v0[0], rt1 = x0[1] - h * v0[1], rt2 = x0[2] - h * v0[2];
   double r0 = DRIFT_FIRST ? sqrt(rt0 * rt0 + rt1 * rt1 + rt2 * rt2) : sqrt(x0[0] * x0[0] + x0[1] * x0[1] + x0[2] * x0[2]);
   double r0inv = 1.0 / r0;
@@ -259,7 +251,7 @@ __device__ __noinline__ void kep_solve_general(const double* x0, const double* v
   }
   for (int j = 0; j < 3; j++) delxv[j] = fm1 * x0[j] + gmh * v0[j];
   for (int j = 0; j < 3; j++) delxv[3 + j] = dfdt * x0[j] + dgdtm1 * v0[j];
-  P.s = gamma / sqb; P.g1 = g1bs; P.g2 = g2bs; P.g3 = g3bs;
+  P.gamma = gamma; P.g1 = g1bs; P.g2 = g2bs; P.g3 = g3bs;
   P.dfdt = dfdt; P.fm1 = fm1; P.gmh = gmh; P.dgdtm1 = dgdtm1; P.r0 = r0; P.r = r; P.r0inv = r0inv; P.rinv = rinv;
   P.k = k; P.h = h; P.beta = beta0; P.eta = eta; P.zeta = zeta;
 }
@@ -279,148 +271,6 @@ __device__ __forceinline__ double stumpff(double z) {
   for (int k = 6; k >= 0; k--) p = fma(-z, p, inv_factorial(NN + 2 * k));
   return p;
 }
-// c_2, c_3 or c_4, a lane's own (n = 0, 1, 2)
-__device__ __forceinline__ double stumpff234(double z, int n) {
-  double p = n == 0 ? inv_factorial(16) : n == 1 ? inv_factorial(17) : inv_factorial(18);
-#pragma unroll
-  for (int k = 6; k >= 0; k--)
-    p = fma(-z, p, n == 0 ? inv_factorial(2 + 2 * k) : n == 1 ? inv_factorial(3 + 2 * k) : inv_factorial(4 + 2 * k));
-  return p;
-}
-
-// FP64 to FP32 (rounded to zero; tiny to zero, huge to infinity) and back by
-// their bit patterns: a conversion instruction runs on the FP64 pipe (0.058 a
-// clock and SM, as an FMA), these on the integer pipes (1.8), and the start
-// needs no rounding.  A zero or subnormal float comes back as about 1e-38.
-__device__ __forceinline__ float to_float(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), mag = hi & 0x7fffffffu;
-  unsigned f = __funnelshift_l(lo, mag, 3) - 0xc0000000u;
-  f = mag < 0x38100000u ? 0u : mag >= 0x47f00000u ? 0x7f800000u : f;
-  return __uint_as_float(f | (hi & 0x80000000u));
-}
-__device__ __forceinline__ double to_double(float x) {
-  const unsigned f = __float_as_uint(x), mag = f & 0x7fffffffu;
-  return __hiloint2double((int)(((mag >> 3) + 0x38000000u) | (f & 0x80000000u)), (int)(f << 29));
-}
-
-// FP32 start of the drift's solve.  With sigma = s r0 / h Kepler's equation
-// r0 s + eta G2 + zeta G3 = h reads sigma + a sigma^2 c_2 + b sigma^3 c_3 = 1
-// at z = w sigma^2; two third-order steps from 1 / (1 + a / 2) leave an error of
-// FP32 rounding for steps up to a tenth of a period.  q: half the ratio of the
-// equation's second to its first derivative at sigma, by s, for the FP64
-// step's second-order term.  Nothing downstream depends on the start beyond
-// the convergence test.
-__device__ __forceinline__ float kep_start(float r0inv, float h, float beta, float eta, float zeta, float* q) {
-  const float t = h * r0inv;
-  const float a = eta * t * r0inv, b = zeta * t * t * r0inv, w = beta * t * t;
-  float sg = a > -1.0f ? __fdividef(1.0f, __fmaf_rn(0.5f, a, 1.0f)) : 1.0f;
-  float half = 0.0f;
-#pragma unroll
-  for (int it = 0; it < 2; it++) {
-    const float s2 = sg * sg, z = w * s2;
-    const float c5 = __fmaf_rn(-z, __fmaf_rn(-z, 2.7557319e-6f, 1.9841270e-4f), 8.3333333e-3f);
-    const float c4 = __fmaf_rn(-z, __fmaf_rn(-z, __fmaf_rn(-z, 2.7557319e-7f, 2.4801587e-5f), 1.3888889e-3f), 4.1666667e-2f);
-    const float c3 = __fmaf_rn(-z, c5, 1.6666667e-1f), c2 = __fmaf_rn(-z, c4, 0.5f);
-    const float c1 = __fmaf_rn(-z, c3, 1.0f), c0 = __fmaf_rn(-z, c2, 1.0f);
-    const float f = __fmaf_rn(b * s2 * sg, c3, __fmaf_rn(a * s2, c2, sg - 1.0f));
-    const float inv = __fdividef(1.0f, __fmaf_rn(b * s2, c2, __fmaf_rn(a * sg, c1, 1.0f)));
-    const float d = f * inv;
-    half = 0.5f * inv * __fmaf_rn(b * sg, c1, a * c0);
-    sg = __fmaf_rn(-d, __fmaf_rn(d, half, 1.0f), sg);
-  }
-  *q = __fdividef(half, t);
-  return sg;
-}
-
-// jac_delxv_gamma! (ahl21.jl:766-890): Kepler drift of the relative orbit
-// (x0, v0) with k = G (m_i + m_j) over h; writes delxv (position and velocity
-// differences, finish - start minus the drift terms).
-//
-// Same quantities as the reference, other steps to them: 86 FP64 instructions
-// (103 for the drift that comes last) where the half-angle iteration took about
-// 480, and 800 for a hyperbolic pair, most of them in five evaluations of sine
-// and cosine (sinh and exp) and in divisions.  FP64 step at the FP32 start:
-// F = r0 s + eta G2 + zeta G3 - h, u = F / r, ds = -(u + u^2 F'' / 2 r); the
-// next term is below u^3 / s^2, so the step that is at most KEP_STEP s long is
-// the last and the G_n move to s + ds by their Taylor series,
-// dG_n / ds = G_{n-1}.  Against binary128 over 3000 draws delxv is off by
-// 2.8e-16 rms (the half-angle iteration: 4.2e-16), star-planet and planet pairs
-// alike.  With kep_derivatives and phi_columns a lone 3-body system's 2000
-// steps went from 241 to 120 ms, a lone 8-body system's 400 from 261 to 167 ms,
-// 4096 three-body systems over 2000 steps from 745 to 532 ms.
-constexpr double KEP_STEP = 0x1p-20;
-template <bool DRIFT_FIRST>
-__device__ __forceinline__ void kep_solve(const double* x0, const double* v0, double k, double h, double* delxv,
-                                          KepParams& P) {
-  double rt[3];
-#pragma unroll
-  for (int q = 0; q < 3; q++) rt[q] = DRIFT_FIRST ? fma(-h, v0[q], x0[q]) : x0[q];
-  const double rr = fma(rt[2], rt[2], fma(rt[1], rt[1], rt[0] * rt[0]));
-  const double vv = fma(v0[2], v0[2], fma(v0[1], v0[1], v0[0] * v0[0]));
-  const double eta = fma(rt[2], v0[2], fma(rt[1], v0[1], rt[0] * v0[0]));
-  const double r0inv = rsqrt_fast(rr);
-  const double r0 = rr * r0inv;
-  const double kr0 = k * r0inv;
-  const double beta = fma(2.0, kr0, -vv);
-  const double zeta = fma(-r0, beta, k);
-  const double t = h * r0inv;
-  float q2;
-  const float sg = kep_start(to_float(r0inv), to_float(h), to_float(beta), to_float(eta), to_float(zeta), &q2);
-  const double q = to_double(q2);
-  double s = t * to_double(sg), ds, y, g0, g1, g2, g3, g4 = 0.0;
-  int iter = 0;
-  bool done = false;
-  do {
-    const double ss = s * s, z = beta * ss;
-    g2 = ss * stumpff<2>(z);
-    g3 = (ss * s) * stumpff<3>(z);
-    if (!DRIFT_FIRST) g4 = (ss * ss) * stumpff<4>(z);
-    g0 = fma(-beta, g2, 1.0);
-    g1 = fma(-beta, g3, s);
-    const double F = fma(zeta, g3, fma(eta, g2, fma(r0, s, -h)));
-    const double r = fma(zeta, g2, fma(eta, g1, r0));
-    y = rcp_seed(r);
-    const double u = F * y;
-    ds = -fma(u, fma(q, u, fma(-r, y, 1.0)), u);
-    s = s + ds;
-    if (!(fabs(z) <= 4.0 * KEP_ZMAX)) break;
-    done = fabs(u) <= KEP_STEP * fabs(s) && fabs(z) <= KEP_ZMAX;
-  } while (!done && ++iter < 6);
-  if (!done) {
-    kep_solve_general<DRIFT_FIRST>(x0, v0, k, h, delxv, P);
-    return;
-  }
-  const double hd = 0.5 * ds;
-  if (!DRIFT_FIRST) g4 = fma(ds, fma(hd, g2, g3), g4);
-  const double g3n = fma(ds, fma(hd, g1, g2), g3);
-  g2 = fma(ds, fma(hd, g0, g1), g2);
-  g3 = g3n;
-  g1 = fma(-beta, g3, s);
-  const double r = fma(zeta, g2, fma(eta, g1, r0));
-  const double rinv = rcp_from(r, y);
-  const double kr = k * rinv;
-  const double dfdt = -(kr0 * rinv) * g1;
-  double fm1, gmh, dgdtm1;
-  if (DRIFT_FIRST) {
-    fm1 = -(kr0 * g2);
-    gmh = kr0 * fma(h, g2, -(r0 * g3));
-    dgdtm1 = (kr0 * rinv) * fma(h, g1, -(r0 * g2));
-  } else {
-    const double h1 = fma(s, g3, -2.0 * g4), h2 = fma(s, g2, -g3);
-    fm1 = kr * fma(-kr0, h1, g2);
-    gmh = kr * fma(r0, h2, eta * h1);
-    dgdtm1 = -(kr * g2);
-  }
-  // the large product (v0's is smaller by h's order) is the one that is not rounded
-#pragma unroll
-  for (int q = 0; q < 3; q++) {
-    delxv[q] = fma(fm1, x0[q], gmh * v0[q]);
-    delxv[3 + q] = fma(dfdt, x0[q], dgdtm1 * v0[q]);
-  }
-  P.s = s; P.g1 = g1; P.g2 = g2; P.g3 = g3;
-  P.dfdt = dfdt; P.fm1 = fm1; P.gmh = gmh; P.dgdtm1 = dgdtm1; P.r0 = r0; P.r = r; P.r0inv = r0inv; P.rinv = rinv;
-  P.k = k; P.h = h; P.beta = beta; P.eta = eta; P.zeta = zeta;
-}
 
 // Derivatives of a solved drift (compute_jacobian_gamma!, ahl21.jl:896-1139,
 // gives the same 6x8 block; here by the chain rule through s).
@@ -435,28 +285,34 @@ __device__ __forceinline__ void kep_solve(const double* x0, const double* v0, do
 // mass derivatives that does not cancel against the masses' own weights.
 // About 150 FP64 instructions, a quarter of the expanded expressions'; the terms
 // are sums of like sign or of different order in h, so none loses digits: K is
-// off by 5.6e-16 rms of its 3x3 blocks (expanded: 8.9e-16), Psi by 1.1e-15
-// (8.8e-16), the derivative by h by 3.0e-16 (4.0e-16), against binary128.
+// off by 7.1e-16 rms of its 3x3 blocks (expanded: 8.9e-16), Psi by 1.2e-15
+// (8.8e-16), the derivative by h by 3.7e-16 (4.0e-16), against binary128.
 struct KepDeriv {
   double a[5], b[5], c[5], d[5];
 };
 template <bool DRIFT_FIRST, bool WITH_H>
 __device__ __forceinline__ void kep_derivatives(const KepParams& P, KepDeriv& o) {
-  const double s = P.s, g1 = P.g1, g2 = P.g2, g3 = P.g3, r0 = P.r0, r0inv = P.r0inv, rinv = P.rinv, k = P.k;
-  const double beta = P.beta, eta = P.eta, zeta = P.zeta, h = P.h;
+  const double r0 = P.r0, r0inv = P.r0inv, rinv = P.rinv, k = P.k;
+  const double beta = P.beta, eta = P.eta, h = P.h, zeta = fma(-r0, beta, k);
+  const double s = P.gamma * rsqrt_fast(fabs(beta));
   const double ss = s * s, z = beta * ss, s3 = ss * s, s4 = ss * ss;
-  double g4, g5, g6;
-  if (fabs(z) <= 1.01 * KEP_ZMAX) {
-    const double c6 = stumpff<6>(z);
-    g4 = s4 * fma(-z, c6, 1.0 / 24.0);
-    g5 = (s4 * s) * stumpff<5>(z);
+  double g2, g3, g4, g5, g6;
+  if (fabs(z) <= KEP_ZMAX) {
+    const double c6 = stumpff<6>(z), c5 = stumpff<5>(z), c4 = fma(-z, c6, 1.0 / 24.0);
+    g2 = ss * fma(-z, c4, 0.5);
+    g3 = s3 * fma(-z, c5, 1.0 / 6.0);
+    g4 = s4 * c4;
+    g5 = (s4 * s) * c5;
     g6 = (s4 * ss) * c6;
   } else {
     const double bi = 1.0 / beta;
+    g2 = P.g2;
+    g3 = P.g3;
     g4 = (0.5 * ss - g2) * bi;
     g5 = (s3 * (1.0 / 6.0) - g3) * bi;
     g6 = (s4 * (1.0 / 24.0) - g4) * bi;
   }
+  const double g1 = fma(-beta, g3, s);
   const double g0 = fma(-beta, g2, 1.0);
   const double h1 = fma(s, g3, -2.0 * g4), h2 = fma(s, g2, -g3);
   const double b1 = -0.5 * h2, b2 = -0.5 * h1, b3 = 0.5 * fma(3.0, g5, -(s * g4));  // dG_n / dbeta

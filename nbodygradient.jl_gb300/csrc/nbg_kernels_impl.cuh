@@ -423,7 +423,8 @@ __device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh)
         if (p % 6 != l || !live) continue;
         double rij[3], f[3];
         for (int k = 0; k < 3; k++) rij[k] = xs.get(3 * N * snap + 3 * i + k) - xs.get(3 * N * snap + 3 * j + k);
-        phis_accel(rij, rsqrt_fast(norm2(rij)), f);
+        const double r2 = norm2(rij);
+        phis_accel(rij, r2, sqrt(r2), f);
         for (int k = 0; k < 3; k++) F[(3 * p + k) * C + col] = f[k];
       }
     __syncwarp();
@@ -523,7 +524,7 @@ __device__ void dq_columns(const GroupArgs& g, int chunk, int first, double* sh)
           aij[k] = a[(3 * i + k) * C] - a[(3 * j + k) * C];
         }
         const double r2 = norm2(rij);
-        phis_corr(rij, r2, rsqrt_fast(r2), aij, is_kick(p) ? 0.0 : mass(i) + mass(j),
+        phis_corr(rij, r2, sqrt(r2), aij, is_kick(p) ? 0.0 : mass(i) + mass(j),
                   is_kick(p) ? phic_coeff(h) : phis_coeff(h), f);
         for (int k = 0; k < 3; k++) G[(3 * p + k) * C + col] = f[k];
       }
@@ -929,17 +930,16 @@ void launch_lanes(const GroupArgs& g, int chunk, cudaStream_t st) {
 template <int N>
 int launch_orbit(const GroupArgs& g, int chunk, cudaStream_t st) {
   // Without a layout of the caller's (nbg_set_producer_layout) a full group's
-  // one-lane warps go three to a block: one warp alone needs registers that three
-  // consumer blocks leave on no SM, and its block waits for one of theirs to end;
-  // which sizes that hits depends on how the consumer's last wave ends. One, two,
-  // three, four warps a block, ms, with derivatives:
-  // N = 3 512 steps 1600 systems 44.3, 44.3, 43.1, 40.4, 1900 61.6, 46.9, 47.0, 47.2,
-  // 2300 63.3, 63.4, 48.9, 49.0, 3100 75.6, 75.9, 76.0, 77.1, 4096 92.1, 85.5, 81.4, 80.2;
-  // N = 2 1024 steps 3000 systems 53.5, 53.6, 40.8, 40.9, 4096 59.0, 59.2, 59.5, 60.2;
-  // N = 4 256 steps 1700 systems 58.8, 47.7, 47.3, 47.6, 2048 66.9, 67.3, 67.2, 68.6.
-  // Without derivatives there is no consumer, and one warp a block is the fastest:
-  // N = 3 1024 steps 4096 systems 53.8, 54.3, 55.5, 58.7; N = 4 512 steps 53.3, 53.9, 54.7, 56.9.
-  const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.grad && g.S >= 1024) ? 3 : 1;
+  // one-lane warps go three to a block, four at two bodies: one warp alone needs
+  // registers that three consumer blocks leave on no SM, and its block waits for
+  // one of theirs to end; which sizes that hits depends on how the consumer's
+  // last wave ends. One, two, three, four warps a block, ms, with derivatives:
+  // N = 2 1024 steps 1300 systems 64.3, 64.5, 63.7, 67.0, 3000 81.4, 75.7, 70.6, 73.5,
+  // 4096 85.0, 83.9, 103.3, 77.0; N = 3 256 steps 1024 52.4, 52.6, 51.3, 53.3,
+  // 3100 64.9, 64.9, 63.3, 65.5, 512 steps 4096 144.2, 139.4, 140.2, 139.1;
+  // N = 4 128 steps 1700 61.5, 61.3, 60.1, 61.8, 3000 74.9, 71.6, 71.3, 80.2.
+  // Without derivatives there is no consumer, and one warp a block is the fastest.
+  const int W = g.pwarps > 0 ? g.pwarps : (!g.team && g.grad && g.S >= 1024) ? (N == 2 ? 4 : 3) : 1;
   if (g.wide) {
     if (g.kick) launch_lanes<N, true>(g, chunk, st);
     else launch_lanes<N, false>(g, chunk, st);

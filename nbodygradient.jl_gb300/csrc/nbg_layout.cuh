@@ -56,23 +56,36 @@ __host__ __device__ inline int trec_size(int N, int tbv) { return tbv ? 21 * N +
 __host__ __device__ inline int snap_count(bool kick) { return kick ? 3 : 2; }
 
 
-// Up to how many running systems of a group the latency-bound forms are taken.  A lanes-form level costs its warp one system's pairs where the
-// one-lane and team forms carry 32 or 32 / (N/2) systems, so the line is where
-// the pairs' levels, (2N - 3) per system, fill the SMs' FP64 pipes.  Measured,
-// us a step, (one lane or team) -> lanes, rows consumer with up to four bodies:
-// N = 3 512 systems 71 -> 60, 1024 84 -> 87; N = 4 512 134 -> 107, 1024 162 -> 173;
-// N = 6 768 440 -> 380; N = 8 384 674 -> 606, 768 935 -> 933; N = 10 384 948 -> 867,
-// 768 1427 -> 1487.  Without derivatives nothing else wants the pipes: N = 3 1024
-// 57 -> 33, 2048 62 -> 58; N = 4 1024 138 -> 80, 2048 112 -> 141; N = 8 768 511 -> 296.
-__host__ inline int rows_limit(int N, int sms) {
-  // six lanes a column: level with one lane a column at 64 columns an SM (96 up
-  // to four bodies, whose lanes form it keeps company); N = 8 96 systems
-  // 417 -> 387, 192 484 -> 510; N = 10 96 627 -> 549, 192 747 -> 792
-  return (N <= 4 ? 96 : 64) * sms / (7 * N);
-}
+// Up to how many running systems of a group the latency-bound forms are taken.
+//
+// Rows consumer: six lanes a column are level with one at 64 columns an SM (96
+// up to four bodies).  us a step: N = 8 96 systems 417 -> 387, 192 484 -> 510;
+// N = 10 96 systems 627 -> 549, 192 747 -> 792.
+__host__ inline int rows_limit(int N, int sms) { return (N <= 4 ? 96 : 64) * sms / (7 * N); }
+
+// Systems whose producer blocks fit on half of the SMs, one block each (two
+// systems of up to three bodies to a block, lanes_systems): as many get SMs of
+// their own.
+__host__ inline int tail_limit(int N, int sms) { return (N <= 3 ? 2 : 1) * (sms / 2 > 32 ? sms / 2 : 32); }
+
+// Lanes producer: a level costs a warp per pair where the one-lane and team
+// forms carry 32 or 32 / (N/2) systems, so the line is where the levels, 2N - 3
+// per system, fill the FP64 pipes, alone or beside the consumer.  us a step, one
+// lane or team -> lanes:
+//   with derivatives    N = 2 512 systems 63 -> 39, 1024 65 -> 63;
+//                       N = 3 152 182 -> 100 on SMs of its own, 200 172 -> 210;
+//                       N = 4 512 423 -> 306, 1024 460 -> 586;
+//                       N = 5 1024 1307 -> 1140, 2048 1383 -> 1638;
+//                       N = 6 512 1434 -> 1055, 1024 1626 -> 1724;
+//                       N = 8 384 2118 -> 1600, 768 2360 -> 2629;
+//                       N = 10 256 2735 -> 1896, 512 3450 -> 3972
+//   without             N = 2 768 59 -> 46, 1024 59 -> 64; N = 3 768 172 -> 170, 1024 174 -> 186;
+//                       N = 4 768 379 -> 323, 1024 381 -> 450; N = 5 512 498 -> 459, 768 630 -> 705;
+//                       N = 8 384 1112 -> 1079, 576 1140 -> 1305; N = 10 256 1380 -> 1288, 384 2273 -> 2426
 __host__ inline int lanes_limit(int N, bool grad, int sms) {
-  if (!grad) return N <= 4 ? (48 * sms / (2 * N - 3) < 2048 ? 48 * sms / (2 * N - 3) : 2048) : 96 * sms / (2 * N - 3);
-  return N <= 4 ? rows_limit(N, sms) : 64 * sms / (2 * N - 3);
+  if (!grad) return N <= 4 ? 5 * sms : 24 * sms / (2 * N - 3);
+  if (N == 3) return tail_limit(N, sms);
+  return N <= 4 ? rows_limit(N, sms) : 48 * sms / (2 * N - 3);
 }
 
 struct GroupArgs {

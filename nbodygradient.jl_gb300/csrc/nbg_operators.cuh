@@ -39,7 +39,7 @@ __device__ __forceinline__ void pair_of_slot(int q, int npk, uint64_t kick, int*
 }
 
 // kepler_driftij_gamma!'s Jacobian part for one pair from its capture; h2 is
-// the drift's half step.  k, zeta and G1 are formed again, as kep_solve does.
+// the drift's half step.
 // With dh.p the derivative by h follows there.
 template <bool DRIFT_FIRST>
 __device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int coff, double m_i, double m_j, double h2,
@@ -49,11 +49,9 @@ __device__ __forceinline__ void pair_record_from_capture(const Rec& cap, int cof
   for (int q = 0; q < PCAP; q++) v[q] = cap.get(coff + q);
   const double *x0 = v, *v0 = v + 3;
   KepParams P;
-  P.s = v[6]; P.g2 = v[7]; P.g3 = v[8]; P.r0 = v[9]; P.r0inv = v[10]; P.rinv = v[PCAP_RINV]; P.beta = v[12]; P.eta = v[13];
+  P.gamma = v[6]; P.g2 = v[7]; P.g3 = v[8]; P.r0 = v[9]; P.r0inv = v[10]; P.rinv = v[PCAP_RINV]; P.beta = v[12]; P.eta = v[13];
   P.fm1 = v[14]; P.gmh = v[15]; P.dfdt = v[16]; P.dgdtm1 = v[17];
   P.k = GNEWT * (m_i + m_j);
-  P.zeta = fma(-P.r0, P.beta, P.k);
-  P.g1 = fma(-P.beta, P.g3, P.s);
   P.h = h2;
   KepDeriv D;
   double K[36], psi[6];

@@ -79,7 +79,7 @@ __device__ __forceinline__ void reset_last(Work<N>& w) {
 template <int N>
 __device__ __forceinline__ void drift(Sys<N>& s, double h) {
 #pragma unroll
-  for (int q = 0; q < 3 * N; q++) kahan_fma(s.x[q], s.xe[q], h, s.v[q]);
+  for (int q = 0; q < 3 * N; q++) kahan(s.x[q], s.xe[q], h * s.v[q]);
 }
 
 // kickfast! (ahl21.jl:337-386 / ahl21_no_grad.jl:35-56)
@@ -261,36 +261,46 @@ __device__ void phic(Sys<N>& s, Work<N>& w, double h, uint64_t kick) {
     }
 }
 
-// phisalpha! (ahl21.jl:558-700 / ahl21_no_grad.jl:110-158) for Kepler pairs,
-// one pair at a time: the accelerations, then the velocity corrections.
-__device__ __forceinline__ double norm2(const double* r) { return fma(r[2], r[2], fma(r[1], r[1], r[0] * r[0])); }
-__device__ __forceinline__ void phis_accel(const double* rij, double rinv, double* f) {
-  const double f2 = (GNEWT * rinv) * (rinv * rinv);
+// A pair's terms of the steps without gradient, each rounded as the reference's
+// expressions are: G r / r^3 of the correctors (ahl21_no_grad.jl:120-127)
+__device__ __forceinline__ double norm2(const double* r) { return r[0] * r[0] + r[1] * r[1] + r[2] * r[2]; }
+__device__ __forceinline__ void phis_accel(const double* rij, double r2, double r1, double* f) {
+  const double fac2 = GNEWT / (r2 * r1);
 #pragma unroll
-  for (int k = 0; k < 3; k++) f[k] = f2 * rij[k];
+  for (int k = 0; k < 3; k++) f[k] = fac2 * rij[k];
 }
-__device__ __forceinline__ void phis_corr(const double* rij, double r2, double rinv, const double* aij, double mij,
+// the corrections (ahl21_no_grad.jl:140-152; with mij = 0 those of :88-99)
+__device__ __forceinline__ void phis_corr(const double* rij, double r2, double r1, const double* aij, double mij,
                                           double coeff, double* f) {
-  const double ri2 = rinv * rinv;
-  const double fac1 = (coeff * rinv) * (ri2 * ri2);
-  const double ardot = fma(aij[2], rij[2], fma(aij[1], rij[1], aij[0] * rij[0]));
-  const double fac2 = fma((2.0 * GNEWT) * mij, rinv, 3.0 * ardot);
+  const double ardot = aij[0] * rij[0] + aij[1] * rij[1] + aij[2] * rij[2];
+  const double fac1 = coeff / (r2 * r2 * r1);
+  const double fac2 = mij != 0.0 ? 2.0 * GNEWT * mij / r1 + 3.0 * ardot : 3.0 * ardot;
 #pragma unroll
-  for (int k = 0; k < 3; k++) f[k] = fac1 * fma(rij[k], fac2, -(r2 * aij[k]));
+  for (int k = 0; k < 3; k++) f[k] = fac1 * (rij[k] * fac2 - r2 * aij[k]);
+}
+// 1 / r^3 of a kick pair (ahl21_no_grad.jl:42-43)
+__device__ __forceinline__ double kick_r3inv(const double* rij) {
+  const double r2inv = 1.0 / norm2(rij);
+  return r2inv * sqrt(r2inv);
 }
 __device__ __forceinline__ double phis_coeff(double h) {  // alpha = 2 (ahl21.jl:47)
   return 2.0 * (h * h * h) / 96.0 * 2.0 * GNEWT;
 }
+__device__ __forceinline__ double phic_coeff(double h) { return h * h * h / 36.0 * GNEWT; }
+
+// phisalpha! (ahl21.jl:558-700 / ahl21_no_grad.jl:110-158) for Kepler pairs,
+// one pair at a time: the accelerations, then the velocity corrections.
 template <int N>
 __device__ __forceinline__ void phis_accel_pair(const Sys<N>& s, double* a, int i, int j) {
   double rij[3], f[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-  phis_accel(rij, rsqrt_fast(norm2(rij)), f);
+  const double r2 = norm2(rij);
+  phis_accel(rij, r2, sqrt(r2), f);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    a[3 * i + k] = fma(-s.m[j], f[k], a[3 * i + k]);
-    a[3 * j + k] = fma(s.m[i], f[k], a[3 * j + k]);
+    a[3 * i + k] = a[3 * i + k] - s.m[j] * f[k];
+    a[3 * j + k] = a[3 * j + k] + s.m[i] * f[k];
   }
 }
 template <int N>
@@ -302,11 +312,11 @@ __device__ __forceinline__ void phis_kick_pair(Sys<N>& s, const double* a, int i
     rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
   }
   const double r2 = norm2(rij);
-  phis_corr(rij, r2, rsqrt_fast(r2), aij, mij, coeff, f);
+  phis_corr(rij, r2, sqrt(r2), aij, mij, coeff, f);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], s.m[j], f[k]);
-    kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -s.m[i], f[k]);
+    kahan(s.v[3 * i + k], s.ve[3 * i + k], s.m[j] * f[k]);
+    kahan(s.v[3 * j + k], s.ve[3 * j + k], (-s.m[i]) * f[k]);
   }
 }
 template <int N>
@@ -329,28 +339,40 @@ __device__ __forceinline__ void plain_kick(Sys<N>& s, double h, uint64_t kick) {
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++) {
       if (!((kick >> pair_bit(i, j, N)) & 1)) continue;
-      double rij[3], f[3];
+      double rij[3];
 #pragma unroll
       for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
-      phis_accel(rij, rsqrt_fast(norm2(rij)), f);
+      const double fac2 = h * GNEWT * kick_r3inv(rij);
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], -(h * s.m[j]), f[k]);
-        kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], h * s.m[i], f[k]);
+        const double fac = fac2 * rij[k];
+        kahan(s.v[3 * i + k], s.ve[3 * i + k], (-s.m[j]) * fac);
+        kahan(s.v[3 * j + k], s.ve[3 * j + k], s.m[i] * fac);
       }
     }
 }
 // phic! without gradient (ahl21_no_grad.jl:62-104): a kick over 2h/3 and the
 // correction, between the pairs of the mask.
-__device__ __forceinline__ double phic_coeff(double h) { return h * h * h / 36.0 * GNEWT; }
 template <int N>
 __device__ __forceinline__ void plain_phic(Sys<N>& s, double* a, double h, uint64_t kick) {
-  plain_kick<N>(s, 2.0 * h / 3.0, kick);
 #pragma unroll
   for (int q = 0; q < 3 * N; q++) a[q] = 0.0;
   for (int i = 0; i < N - 1; i++)
-    for (int j = i + 1; j < N; j++)
-      if ((kick >> pair_bit(i, j, N)) & 1) phis_accel_pair<N>(s, a, i, j);
+    for (int j = i + 1; j < N; j++) {
+      if (!((kick >> pair_bit(i, j, N)) & 1)) continue;
+      double rij[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
+      const double r3inv = kick_r3inv(rij);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const double fac = GNEWT * rij[k] * r3inv, facv = fac * 2.0 * h / 3.0;
+        kahan(s.v[3 * i + k], s.ve[3 * i + k], (-s.m[j]) * facv);
+        kahan(s.v[3 * j + k], s.ve[3 * j + k], s.m[i] * facv);
+        a[3 * i + k] = a[3 * i + k] - s.m[j] * fac;
+        a[3 * j + k] = a[3 * j + k] + s.m[i] * fac;
+      }
+    }
   for (int i = 0; i < N - 1; i++)
     for (int j = i + 1; j < N; j++)
       if ((kick >> pair_bit(i, j, N)) & 1) phis_kick_pair<N>(s, a, i, j, 0.0, phic_coeff(h));
@@ -470,7 +492,7 @@ __device__ void phisalpha_operator(const Sys<N>& s, Work<N>& w, double h, uint64
         rij[k] = s.x[3 * i + k] - s.x[3 * j + k];
       }
       const double r2 = norm2(rij);
-      phis_corr(rij, r2, rsqrt_fast(r2), aij, s.m[i] + s.m[j], coeff, f);
+      phis_corr(rij, r2, sqrt(r2), aij, s.m[i] + s.m[j], coeff, f);
       for (int k = 0; k < 3; k++) {
         w.dqop[3 * i + k] = fma(hi3 * s.m[j], f[k], w.dqop[3 * i + k]);
         w.dqop[3 * j + k] = fma(-hi3 * s.m[i], f[k], w.dqop[3 * j + k]);
@@ -481,7 +503,7 @@ __device__ void phisalpha_operator(const Sys<N>& s, Work<N>& w, double h, uint64
 // Writes one solved pair's capture (pair_record_from_capture reads it).
 __device__ __forceinline__ void put_capture(const Rec& cap, int coff, const double* x0, const double* v0,
                                             const KepParams& P) {
-  const double pv[PCAP] = {x0[0], x0[1], x0[2], v0[0],  v0[1], v0[2], P.s,   P.g2,   P.g3,
+  const double pv[PCAP] = {x0[0], x0[1], x0[2], v0[0],  v0[1], v0[2], P.gamma, P.g2, P.g3,
                            P.r0,  P.r0inv, P.rinv, P.beta, P.eta, P.fm1, P.gmh, P.dfdt, P.dgdtm1};
 #pragma unroll
   for (int q = 0; q < PCAP; q++) cap.put(coff + q, pv[q]);
@@ -505,17 +527,17 @@ __device__ __forceinline__ bool kepler_pair(Sys<N>& s, int i, int j, double h2, 
   }
   kep_solve<DRIFT_FIRST>(x0, v0, gm, h2, delxv, P);
   if (cap.p) put_capture(cap, coff, x0, v0, P);
-  const double mijinv = rcp_fast(mij);
+  const double mijinv = 1.0 / mij;
   const double mi = s.m[i] * mijinv, mj = s.m[j] * mijinv;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    kahan_fma(s.x[3 * i + k], s.xe[3 * i + k], mj, delxv[k]);
-    kahan_fma(s.x[3 * j + k], s.xe[3 * j + k], -mi, delxv[k]);
+    kahan(s.x[3 * i + k], s.xe[3 * i + k], mj * delxv[k]);
+    kahan(s.x[3 * j + k], s.xe[3 * j + k], (-mi) * delxv[k]);
   }
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    kahan_fma(s.v[3 * i + k], s.ve[3 * i + k], mj, delxv[3 + k]);
-    kahan_fma(s.v[3 * j + k], s.ve[3 * j + k], -mi, delxv[3 + k]);
+    kahan(s.v[3 * i + k], s.ve[3 * i + k], mj * delxv[3 + k]);
+    kahan(s.v[3 * j + k], s.ve[3 * j + k], (-mi) * delxv[3 + k]);
   }
   return true;
 }

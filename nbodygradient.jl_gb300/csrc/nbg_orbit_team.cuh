@@ -53,7 +53,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run,
   if (run)
     for (int q = t; q < 3 * N; q += L) {
       if (vs.p) vs.put(q, s.v[q]);
-      kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+      kahan(s.x[q], s.xe[q], h2 * s.v[q]);
     }
   __syncwarp();
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
@@ -90,7 +90,7 @@ __device__ __forceinline__ void team_step(Sys<N>& s, double* a, int t, bool run,
   if (run)
     for (int q = t; q < 3 * N; q += L) {
       if (vs.p) vs.put(3 * N + q, s.v[q]);
-      kahan_fma(s.x[q], s.xe[q], h2, s.v[q]);
+      kahan(s.x[q], s.xe[q], h2 * s.v[q]);
     }
   __syncwarp();
 }
@@ -187,27 +187,29 @@ __global__ void __launch_bounds__(PROD_BS * PROD_MAX_WARPS) orbit_team_kernel(Gr
 // ------------------------------------------------------------ pairs on lanes
 //
 // Orbit producer for latency-bound chunks (up to lanes_limit systems of the
-// group still running): one block per system (two systems of two or three
-// bodies), sixteen lanes per pair solve.
+// group still running): one block per system and one warp per pair of a level,
+// or two systems of two or three bodies (whose levels have one pair) to a warp.
 // A warp issues one FP64 instruction per 64 cycles however independent its
 // instructions are, and with few systems nothing else fills the SM, so a step
 // takes as long as its longest warp's FP64 instructions; spreading a solve's
-// independent pieces over lanes makes them one instruction each:
+// independent pieces over sixteen lanes makes them one instruction each:
 //   * lanes 0-5 hold the pair's relative coordinates, lanes 0-5 and 6-11 the
 //     two bodies' (one subtraction, one Kahan sum instead of six and twelve);
-//   * the three dot products, the two Stumpff polynomials, G2 and G3, G0 and
-//     G1, Kepler's equation and r, and the four coefficients of the result are
-//     evaluated side by side, each by its own lanes, and shuffled to all;
-//   * the pairs of a level (equal i + j, see above) go to the block's half
-//     warps, and phisalpha!'s pair terms to one lane each before each body sums
-//     its own in pair order.
-// 57 FP64 instructions a level instead of a one-lane solve's 146.  Every value is
-// formed by the operations of kep_solve, phisalpha and kahan_fma in the same
-// order, so the results are bitwise those of the other forms.
-// One system alone, before (a pair solve on one lane or two) and after: 301 steps
-// of five bodies without derivatives 30.2 -> 15.4 ms, 2000 steps of three bodies
-// with transits 97 -> 67 ms (then bound by the consumer, jacobian_rows_kernel).
-__host__ __device__ constexpr int lanes_warps(int N) { return (N / 2 + 1) / 2 > 0 ? (N / 2 + 1) / 2 : 1; }
+//   * the three dot products, 1 / beta and 6 / zeta, the cubic's coefficients,
+//     the sine and cosine series, numerator and denominator of the Newton
+//     update, G1, G3, H1 and H2, the sum of r and the four coefficients of the
+//     result are evaluated side by side, each by its own lanes, and shuffled to
+//     all;
+//   * phisalpha!'s pair terms go to one lane each before each body sums its own
+//     in pair order.
+// Every value is formed by the operations of kep_solve, phisalpha and kahan in
+// the same order, so the results are bitwise those of the other forms.  From
+// four bodies on a pair has a warp, whose upper lanes repeat the lower ones and
+// write nothing (an FP64 instruction costs the same): a bound and a hyperbolic
+// pair in one warp would wait for each other.
+// One system alone, a solve on one lane or two -> here: 301 steps of five bodies
+// without derivatives 84 -> 56 ms, 400 of eight with transits 261 -> 146 ms.
+__host__ __device__ constexpr int lanes_warps(int N) { return N <= 3 ? 1 : N / 2; }
 // A level of two or three bodies has one pair: a system then takes a half warp.
 __host__ __device__ constexpr int lanes_systems(int N) { return N <= 3 ? 2 : 1; }
 __host__ __device__ constexpr int lanes_each(int N) { return 32 * lanes_warps(N) / lanes_systems(N); }
@@ -218,7 +220,7 @@ struct LanesShared {
   double a[3 * N], ac[3 * N], g[N];
   long long cnt[N];
   double pk[N * (N - 1) / 2], pmi[N * (N - 1) / 2], pmj[N * (N - 1) / 2];  // k, m_i / (m_i + m_j), m_j / (m_i + m_j)
-  double f[N * (N - 1) / 2][3];
+  double f[N * (N - 1) / 2][3], fk[N * (N - 1) / 2][3];
 };
 
 template <int N>
@@ -227,24 +229,40 @@ __device__ __forceinline__ void lanes_sync() {
   else __syncthreads();
 }
 
-// One pair of a sweep on the sixteen lanes hl = 0..15 of a half warp.  Both
-// halves of a warp run the same instructions, so that its two pairs share their
-// issue slots; a half without a pair (act false) repeats pair (0, 1) and writes
-// nothing.  Only a solve that needs more than one FP64 step leaves the other
-// half.
+// The coefficients of G3, H1 and H2 (kGHCoef), by lane.
+template <int Q>
+__device__ __forceinline__ double gh_coef(int n) {
+  constexpr double g3[11] = {0x1.0000000000000p+0, 0x1.999999999999ap-5, 0x1.3813813813814p-10, 0x1.1566abc011567p-16, 0x1.42cb40df7f3abp-23, 0x1.08db48ebe51c7p-30, 0x1.42df6ed66ca17p-38, 0x1.2fe15942481f8p-46, 0x1.c6ee8e9c1e203p-55, 0x1.154ab3925b815p-63, 0x1.189470e50aa13p-72};
+  constexpr double h1[11] = {0x1.0000000000000p+0, 0x1.1111111111111p-4, 0x1.d41d41d41d41dp-10, 0x1.bbd779334ef0bp-16, 0x1.0cfeb60f94b0ep-22, 0x1.c60a33dd88c31p-30, 0x1.1a8380fb9f0d4p-37, 0x1.0e1da4acb1e32p-45, 0x1.99704d261b1cfp-54, 0x1.f82abadb8f19bp-63, 0x1.0132bcd1f4692p-71};
+  constexpr double h2[11] = {0x1.0000000000000p+0, 0x1.999999999999ap-4, 0x1.d41d41d41d41dp-9, 0x1.1566abc011567p-14, 0x1.937e11175f095p-21, 0x1.8d48ed61d7aabp-28, 0x1.1a8380fb9f0d4p-35, 0x1.2fe15942481f8p-43, 0x1.ffcc606fa1e43p-52, 0x1.5a9d6076f261ap-60, 0x1.81cc1b3aee9dbp-69};
+  return n == 0 ? g3[Q] : n == 1 ? h1[Q] : h2[Q];
+}
+template <int Q>
+__device__ __forceinline__ double gh_horner_of(int n, double x2, double p) {
+  p = fma(p, x2, gh_coef<Q>(n));
+  if constexpr (Q > 0) return gh_horner_of<Q - 1>(n, x2, p);
+  return p;
+}
+
+// One pair of a sweep on the sixteen lanes hl = 0..15 of a half warp.  The whole
+// warp runs the same instructions: its other half has the other system's pair
+// (N <= 3) or repeats this one (write false).  A half without a pair (act
+// false) repeats pair (0, 1) of its own system and writes nothing.
 template <int N, bool DRIFT_FIRST>
 __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, bool act, double h, const Rec& cap,
-                                           int coff, int hl) {
+                                           int coff, int hl, bool write) {
+  constexpr unsigned ALL = 0xffffffffu;
   const int pb = pair_bit(i, j, N);
   const double k = sh.pk[pb];
   if (k == 0.0) {
-    if (act && cap.p && hl == 0) cap.put(coff + PCAP_RINV, 0.0);
+    if (act && write && cap.p && hl == 0) cap.put(coff + PCAP_RINV, 0.0);
     act = false;
   }
-  unsigned mask = 0xffffffffu;
-  auto from = [&](double v, int src) { return __shfl_sync(mask, v, src, 16); };
+  if (!__any_sync(ALL, act)) return;
+  auto from = [](double v, int src) { return __shfl_sync(ALL, v, src, 16); };
   double* q = sh.st.x;  // x, v, xe, ve of Sys<N> in a row, 3N each
-  const int c = hl % 6, k3 = hl % 3;
+  const int c = hl % 6, k3 = hl % 3, w4 = hl & 3;
+  const bool odd = hl & 1;
   const int at = (c < 3 ? 0 : 3 * N) + k3;
   const double qi = q[at + 3 * i], qj = q[at + 3 * j], d = qi - qj;
   // lanes 0-5 carry body i's coordinates, 6-11 body j's
@@ -259,7 +277,7 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
   }
   const double xk = k3 == 0 ? X[0] : k3 == 1 ? X[1] : X[2], vk = k3 == 0 ? V[0] : k3 == 1 ? V[1] : V[2];
   if (DRIFT_FIRST) {
-    const double rt = fma(-h, vk, xk);
+    const double rt = xk - h * vk;
 #pragma unroll
     for (int w = 0; w < 3; w++) R[w] = from(rt, w);
   } else {
@@ -274,112 +292,184 @@ __device__ __forceinline__ void lanes_pair(LanesShared<N>& sh, int i, int j, boo
       A[w] = k3 == 1 ? V[w] : R[w];
       B[w] = k3 == 0 ? R[w] : V[w];
     }
-    const double dot = fma(A[2], B[2], fma(A[1], B[1], A[0] * B[0]));
+    const double dot = A[0] * B[0] + A[1] * B[1] + A[2] * B[2];
     rr = from(dot, 0);
     vv = from(dot, 1);
     eta = from(dot, 2);
   }
-  const double r0inv = rsqrt_fast(rr);
-  const double r0 = rr * r0inv;
-  const double kr0 = k * r0inv;
-  const double beta = fma(2.0, kr0, -vv);
-  const double zeta = fma(-r0, beta, k);
-  const double t = h * r0inv;
-  float q2;
-  const float sg = kep_start(to_float(r0inv), to_float(h), to_float(beta), to_float(eta), to_float(zeta), &q2);
-  const double q2d = to_double(q2);
-  const int w4 = hl & 3;
-  const bool odd = hl & 1;
-  double s = t * to_double(sg), ds, y, g0, g1, g2, g3, g4 = 0.0;
-  bool done = false, far = false;
-  auto iterate = [&]() {
-    const double ss = s * s, z = beta * ss;
-    const double scale = ss * (w4 == 0 ? 1.0 : w4 == 1 ? s : ss);
-    const double g = scale * stumpff234(z, w4);  // G2, G3, G4 by w4
-    g2 = from(g, 0);
-    g3 = from(g, 1);
-    if (!DRIFT_FIRST) g4 = from(g, 2);
-    const double g01 = fma(-beta, odd ? g3 : g2, odd ? s : 1.0);
-    g0 = from(g01, 0);
-    g1 = from(g01, 1);
-    const double first = fma(r0, s, -h);  // in the shuffles' shadow
-    const double fr = fma(zeta, odd ? g2 : g3, fma(eta, odd ? g1 : g2, odd ? r0 : first));
-    const double r = from(fr, 1);
-    y = rcp_seed(r);
-    const double ue = fma(odd ? -r : fr, y, odd ? 1.0 : 0.0);  // F / r to the seed's digits, and what they lack
-    const double u = from(ue, 0);
-    ds = -fma(u, fma(q2d, u, from(ue, 1)), u);
-    s = s + ds;
-    far = !(fabs(z) <= 4.0 * KEP_ZMAX);
-    done = fabs(u) <= KEP_STEP * fabs(s) && fabs(z) <= KEP_ZMAX;
-  };
-  iterate();
-  if (act && !done) {
-    mask = 0xffffu << (threadIdx.x & 16);
-    for (int iter = 1; iter < 6 && !done && !far; iter++) iterate();
-    mask = 0xffffffffu;
-  }
-  __syncwarp();
-  double del, val;  // val: fm1, gmh, dfdt, dgdtm1 by hl & 3
-  KepParams P;
+  const double r0 = sqrt(rr);
+  const double r0inv = 1.0 / r0;
+  const double beta = 2.0 * k * r0inv - vv;
+  const double signb = jsign(beta);
+  const bool plus = signb > 0.0;  // products with signb = +-1 are changes of sign
+  const double sqb = sqrt(signb * beta);
+  const double rb = r0 * beta;
+  const double zeta = k - rb;
+  // the solve's other branches (zeta or beta zero): all of it on every lane
+  const bool plain = act && !(zeta != 0.0 && beta != 0.0);
+  const bool solve = act && !plain;
+  double betainv, gamma;
   {
-    const double hd = 0.5 * ds;
-    if (!DRIFT_FIRST) g4 = fma(ds, fma(hd, g2, g3), g4);
-    const double gn = fma(ds, fma(hd, odd ? g1 : g0, odd ? g2 : g1), odd ? g3 : g2);
-    g2 = from(gn, 0);
-    g3 = from(gn, 1);
-    g1 = fma(-beta, g3, s);
-    const double r = fma(zeta, g2, fma(eta, g1, r0));
-    const double rinv = rcp_from(r, y);
-    const double krr = kr0 * rinv;
-    double pre, mul;
-    bool neg;
-    if (DRIFT_FIRST) {
-      const double ga = (w4 & 2) ? g1 : g2, gb = (w4 & 2) ? g2 : g3;
-      const double both = fma(h, ga, -(r0 * gb));
-      pre = (w4 & 2) ? krr : kr0;
-      mul = (w4 & 1) ? both : ga;
-      neg = !(w4 & 1);
+    const double inv = (odd ? 6.0 : 1.0) / (odd ? zeta : beta);
+    betainv = from(inv, 0);
+    const double zinv = from(inv, 1);
+    const double hs = plus ? -h : h;
+    // cubic1's arguments a, b, c on lanes 0, 1, 2
+    const double first = (w4 == 2 ? hs : 0.5) * (w4 == 2 ? beta : eta);
+    const double arg = ((w4 == 1 ? rb : first) * (w4 == 1 ? signb : sqb)) * zinv;
+    const double third = arg * THIRD;
+    const double b = from(arg, 1), cc = from(arg, 2), a3 = from(third, 0);
+    const double a3sq = a3 * a3;
+    const double Q = a3sq - from(third, 1);
+    const double pr = (odd ? -a3 : a3sq) * (odd ? b : a3);
+    const double Rc = from(pr, 0) + 0.5 * (from(pr, 1) + cc);
+    const double sq = (odd ? Q : Rc) * (odd ? Q : Rc);
+    const double R2 = from(sq, 0), Q3 = from(sq, 1) * Q;
+    if (R2 < Q3) {
+      gamma = -cc / b;
     } else {
-      const double kr = k * rinv;
-      const double h12 = fma(s, odd ? g2 : g3, odd ? -g3 : -2.0 * g4);
-      const double h1 = from(h12, 0), h2 = from(h12, 1);
-      const double eh = eta * h1;
-      const double ab = fma(w4 == 0 ? -kr0 : r0, w4 == 0 ? h1 : h2, w4 == 0 ? g2 : eh);
-      pre = (w4 == 2) ? krr : kr;
-      mul = (w4 < 2) ? ab : (w4 == 2) ? g1 : g2;
-      neg = w4 >= 2;
+      const double A = (-jsign(Rc)) * cbrt(fabs(Rc) + sqrt(R2 - Q3));
+      const double B = (A == 0.0) ? 0.0 : Q / A;
+      gamma = A + B - a3;
     }
-    val = pre * mul;
-    if (neg) val = -val;
-    P.s = s; P.g1 = g1; P.g2 = g2; P.g3 = g3; P.r0 = r0; P.r0inv = r0inv; P.rinv = rinv; P.beta = beta; P.eta = eta;
-    P.zeta = zeta;
-    const double cx = from(val, c < 3 ? 0 : 2), cv = from(val, c < 3 ? 1 : 3);
-    del = fma(cx, xk, cv * vk);
   }
-  if (act && !done) {
+  // the Newton update's numerator on even lanes, its denominator on odd ones
+  const double e2 = plus ? 2.0 * eta : -(2.0 * eta);
+  const double pc = sqb * (odd ? h : e2);
+  const double c3 = from(pc, 0), c4 = -from(pc, 1) * beta;
+  const double z2 = 2.0 * zeta;
+  const double a1 = odd ? (plus ? z2 : -z2) : k, a2 = odd ? c3 : -z2;
+  const bool ell = beta > 0.0;
+  const bool any_ell = __any_sync(ALL, solve && ell), any_hyp = __any_sync(ALL, solve && !ell);
+  double sx = 0.0, cx = 0.0;
+  auto functions = [&](double x) {  // sine and cosine of x, or their hyperbolic counterparts
+    if (any_ell) {
+      const double x2 = x * x;
+      double p = odd ? -0x1.6827863b97d97p-53 : 0x1.952c77030ad4ap-49;
+      p = fma(p, x2, odd ? 0x1.ae7f3e733b81fp-45 : -0x1.ae7f3e733b81fp-41);
+      p = fma(p, x2, odd ? -0x1.93974a8c07c9dp-37 : 0x1.6124613a86d09p-33);
+      p = fma(p, x2, odd ? 0x1.1eed8eff8d898p-29 : -0x1.ae64567f544e4p-26);
+      p = fma(p, x2, odd ? -0x1.27e4fb7789f5cp-22 : 0x1.71de3a556c734p-19);
+      p = fma(p, x2, odd ? 0x1.a01a01a01a01ap-16 : -0x1.a01a01a01a01ap-13);
+      p = fma(p, x2, odd ? -0x1.6c16c16c16c17p-10 : 0x1.1111111111111p-7);
+      p = fma(p, x2, odd ? 0x1.5555555555555p-5 : -0x1.5555555555555p-3);
+      const double b = x2 * (odd ? x2 : x);
+      const double one = fma(-0.5, x2, 1.0);
+      const double v = fma(b, p, odd ? one : x);
+      sx = from(v, 0);
+      cx = from(v, 1);
+      if (ell && fabs(x) > 0.78539816339744831) sincos(x, &sx, &cx);
+    }
+    if (any_hyp && !ell) {
+      sx = sinh(x);
+      cx = exp(-x) + sx;
+    }
+  };
+  {
+    double gamma1 = 2.0 * gamma, gamma2 = 3.0 * gamma;
+    int iter = 0;
+    bool done = !solve;
+#pragma unroll 1
+    while (__any_sync(ALL, !done)) {
+      if (!done) {
+        gamma2 = gamma1;
+        gamma1 = gamma;
+      }
+      functions(0.5 * gamma);
+      const double ss = sx * sx;
+      double acc = a1 * (odd ? ss : gamma) + (a2 * sx) * cx;
+      acc = acc + (odd ? rb : c3 * ss);
+      const double acc4 = acc + c4;
+      acc = odd ? acc : acc4;
+      const double num = from(acc, 0), den = from(acc, 1);
+      const double next = gamma - num / den;
+      if (!done) {
+        gamma = next;
+        iter += 1;
+        done = iter >= 20 || gamma == gamma2 || gamma == gamma1;
+      }
+    }
+  }
+  functions(0.5 * gamma);
+  const bool big = solve && !(gamma < 0.5);
+  double g0, g1, g2, g3, h1 = 0.0, h2 = 0.0;
+  {  // lanes by w4: G3, H1, H2 and, on 3, G2, beta G2 and G1
+    const double sq = (w4 == 3 ? sx : gamma) * (w4 == 3 ? sx : gamma);
+    const double x2 = plus ? -sq : sq, s2 = plus ? 2.0 * sq : -(2.0 * sq);
+    const double p1 = (w4 == 3 ? s2 : w4 == 1 ? beta : w4 == 0 ? 6.0 : 3.0) * (w4 == 3 ? betainv : beta);
+    g2 = from(p1, 3);
+    const double p2 = (w4 == 3 ? beta : p1) * (w4 == 3 ? g2 : w4 == 1 ? 12.0 : sqb);
+    g0 = 1.0 - from(p2, 3);
+    const double num = (w4 == 3 ? 2.0 * sx : w4 == 1 ? x2 : -x2) * (w4 == 3 ? cx : w4 == 1 ? x2 : gamma);
+    const double quot = num / (w4 == 3 ? sqb : p2);
+    g1 = from(quot, 3);
+    const double val = gh_horner_of<9>(w4, x2, gh_coef<10>(w4)) * quot;
+    g3 = from(val, 0);
+    if (!DRIFT_FIRST) {
+      h1 = from(val, 1);
+      h2 = from(val, 2);
+    }
+    if (big) {
+      const GH gh = gh_functions<DRIFT_FIRST ? GH_G3 : (GH_G3 | GH_H1 | GH_H2)>(gamma, beta, sqb);
+      g3 = gh.g3;
+      h1 = gh.h1;
+      h2 = gh.h2;
+    }
+    __syncwarp();
+  }
+  const double rp = (w4 == 0 ? r0 : w4 == 1 ? eta : k) * (w4 == 0 ? g0 : w4 == 1 ? g1 : g2);
+  const double r = from(rp, 0) + from(rp, 1) + from(rp, 2);
+  const double rinv = 1.0 / r;
+  double val;  // fm1, gmh, dfdt, dgdtm1 by w4
+  if (DRIFT_FIRST) {
+    double pre = ((w4 & 1) ? k : -k) * (w4 == 2 ? g1 : r0inv);
+    const double pr = pre * rinv;
+    pre = (w4 & 2) ? pr : pre;
+    const double a = h * (w4 == 1 ? g2 : g1), b = r0 * (w4 == 1 ? g3 : g2);
+    val = pre * (w4 == 0 ? g2 : w4 == 2 ? r0inv : a - b);
+  } else {
+    double pre = (w4 < 2 ? k : -k) * (w4 == 2 ? g1 : rinv);
+    const double pr = pre * rinv;
+    pre = w4 == 2 ? pr : pre;
+    const double a = (w4 == 0 ? k : eta) * (w4 == 0 ? r0inv : h1);
+    const double b = (w4 == 0 ? a : r0) * (w4 == 0 ? h1 : h2);
+    const double in = (w4 == 0 ? g2 : a) + (w4 == 0 ? -b : b);
+    val = pre * (w4 < 2 ? in : w4 == 2 ? r0inv : g2);
+  }
+  double del;
+  {  // the products with x0 on lanes 0-5, with v0 on 6-11
+    const double prod = from(val, (c < 3 ? 0 : 2) + (hl < 6 ? 0 : 1)) * (hl < 6 ? xk : vk);
+    del = from(prod, c) + from(prod, 6 + c);
+  }
+  double cg = gamma, cg2 = g2, cg3 = g3, crinv = rinv;
+  if (plain) {
+    KepParams P;
     double delxv[6];
-    kep_solve_general<DRIFT_FIRST>(X, V, k, h, delxv, P);
+    kep_solve<DRIFT_FIRST>(X, V, k, h, delxv, P);
     val = w4 == 0 ? P.fm1 : w4 == 1 ? P.gmh : w4 == 2 ? P.dfdt : P.dgdtm1;
+    cg = P.gamma;
+    cg2 = P.g2;
+    cg3 = P.g3;
+    crinv = P.rinv;
     del = delxv[0];
 #pragma unroll
     for (int w = 1; w < 6; w++) del = (c == w) ? delxv[w] : del;
   }
-  if (act && hl < 12) {
-    kahan_fma(own_q, own_e, weight, del);
+  if (act && write && hl < 12) {
+    kahan(own_q, own_e, weight * del);
     q[id] = own_q;
     q[6 * N + id] = own_e;
   }
-  if (act && cap.p) {  // in put_capture's order: lanes 0-5 x0 and v0, 6-13 the solve, then 0-3 the coefficients
+  if (act && write && cap.p) {  // in put_capture's order: lanes 0-5 x0 and v0, 6-13 the solve, then 0-3 the coefficients
     double own = d;
-    own = hl == 6 ? P.s : own;
-    own = hl == 7 ? P.g2 : own;
-    own = hl == 8 ? P.g3 : own;
-    own = hl == 9 ? P.r0 : own;
-    own = hl == 10 ? P.r0inv : own;
-    own = hl == 11 ? P.rinv : own;
-    own = hl == 12 ? P.beta : own;
-    own = hl == 13 ? P.eta : own;
+    own = hl == 6 ? cg : own;
+    own = hl == 7 ? cg2 : own;
+    own = hl == 8 ? cg3 : own;
+    own = hl == 9 ? r0 : own;
+    own = hl == 10 ? r0inv : own;
+    own = hl == 11 ? crinv : own;
+    own = hl == 12 ? beta : own;
+    own = hl == 13 ? eta : own;
     double* to = cap.p + (unsigned)((coff + hl) * cap.stride);  // below 2^31: 2 P PCAP slots
     if (hl < 14) *to = own;
     if (hl < 4) to[(unsigned)(14 * cap.stride)] = val;
@@ -394,7 +484,8 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
                                            const Rec& cap, const Rec& xs, const Rec& vs) {
   constexpr int P = N * (N - 1) / 2, T = lanes_each(N);
   static_assert(P <= T && 3 * N <= T, "one lane per pair and per coordinate");
-  const int half = t >> 4, hl = t & 15;
+  const int slot = t / (N <= 3 ? 16 : 32), hl = t & 15;
+  const bool write = N <= 3 || !(t & 16);
   const double h2 = 0.5 * h;
   const bool coord = run && t < 3 * N, pair = run && t < P;
   Sys<N>& st = sh.st;
@@ -407,32 +498,35 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
   const bool kicked = KICK && pair && ((kick >> t) & 1);
   auto pair_at = [&](int o) { return o < b ? pair_bit(o, b, N) : pair_bit(b, o, N); };
   auto is_kick = [&](int o) { return KICK && ((kick >> pair_at(o)) & 1); };
-  double rij[3], r2 = 0.0, rinv = 0.0;
-  auto force = [&](bool which) {  // G r / r^3 of pair t
-    if (!which) return;
+  double rij[3], r2 = 0.0, r1 = 0.0;
+  auto apart = [&]() {
 #pragma unroll
     for (int q = 0; q < 3; q++) rij[q] = st.x[3 * pi + q] - st.x[3 * pj + q];
-    r2 = norm2(rij);
-    rinv = rsqrt_fast(r2);
-    phis_accel(rij, rinv, sh.f[t]);
   };
-  auto kick_v = [&](double hk) {  // the kicked pairs' velocity changes, by body and in pair order
+  auto kick_force = [&](double hk) {  // of pair t over hk
+    if (!kicked) return;
+    apart();
+    const double fac2 = hk * GNEWT * kick_r3inv(rij);
+#pragma unroll
+    for (int q = 0; q < 3; q++) sh.fk[t][q] = fac2 * rij[q];
+  };
+  auto kick_v = [&]() {  // the kicked pairs' velocity changes, by body and in pair order
     if (!coord) return;
     double v = st.v[t], ve = st.ve[t];
     for (int o = 0; o < N; o++)
-      if (o != b && is_kick(o)) kahan_fma(v, ve, o < b ? hk * st.m[o] : -(hk * st.m[o]), sh.f[pair_at(o)][w]);
+      if (o != b && is_kick(o)) kahan(v, ve, (o < b ? st.m[o] : -st.m[o]) * sh.fk[pair_at(o)][w]);
     st.v[t] = v;
     st.ve[t] = ve;
   };
   if (KICK) {
     if (xs.p && coord) xs.put(3 * N + t, st.x[t]);
-    force(kicked);
+    kick_force(h / 6.0);
     lanes_sync<N>();
-    kick_v(h / 6.0);
+    kick_v();
   }
   if (coord) {
     if (vs.p) vs.put(t, st.v[t]);
-    kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+    kahan(st.x[t], st.xe[t], h2 * st.v[t]);
   }
   lanes_sync<N>();
   // a Kepler pair's capture slot: the ones before it in sweep order
@@ -441,23 +535,38 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
 #pragma unroll 1
   for (int lev = 1; lev <= 2 * N - 3; lev++) {
     int i = 0, j = 1;
-    bool act = level_pair<N>(lev, half, &i, &j) && run;
+    bool act = level_pair<N>(lev, slot, &i, &j) && run;
     const int pb = pair_bit(i, j, N);
     if (KICK) act = act && !((kick >> pb) & 1);
-    if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, slot_of(pb) * PCAP, hl);
+    if (__any_sync(0xffffffffu, act)) lanes_pair<N, true>(sh, i, j, act, h2, cap, slot_of(pb) * PCAP, hl, write);
     lanes_sync<N>();
   }
   if (xs.p && coord) xs.put(t, st.x[t]);
-  force(pair);
+  if (pair) {
+    apart();
+    r2 = norm2(rij);
+    r1 = sqrt(r2);
+    if (kicked) {
+      const double r3inv = kick_r3inv(rij);
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const double fac = GNEWT * rij[q] * r3inv;
+        sh.f[t][q] = fac;
+        sh.fk[t][q] = fac * 2.0 * h / 3.0;
+      }
+    } else {
+      phis_accel(rij, r2, r1, sh.f[t]);
+    }
+  }
   lanes_sync<N>();
-  if (KICK) kick_v(2.0 * h / 3.0);
+  if (KICK) kick_v();
   if (coord) {
     double a = 0.0, ac = 0.0;  // by the Kepler pairs and by the kicked ones
     for (int o = 0; o < N; o++)
       if (o != b) {
         const double f = sh.f[pair_at(o)][w], m = o < b ? st.m[o] : -st.m[o];
-        if (is_kick(o)) ac = fma(m, f, ac);
-        else a = fma(m, f, a);
+        if (is_kick(o)) ac = ac + m * f;
+        else a = a + m * f;
       }
     sh.a[t] = a;
     if (KICK) sh.ac[t] = ac;
@@ -469,14 +578,14 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
     double aij[3];
 #pragma unroll
     for (int q = 0; q < 3; q++) aij[q] = a[3 * pi + q] - a[3 * pj + q];
-    phis_corr(rij, r2, rinv, aij, kicked ? 0.0 : st.m[pi] + st.m[pj], kicked ? phic_coeff(h) : phis_coeff(h), sh.f[t]);
+    phis_corr(rij, r2, r1, aij, kicked ? 0.0 : st.m[pi] + st.m[pj], kicked ? phic_coeff(h) : phis_coeff(h), sh.f[t]);
   }
   lanes_sync<N>();
   if (coord) {
     double v = st.v[t], ve = st.ve[t];
     for (int pass = KICK ? 0 : 1; pass < 2; pass++)  // the kicked pairs' corrections, then the Kepler pairs'
       for (int o = 0; o < N; o++)
-        if (o != b && is_kick(o) == (pass == 0)) kahan_fma(v, ve, o < b ? -st.m[o] : st.m[o], sh.f[pair_at(o)][w]);
+        if (o != b && is_kick(o) == (pass == 0)) kahan(v, ve, (o < b ? -st.m[o] : st.m[o]) * sh.f[pair_at(o)][w]);
     st.v[t] = v;
     st.ve[t] = ve;
   }
@@ -484,23 +593,23 @@ __device__ __forceinline__ void lanes_step(LanesShared<N>& sh, int t, bool run, 
 #pragma unroll 1
   for (int lev = 2 * N - 3; lev >= 1; lev--) {
     int i = 0, j = 1;
-    bool act = level_pair<N>(lev, half, &i, &j) && run;
+    bool act = level_pair<N>(lev, slot, &i, &j) && run;
     const int pb = pair_bit(i, j, N);
     if (KICK) act = act && !((kick >> pb) & 1);
     if (__any_sync(0xffffffffu, act))
-      lanes_pair<N, false>(sh, i, j, act, h2, cap, (npk + (npk - 1 - slot_of(pb))) * PCAP, hl);
+      lanes_pair<N, false>(sh, i, j, act, h2, cap, (npk + (npk - 1 - slot_of(pb))) * PCAP, hl, write);
     lanes_sync<N>();
   }
   if (coord) {
     if (vs.p) vs.put(3 * N + t, st.v[t]);
-    kahan_fma(st.x[t], st.xe[t], h2, st.v[t]);
+    kahan(st.x[t], st.xe[t], h2 * st.v[t]);
   }
   lanes_sync<N>();
   if (KICK) {
     if (xs.p && coord) xs.put(6 * N + t, st.x[t]);
-    force(kicked);
+    kick_force(h / 6.0);
     lanes_sync<N>();
-    kick_v(h / 6.0);
+    kick_v();
     lanes_sync<N>();
   }
 }
@@ -519,14 +628,17 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
   const int most = lanes_systems(N) > 1 ? max(nk, __shfl_xor_sync(0xffffffffu, nk, 16)) : nk;
   if (most == 0) return;
   Sys<N>& st = sh.st;
+  // a slot without a system beside one that runs gets ordinary numbers: division
+  // and square root of a zero or a NaN leave the short path, and its half warp
+  // runs with the other's
   if (t < 3 * N) {
-    st.x[t] = valid ? g.x[t * S + s] : 0.0;
-    st.v[t] = valid ? g.v[t * S + s] : 0.0;
+    st.x[t] = valid ? g.x[t * S + s] : (t % 3 == 0) ? t / 3 : 0.0;
+    st.v[t] = valid ? g.v[t * S + s] : (t % 3 == 1) ? 0.01 * (t / 3) : 0.0;
     st.xe[t] = valid ? g.xe[t * S + s] : 0.0;
     st.ve[t] = valid ? g.ve[t * S + s] : 0.0;
   }
   if (t < N) {
-    st.m[t] = valid ? g.m[t * S + s] : 0.0;
+    st.m[t] = valid ? g.m[t * S + s] : 1.0;
     sh.g[t] = valid ? g.gsave[t * S + s] : 0.0;
     sh.cnt[t] = valid ? g.count[t * S + s] : 0;
   }
@@ -537,7 +649,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) orbit_lanes_kernel(GroupA
       i++;
       j += i + 1 - N;
     }
-    const double mij = st.m[i] + st.m[j], inv = rcp_fast(mij);
+    const double mij = st.m[i] + st.m[j], inv = 1.0 / mij;
     sh.pk[t] = GNEWT * mij;
     sh.pmi[t] = st.m[i] * inv;
     sh.pmj[t] = st.m[j] * inv;

@@ -1,8 +1,8 @@
 // nbg_search.cuh -- transit searches of kick-free groups: findtransit!
 // (src/transits/timing.jl:31-109) for a detection queued by the orbit producer.
 //
-// Newton iterations on partial AHL21 steps from the detecting step's start
-// state, on x and v alone, with the physical time derivative of g
+// Newton iterations on partial AHL21 steps from the state at the detecting step's
+// end, on x and v alone, with the physical time derivative of g
 // (gdot_physical) where the reference builds the full gradient step to read g's
 // step derivative: both reach the same root of g to rounding.  With grad the
 // converged partial step's captures become pair records, dq/dt is carried
@@ -25,20 +25,13 @@ namespace nbg {
 
 constexpr int SEARCH_ITMAX = 20;
 
-// Whether a search may stop after a step dt (the one before: prev): the
-// reference stops when an iterate repeats; a step that linear convergence at
-// the rate just seen would follow by one below an ulp of h is the last already.
-__device__ __forceinline__ bool search_done(double dt, double prev, double h, int iter) {
-  return iter > 1 && dt * dt <= 0x1p-54 * fabs(h) * fabs(prev);
-}
-
 // Sky-plane g and its physical time derivative from the two bodies'
 // accelerations (timing.jl:141-144): |dv|^2 plus the relative acceleration.
 template <int N>
 __device__ __forceinline__ double gdot_from(const Sys<N>& s, int i, int j, const double* ai, const double* aj) {
   const double dvx = s.v[3 * j] - s.v[3 * i], dvy = s.v[3 * j + 1] - s.v[3 * i + 1];
   const double dx = s.x[3 * j] - s.x[3 * i], dy = s.x[3 * j + 1] - s.x[3 * i + 1];
-  return fma(dy, aj[1] - ai[1], fma(dx, aj[0] - ai[0], fma(dvy, dvy, dvx * dvx)));
+  return dvx * dvx + dvy * dvy + dx * (aj[0] - ai[0]) + dy * (aj[1] - ai[1]);
 }
 // acceleration of body c by body b in the sky plane
 template <int N>
@@ -46,8 +39,8 @@ __device__ __forceinline__ void sky_pull(const Sys<N>& s, int b, int c, double* 
   double d[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) d[k] = s.x[3 * b + k] - s.x[3 * c + k];
-  const double ri = rsqrt_fast(norm2(d));
-  const double w = (GNEWT * s.m[b]) * (ri * (ri * ri));
+  const double r2 = norm2(d);
+  const double w = GNEWT * s.m[b] / (r2 * sqrt(r2));
   f[0] = w * d[0];
   f[1] = w * d[1];
 }
@@ -334,12 +327,12 @@ __device__ __forceinline__ void put_search(const GroupArgs& g, double* tr, doubl
     tr[(size_t)(7 * N) * S] = gd;
     return;
   }
-  const double vsky = sqrt(fma(dvy, dvy, dvx * dvx));
+  const double vsky = sqrt(dvx * dvx + dvy * dvy);
   tr[(size_t)(21 * N) * S] = gd;
   tr[(size_t)(21 * N + 1) * S] = vsky;
   tr[(size_t)(21 * N + 2) * S] = fma(dvy, qb[4] - qt[4], dvx * (qb[3] - qt[3])) / vsky;
   ttout[1] = vsky;
-  ttout[2] = fma(dy, dy, dx * dx);
+  ttout[2] = dx * dx + dy * dy;
 }
 
 // A task of the queue.
@@ -374,8 +367,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
     const SearchTask k = search_task<N>(g, idx);
     const double* tf = g.task_f + (size_t)idx * (12 * N + 2);
     Sys<N> wk;
-    double a[3 * N], dt0 = k.dt0, prev = 0.0, stmp = 0.0, tt1 = dt0 + 1.0, tt2 = dt0 + 2.0;
-    const double h = g.h[k.s];
+    double a[3 * N], dt0 = k.dt0, stmp = 0.0, tt1 = dt0 + 1.0, tt2 = dt0 + 2.0;
     int iter = 0;
     for (int q = 0; q < N; q++) wk.m[q] = g.m[q * S + k.s];
     auto start = [&]() {
@@ -395,8 +387,7 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       const double dt = -gs / gd;
       kahan(dt0, stmp, dt);
       iter += 1;
-      if (iter >= SEARCH_ITMAX || dt0 == tt1 || dt0 == tt2 || search_done(dt, prev, h, iter)) break;
-      prev = dt;
+      if (iter >= SEARCH_ITMAX || dt0 == tt1 || dt0 == tt2) break;
     }
     if (iter >= SEARCH_ITMAX) atomicOr(g.status + k.s, NBG_STATUS_NEWTON_ITMAX);
     double* ttout = g.tt + g.off_tt[g.sysidx[k.s]] + (long long)(g.tbv ? 3 : 1) * (k.ib + (long long)N * k.c);
@@ -423,8 +414,8 @@ __global__ void __launch_bounds__(TRANSIT_BS) transit_kernel(GroupArgs g, int ch
       // b_sky^2 of the last Newton iteration's state
       const double dvx = wk.v[3 * k.ib] - wk.v[3 * k.ti], dvy = wk.v[3 * k.ib + 1] - wk.v[3 * k.ti + 1];
       const double dx = wk.x[3 * k.ib] - wk.x[3 * k.ti], dy = wk.x[3 * k.ib + 1] - wk.x[3 * k.ti + 1];
-      ttout[1] = sqrt(fma(dvy, dvy, dvx * dvx));
-      ttout[2] = fma(dy, dy, dx * dx);
+      ttout[1] = sqrt(dvx * dvx + dvy * dvy);
+      ttout[2] = dx * dx + dy * dy;
     }
     ttout[0] = k.t + dt0;
   }
@@ -527,7 +518,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
       pj += pi + 1 - N;
     }
     if (t < P) {
-      const double mij = wk.m[pi] + wk.m[pj], inv = rcp_fast(mij);
+      const double mij = wk.m[pi] + wk.m[pj], inv = 1.0 / mij;
       sh.l.pk[t] = GNEWT * mij;
       sh.l.pmi[t] = wk.m[pi] * inv;
       sh.l.pmj[t] = wk.m[pj] * inv;
@@ -541,8 +532,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
       }
       lanes_sync<N>();
     };
-    const double h = g.h[k.s];
-    double dt0 = k.dt0, prev = 0.0, stmp = 0.0, tt1 = dt0 + 1.0, tt2 = dt0 + 2.0;
+    double dt0 = k.dt0, stmp = 0.0, tt1 = dt0 + 1.0, tt2 = dt0 + 2.0;
     int iter = 0;
     bool active = true;
     // every search of the block steps until the last has converged
@@ -572,8 +562,7 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
         const double dt = -gs / gd;
         kahan(dt0, stmp, dt);
         iter += 1;
-        if (iter >= SEARCH_ITMAX || dt0 == tt1 || dt0 == tt2 || search_done(dt, prev, h, iter)) active = false;
-        prev = dt;
+        if (iter >= SEARCH_ITMAX || dt0 == tt1 || dt0 == tt2) active = false;
       }
       lanes_sync<N>();
     }
@@ -700,8 +689,8 @@ __global__ void __launch_bounds__(32 * lanes_warps(N)) transit_lanes_kernel(Grou
     } else if (g.tbv && has && t == 0) {
       const double dvx = wk.v[3 * k.ib] - wk.v[3 * k.ti], dvy = wk.v[3 * k.ib + 1] - wk.v[3 * k.ti + 1];
       const double dx = wk.x[3 * k.ib] - wk.x[3 * k.ti], dy = wk.x[3 * k.ib + 1] - wk.x[3 * k.ti + 1];
-      ttout[1] = sqrt(fma(dvy, dvy, dvx * dvx));
-      ttout[2] = fma(dy, dy, dx * dx);
+      ttout[1] = sqrt(dvx * dvx + dvy * dvy);
+      ttout[2] = dx * dx + dy * dy;
     }
     if (has && t == 0) ttout[0] = k.t + dt0;
     lanes_sync<N>();
