@@ -285,7 +285,7 @@ __device__ __forceinline__ double stumpff(double z) {
 // mass derivatives that does not cancel against the masses' own weights.
 // About 150 FP64 instructions, a quarter of the expanded expressions'; the terms
 // are sums of like sign or of different order in h, so none loses digits: K is
-// off by 7.1e-16 rms of its 3x3 blocks (expanded: 8.9e-16), Psi by 1.2e-15
+// off by 7.1e-16 rms of its 3x3 blocks (expanded: 8.9e-16), Psi by 8.6e-16
 // (8.8e-16), the derivative by h by 3.7e-16 (4.0e-16), against binary128.
 struct KepDeriv {
   double a[5], b[5], c[5], d[5];
@@ -318,9 +318,13 @@ __device__ __forceinline__ void kep_derivatives(const KepParams& P, KepDeriv& o)
   const double b1 = -0.5 * h2, b2 = -0.5 * h1, b3 = 0.5 * fma(3.0, g5, -(s * g4));  // dG_n / dbeta
   const double rp = fma(eta, g0, zeta * g1);                                        // dr / ds
   const double kr0 = k * r0inv;
-  // by r0, eta, beta, k, h: s, r and, at fixed s, G_1, G_2
-  const double ds[5] = {-(g1 * rinv), -(g2 * rinv), -(fma(k, b3, fma(eta, b2, r0 * b1)) * rinv), -(g3 * rinv), rinv};
-  const double rq[4] = {g0, g1, fma(-r0, g2, fma(eta, b1, zeta * b2)), g2};
+  // s, and r at fixed s, by r0, eta, beta, k, h.  By k with beta = 2 k / r0 - v^2
+  // moving along, so that zeta falls as k grows: its terms then differ in order
+  // of h, where those at fixed beta and by beta would cancel to a fifth
+  const double ri2 = 2.0 * r0inv, kb1 = ri2 * b1, kb2 = ri2 * b2, kb3 = ri2 * b3;
+  const double ds[5] = {-(g1 * rinv), -(g2 * rinv), -(fma(k, b3, fma(eta, b2, r0 * b1)) * rinv),
+                        fma(-zeta, kb3, fma(-eta, kb2, g3)) * rinv, rinv};
+  const double rq[4] = {g0, g1, fma(-r0, g2, fma(eta, b1, zeta * b2)), fma(eta, kb1, fma(zeta, kb2, -g2))};
   constexpr int NQ = WITH_H ? 5 : 4;
   const double g2r = g2 * rinv, g1r = g1 * rinv, rr0 = r0inv * rinv;
   double al = 0.0, as = 0.0, bb = 0.0, bs = 0.0, hb1 = 0.0, hb2 = 0.0;
@@ -335,26 +339,29 @@ __device__ __forceinline__ void kep_derivatives(const KepParams& P, KepDeriv& o)
 #pragma unroll
   for (int q = 0; q < NQ; q++) {
     const double r_q = (q < 4) ? fma(rp, ds[q], rq[q]) : rp * ds[q];
-    const double dg2 = (q == 2) ? fma(g1, ds[q], b2) : g1 * ds[q];
-    const double dg1 = (q == 2) ? fma(g0, ds[q], b1) : g0 * ds[q];
+    const double dg2 = (q == 2) ? fma(g1, ds[q], b2) : (q == 3) ? fma(g1, ds[q], kb2) : g1 * ds[q];
+    const double dg1 = (q == 2) ? fma(g0, ds[q], b1) : (q == 3) ? fma(g0, ds[q], kb1) : g0 * ds[q];
     o.d[q] = rinv * fma(g2r, r_q, -dg2);
     o.c[q] = rr0 * fma(g1r, r_q, -dg1);
     if (q == 0) o.c[q] = fma(r0inv, g1r * r0inv, o.c[q]);
     if (DRIFT_FIRST) {
       o.a[q] = -(r0inv * dg2);
       if (q == 0) o.a[q] = fma(r0inv * r0inv, g2, o.a[q]);
-      o.b[q] = (q == 2) ? fma(-g2, ds[q], -b3) : -(g2 * ds[q]);
+      o.b[q] = (q == 2) ? fma(-g2, ds[q], -b3) : (q == 3) ? fma(-g2, ds[q], -kb3) : -(g2 * ds[q]);
     } else {
       double aq = as * ds[q], bq = bs * ds[q];
       if (q == 0) { aq = fma(kr0 * r0inv, h1, aq); bq = bq + h2; }
       if (q == 1) bq = bq + h1;
       if (q == 2) { aq = aq + fma(-kr0, hb1, b2); bq = bq + fma(r0, hb2, eta * hb1); }
-      if (q == 3) aq = fma(-r0inv, h1, aq);
+      if (q == 3) {
+        aq = aq + fma(-kr0 * ri2, hb1, fma(-r0inv, h1, kb2));
+        bq = fma(ri2, fma(r0, hb2, eta * hb1), bq);
+      }
       o.a[q] = rinv * fma(-al, r_q, aq);
       o.b[q] = rinv * fma(-bb, r_q, bq);
     }
   }
-  const double kk = 2.0 * kr0 * r0inv * r0inv, ri2 = 2.0 * r0inv, gk = GNEWT * k, vv = fma(2.0, kr0, -beta);
+  const double kk = 2.0 * kr0 * r0inv * r0inv, gk = GNEWT * k, vv = fma(2.0, kr0, -beta);
   double* const f[4] = {o.a, o.b, o.c, o.d};
 #pragma unroll
   for (int w = 0; w < 4; w++) {
@@ -363,7 +370,7 @@ __device__ __forceinline__ void kep_derivatives(const KepParams& P, KepDeriv& o)
     S[0] = k * fma(-kk, sb, S[0] * r0inv);
     S[1] = k * S[1];
     S[2] = -2.0 * k * sb;
-    S[3] = gk * fma(ri2, sb, S[3]);
+    S[3] = gk * S[3];
     if (WITH_H) S[4] = DRIFT_FIRST ? fma(k, S[4], -fma(eta, S[0], vv * S[1])) : k * S[4];
   }
   (void)h;
