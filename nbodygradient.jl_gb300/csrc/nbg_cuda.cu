@@ -733,10 +733,10 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     nev += 2;
     return r;
   };
-  // The transit searches of a chunk take the team form once few of the
+  // The transit searches of a chunk take a block's lanes each once few of the
   // group's systems still run (the long tail of an uneven batch, where the
-  // searches are latency-bound); while many run, one lane per search keeps
-  // every lane busy.  The same kernels' results either way (bitwise).
+  // searches are latency-bound), whatever form the producer is set to; while
+  // many run, one lane per search keeps every lane busy.  Bitwise the same.
   //
   // In the same tail the group's orbit producer runs on SMs of its own: its
   // blocks ask for 210 KB of shared memory, and from the first tail chunk on
@@ -761,7 +761,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   };
   auto search_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    gx.search_lanes = use_wide(ctx->orbit_team, active_at(q, c) <= tail_max) ? 1 : 0;
+    gx.search_lanes = (ctx->orbit_team == 2 || active_at(q, c) <= tail_max) ? 1 : 0;
     if (tail_any) gx.guard_smem = std::max(gx.guard_smem, 18 * 1024);
     return gx;
   };

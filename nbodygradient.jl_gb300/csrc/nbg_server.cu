@@ -624,13 +624,12 @@ int service_group(nbg_server* srv, int gi) {
   NBG_CUDA(cudaStreamWaitEvent(stt, G->ev_orb[par], 0));
   NBG_CUDA(cudaStreamWaitEvent(sw, G->ev_orb[par], 0));
   {
-    // a block's lanes per search while few slots are running, from five bodies on:
-    // below, a search on one lane ends within the producer's next chunk (32
-    // steps by default), and the lanes would only take pipe time from the groups
-    // beside it
+    // a block's lanes per search while few slots are running, from four bodies on:
+    // below, a step is a chain of one pair after another in either form, a search
+    // on one lane ends within the producer's next chunk (32 steps by default),
+    // and the lanes would only take pipe time from the groups beside it
     GroupArgs gs = gc;
-    gs.search_lanes =
-        N >= 5 && use_wide(srv->cfg.orbit_team, G->active <= std::max(32, srv->sm_count / 2)) ? 1 : 0;
+    gs.search_lanes = N >= 4 && G->active <= std::max(32, srv->sm_count / 2) ? 1 : 0;
     if ((rc = launch_group_transit(N, gs, (int)c, stt))) return rc;
   }
   NBG_CUDA(cudaEventRecord(G->ev_tr[par], stt));

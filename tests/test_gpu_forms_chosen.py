@@ -1,0 +1,40 @@
+"""Which form of a kernel a call takes, where only its time tells: the results of all forms are bitwise the same.
+
+A form for few systems is several times faster than the one for full groups on a lone system, so a factor of 1.6
+between two times of the same work separates them.
+"""
+import numpy as np
+import pytest
+
+import nbg
+from conftest import has_gpu
+from nbg import workloads as W
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not has_gpu(), reason="needs a CUDA GPU")]
+
+
+def lone(ctx, n, steps, grad=True):
+    """The device times (total, orbit, transits, Jacobian) of one system of n bodies, the least of three calls."""
+    els, hs, _ = W.batch_uneven(1, seed=40 + n, nmin=n, nmax=n)
+    b = nbg.Batch([n], 0, hs, [hs[0] * steps], [steps], grad)
+    best = None
+    for _ in range(4):
+        b.set_system(0, nbg.State(W.ic_of(els[0])), nbg.TransitTiming(hs[0] * steps, W.ic_of(els[0]), ntt=steps))
+        b.run(ctx)
+        t = np.array(ctx.last_timing())
+        best = t if best is None else np.minimum(best, t)
+    assert b.arrays["count"].sum() > 0
+    return best
+
+
+@pytest.mark.parametrize("n", [5, 8])
+def test_few_searches_take_a_blocks_lanes_in_every_mode(n):
+    """The searches of few systems are as fast with a one-lane or team producer as with the lanes one."""
+    took = {}
+    for mode in (0, 1, 2):
+        ctx = nbg.Context(0)
+        ctx.set_orbit_team(mode)
+        ctx.set_profiling(1)
+        took[mode] = lone(ctx, n, 120)[2]
+        ctx.close()
+    assert took[0] < 1.6 * took[2] and took[1] < 1.6 * took[2], took
