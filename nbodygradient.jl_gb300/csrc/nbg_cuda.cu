@@ -390,18 +390,17 @@ namespace nbg {
 // critical path. One lane -> team, ms: 5 bodies 2048 systems 128 steps 56.3 -> 52.7,
 // 8 bodies 1024 systems 64 steps 61.5 -> 57.4, 10 bodies 1024 systems 32 steps 61.6 -> 54.8.
 // Modes (nbg_set_orbit_team): -1 automatic, 0 one lane, 1 team, 2 the wide
-// forms always, 3 team with the wide forms in latency-bound chunks.
+// forms always, 3 team with the wide forms in latency-bound chunks; and the
+// autotuner's ONE_LANE_WIDE: one lane with the wide forms in latency-bound chunks.
 bool use_team(int mode, int N, unsigned long long kick) {
-  if (kick) return false;
+  if (kick || mode == ONE_LANE_WIDE) return false;
   return mode > 0 || (mode < 0 && N >= 5);
 }
 
 // The forms for latency-bound chunks (sixteen lanes per pair solve, six per
 // column of jac_step): always in mode 2, in the latency-bound chunks (few
-// systems running) in modes -1 and 3.
-bool use_wide(int mode, bool latency_bound) {
-  return mode == 2 || ((mode < 0 || mode == 3) && latency_bound);
-}
+// systems running) in modes -1, 3 and ONE_LANE_WIDE.
+bool use_wide(int mode, bool latency_bound) { return mode == 2 || ((mode < 0 || mode >= 3) && latency_bound); }
 }  // namespace nbg
 
 namespace {
@@ -2107,9 +2106,9 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   // difference of two trial lengths would understate a step's time.
   int wchunk = 0;
   for (const Cand& cd : cands) wchunk = std::max(wchunk, cd.chunk);
-  // a team or one lane; the forms for latency-bound chunks beside the team and,
-  // in a batch of up to four bodies, where the choice is not between the two
-  auto mode_of = [&](bool team) { return team ? 3 : any_team ? 0 : -1; };
+  // a team or one lane for full groups, with the forms for latency-bound chunks
+  // beside either: the choice stays on the context, for calls of any size
+  auto mode_of = [](bool team) { return team ? 3 : ONE_LANE_WIDE; };
   for (int wteam : {0, 3}) {
     if (wteam && !any_team) continue;
     ctx->chunk_steps = wchunk;

@@ -29,7 +29,8 @@ long long steps_of(double h, double tmax);
 double check_step(double t0, double tmax);
 
 // Whether a group of N bodies with kick-pair mask `kick` uses the team form
-// of the orbit producer (mode: -1 automatic, 0 never, 1 whenever possible).
+// of the orbit producer (mode: -1 automatic, 0 never, 1 whenever possible, ...).
+constexpr int ONE_LANE_WIDE = 4;  // a mode beside nbg_set_orbit_team's, left by the autotuner
 bool use_team(int mode, int N, unsigned long long kick);
 bool use_wide(int mode, bool latency_bound);
 

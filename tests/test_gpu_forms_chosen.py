@@ -38,3 +38,30 @@ def test_few_searches_take_a_blocks_lanes_in_every_mode(n):
         took[mode] = lone(ctx, n, 120)[2]
         ctx.close()
     assert took[0] < 1.6 * took[2] and took[1] < 1.6 * took[2], took
+
+
+def tuned(n, count, steps, trial_steps):
+    """A context after autotuning on `count` systems of n bodies, and the report."""
+    import torch
+    els, hs, _ = W.batch_uneven(count, seed=9, nmin=n, nmax=n)
+    b = nbg.Batch([n] * count, 0, hs, [h * steps for h in hs], [steps // 10 + 4] * count, True)
+    for q, (x, v, jac) in enumerate(nbg.init_nbody_batch([W.ic_of(el) for el in els])):
+        b.view("x", q)[:], b.view("v", q)[:] = x.ravel(order="F"), v.ravel(order="F")
+        b.view("m", q)[:] = els[q][:, 0]
+        b.view("jac_init", q)[:] = jac.ravel(order="F")
+        b.view("jac_step", q)[:: 7 * n + 1] = 1.0
+    dev = {k: torch.from_numpy(a).cuda() for k, a in b.arrays.items()}
+    ctx = nbg.Context(0)
+    return ctx, b, dev, b.autotune_device(dev, ctx, trial_steps=trial_steps)
+
+
+def test_a_lone_system_after_autotuning_takes_the_forms_for_few_systems():
+    """Tuned on a full batch of four-body systems, where one lane a system is the fastest producer."""
+    fresh = nbg.Context(0)
+    before = lone(fresh, 8, 120)[0]
+    fresh.close()
+    ctx, _, _, report = tuned(4, 1500, 64, 16)
+    assert report[0]["ms"] > 0
+    after = lone(ctx, 8, 120)[0]
+    ctx.close()
+    assert after < 1.6 * before, (before, after, report[0])
