@@ -432,7 +432,8 @@ int nbg_last_timing(nbg_context* ctx, double* total_ms, double* orbit_ms, double
  * for T = trial_steps and 2 trial_steps, on device copies (the caller's
  * arrays are not modified) -- for each candidate mapping: steps per chunk
  * {64, 128} x orbit producer form {one lane per system, team of lanes} x
- * producer block layout {one warp; four warps} (nbg_set_producer_layout).  The
+ * producer block layout {the default; four warps; four warps holding 200 KB of
+ * shared memory, operator and search blocks 32 KB} (nbg_set_producer_layout).  The
  * two trial times give the loop's fill and drain and its time per step with
  * the whole batch active.  For a batch of uneven length (its shortest system
  * under half its longest) two more trials run only the systems with its
@@ -489,8 +490,9 @@ int nbg_set_orbit_team(nbg_context* ctx, int mode);
  * operator-record and transit-search block.  Blocks cannot share an SM when
  * their shared memory exceeds the SM's 227 KB, so smem_kb = 200 with
  * guard_kb = 32 keeps the throughput kernels off the SMs that run the
- * latency-bound producer.  Default: no shared memory held, one warp a block,
- * three in a one-lane group with derivatives of 1024 systems or more. */
+ * latency-bound producer.  Default 1, 0, 0, which stands for the fastest number
+ * of warps at the group's size: one, or three or four in a one-lane group with
+ * derivatives of 1024 systems or more. */
 int nbg_set_producer_layout(nbg_context* ctx, int warps_per_block, int smem_kb, int guard_kb);
 
 /* Profiling (no reference counterpart).

@@ -267,7 +267,7 @@ struct nbg_context {
   int overlap = 1;  // orbit producer on its own stream, one chunk ahead of the rest
   int orbit_spw = 0;  // 0: automatic
   int orbit_team = -1;  // -1: automatic (teams for N >= 5), 0: one lane per system, 1: teams for every N
-  int prod_warps = 0, prod_smem_kb = 0, guard_smem_kb = 0;  // orbit producer block layout
+  int prod_warps = 1, prod_smem_kb = 0, guard_smem_kb = 0;  // orbit producer block layout (1, 0, 0: by group size)
   int sm_count = 0;
   double last_total_ms = 0, last_orbit_ms = 0, last_jac_ms = 0, last_transit_ms = 0, last_ops_ms = 0;
   double last_host_ms = 0;  // host time spent enqueueing the chunk loop
@@ -551,7 +551,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     // the most FP64 issue slots to the kernels running beside the producer.
     // Without overlap a small batch is spread over about two warps per SM.
     g.team = use_team(ctx->orbit_team, N, gp.kick) && ctx->orbit_spw == 0;
-    g.pwarps = ctx->prod_warps;
+    g.pwarps = ctx->prod_warps == 1 && ctx->prod_smem_kb == 0 ? 0 : ctx->prod_warps;
     g.prod_smem = ctx->prod_smem_kb * 1024;
     g.guard_smem = ctx->guard_smem_kb * 1024;
     if (ctx->orbit_spw > 0) {
@@ -766,8 +766,10 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   };
   auto orbit_args = [&](size_t q, const GroupArgs& g, long long c) {
     GroupArgs gx = g;
-    if (active_at(q, c) <= tail_limit(g.N, ctx->sm_count)) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
     gx.wide = use_wide(ctx->orbit_team, active_at(q, c) <= lanes_limit(g.N, g.grad, ctx->sm_count)) ? 1 : 0;
+    if (active_at(q, c) <= tail_limit(g.N, ctx->sm_count)) gx.prod_smem = std::max(gx.prod_smem, 210 * 1024);
+    // a layout that holds an SM per block is meant for blocks of many systems
+    else if (gx.wide) gx.prod_smem = 0;
     return gx;
   };
   auto jac_args = [&](size_t q, const GroupArgs& g, long long c) {
@@ -2082,11 +2084,12 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   for (int chunk : {64, 128})
     for (int team : {0, 1}) {
       if (team && !any_team) continue;
-      // producer blocks of one warp or of four (4096 three-body systems over
-      // 2000 steps: 366 and 307 ms; with 200 KB of shared memory held beside
-      // the four, 317)
+      // producer blocks by group size (launch_orbit), of four warps, and of four
+      // on SMs of their own: 4096 three-body systems over 512 steps 137, 135 and
+      // 130 ms; 2048 five-body systems over 96 steps 126, 118 and 87
       cands.push_back({chunk, team, 0, 1, 0, 0});
       cands.push_back({chunk, team, 0, 4, 0, 0});
+      cands.push_back({chunk, team, 0, 4, 200, 32});
     }
   const int save_chunk = ctx->chunk_steps, save_team = ctx->orbit_team, save_spw = ctx->orbit_spw;
   const int save_pw = ctx->prod_warps, save_sm = ctx->prod_smem_kb, save_gd = ctx->guard_smem_kb;

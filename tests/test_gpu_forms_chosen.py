@@ -5,6 +5,7 @@ between two times of the same work separates them.
 """
 import numpy as np
 import pytest
+import torch
 
 import nbg
 from conftest import has_gpu
@@ -42,7 +43,6 @@ def test_few_searches_take_a_blocks_lanes_in_every_mode(n):
 
 def tuned(n, count, steps, trial_steps):
     """A context after autotuning on `count` systems of n bodies, and the report."""
-    import torch
     els, hs, _ = W.batch_uneven(count, seed=9, nmin=n, nmax=n)
     b = nbg.Batch([n] * count, 0, hs, [h * steps for h in hs], [steps // 10 + 4] * count, True)
     for q, (x, v, jac) in enumerate(nbg.init_nbody_batch([W.ic_of(el) for el in els])):
@@ -65,3 +65,29 @@ def test_a_lone_system_after_autotuning_takes_the_forms_for_few_systems():
     after = lone(ctx, 8, 120)[0]
     ctx.close()
     assert after < 1.6 * before, (before, after, report[0])
+
+
+def test_autotuner_tries_the_default_layout_and_producers_on_sms_of_their_own():
+    ctx, b, dev, report = tuned(5, 64, 48, 8)
+    tried = {(r["producer_warps"], r["producer_smem_kb"]) for r in report}
+    ctx.close()
+    assert tried == {(1, 0), (4, 0), (4, 200)}
+
+
+def test_a_layout_for_full_groups_does_not_hold_up_the_forms_for_few_systems():
+    """400 four-body systems: their blocks of the lanes form, each with an SM to itself, would run in three waves."""
+    took = []
+    for layout in ((1, 0, 0), (4, 200, 32)):
+        ctx, b, dev, _ = tuned(4, 400, 64, 8)
+        ctx.set_tuning(64)
+        ctx.set_orbit_team(-1)
+        ctx.set_producer_layout(*layout)
+        best = []
+        for _ in range(3):
+            work = {k: t.clone() for k, t in dev.items()}
+            torch.cuda.synchronize()  # the call runs on the library's own streams
+            b.run_device(work, ctx)
+            best.append(ctx.last_timing()[0])
+        took.append(min(best))
+        ctx.close()
+    assert took[1] < 1.3 * took[0], took
