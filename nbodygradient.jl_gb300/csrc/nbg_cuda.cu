@@ -264,6 +264,7 @@ struct nbg_context {
   cudaStream_t stream = nullptr;
   std::map<std::string, Buf> pool;
   int chunk_steps = 64;
+  bool whole_chunks = false;  // short calls take chunk_steps as they are, too (the autotuner's trials)
   int overlap = 1;  // orbit producer on its own stream, one chunk ahead of the rest
   int orbit_spw = 0;  // 0: automatic
   int orbit_team = -1;  // -1: automatic (teams for N >= 5), 0: one lane per system, 1: teams for every N
@@ -486,7 +487,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   int K = std::max(1, ctx->chunk_steps);
   long long longest = 0;
   for (auto& kv : groups) longest = std::max(longest, kv.second.max_steps);
-  K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
+  if (!ctx->whole_chunks) K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
   for (auto& kv : groups) {
     const GroupPlan& gp = kv.second;
     if (!gp.grad) continue;
@@ -2095,6 +2096,8 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   const int save_pw = ctx->prod_warps, save_sm = ctx->prod_smem_kb, save_gd = ctx->guard_smem_kb;
   const int save_prof = ctx->profile;
   ctx->profile = 0;
+  // a trial stands for a long integration: it runs at the candidate's chunk
+  ctx->whole_chunks = true;
   int best = -1, nrep = 0;
   double best_ms = 1e300;
   std::vector<double> cand_ms;
@@ -2185,6 +2188,7 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
     }
   }
   ctx->profile = save_prof;
+  ctx->whole_chunks = false;
   // the chosen candidate first in the report
   if (!rc && best > 0 && report && best < std::min(nrep, report_len)) std::swap(report[0], report[best]);
   if (rc || best < 0) {

@@ -91,3 +91,16 @@ def test_a_layout_for_full_groups_does_not_hold_up_the_forms_for_few_systems():
         took.append(min(best))
         ctx.close()
     assert took[1] < 1.3 * took[0], took
+
+
+def test_autotuner_trials_run_at_the_candidates_chunk():
+    """The last trial, 128 steps at a chunk of 128, is one chunk: fewer launches than a call of 128 steps takes, which
+    is cut into four chunks so that they overlap."""
+    ctx, b, dev, report = tuned(3, 64, 128, 64)
+    trial = ctx.last_launch_count()
+    assert max(r["chunk_steps"] for r in report) == 128
+    ctx.set_tuning(128)
+    b.run_device(dev, ctx)
+    call = ctx.last_launch_count()
+    ctx.close()
+    assert trial < call, (trial, call)
