@@ -25,6 +25,7 @@
 
 #include "../../include/nbg.h"
 #include "nbg_internal.cuh"
+#include "nbg_staging.hpp"
 
 using namespace nbg;
 
@@ -259,6 +260,8 @@ struct NoallocPlan {
 
 }  // namespace
 
+constexpr size_t kStageMax = 4u << 20;  // page-locked bytes that a context keeps for staging, each block
+
 struct nbg_context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -284,28 +287,16 @@ struct nbg_context {
   std::vector<cudaStream_t> hstreams;
   std::vector<cudaEvent_t> sync_events;  // cross-stream ordering, no timing
   NoallocPlan* noalloc = nullptr;         // host plan of the allocation-free entry point
-  // pinned host memory that a call's small arrays go through, one copy for all
-  // of them: 0 the plan's, 1 the caller's arrays (grow-only, kStageMax at most)
-  struct Pinned {
-    unsigned char* p = nullptr;
-    size_t bytes = 0;
-  } pinned[2];
-  int pin(int which, size_t bytes, unsigned char** out) {
-    Pinned& b = pinned[which];
-    if (b.bytes < bytes) {
-      if (b.p) cudaFreeHost(b.p);
-      b.p = nullptr;
-      b.bytes = 0;
-      const size_t want = std::max<size_t>(bytes, 64 * 1024);
-      if (cudaHostAlloc((void**)&b.p, want, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(NBG_ENOMEM, "cudaHostAlloc(%zu bytes)", want);
-      }
-      b.bytes = want;
-    }
-    *out = b.p;
-    return NBG_OK;
+  // page-locked memory that a call's small arrays go through, one copy for all of
+  // them: 0 the plan's, 1 the caller's arrays
+  static void* pinned_alloc(size_t n) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, n, cudaHostAllocDefault) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
   }
+  static void pinned_free(void* p) { cudaFreeHost(p); }
+  StagingBlock pinned[2] = {{pinned_alloc, pinned_free, kStageMax}, {pinned_alloc, pinned_free, kStageMax}};
 
   int sync_event(size_t i, cudaEvent_t* out) {
     while (sync_events.size() <= i) {
@@ -499,13 +490,18 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     const int kmax = (int)std::min(4096.0, std::floor(4294967296.0 / per_step));
     K = std::min(K, std::max(std::min(K, 8), kmax));
   }
-  // ---- the plan's small arrays (offsets, each group's scalars): written to
-  // pinned memory and copied as one block
+  // ---- the plan's small arrays (offsets, each group's scalars): gathered on the
+  // host and copied as one block
   size_t plan_bytes = 0;
   for (auto& kv : groups) plan_bytes += ((kv.second.systems.size() + 31) / 32) * 32 * (5 * 8 + 4 * 4) + 9 * 64;
   plan_bytes += (size_t)nsys * (sizeof(SysOff) + 24) + 4 * 64;
-  unsigned char *plan, *d_plan;
-  if ((rc = ctx->pin(0, plan_bytes, &plan)) || (rc = ctx->get("plan", plan_bytes, &d_plan))) return rc;
+  unsigned char *plan = ctx->pinned[0].get(plan_bytes), *d_plan;
+  std::vector<unsigned char> pageable;
+  if (!plan) {
+    pageable.resize(plan_bytes);
+    plan = pageable.data();
+  }
+  if ((rc = ctx->get("plan", plan_bytes, &d_plan))) return rc;
   size_t plan_at = 0;
   auto part = [&](auto** dev, size_t count) {  // room for count values; *dev their device address
     using T = std::remove_reference_t<decltype(**dev)>;
@@ -987,9 +983,8 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
 // A host call's arrays: what goes in, out or both, in one device block.  Up to
 // kStageMax in all they go through the context's pinned memory in one copy each
 // way (a copy of its own for each array of a small system costs more than the
-// bytes: 16 steps of two bodies 473 -> 358 us a call); larger ones are copied from and
-// to where they are.
-constexpr size_t kStageMax = 4u << 20;
+// bytes: 16 steps of two bodies 473 -> 358 us a call); larger ones, and all where
+// no pinned memory is to be had, are copied from and to where they are.
 struct HostArrays {
   struct Array {
     const void* in;
@@ -998,7 +993,7 @@ struct HostArrays {
   };
   std::vector<Array> arrays;
   size_t total = 0, out_end = 0;
-  unsigned char* dev = nullptr;
+  unsigned char *dev = nullptr, *host = nullptr;  // host: the staged copy, if any
 
   // null `in`: zeros on the device; `out` arrays first
   void add(const void* in, void* out, size_t bytes) {
@@ -1009,13 +1004,11 @@ struct HostArrays {
   int upload(nbg_context* ctx, const char* name) {
     int rc;
     if ((rc = ctx->get(name, total, &dev))) return rc;
-    if (total <= kStageMax) {
-      unsigned char* p;
-      if ((rc = ctx->pin(1, total, &p))) return rc;
+    if ((host = ctx->pinned[1].get(total))) {
       for (auto& a : arrays)
-        if (a.in) memcpy(p + a.at, a.in, a.bytes);
-        else memset(p + a.at, 0, a.bytes);
-      NBG_CUDA(cudaMemcpyAsync(dev, p, total, cudaMemcpyHostToDevice, ctx->stream));
+        if (a.in) memcpy(host + a.at, a.in, a.bytes);
+        else memset(host + a.at, 0, a.bytes);
+      NBG_CUDA(cudaMemcpyAsync(dev, host, total, cudaMemcpyHostToDevice, ctx->stream));
       return NBG_OK;
     }
     for (auto& a : arrays)
@@ -1024,16 +1017,15 @@ struct HostArrays {
     return NBG_OK;
   }
   int download(nbg_context* ctx) {
-    const bool staged = total <= kStageMax;
-    if (staged)
-      NBG_CUDA(cudaMemcpyAsync(ctx->pinned[1].p, dev, out_end, cudaMemcpyDeviceToHost, ctx->stream));
+    if (host)
+      NBG_CUDA(cudaMemcpyAsync(host, dev, out_end, cudaMemcpyDeviceToHost, ctx->stream));
     else
       for (auto& a : arrays)
         if (a.out) NBG_CUDA(cudaMemcpyAsync(a.out, dev + a.at, a.bytes, cudaMemcpyDeviceToHost, ctx->stream));
     NBG_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (staged)
+    if (host)
       for (auto& a : arrays)
-        if (a.out) memcpy(a.out, ctx->pinned[1].p + a.at, a.bytes);
+        if (a.out) memcpy(a.out, host + a.at, a.bytes);
     return NBG_OK;
   }
   template <class T>
@@ -1499,8 +1491,7 @@ int nbg_destroy(nbg_context* ctx) {
   for (cudaStream_t s2 : ctx->hstreams) cudaStreamSynchronize(s2);
   for (auto& kv : ctx->pool)
     if (kv.second.p) cudaFree(kv.second.p);
-  for (auto& b : ctx->pinned)
-    if (b.p) cudaFreeHost(b.p);
+  for (auto& b : ctx->pinned) b.free();
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);
   for (auto e : ctx->prof_events) cudaEventDestroy(e);
