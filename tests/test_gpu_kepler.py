@@ -249,3 +249,68 @@ def test_drift_and_derivatives(device, name, drift_first):
         assert rms <= bound, (q, rms)
         if name in ("bound", "planets"):
             assert float(err[q].max()) <= 8 * bound, (q, float(err[q].max()))
+
+
+ELEMENTARY = r'''
+#include <cstdio>
+#include <vector>
+#include "nbg_kepler.cuh"
+using namespace nbg;
+__global__ void run(int n, const double* x, const double* z, double* out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  double* o = out + (size_t)t * 7;
+  o[0] = rcp_fast(x[t]);
+  o[1] = rsqrt_fast(fabs(x[t]));
+  o[2] = stumpff<2>(z[t]);
+  o[3] = stumpff<3>(z[t]);
+  o[4] = stumpff<4>(z[t]);
+  o[5] = stumpff<5>(z[t]);
+  o[6] = stumpff<6>(z[t]);
+}
+int main(int argc, char** argv) {
+  FILE* f = fopen(argv[1], "rb");
+  int n = 0;
+  if (!f || fread(&n, sizeof(int), 1, f) != 1 || n <= 0 || n > (1 << 22)) return 2;
+  std::vector<double> in((size_t)n * 2), out((size_t)n * 7);
+  if (fread(in.data(), 8, in.size(), f) != in.size()) return 3;
+  fclose(f);
+  double *di, *dout;
+  if (cudaMalloc(&di, in.size() * 8) != cudaSuccess || cudaMalloc(&dout, out.size() * 8) != cudaSuccess) return 4;
+  cudaMemcpy(di, in.data(), in.size() * 8, cudaMemcpyHostToDevice);
+  run<<<(n + 127) / 128, 128>>>(n, di, di + n, dout);
+  if (cudaMemcpy(out.data(), dout, out.size() * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return 5;
+  f = fopen(argv[2], "wb");
+  fwrite(out.data(), 8, out.size(), f);
+  fclose(f);
+  return 0;
+}
+'''
+
+
+def test_reciprocal_root_and_stumpff_sums():
+    """rcp_fast and rsqrt_fast over 2^-300 to 2^300 and the Stumpff sums over |z| <= KEP_ZMAX, against long double.
+
+    u = 2^-53.  rcp_fast: the last FMA's rounding, u, and e's own error times the seed's (below u / 1000).  rsqrt_fast:
+    that and half of the rounding of x y, which e carries whole: 1.5 u.  stumpff: the last sum's rounding and its
+    coefficient's, 2 u, and z c_{n+2} / c_n <= 0.05 of as much again, and the truncation, below 0.2 u."""
+    rng, n = np.random.default_rng(5), 1 << 17
+    x = np.exp2(rng.uniform(-300, 300, n)) * rng.choice([-1.0, 1.0], n)
+    z = rng.uniform(-0.6, 0.6, n)
+    z[:3] = 0.0, 0.6, -0.6
+    with tempfile.TemporaryDirectory() as tmp:
+        src, exe, a, b = (os.path.join(tmp, q) for q in ("e.cu", "e", "in", "out"))
+        with open(src, "w") as f:
+            f.write(ELEMENTARY)
+        subprocess.run(["nvcc", "-gencode", "arch=compute_103a,code=sm_103a", "-O3", "--fmad=false",
+                        "-I", os.path.join(PKG_DIR, "csrc"), "-o", exe, src], check=True)
+        with open(a, "wb") as f:
+            f.write(np.int32(n).tobytes() + x.tobytes() + z.tobytes())
+        subprocess.run([exe, a, b], check=True)
+        got = np.fromfile(b).reshape(n, 7).astype(LD)
+    u = LD(2) ** -53
+    off = lambda g, r: float((np.abs(g - r) / np.abs(r)).max() / u)  # noqa: E731
+    assert off(got[:, 0], 1 / x.astype(LD)) <= 1.01
+    assert off(got[:, 1], 1 / np.sqrt(np.abs(x).astype(LD))) <= 1.51
+    for k in range(2, 7):
+        assert off(got[:, k], stumpff(k, z.astype(LD))[0]) <= 2.4, k
