@@ -413,7 +413,8 @@ int nbg_server_stop(nbg_server* srv);
  * depend on them.
  * chunk_steps: integration steps per producer/consumer chunk (default 64,
  *   shortened for batches whose per-chunk operator records would pass
- *   4 GiB; 0 keeps the current value);
+ *   4 GiB and, with overlap, to a quarter of a short call's steps, 16 at
+ *   least; 0 keeps the current value);
  * overlap: 1 (default) runs the orbit producer on its own stream one chunk
  *   ahead of the transit searches, operator kernels and Jacobian consumer
  *   (three streams per group of systems); 0 runs everything on one stream;

@@ -478,7 +478,8 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   int K = std::max(1, ctx->chunk_steps);
   long long longest = 0;
   for (auto& kv : groups) longest = std::max(longest, kv.second.max_steps);
-  if (!ctx->whole_chunks) K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
+  if (ctx->overlap && !ctx->whole_chunks)
+    K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
   for (auto& kv : groups) {
     const GroupPlan& gp = kv.second;
     if (!gp.grad) continue;

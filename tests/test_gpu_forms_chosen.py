@@ -104,3 +104,15 @@ def test_autotuner_trials_run_at_the_candidates_chunk():
     call = ctx.last_launch_count()
     ctx.close()
     assert trial < call, (trial, call)
+
+
+def test_a_short_call_without_overlap_is_one_chunk():
+    """Chunks of a quarter of a short call's steps are for overlapping them: on one stream 64 steps stay one chunk."""
+    count = {}
+    for overlap in (0, 1):
+        ctx = nbg.Context(0)
+        ctx.set_tuning(64, overlap)
+        lone(ctx, 3, 64)
+        count[overlap] = ctx.last_launch_count()
+        ctx.close()
+    assert count[0] < count[1], count
