@@ -433,8 +433,8 @@ int nbg_last_timing(nbg_context* ctx, double* total_ms, double* orbit_ms, double
  * for T = trial_steps and 2 trial_steps, on device copies (the caller's
  * arrays are not modified) -- for each candidate mapping: steps per chunk
  * {64, 128} x orbit producer form {one lane per system, team of lanes} x
- * producer block layout {the default; four warps; four warps holding 200 KB of
- * shared memory, operator and search blocks 32 KB} (nbg_set_producer_layout).  The
+ * producer block layout {the default; four warps holding 200 KB of shared
+ * memory, operator and search blocks 32 KB} (nbg_set_producer_layout).  The
  * two trial times give the loop's fill and drain and its time per step with
  * the whole batch active.  For a batch of uneven length (its shortest system
  * under half its longest) two more trials run only the systems with its

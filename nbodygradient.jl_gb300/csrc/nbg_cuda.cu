@@ -2077,11 +2077,11 @@ int nbg_autotune_device(nbg_context* ctx, int nsys, const nbg_system_desc* desc,
   for (int chunk : {64, 128})
     for (int team : {0, 1}) {
       if (team && !any_team) continue;
-      // producer blocks by group size (launch_orbit), of four warps, and of four
-      // on SMs of their own: 4096 three-body systems over 512 steps 137, 135 and
-      // 130 ms; 2048 five-body systems over 96 steps 126, 118 and 87
+      // producer blocks by group size (launch_orbit), and of four warps on SMs of
+      // their own: 4096 three-body systems over 512 steps 137 and 130 ms, 2048
+      // five-body systems over 96 steps 126 and 87, 1024 eight-body systems over
+      // 64 steps 149 and 164
       cands.push_back({chunk, team, 0, 1, 0, 0});
-      cands.push_back({chunk, team, 0, 4, 0, 0});
       cands.push_back({chunk, team, 0, 4, 200, 32});
     }
   const int save_chunk = ctx->chunk_steps, save_team = ctx->orbit_team, save_spw = ctx->orbit_spw;
