@@ -1671,6 +1671,10 @@ static int batch_host_device(nbg_context* ctx, int nsys, const nbg_system_desc* 
   const int nr = tbv ? 3 : 1;
   if (!ctx) return set_error(NBG_EINVAL, "ctx is NULL");
   if (nsys <= 0 || !desc) return set_error(NBG_EINVAL, "nsys = %d", nsys);
+  // a null entry of HostArrays means zeros, or nothing to bring back
+  if (!t || !x || !v || !m || !xerror || !verror || !jac_step || !jac_error || !dqdt || !pair || !jac_init || !tt ||
+      !dtdq0 || !dtdelements || !count)
+    return set_error(NBG_EINVAL, "NULL array argument");
   NBG_CUDA(cudaSetDevice(ctx->device));
   long long ax = 0, am = 0, aJ = 0, adq = 0, ap = 0, att = 0, adq0 = 0;
   for (int s = 0; s < nsys; s++) {
