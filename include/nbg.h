@@ -295,7 +295,7 @@ int nbg_batch_integrate_transits_device(nbg_context* ctx, int nsys, const nbg_sy
  * producer / consumer overlap of the other batched entry points, and its
  * chunk shrinks when the working set would not fit; expect it to be slower
  * than nbg_batch_integrate_transits_device on the same batch (measured: 128
- * 3-body systems, 2000 steps, 473 ms against 326 ms, 1.45 times as long).
+ * 3-body systems, 2000 steps, 388 ms against 174 ms, 2.2 times as long).
  *
  * Every call on a device shares
  * the one array and finds the previous call's contents in it (the call
@@ -414,7 +414,8 @@ int nbg_server_stop(nbg_server* srv);
  * chunk_steps: integration steps per producer/consumer chunk (default 64,
  *   shortened for batches whose per-chunk operator records would pass
  *   4 GiB and, with overlap, to a quarter of a short call's steps, 16 at
- *   least; 0 keeps the current value);
+ *   least, but where full groups of four bodies or more search for transits;
+ *   0 keeps the current value);
  * overlap: 1 (default) runs the orbit producer on its own stream one chunk
  *   ahead of the transit searches, operator kernels and Jacobian consumer
  *   (three streams per group of systems); 0 runs everything on one stream;

@@ -474,12 +474,23 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   // Steps per chunk: the context's setting, shortened (not below 8) where a
   // group's operator records for one chunk would pass 4 GiB per buffer half.
   // A short call takes a quarter of its steps, so that its producer, searches
-  // and consumer still overlap (a recorded trajectory of 62 steps 2.5 -> 2.0 ms).
+  // and consumer overlap: 62 steps of one eight-body system with transits
+  // 27.1 -> 24.8 ms, 64 of 4096 three-body systems 28.0 -> 24.3, but of a recorded
+  // three-body trajectory 6.8 -> 7.0.  Not from four bodies on where the searches
+  // take one lane each (more than tail_max systems): a chunk's searches then last
+  // as long as 20 steps of a one-lane producer, whatever its length, and four of
+  // them one after another longer than the producer: 64 steps of 1024 systems of
+  // six bodies 70 ms instead of 102, of eight 119 instead of 152, 128 steps of 2048
+  // of four without derivatives 50 instead of 71.
   int K = std::max(1, ctx->chunk_steps);
+  const int tail_max = std::max(32, ctx->sm_count / 2);
   long long longest = 0;
-  for (auto& kv : groups) longest = std::max(longest, kv.second.max_steps);
-  if (ctx->overlap && !ctx->whole_chunks)
-    K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
+  bool quarter = ctx->overlap && !ctx->whole_chunks;
+  for (auto& kv : groups) {
+    longest = std::max(longest, kv.second.max_steps);
+    if (!plain && kv.second.N >= 4 && ctx->orbit_team != 2 && (int)kv.second.systems.size() > tail_max) quarter = false;
+  }
+  if (quarter) K = (int)std::min<long long>(K, std::max<long long>(std::min(K, 16), (longest + 3) / 4));
   for (auto& kv : groups) {
     const GroupPlan& gp = kv.second;
     if (!gp.grad) continue;
@@ -742,7 +753,6 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
   // 24 KB or more).  A producer warp then has its SM's FP64 pipe to itself
   // instead of sharing it with the throughput kernels of the other groups;
   // while many systems run, the layout stays the autotuner's.
-  const int tail_max = std::max(32, ctx->sm_count / 2);
   bool tail_any = false;
   auto active_at = [&](size_t q, long long c) -> long long {
     const std::vector<long long>& st_q = gsteps[q];
@@ -984,7 +994,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
 // A host call's arrays: what goes in, out or both, in one device block.  Up to
 // kStageMax in all they go through the context's pinned memory in one copy each
 // way (a copy of its own for each array of a small system costs more than the
-// bytes: 16 steps of two bodies 473 -> 358 us a call); larger ones, and all where
+// bytes: 16 steps of two bodies 0.85 -> 0.77 ms a call); larger ones, and all where
 // no pinned memory is to be had, are copied from and to where they are.
 struct HostArrays {
   struct Array {

@@ -116,3 +116,21 @@ def test_a_short_call_without_overlap_is_one_chunk():
         count[overlap] = ctx.last_launch_count()
         ctx.close()
     assert count[0] < count[1], count
+
+
+@pytest.mark.parametrize("n, count, cut", [(3, 200, True), (4, 40, True), (4, 200, False), (6, 200, False)])
+def test_short_calls_of_full_groups_keep_their_chunk(n, count, cut):
+    """From four bodies on, where each search takes one lane and lasts as long whatever the chunk, 64 steps are one
+    chunk, as without overlap; fewer bodies or few systems overlap in four."""
+    els, hs, _ = W.batch_uneven(count, seed=3, nmin=n, nmax=n)
+    b = nbg.Batch([n] * count, 0, hs, [h * 64 for h in hs], [10] * count, False)
+    launches = {}
+    for overlap in (0, 1):
+        ctx = nbg.Context(0)
+        ctx.set_tuning(64, overlap)
+        for q, el in enumerate(els):
+            b.set_system(q, nbg.State(W.ic_of(el)), nbg.TransitTiming(hs[q] * 64, W.ic_of(el), ntt=10))
+        b.run(ctx)
+        launches[overlap] = ctx.last_launch_count()
+        ctx.close()
+    assert (launches[0] < launches[1]) == cut, launches
