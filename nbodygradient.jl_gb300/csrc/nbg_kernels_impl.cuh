@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(OPS_BS) operator_phi_kernel(GroupArgs g, int c
   for (int q = 0; q < N; q++) m[q] = g.m[q * S + s];
   for (int q = 0; q < 12 * N; q++) acc[q] = 0.0;
   // the consumer reads position columns of J_d - J_0 only, none of body 0's
-  // (4096 three-body systems over 2000 steps: 291.2 -> 287.9 ms)
+  // (4096 three-body systems over 2000 steps: 551 -> 535 ms)
   if (d == 0) phi_columns<N, false>(x, a, m, h, 0, d, acc);
   else phi_columns<N>(x, a, m, h, 0, d, acc);
   const int off_phi = g.npk * PREC;
@@ -649,8 +649,9 @@ __global__ void __launch_bounds__(cons_bs(N), 3 * 128 / cons_bs(N)) jacobian_chu
 // one (cp.async), so no trip to memory is waited out.  Per column the FP64 work
 // is that of the one-lane form within a tenth, and every value is formed by the
 // same operations in the same order: bitwise the same columns.
-// One system alone, before and after: 400 steps of eight bodies with transits
-// 121 -> 55 ms, 2000 of three 67 -> 54 ms, 203 of six 33 -> 20 ms.
+// One system alone, one lane a column -> six: 400 steps of eight bodies with
+// transits 161 -> 148 ms, 2000 of three 193 -> 191 ms, 203 of six 57 -> 52 ms
+// (its consumer 0.26 -> 0.044 ms a step at eight bodies, 0.030 -> 0.0065 at three).
 constexpr int ROWS_COLS = 5, ROWS_WARPS = 2;
 __host__ __device__ constexpr int rows_plain_warps(int N) { return (6 * N + ROWS_COLS - 1) / ROWS_COLS; }
 __host__ __device__ constexpr int rows_warps(int N) { return rows_plain_warps(N) + (N + ROWS_COLS - 1) / ROWS_COLS; }
@@ -1002,8 +1003,16 @@ int launch_transit(const GroupArgs& g, int chunk, cudaStream_t st) {
     allow_smem(transit_lanes_kernel<N>, smem);
     transit_lanes_kernel<N><<<g.tgrid / TRANSIT_BS, 32 * lanes_warps(N), smem, st>>>(g, chunk);
   } else {
-    allow_smem(transit_kernel<N>, g.guard_smem);
-    transit_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, g.guard_smem, st>>>(g, chunk);
+    // An SM that runs blocks without shared memory gives it to L1, and a team or
+    // lanes producer's block waits until that SM idles: the next chunk's then crowd
+    // on a few.  Where no consumer block (24 KB or more) sees to it, the searches
+    // ask for some themselves, 12 blocks an SM as its registers allow 8.  Without ->
+    // with, no derivatives, 128 steps, ms: 2048 systems of five bodies 122 -> 64,
+    // 1024 of six 143 -> 79, of eight 213 -> 118; one-lane producers are level
+    // (2048 of four 50.0).
+    const int smem = g.grad ? g.guard_smem : std::max(g.guard_smem, 18 * 1024);
+    allow_smem(transit_kernel<N>, smem);
+    transit_kernel<N><<<g.tgrid / TRANSIT_BS, TRANSIT_BS, smem, st>>>(g, chunk);
   }
   return 0;
 }
