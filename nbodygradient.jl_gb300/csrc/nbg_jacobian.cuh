@@ -88,8 +88,8 @@ __device__ __forceinline__ void fold_all(double* J, double* E) {
 // of jac_step where a Kahan sum at every update leaves 3.3e-13 and 2.5e-13.
 // Per column and pair 66 FP64 instructions instead of 102, and no folds; per
 // column-step at three bodies 600 instead of 864.  FP64 issue bounds the
-// kernel: 4096 three-body systems over 2000 steps went from 532 to 361 ms a
-// pass, 1024 eight-body systems over 200 steps from 273 to 202 ms.
+// kernel: over 4096 three-body systems and 2000 steps its launches, one after
+// another, went from 327 to 219 ms.
 //
 // The corrector's and the kicks' operators depend on position differences alone
 // (the sum of their blocks over all bodies is zero), so they are applied to

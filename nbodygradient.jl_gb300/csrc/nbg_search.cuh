@@ -12,11 +12,9 @@
 // Two forms, bitwise the same: one lane per search (many searches), and a
 // block's lanes per search (orbit_lanes_kernel's layout) while few systems run
 // and a search's latency counts.  Both are bound by the FP64 instructions one
-// warp issues after another.  A search of eight bodies on a team of lanes, with
-// the gradient step and the dense corrector block on one of them, took 5.1 ms;
-// on the block's lanes: 203 mixed systems over 80 steps 41.6 -> 22.6 ms a pass, 400
-// steps of one 8-body system 48 -> 36 ms, 24 served requests 47 -> 29 ms; on one
-// lane: 1024 eight-body systems over 200 steps 185 -> 170 ms.
+// warp issues after another.  One lane -> a block's lanes, ms: 203 mixed systems
+// over 80 steps 92 -> 47, one system over 400 steps of eight bodies 158 -> 148,
+// over 203 of six with TransitParameters 56 -> 53.
 #pragma once
 #include "nbg_jacobian.cuh"
 #include "nbg_orbit_team.cuh"
