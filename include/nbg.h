@@ -492,9 +492,10 @@ int nbg_set_orbit_team(nbg_context* ctx, int mode);
  * operator-record and transit-search block.  Blocks cannot share an SM when
  * their shared memory exceeds the SM's 227 KB, so smem_kb = 200 with
  * guard_kb = 32 keeps the throughput kernels off the SMs that run the
- * latency-bound producer.  Default 1, 0, 0, which stands for the fastest number
- * of warps at the group's size: one, or three or four in a one-lane group with
- * derivatives of 1024 systems or more. */
+ * latency-bound producer.  Default 1, 0, 0, which stands for the fastest layout
+ * at the group's size: one warp, or three or four in a one-lane group with
+ * derivatives of 1024 systems or more, or 4, 200, 32 for a full team group with
+ * derivatives whose blocks then hold no more than half of the SMs. */
 int nbg_set_producer_layout(nbg_context* ctx, int warps_per_block, int smem_kb, int guard_kb);
 
 /* Profiling (no reference counterpart).

@@ -379,8 +379,10 @@ namespace {
 namespace nbg {
 // Team producer (a team of lanes per system) for full kick-free groups: automatic
 // from five bodies on, where the level-parallel sweeps shorten the step's
-// critical path. One lane -> team, ms: 5 bodies 2048 systems 128 steps 56.3 -> 52.7,
-// 8 bodies 1024 systems 64 steps 61.5 -> 57.4, 10 bodies 1024 systems 32 steps 61.6 -> 54.8.
+// critical path. One lane -> team, ms: with derivatives 5 bodies 1100 systems 512
+// steps 349 -> 276, 6 bodies 1024 systems 400 steps 418 -> 318, 8 bodies 1024 systems
+// 64 steps 176 -> 119; without 5 bodies 2048 systems 128 steps 82 -> 64, 8 bodies
+// 1024 systems 64 steps 121 -> 72.
 // Modes (nbg_set_orbit_team): -1 automatic, 0 one lane, 1 team, 2 the wide
 // forms always, 3 team with the wide forms in latency-bound chunks; and the
 // autotuner's ONE_LANE_WIDE: one lane with the wide forms in latency-bound chunks.
@@ -536,6 +538,7 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     }
   }
   // ---- per-group device state
+  int own_sms = 0;  // SMs that producers hold for themselves
   std::vector<GroupArgs> gargs;
   std::vector<GroupArgs> ghalf;  // the same groups on the second half of the per-chunk buffers
   int* d_bad;
@@ -563,6 +566,24 @@ int run_batch(nbg_context* ctx, int nsys, const nbg_system_desc* desc, const dou
     g.pwarps = ctx->prod_warps == 1 && ctx->prod_smem_kb == 0 ? 0 : ctx->prod_warps;
     g.prod_smem = ctx->prod_smem_kb * 1024;
     g.guard_smem = ctx->guard_smem_kb * 1024;
+    // A team's one-warp blocks need registers that three consumer blocks leave on
+    // no SM.  A full group with derivatives therefore takes SMs of its own for
+    // them, four warps a block, up to half of the SMs in all, where a chunk's
+    // producer and consumer run side by side (more than one chunk).  One warp a
+    // block -> SMs of its own, ms: N = 5 1100 systems 512 steps 644 -> 276, 128 steps
+    // 135 -> 87, 3500 systems 256 steps 350 -> 237; N = 6 1024 systems 100 steps
+    // 114 -> 96, 400 steps 566 -> 318; N = 8 1024 systems 256 steps 541 -> 336;
+    // in one chunk N = 8 1024 systems 119 -> 128, N = 10 118 -> 131.
+    if (g.pwarps == 0 && g.team && g.grad && ctx->overlap && gp.max_steps > K &&
+        nsg > lanes_limit(N, true, ctx->sm_count)) {
+      const int each = PROD_MAX_WARPS * (PROD_BS / team_lanes(N)), blocks = (nsg + each - 1) / each;
+      if (own_sms + blocks <= ctx->sm_count / 2) {
+        own_sms += blocks;
+        g.pwarps = PROD_MAX_WARPS;
+        g.prod_smem = 200 * 1024;
+        g.guard_smem = std::max(g.guard_smem, 32 * 1024);
+      }
+    }
     if (ctx->orbit_spw > 0) {
       g.spw = ctx->orbit_spw;
     } else if (ctx->overlap) {

@@ -38,6 +38,7 @@ __host__ __device__ inline int search_scratch(int N, int npk, bool kick) {
 
 constexpr int PROD_BS = 32;     // orbit producer: threads per warp-sized unit of work
 constexpr int PROD_MAX_WARPS = 4;  // orbit producer: up to 4 independent warps per block
+__host__ __device__ constexpr int team_lanes(int N) { return N / 2 > 1 ? N / 2 : 1; }  // lanes of a system's team
 // Jacobian consumer: columns per block.  96 N bytes of shared memory a column:
 // four warps a block, two from nine bodies on, so that six or more warps fit an
 // SM (227 KB) at every N; every block holds 24 KB or more.

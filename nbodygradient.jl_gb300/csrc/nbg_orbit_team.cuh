@@ -26,8 +26,6 @@
 
 namespace nbg {
 
-__host__ __device__ constexpr int team_lanes(int N) { return N / 2 > 1 ? N / 2 : 1; }
-
 // The pair of level `lev` (i + j == lev) that lane t of a team takes, if any.
 template <int N>
 __device__ __forceinline__ bool level_pair(int lev, int t, int* i, int* j) {

@@ -134,3 +134,33 @@ def test_short_calls_of_full_groups_keep_their_chunk(n, count, cut):
         launches[overlap] = ctx.last_launch_count()
         ctx.close()
     assert (launches[0] < launches[1]) == cut, launches
+
+
+def test_full_team_groups_on_sms_of_their_own():
+    """A full team group's default layout, on SMs of its own, against one of two warps a block anywhere: the same bits,
+    and not slower (1.15 for noise; without SMs of its own this takes half as long again)."""
+    n, count, steps = 6, 1100, 256
+    els, hs, _ = W.batch_uneven(count, seed=5, nmin=n, nmax=n)
+    b = nbg.Batch([n] * count, 0, hs, [h * steps for h in hs], [steps // 10 + 4] * count, True)
+    start = nbg.init_nbody_batch([W.ic_of(el) for el in els])
+    got, took = [], []
+    for layout in ((1, 0, 0), (2, 0, 0)):
+        ctx = nbg.Context(0)
+        ctx.set_producer_layout(*layout)
+        times = []
+        for _ in range(3):
+            for k in b.arrays:
+                b.arrays[k][...] = 0
+            for q, (x, v, jac) in enumerate(start):
+                b.view("x", q)[:], b.view("v", q)[:] = x.ravel(order="F"), v.ravel(order="F")
+                b.view("m", q)[:] = els[q][:, 0]
+                b.view("jac_init", q)[:] = jac.ravel(order="F")
+                b.view("jac_step", q)[:: 7 * n + 1] = 1.0
+            b.run(ctx)
+            times.append(ctx.last_timing()[0])
+        got.append({k: a.copy() for k, a in b.arrays.items()})
+        took.append(min(times))
+        ctx.close()
+    for k in got[0]:
+        np.testing.assert_array_equal(got[0][k], got[1][k], err_msg=k)
+    assert took[0] < 1.15 * took[1], took
